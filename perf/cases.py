@@ -126,16 +126,26 @@ def _frames_of_step(case):
     return (10 * np.arange(case["origins"])[:, None] + np.arange(case["points"])[None, :]).astype(np.int32).ravel()
 
 
+def _box(nmol, frames, seed):
+    """A synthetic trajectory; the generator gives up on a start where a molecule has no room."""
+    for again in range(50):
+        try:
+            return cg.synth_trajectory(nmol, frames, seed=seed + 10_000_019 * again)
+        except cg.CirError:
+            pass
+    raise RuntimeError("no trajectory of %d molecules from seed %d" % (nmol, seed))
+
+
 def _trajectories(case, seed):
     """The library's synthetic trajectories: [(xyz (frames, atoms, 3), boxes (frames, 3))], float32."""
     nf = case["frames"] if case["kind"] in ("hamiltonian", "frame") else int(_frames_of_step(case).max()) + 1
     out = []
     for i, nmol in enumerate(_sizes(case)):
         if case["kind"] == "frame":      # the current frames of independent trajectories
-            parts = [cg.synth_trajectory(nmol, 1, seed=1000 * seed + f + 1) for f in range(nf)]
+            parts = [_box(nmol, 1, 1000 * seed + f + 1) for f in range(nf)]
             xyz, box = np.concatenate([p[0] for p in parts]), parts[0][1]
         else:
-            xyz, box = cg.synth_trajectory(nmol, nf, seed=1000 * seed + i + 1)
+            xyz, box = _box(nmol, nf, 1000 * seed + i + 1)
         out.append((xyz, np.tile(np.asarray(box, np.float32), (nf, 1))))
     return out
 
