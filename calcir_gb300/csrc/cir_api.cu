@@ -55,7 +55,8 @@ enum {
     B_XYZ, B_BOX, B_FIDX, B_CXYZ, B_CBOX,          // run: frames and their gather
     B_A, B_W, B_M, B_F, B_G, B_M0,                 // run: matrices
     B_TCF, B_HCNT, B_HIPR, B_HMIPR, B_OOR, B_SW, B_MU2, B_SWEEPS, B_ROT, B_PAD,
-    B_FFT0, B_FFT1, B_FFTY, B_FFTX, B_PROF, B_DE, B_ERR, B_DC, B_TUNE,
+    B_FFT0, B_FFT1, B_FFTY, B_FFTX,  // lineshape: Stockham work, adjoint, rows, input
+    B_PROF, B_DE, B_ERR, B_DC, B_TUNE,
     B_PSI, B_LAM, B_PA, B_PB, B_SEG, B_CKPT, B_R, B_T, B_GRAD,   // differentiation form
     B_VS, B_FS,                                    // split-BF16 propagation operands
     B_UFR,                                         // run: distinct frames of a chunk and their multiplicity
@@ -86,6 +87,8 @@ struct cir_ctx {
     cir_stats stats;
     cudaEvent_t ev[8];
     CirMaps maps;
+    LsRows ls;                            // printed lineshape rows and their frequencies
+    std::vector<float> ls_omega;
     std::map<GemmShape, int> gemm_tile;   // autotuner: SIMT tile shape per product shape
     // autotuner, mixed forms: tile width of each split-BF16 product shape (M, N, K, batch,
     // epilogue, output form, fused contraction) and tridiagonalisation blocks per SM per order
@@ -205,6 +208,37 @@ static bool all_finite(const float *x, size_t n) {
     return true;
 }
 
+// The rows of the three lineshape files (calcIR.cu:890-919).  Each part of the selection runs
+// over falling frequencies, so it keeps an end of its range: the first from i0 up, the second
+// below cnt2.  Fixed by the parameters: made once per context, with their frequencies.
+static LsRows ls_rows(const cir_params *p, std::vector<float> &omega) {
+    const int n = p->ntcfpoints + p->nzeros;
+    const float factor = (float)(2 * CIR_PI * CIR_HBAR / (p->dt * (float)n));
+    LsRows r{n, n, 0, 0, factor * (float)n};
+    auto freq1 = [&](int i) { return -1 * (i - p->ntcfpoints - p->nzeros) * factor + p->avef; };
+    auto freq2 = [&](int i) { return -1 * i * factor + p->avef; };
+    int lo = n / 2, hi = n;                       // the first i with freq1(i) <= omegaStop
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (freq1(mid) <= (float)p->omegaStop) hi = mid;
+        else lo = mid + 1;
+    }
+    r.i0 = lo;
+    r.cnt1 = n - lo;
+    lo = 0;                                       // the first i with freq2(i) < omegaStart
+    hi = p->ntcfpoints + p->nzeros / 2;
+    while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (freq2(mid) >= (float)p->omegaStart) lo = mid + 1;
+        else hi = mid;
+    }
+    r.cnt2 = lo;
+    omega.resize(r.cnt1 + r.cnt2);
+    for (int i = 0; i < r.cnt1; i++) omega[i] = freq1(r.i0 + i);
+    for (int i = 0; i < r.cnt2; i++) omega[r.cnt1 + i] = freq2(i);
+    return r;
+}
+
 extern "C" int cir_create(const cir_params *p, int natoms, cir_ctx **out) {
     if (!p || !out) return cir_fail(CIR_ERR_ARG, "cir_create: null pointer");
     *out = nullptr;
@@ -229,6 +263,7 @@ extern "C" int cir_create(const cir_params *p, int natoms, cir_ctx **out) {
     c->n = n;
     c->ld = (n + 3) & ~3;
     cir_maps(q.map, q.ispecies, &c->maps);
+    c->ls = ls_rows(&c->p, c->ls_omega);
     memset(&c->stats, 0, sizeof c->stats);
     cudaError_t e = cudaGetDevice(&c->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
@@ -751,56 +786,31 @@ extern "C" int cir_spectral_density(cir_ctx *c, int n, const float *V, const flo
     return CIR_OK;
 }
 
-// Frequency axis and intensity rows of the three lineshape files (calcIR.cu:890-919);
-// y = C2R transform (length n) of one damped TCF.
-static int lineshape_rows(const cir_params *p, const double *y, float *omega, float *inten) {
-    const int n = p->ntcfpoints + p->nzeros;
-    const float factor = (float)(2 * CIR_PI * CIR_HBAR / (p->dt * (float)n));
-    const float norm = factor * (float)n;
-    int cnt = 0;
-    for (int i = n / 2; i < n; i++) {
-        const float freq = -1 * (i - p->ntcfpoints - p->nzeros) * factor + p->avef;
-        if (freq <= (float)p->omegaStop) {
-            if (omega) omega[cnt] = freq;
-            if (inten) inten[cnt] = (float)y[i] / norm;
-            cnt++;
-        }
-    }
-    for (int i = 0; i < p->ntcfpoints + p->nzeros / 2; i++) {
-        const float freq = -1 * i * factor + p->avef;
-        if (freq >= (float)p->omegaStart) {
-            if (omega) omega[cnt] = freq;
-            if (inten) inten[cnt] = (float)y[i] / norm;
-            cnt++;
-        }
-    }
-    return cnt;
-}
-
-static int c2r_dev(cir_ctx *c, const double *tcf_host, std::vector<double> &y) {
-    const int n = c->p.ntcfpoints + c->p.nzeros;
-    const int nx = c->p.ntcfpoints;
-    CK(c->buf[B_FFT0].ensure((size_t)n * 16));
-    CK(c->buf[B_FFT1].ensure((size_t)n * 16));
-    CK(c->buf[B_FFTY].ensure((size_t)n * 8));
-    CK(c->buf[B_FFTX].ensure((size_t)nx * 16));
-    CK(cudaMemcpyAsync(c->buf[B_FFTX].p, tcf_host, (size_t)nx * 16, cudaMemcpyHostToDevice, c->stream));
+// Rows of nq damped TCFs (host, [nq][ntcfpoints] complex) into the device buffer B_FFTY.
+static int lineshape_dev(cir_ctx *c, const double *tcf_host, int nq, const LsRows &r) {
+    const int K = c->p.ntcfpoints;
+    const size_t work = cir_lineshape_work_bytes(K, r.n);
+    if (work) CK(c->buf[B_FFT0].ensure(work));
+    CK(c->buf[B_FFTY].ensure((size_t)nq * (r.cnt1 + r.cnt2) * 4 + 16));
+    CK(c->buf[B_FFTX].ensure((size_t)nq * K * 16));
+    CK(cudaMemcpyAsync(c->buf[B_FFTX].p, tcf_host, (size_t)nq * K * 16, cudaMemcpyHostToDevice, c->stream));
     int launches = 0;
-    CK(cir_launch_c2r(c->buf[B_FFTX].as<double>(), nx, n, c->buf[B_FFT0].as<double>(), c->buf[B_FFT1].as<double>(),
-                      c->buf[B_FFTY].as<double>(), c->stream, &launches));
+    CK(cir_launch_lineshape(c->buf[B_FFTX].as<double>(), nq, K, r, work ? c->buf[B_FFT0].p : nullptr,
+                            c->buf[B_FFTY].as<float>(), c->stream, &launches));
     count_launch(c, launches);
-    y.resize(n);
-    CK(cudaMemcpyAsync(y.data(), c->buf[B_FFTY].p, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     return CIR_OK;
 }
 
 extern "C" int cir_lineshape(cir_ctx *c, const double *tcf, float *omega, float *intensity, int *nls) {
     if (!c || !tcf) return cir_fail(CIR_ERR_ARG, "cir_lineshape: bad argument");
-    std::vector<double> y;
-    int rc = c2r_dev(c, tcf, y);
+    const LsRows &r = c->ls;
+    const int cnt = r.cnt1 + r.cnt2;
+    int rc = lineshape_dev(c, tcf, 1, r);
     if (rc) return rc;
-    const int cnt = lineshape_rows(&c->p, y.data(), omega, intensity);
+    if (omega && cnt) memcpy(omega, c->ls_omega.data(), (size_t)cnt * 4);   // while the kernel runs
+    if (intensity && cnt)
+        CK(cudaMemcpyAsync(intensity, c->buf[B_FFTY].p, (size_t)cnt * 4, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     if (nls) *nls = cnt;
     return CIR_OK;
 }
@@ -1372,27 +1382,35 @@ struct GroupJob {
             if (hst[i]) return cir_fail(CIR_ERR_NOCONVERGE, "eigensolver sweep cap reached");
         if (p.precision != CIR_PREC_FP32 && (rc = check_kernel_flag(c))) return rc;
 
+        // damped correlation sums of every trajectory, their lineshapes in one launch
+        // (calcIR.cu:786-827, 890-919); the host fills the other outputs meanwhile
+        std::vector<double> damped((size_t)T * 6 * K);
         for (int tr = 0; tr < T; tr++) {
             cir_result *r = res + tr;
-            const double *sw_t = hsw.data() + (size_t)tr * nomega, *ipr_t = hipr.data() + (size_t)tr * nomega,
-                         *mipr_t = hmipr.data() + (size_t)tr * nomega;
-            const unsigned long long *cnt_t = hcnt.data() + (size_t)tr * nomega;
+            double *dp = damped.data() + (size_t)tr * 6 * K;
             // sum over origins, T1 damping and 1/nsamples (calcIR.cu:777-782, 798-802, 815-819)
-            std::vector<double> damped[3];
-            for (int q = 0; q < 3; q++) damped[q].assign((size_t)2 * K, 0.0);
             for (int k = 0; k < K; k++) {
                 CompSum sum[6];
                 for (int s = tr * S; s < (tr + 1) * S; s++)
                     for (int q = 0; q < 6; q++) sum[q].add(htcf[((size_t)s * K + k) * 6 + q]);
                 const double dcy = exp(-1.0 * k * p.dt / (2.0 * p.t1)) / (1. * S);
                 for (int q = 0; q < 3; q++) {
-                    damped[q][2 * k] = sum[2 * q].value() * dcy;
-                    damped[q][2 * k + 1] = sum[2 * q + 1].value() * dcy;
+                    dp[(size_t)2 * (q * K + k)] = sum[2 * q].value() * dcy;
+                    dp[(size_t)2 * (q * K + k) + 1] = sum[2 * q + 1].value() * dcy;
                 }
             }
             double *outs[3] = {r->tcf_ir, r->tcf_vv, r->tcf_vh};
             for (int q = 0; q < 3; q++)
-                if (outs[q]) memcpy(outs[q], damped[q].data(), (size_t)2 * K * 8);
+                if (outs[q]) memcpy(outs[q], dp + (size_t)2 * q * K, (size_t)2 * K * 8);
+        }
+        const LsRows &lr = c->ls;
+        const int nls = lr.cnt1 + lr.cnt2;
+        if ((rc = lineshape_dev(c, damped.data(), 3 * T, lr))) return rc;
+        for (int tr = 0; tr < T; tr++) {
+            cir_result *r = res + tr;
+            const double *sw_t = hsw.data() + (size_t)tr * nomega, *ipr_t = hipr.data() + (size_t)tr * nomega,
+                         *mipr_t = hmipr.data() + (size_t)tr * nomega;
+            const unsigned long long *cnt_t = hcnt.data() + (size_t)tr * nomega;
             // spectral density and frequency distributions (calcIR.cu:831-839)
             const float norm = (float)(n * S * K);
             for (int i = 0; i < nomega; i++) {
@@ -1403,19 +1421,19 @@ struct GroupJob {
                 if (r->rw) r->rw[i] = ((float)(ipr_t[i] / p.omegaStep) / norm) / pw;
                 if (r->rmw) r->rmw[i] = ((float)(mipr_t[i] / p.omegaStep) / norm) / pw;
             }
-            // lineshapes (calcIR.cu:786-827, 890-919)
-            float *lsv[3] = {r->ls_ir, r->ls_vv, r->ls_vh};
-            int nls = 0;
-            for (int q = 0; q < 3; q++) {
-                std::vector<double> y;
-                int rc3 = c2r_dev(c, damped[q].data(), y);
-                if (rc3) return rc3;
-                nls = lineshape_rows(&p, y.data(), q == 0 ? r->ls_omega : nullptr, lsv[q]);
-            }
             r->nls = nls;
+            if (r->ls_omega && nls) memcpy(r->ls_omega, c->ls_omega.data(), (size_t)nls * 4);
             r->bins_out_of_range = (long long)oor[tr];
             r->frame_steps_per_s = ms_total > 0 ? steps / (ms_total * 1e-3) : 0.0;
         }
+        for (int tr = 0; tr < T; tr++) {
+            float *lsv[3] = {res[tr].ls_ir, res[tr].ls_vv, res[tr].ls_vh};
+            for (int q = 0; q < 3; q++)
+                if (lsv[q] && nls)
+                    CK(cudaMemcpyAsync(lsv[q], c->buf[B_FFTY].as<float>() + (size_t)(3 * tr + q) * nls, (size_t)nls * 4,
+                                       cudaMemcpyDeviceToHost, c->stream));
+        }
+        CK(cudaStreamSynchronize(c->stream));
         return CIR_OK;
     }
 };
@@ -1861,20 +1879,6 @@ extern "C" int cir_set_coeffs(cir_ctx *c, const float *t) {
     return CIR_OK;
 }
 
-// Positions in the C2R output of the printed lineshape rows (the selection of lineshape_rows),
-// and the intensity normalisation.
-static std::vector<int> lineshape_index(const cir_params *p, float *norm_out) {
-    const int n = p->ntcfpoints + p->nzeros;
-    const float factor = (float)(2 * CIR_PI * CIR_HBAR / (p->dt * (float)n));
-    *norm_out = factor * (float)n;
-    std::vector<int> idx;
-    for (int i = n / 2; i < n; i++)
-        if (-1 * (i - p->ntcfpoints - p->nzeros) * factor + p->avef <= (float)p->omegaStop) idx.push_back(i);
-    for (int i = 0; i < p->ntcfpoints + p->nzeros / 2; i++)
-        if (-1 * i * factor + p->avef >= (float)p->omegaStart) idx.push_back(i);
-    return idx;
-}
-
 // x <- V_k exp(i L_k dt/hbar) V_k^T x for S origins, x n x 9 complex (row-major, 18 floats per
 // row); FP32 SIMT GEMMs.  V: origin s at V + s*sV, w likewise; tmp: S x n x 18.
 static int psi_propagate(cir_ctx *c, int S, int n, int ld, const float *V, long long sV, const float *w, long long sw,
@@ -1896,10 +1900,9 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     const cir_params &p = c->p;
     const int S = p.nsamples, K = p.ntcfpoints, n = c->n, ld = c->ld;
     const long long steps = (long long)S * K;
-    float norm = 0.f;
-    const std::vector<int> rows = lineshape_index(&p, &norm);
-    if (nls != (int)rows.size())
-        return cir_fail(CIR_ERR_ARG, "cir_loss_grad: %d target rows, the lineshape has %zu", nls, rows.size());
+    const LsRows &lr = c->ls;
+    if (nls != lr.cnt1 + lr.cnt2)
+        return cir_fail(CIR_ERR_ARG, "cir_loss_grad: %d target rows, the lineshape has %d", nls, lr.cnt1 + lr.cnt2);
     std::vector<int> fidx(steps);
     for (long long i = 0; i < steps; i++) {
         const int f = frame_of_step ? frame_of_step[i] : (int)i;
@@ -2017,46 +2020,35 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     CK(cudaStreamSynchronize(c->stream));
     for (int i = 0; i < nb; i++)
         if (hst[i]) return cir_fail(CIR_ERR_NOCONVERGE, "eigensolver sweep cap reached");
-    std::vector<double> dcy(K), X[2];
-    for (int q = 0; q < 2; q++) X[q].assign((size_t)2 * K, 0.0);
+    std::vector<double> dcy(K), X((size_t)4 * K, 0.0);
     for (int k = 0; k < K; k++) {
         dcy[k] = exp(-1.0 * k * p.dt / (2.0 * p.t1)) / (1. * S);
         CompSum sum[4];                              // IR (terms 0, 1) and VV (terms 2, 3)
         for (int s = 0; s < S; s++)
             for (int q = 0; q < 4; q++) sum[q].add(htcf[((size_t)s * K + k) * 6 + q]);
         for (int q = 0; q < 2; q++) {
-            X[q][2 * k] = sum[2 * q].value() * dcy[k];
-            X[q][2 * k + 1] = sum[2 * q + 1].value() * dcy[k];
+            X[(size_t)2 * (q * K + k)] = sum[2 * q].value() * dcy[k];
+            X[(size_t)2 * (q * K + k) + 1] = sum[2 * q + 1].value() * dcy[k];
         }
     }
-    const int nfft = p.ntcfpoints + p.nzeros;
-    const float *tg[2] = {target_ir, target_vv};
-    double L = 0.0;
+    // the loss and dL/dX of both spectra (k_fft.cu), then through the damping and 1/nsamples
+    if ((rc = lineshape_dev(c, X.data(), 2, lr))) return rc;
+    CK(c->buf[B_FFT1].ensure((size_t)nls * (16 + 8) + (size_t)(4 * K + 1) * 8));
+    double *dy = c->buf[B_FFT1].as<double>(), *dl = dy + 2 * (size_t)nls, *dg = dl + 1;
+    float *tgt = reinterpret_cast<float *>(dg + 4 * (size_t)K);
+    CK(cudaMemcpyAsync(tgt, target_ir, (size_t)nls * 4, cudaMemcpyDefault, c->stream));
+    CK(cudaMemcpyAsync(tgt + nls, target_vv, (size_t)nls * 4, cudaMemcpyDefault, c->stream));
+    CK(cir_launch_ls_adjoint(c->buf[B_FFTY].as<float>(), tgt, K, lr, dy, dl, dg, c->stream, &launches));
+    std::vector<double> lg((size_t)4 * K + 1);
+    CK(cudaMemcpyAsync(lg.data(), dl, lg.size() * 8, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    const double L = lg[0];
     std::vector<double> gre[2], gim[2];
-    for (int q = 0; q < 2; q++) {
-        std::vector<double> y;
-        if ((rc = c2r_dev(c, X[q].data(), y))) return rc;
-        gre[q].assign(K, 0.0);
-        gim[q].assign(K, 0.0);
-        // dL/dX_k = sum over rows of dL/dy_i dy_i/dX_k; y_i = Re X_0 + 2 sum_k Re(X_k e^{2 pi i ik/n})
-        for (size_t r = 0; r < rows.size(); r++) {
-            const int i = rows[r];
-            const double ls = (float)y[i] / norm;      // the printed value, as lineshape_rows makes it
-            const double d = ls - tg[q][r];
-            L += d * d;
-            const double dy = 2.0 * d / norm;
-            gre[q][0] += dy;
-            for (int k = 1; k < K; k++) {
-                const double ang = 2.0 * CIR_PI * (double)((long long)i * k % nfft) / nfft;
-                gre[q][k] += 2.0 * dy * cos(ang);
-                gim[q][k] -= 2.0 * dy * sin(ang);
-            }
+    for (int q = 0; q < 2; q++)
+        for (int k = 0; k < K; k++) {
+            gre[q].push_back(lg[1 + (size_t)2 * (q * K + k)] * dcy[k]);
+            gim[q].push_back(lg[2 + (size_t)2 * (q * K + k)] * dcy[k]);
         }
-        for (int k = 0; k < K; k++) {              // through the damping and 1/nsamples
-            gre[q][k] *= dcy[k];
-            gim[q][k] *= dcy[k];
-        }
-    }
     // backward, one segment of CKPT steps at a time, last segment first
     const float tau = (float)(p.dt / CIR_HBAR);
     DthetaArgs dt{};

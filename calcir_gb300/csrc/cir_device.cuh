@@ -275,10 +275,22 @@ cudaError_t cir_launch_spectral(const float *V, int ld, const float *w, const fl
                                 float *mu2_scratch, double *Sw, int nomega, float omegaStart, int omegaStep,
                                 float t1, float avef, cudaStream_t s, int *launches);
 
-// unnormalised inverse real DFT (cuFFT C2R convention) of X[0..n/2] (complex double)
-// into y[n], by a mixed-radix Stockham FFT in double precision
-cudaError_t cir_launch_c2r(const double *X, int nx, int n, double *work0, double *work1, double *y,
-                           cudaStream_t s, int *launches);
+// The printed rows of a lineshape: outputs i0 .. i0 + cnt1 - 1 of the transform of length n,
+// then outputs 0 .. cnt2 - 1, each over norm (cir_api.cu ls_rows).
+struct LsRows {
+    int n, i0, cnt1, cnt2;
+    float norm;
+};
+// rows [nq][cnt1 + cnt2] of nq damped TCFs X [nq][K] (complex double): the unnormalised inverse
+// real DFT (cuFFT C2R convention) of the zero-padded TCFs; work: cir_lineshape_work_bytes (null
+// when 0)
+size_t cir_lineshape_work_bytes(int K, int n);
+cudaError_t cir_launch_lineshape(const double *X, int nq, int K, const LsRows &r, void *work, float *out,
+                                 cudaStream_t s, int *launches);
+// L = sum (rows - target)^2 over two spectra and dL/dX [2][K] (complex) into g; dy: scratch
+// [2][cnt1 + cnt2]
+cudaError_t cir_launch_ls_adjoint(const float *rows, const float *target, int K, const LsRows &r, double *dy,
+                                  double *loss, double *g, cudaStream_t s, int *launches);
 
 // F = I for nprop complex matrices
 cudaError_t cir_launch_identity(float *F, int n, int ldf, long long sF, int batch, cudaStream_t s, int *launches);

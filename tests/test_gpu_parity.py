@@ -433,3 +433,20 @@ def test_run_mixed_precision_forms(lib, case, precision):
     print(case, precision, {k: f"{v:.2e}" for k, v in errs.items()})
     for k, v in errs.items():
         assert v < MIXED_TOL, (k, v)
+
+
+# the direct sum's tiles (64 and 256 terms, 64 output pairs) and its remainders, and the
+# mixed-radix transform above 40 terms per unit of n's factor sum (n = 4200: 26, 40 * 26 = 1040)
+@pytest.mark.parametrize("ntcf,nzeros", [(1, 1), (2, 0), (3, 1), (64, 63), (65, 64), (66, 191), (257, 255), (258, 511),
+                                         (322, 4001), (1000, 3200), (2000, 2200)])
+def test_lineshape_forms(lib, ntcf, nzeros):
+    rng = np.random.default_rng(ntcf + nzeros)
+    p = lib.default_params(species="H2O", ntcfpoints=ntcf, nzeros=nzeros, omegaStart=2000, omegaStop=5000, avef=3415.0)
+    tcf = (rng.standard_normal(ntcf) + 1j * rng.standard_normal(ntcf)) * np.exp(-np.arange(ntcf) / 40)
+    prm = {"ntcfpoints": ntcf, "nzeros": nzeros, "dt": 0.010, "avef": 3415.0, "omegaStart": 2000, "omegaStop": 5000}
+    with lib.Engine(p, 8) as eng:
+        om, val = eng.lineshape(tcf)
+    om_ref, val_ref = O.lineshape_rows(prm, O.c2r(tcf, ntcf + nzeros))
+    np.testing.assert_array_equal(om, om_ref.astype(np.float32))
+    # four FP32 roundings (the sum, the axis step, the norm and the quotient), 6e-8 each
+    assert O.rel_l2(val, val_ref) < 5e-7
