@@ -160,8 +160,8 @@ static void eigh_profile_report(const unsigned long long *dev, int nmat, cudaStr
                         "%.3f roots %.3f z and norms %.3f ranking %.3f rotation %.3f\n",
                 mp[0] / nmat * 1e-6, mp[1] / nmat * 1e-6, mp[2] / nmat * 1e-6, mp[3] / nmat * 1e-6, mp[4] / nmat * 1e-6);
     if (tqp[0] + tqp[2] > 0)
-        fprintf(stderr, "eigh profile: tridiagonalisation phases, mean per block (ms): column %.3f reflector %.3f "
-                        "symv %.3f panel dots %.3f w %.3f trailing update %.3f\n",
+        fprintf(stderr, "eigh profile: tridiagonalisation phases, mean per matrix (ms): exchange %.3f reflector %.3f "
+                        "symv %.3f panel dots %.3f w %.3f symv with update %.3f\n",
                 tqp[0] / nmat * 1e-6, tqp[1] / nmat * 1e-6, tqp[2] / nmat * 1e-6, tqp[3] / nmat * 1e-6,
                 tqp[4] / nmat * 1e-6, tqp[5] / nmat * 1e-6);
 }

@@ -104,10 +104,10 @@ struct EighArgs {
     // tridiagonalisation, of forming Q, of the QR iteration and of the ordering (0-6), then the
     // chase and apply times (ns), rotations, the chase's block-search time (ns) and sweeps
     // (7-11; on the divide-and-conquer path: the merges' time in setup and deflation, secular
-    // roots, z and norms, ranking and rotation, summed over a matrix's merges), then the blocked
-    // tridiagonalisation's time (ns) in its column fetch, reflector, symmetric matrix-vector
-    // product, panel dot products, w and trailing update (12-17), then the secular equation's
-    // iterations and roots (18-19)
+    // roots, z and norms, ranking and rotation, summed over a matrix's merges), then the
+    // tridiagonalisation's time (ns) in its cluster exchange, reflector, symmetric matrix-vector
+    // product, panel dot products, w and the products that update the matrix (12-17), then the
+    // secular equation's iterations and roots (18-19)
     unsigned long long *phase_ns;
     // optional FP64 refinement of the eigenpairs on the divide-and-conquer path (k_refine.cu),
     // on when Href is not null: Href holds a copy of the input matrices (same strides as A), RW
@@ -118,9 +118,6 @@ struct EighArgs {
     // fault drills (tests only, 0 = off): the split-BF16 GEMMs' stall (SplitGemmArgs::test_stall)
     // and a cap on the QR sweeps of each divide-and-conquer leaf
     int test_stall, test_sweep_cap;
-    // set by the launcher: 1 walks the tiles of the tridiagonalisation's matrix-vector
-    // products in reverse order on alternate columns (CIR_TQ_ORDER=0 keeps one order)
-    int tq_order;
     // thread blocks of the tridiagonalisation per SM: 0 the kernel's own occupancy, or a
     // smaller count enforced through its shared-memory request (the autotuner's choice)
     int tq_blocks;

@@ -1,14 +1,11 @@
 // Batched symmetric eigensolver for the exciton Hamiltonians (replaces magma_ssyevd_gpu,
-// calcIR.cu:420-448).  Three kernels, each with one thread block per matrix, so the SMs
-// work on independent frames at once: k_eigh_tq (phase 1), k_eigh_formq (phase 2) and
+// calcIR.cu:420-448).  After the tridiagonalisation (phase 1) two kernels, each with one thread
+// block per matrix, so the SMs work on independent frames at once: k_eigh_formq (phase 2) and
 // k_eigh_qr (phases 3-4, 128 threads: one chasing warp and three applying warps, three
 // blocks per SM so that three bulge chases overlap on every SM).
 //
-//  1. Householder tridiagonalisation Q^T H Q = T (reflectors stored below the subdiagonal,
-//     as LAPACK sytrd).  Orders above 256: blocked, lower storage, panels of TB_NB columns
-//     (tiled symmetric matrix-vector products, one rank-2*TB_NB update per panel).  Smaller
-//     orders: the rank-2 update of step k-1 and the matrix-vector product of step k share
-//     one read/write pass over the trailing block.
+//  1. Householder tridiagonalisation Q^T H Q = T (k_tridiag.cu; reflectors stored below the
+//     subdiagonal, as LAPACK sytrd).
 //  2. Q is formed explicitly in Z by backward accumulation of the reflectors in compact WY
 //     blocks, each warp holding its rows of the block's reflectors in registers.  (The
 //     divide-and-conquer path, a.DC set, skips phases 2-4: it solves the tridiagonal
@@ -51,44 +48,9 @@ __device__ __forceinline__ void cp_async4(float *dst, const float *src, bool val
     const int sz = valid ? 4 : 0;   // 0: fill with zeros
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
 }
-// 16-byte asynchronous global-to-shared copy (zero fill when !valid)
-__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool valid) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    const int sz = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// request the 128-byte line holding p into L2 (no data returned, no register held)
-__device__ __forceinline__ void prefetch_l2(const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Blocked tridiagonalisation (orders above 256): panels of TB_NB columns, LAPACK sytrd/latrd
-// with lower storage.  Within a panel each column's matrix-vector product reads the lower
-// triangle of the trailing block as it stood at the start of the panel and corrects for the
-// panel's earlier columns with V and W; after the panel the trailing block is updated once,
-// A -= V W^T + W V^T, in TB_KC-column steps staged in shared memory.
-constexpr int TB_NB = 32;      // panel width
-constexpr int TB_KC = 8;       // panel columns per staged step of the trailing update
-constexpr int TB_ROWS = 128;   // rows of a trailing-update tile
-
-__host__ __device__ constexpr int tb_cols(int nt) { return 4 * (nt / 16); }   // its columns
-__host__ __device__ constexpr int tb_stage(int nt) { return TB_KC * (2 * TB_ROWS + 2 * tb_cols(nt)); }
-
-// floats of phase 1's shared work area: the four vectors of the unblocked path, or the
-// blocked state (x, one partial product per warp, the staging tiles aliasing those, 4 panel
-// vectors)
-__host__ __device__ inline size_t tq_union_floats(int n, int nt, bool blocked) {
-    const size_t n4 = (size_t)((n + 3) & ~3), n32 = (size_t)((n + 31) & ~31);
-    if (!blocked) return 4 * n4;
-    const size_t yw = n32 * (nt / 32), st = 2 * (size_t)tb_stage(nt);   // two staging buffers
-    return n32 + (yw > st ? yw : st) + 4 * TB_NB;
-}
-
-size_t tq_smem_bytes(int n, int nt, bool blocked) {
-    const size_t n4 = (size_t)((n + 3) & ~3);
-    return sizeof(float) * (3 * n4 + tq_union_floats(n, nt, blocked) + 64);
-}
 
 // d, e, ranks, the group bookkeeping, then the appliers' column ring (QR_AHEAD+1 slots of
 // rows x applying threads)
@@ -99,22 +61,6 @@ __host__ __device__ inline size_t qr_ring_offset_floats(int n) {
 
 size_t qr_smem_bytes(int n, int nt, int rows) {
     return sizeof(float) * (qr_ring_offset_floats(n) + (size_t)(QR_AHEAD + 1) * rows * (nt - 32));
-}
-
-template <int NT>
-__device__ __forceinline__ float block_sum(float v, float *red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = warp_sum(v);
-    __syncthreads();               // red may still be read from the previous call
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        float t = lane < NT / 32 ? red[lane] : 0.f;
-        t = warp_sum(t);
-        if (lane == 0) red[32] = t;
-    }
-    __syncthreads();
-    return red[32];
 }
 
 __device__ __forceinline__ bool negligible(float e, float d0, float d1, float tiny) {
@@ -308,617 +254,6 @@ __device__ __forceinline__ void apply_group(float *Z, int ld, const int (&row)[R
                 if (row[j] >= 0) __stcg(Z + (size_t)c * ld + row[j], w[j][v]);
         }
     }
-}
-
-// ---- blocked tridiagonalisation (phase 1 for orders above 256) ----
-
-// y += A x on one 32 x 32 tile (I, J), I >= J, of the lower triangle, for both halves of
-// the symmetric matrix: A_IJ x_J into rows 32I.., A_IJ^T x_I into rows 32J...  Lane
-// (g, h) = (lane & 7, lane >> 3) loads rows 32I+4g..+3 of columns 32J+8h..+7 with 16-byte
-// accesses (each load instruction covers four whole 128-byte column segments).  The row
-// sums are reduced over h and the column sums over g by halving exchanges, after which lane
-// (g, h) owns row 32I+4g+h and column 32J+8h+g; both are added to this warp's own partial
-// product ywp, so no two lanes or warps write one word.  CHECK: diagonal tile (only r >= c
-// counted, the diagonal once) or a tile reaching past row n-1 (rows/columns >= n masked;
-// the padding rows below n may hold anything).
-template <bool CHECK>
-__device__ __forceinline__ void symv_tile(const float *__restrict__ A, int ld, int n, int I, int J,
-                                          const float *x, float *ywp, int lane) {
-    const int g = lane & 7, h = lane >> 3;
-    const int r0 = 32 * I + 4 * g, c0 = 32 * J + 8 * h;
-    float4 a[8];
-    #pragma unroll
-    for (int t = 0; t < 8; t++) {
-        if (!CHECK || (r0 < n && c0 + t < n)) a[t] = __ldcg(reinterpret_cast<const float4 *>(A + (size_t)(c0 + t) * ld + r0));
-        else a[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    const float4 xr4 = *reinterpret_cast<const float4 *>(x + r0);
-    const float4 xc0 = *reinterpret_cast<const float4 *>(x + c0);
-    const float4 xc1 = *reinterpret_cast<const float4 *>(x + c0 + 4);
-    const float xr[4] = {xr4.x, xr4.y, xr4.z, xr4.w};
-    const float xc[8] = {xc0.x, xc0.y, xc0.z, xc0.w, xc1.x, xc1.y, xc1.z, xc1.w};
-    float yr[4] = {0.f, 0.f, 0.f, 0.f}, yc[8];
-    #pragma unroll
-    for (int t = 0; t < 8; t++) {
-        float av[4] = {a[t].x, a[t].y, a[t].z, a[t].w};
-        float s = 0.f;
-        #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            float ar = av[q], ac = av[q];
-            if (CHECK) {
-                const int r = r0 + q, c = c0 + t;
-                const bool ok = r < n && c < n;
-                ar = (ok && (I != J || r >= c)) ? ar : 0.f;
-                ac = (ok && (I != J || r > c)) ? ac : 0.f;
-            }
-            yr[q] = fmaf(ar, xc[t], yr[q]);
-            s = fmaf(ac, xr[q], s);
-        }
-        yc[t] = s;
-    }
-    // column sums over g (lane bits 0-2): keep the upper half where the bit is set
-    #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const bool up = lane & 4;
-        const float send = up ? yc[i] : yc[i + 4], keep = up ? yc[i + 4] : yc[i];
-        yc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-    }
-    #pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const bool up = lane & 2;
-        const float send = up ? yc[i] : yc[i + 2], keep = up ? yc[i + 2] : yc[i];
-        yc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-    }
-    {
-        const bool up = lane & 1;
-        const float send = up ? yc[0] : yc[1], keep = up ? yc[1] : yc[0];
-        yc[0] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-    }
-    // row sums over h (lane bits 3-4)
-    #pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const bool up = lane & 16;
-        const float send = up ? yr[i] : yr[i + 2], keep = up ? yr[i + 2] : yr[i];
-        yr[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-    {
-        const bool up = lane & 8;
-        const float send = up ? yr[0] : yr[1], keep = up ? yr[1] : yr[0];
-        yr[0] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    ywp[r0 + h] += yr[0];
-    ywp[c0 + g] += yc[0];
-}
-
-// Trailing update after a panel: A[r][c] -= sum_j V[r][j] W[c][j] + W[r][j] V[c][j] for
-// q0 <= c <= r < n (lower triangle only), V = the panel's reflectors (columns p0.. of A,
-// with the unit element stored), W = the panel's W columns (Wb, leading dimension ld).
-// Tiles of TB_ROWS x BC on a grid starting at q0 rounded down to 4; thread (tr, tc) owns
-// rows 4tr..+3 and 64+4tr..+3 and columns 4tc..+3 of a tile.  V and W rows of the tile's
-// rows and columns are staged TB_KC panel columns at a time.
-template <int NT>
-__device__ void trail_update(float *__restrict__ A, const float *__restrict__ Wb, int n, int ld, int p0,
-                             int nb, float *stage) {
-    constexpr int BC = tb_cols(NT);
-    constexpr int F4 = (2 * TB_ROWS + 2 * BC) / 4;     // staged float4 per panel column
-    const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-    const int q0 = p0 + nb;
-    const int R0 = q0 & ~3;
-    const int mr = n - R0;
-    const int ti = (mr + TB_ROWS - 1) / TB_ROWS, tj = (mr + BC - 1) / BC;
-    constexpr int TBS = tb_stage(NT);                 // floats of one staging buffer
-    for (int I = 0; I < ti; I++) {
-        const int jmax = min(tj - 1, (TB_ROWS * I + TB_ROWS - 1) / BC);
-        for (int J = 0; J <= jmax; J++) {
-            const int rb = R0 + TB_ROWS * I, cb = R0 + BC * J;
-            const bool full = rb + TB_ROWS <= n && cb + BC <= n && cb >= q0 && cb + BC - 1 <= rb;
-            float a[8][4];
-            #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int c = cb + 4 * tc + j;
-                #pragma unroll
-                for (int hh = 0; hh < 2; hh++) {
-                    const int r = rb + 64 * hh + 4 * tr;
-                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (full || (r < n && c < n)) v = __ldcg(reinterpret_cast<const float4 *>(A + (size_t)c * ld + r));
-                    a[4 * hh + 0][j] = v.x; a[4 * hh + 1][j] = v.y; a[4 * hh + 2][j] = v.z; a[4 * hh + 3][j] = v.w;
-                }
-            }
-            // V and W rows of the tile's rows and columns, TB_KC panel columns at a time, copied
-            // by cp.async into one of two buffers while the other is in use
-            auto stage_chunk = [&](int j0, int buf) {
-                const int kc = min(TB_KC, nb - j0);
-                float *Vr = stage + buf * TBS, *Wr = Vr + TB_KC * TB_ROWS, *Vc = Wr + TB_KC * TB_ROWS, *Wc = Vc + TB_KC * BC;
-                for (int idx = tid; idx < kc * F4; idx += NT) {
-                    const int jj = idx / F4, o = idx - jj * F4;
-                    int row, part;
-                    if (o < TB_ROWS / 4) { part = 0; row = rb + 4 * o; }
-                    else if (o < TB_ROWS / 2) { part = 1; row = rb + 4 * (o - TB_ROWS / 4); }
-                    else if (o < TB_ROWS / 2 + BC / 4) { part = 2; row = cb + 4 * (o - TB_ROWS / 2); }
-                    else { part = 3; row = cb + 4 * (o - TB_ROWS / 2 - BC / 4); }
-                    const float *src = (part == 0 || part == 2) ? A + (size_t)(p0 + j0 + jj) * ld
-                                                                : Wb + (size_t)(j0 + jj) * ld;
-                    float *dst = part == 0 ? Vr + jj * TB_ROWS + (row - rb)
-                               : part == 1 ? Wr + jj * TB_ROWS + (row - rb)
-                               : part == 2 ? Vc + jj * BC + (row - cb)
-                                           : Wc + jj * BC + (row - cb);
-                    cp_async16(dst, row < n ? src + row : src, row < n);
-                }
-                cp_async_commit();
-            };
-            __syncthreads();   // the previous tile's reads of both buffers are done
-            stage_chunk(0, 0);
-            for (int j0 = 0, buf = 0; j0 < nb; j0 += TB_KC, buf ^= 1) {
-                const int kc = min(TB_KC, nb - j0);
-                if (j0 + TB_KC < nb) {
-                    stage_chunk(j0 + TB_KC, buf ^ 1);
-                    cp_async_wait<1>();
-                } else {
-                    cp_async_wait<0>();
-                }
-                __syncthreads();   // every thread's copies of this chunk are in
-                const float *Vr = stage + buf * TBS, *Wr = Vr + TB_KC * TB_ROWS, *Vc = Wr + TB_KC * TB_ROWS,
-                            *Wc = Vc + TB_KC * BC;
-                for (int jj = 0; jj < kc; jj++) {
-                    const float4 v0 = *reinterpret_cast<const float4 *>(Vr + jj * TB_ROWS + 4 * tr);
-                    const float4 v1 = *reinterpret_cast<const float4 *>(Vr + jj * TB_ROWS + 64 + 4 * tr);
-                    const float4 w0 = *reinterpret_cast<const float4 *>(Wr + jj * TB_ROWS + 4 * tr);
-                    const float4 w1 = *reinterpret_cast<const float4 *>(Wr + jj * TB_ROWS + 64 + 4 * tr);
-                    const float4 vc4 = *reinterpret_cast<const float4 *>(Vc + jj * BC + 4 * tc);
-                    const float4 wc4 = *reinterpret_cast<const float4 *>(Wc + jj * BC + 4 * tc);
-                    const float vr[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-                    const float wr[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-                    const float vc[4] = {vc4.x, vc4.y, vc4.z, vc4.w};
-                    const float wc[4] = {wc4.x, wc4.y, wc4.z, wc4.w};
-                    #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        #pragma unroll
-                        for (int j = 0; j < 4; j++) a[i][j] = fmaf(-vr[i], wc[j], fmaf(-wr[i], vc[j], a[i][j]));
-                }
-                __syncthreads();   // this buffer is refilled by the next chunk's copies
-            }
-            #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int c = cb + 4 * tc + j;
-                #pragma unroll
-                for (int hh = 0; hh < 2; hh++) {
-                    const int r = rb + 64 * hh + 4 * tr;
-                    float *dst = A + (size_t)c * ld + r;
-                    if (full) {
-                        __stcg(reinterpret_cast<float4 *>(dst),
-                               make_float4(a[4 * hh][j], a[4 * hh + 1][j], a[4 * hh + 2][j], a[4 * hh + 3][j]));
-                    } else if (c < n && c >= q0) {
-                        #pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            if (r + q < n && r + q >= c) dst[q] = a[4 * hh + q][j];
-                    }
-                }
-            }
-        }
-    }
-}
-
-// Phase 1 for orders above 256 (LAPACK ssytrd with lower storage, panels of TB_NB columns;
-// the same reflectors, d, e and tau conventions as the unblocked path).  Wb (TB_NB columns
-// of leading dimension ld) holds the panel's W; x, ywall (one partial product of order n32
-// per warp), pv (4 x TB_NB) and stage (aliasing ywall) are shared memory.
-template <int NT, int NMAX>
-__device__ void tridiag_blocked(float *__restrict__ A, float *__restrict__ Wb, int n, int ld, float *d, float *e,
-                                float *tau, float *x, float *ywall, float *pv, float *red, unsigned long long *pt,
-                                int tq_order) {
-    constexpr int NW = NT / 32;
-    constexpr int RW = (NMAX + NT - 1) / NT;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n32 = (n + 31) & ~31;
-    const int tn = n32 >> 5;
-    float *sv = pv, *sw = pv + TB_NB, *t1 = pv + 2 * TB_NB, *t2 = pv + 3 * TB_NB;
-    float *ywp = ywall + (size_t)warp * n32;
-    for (int i = tid; i < n32; i += NT) x[i] = 0.f;
-    __syncthreads();
-    // optional per-phase timers (pt[12..17]), read by thread 0 after a block-wide barrier
-    unsigned long long tlast = (pt && tid == 0) ? globaltimer_ns() : 0ull;
-    auto mark = [&](int slot) {
-        if (!pt) return;
-        __syncthreads();
-        if (tid == 0) {
-            const unsigned long long t = globaltimer_ns();
-            pt[slot] += t - tlast;
-            tlast = t;
-        }
-    };
-    const int nref = n - 2;       // columns 0 .. n-3 carry reflectors
-    for (int p0 = 0; p0 < nref; p0 += TB_NB) {
-        const int nb = min(TB_NB, nref - p0);
-        float xn2 = 0.f;   // |column k below k+1|^2; after the first column of a panel it comes
-                           // from the previous column's step (d), which also leaves d[k], the
-                           // alpha in red[48] and the rest of the column in x
-        for (int kk = 0; kk < nb; kk++) {
-            const int k = p0 + kk;
-            if (kk == 0) {
-                // (a) column k (rows k..n-1): the panel's first, unaffected by its reflectors
-                float part = 0.f;
-                for (int r = k + tid; r < n; r += NT) {
-                    const float v = A[(size_t)k * ld + r];
-                    if (r == k) d[k] = v;
-                    else if (r == k + 1) red[48] = v;
-                    else { x[r] = v; part += v * v; }
-                }
-                xn2 = block_sum<NT>(part, red);
-            }
-            mark(12);
-            // (b) the reflector (slarfg convention: v[0] = 1, beta = -sign(alpha)*norm)
-            if (tid == 0) {
-                const float alpha = red[48];
-                float t = 0.f, beta = alpha, scale = 0.f;
-                if (xn2 > 0.f) {
-                    beta = -copysignf(sqrtf(alpha * alpha + xn2), alpha);
-                    t = (beta - alpha) / beta;
-                    scale = 1.f / (alpha - beta);
-                }
-                tau[k] = t;
-                e[k] = beta;
-                red[49] = scale;
-            }
-            __syncthreads();
-            const float scale = red[49];
-            const float tk = tau[k];
-            // v (unit element at k+1, stored in A during the panel) into x; x[k] cleared
-            for (int r = k + tid; r < n; r += NT) {
-                const float v = r == k ? 0.f : (r == k + 1 ? 1.f : x[r] * scale);
-                x[r] = v;
-                if (r > k) A[(size_t)k * ld + r] = v;
-            }
-            const int j0 = (k + 1) >> 5;
-            for (int i = 32 * j0 + lane; i < n32; i += 32) ywp[i] = 0.f;
-            __syncthreads();
-            mark(13);
-            // (c) y = A22 v on the panel-start trailing block, plus t1 = W^T v, t2 = V^T v.
-            // Within a panel consecutive columns read the same tiles (A is not updated until the
-            // panel ends), so alternate columns walk them in opposite orders: a column starts on
-            // the tiles the previous column (or the trailing update, for a panel's first column)
-            // read last, which are the ones most likely still in L2.
-            {
-                const int tt = tn - j0;
-                const int ntiles = tt * (tt + 1) / 2;
-                const bool rev = tq_order && (kk & 1) == 0;
-                // tile of position L of the row-major enumeration of the lower triangle
-                auto tile_of = [&](int L, int &Ii, int &Jj) {
-                    int i = (int)((sqrtf(8.f * (float)L + 1.f) - 1.f) * 0.5f);
-                    while (i * (i + 1) / 2 > L) i--;
-                    while ((i + 1) * (i + 2) / 2 <= L) i++;
-                    Ii = i;
-                    Jj = L - i * (i + 1) / 2;
-                };
-                for (int q = warp; q < ntiles; q += NW) {
-                    int Ii, Jj;
-                    tile_of(rev ? ntiles - 1 - q : q, Ii, Jj);
-                    if (q + NW < ntiles) {   // this warp's next tile: its lines are requested into L2
-                        int In, Jn;
-                        tile_of(rev ? ntiles - 1 - (q + NW) : q + NW, In, Jn);
-                        const int c = 32 * (j0 + Jn) + lane;
-                        if (c < n) prefetch_l2(A + (size_t)c * ld + 32 * (j0 + In));
-                    }
-                    const int I = j0 + Ii, J = j0 + Jj;
-                    if (I == J || 32 * I + 32 > n) symv_tile<true>(A, ld, n, I, J, x, ywp, lane);
-                    else symv_tile<false>(A, ld, n, I, J, x, ywp, lane);
-                }
-            }
-            mark(14);
-            for (int dq = warp; dq < 2 * kk; dq += NW) {
-                const float *col = dq < kk ? Wb + (size_t)dq * ld : A + (size_t)(p0 + dq - kk) * ld;
-                float s = 0.f;
-                float s2 = 0.f;            // two chains, four loads in flight per lane
-                int r = k + 1 + lane;
-                for (; r + 32 < n; r += 64) {
-                    s = fmaf(col[r], x[r], s);
-                    s2 = fmaf(col[r + 32], x[r + 32], s2);
-                }
-                if (r < n) s = fmaf(col[r], x[r], s);
-                s += s2;
-                s = warp_sum(s);
-                if (lane == 0) {
-                    if (dq < kk) t1[dq] = s;
-                    else t2[dq - kk] = s;
-                }
-            }
-            __syncthreads();
-            mark(15);
-            // (d) w = tau (y - V t1 - W t2), then w -= (tau/2)(w.v) v, into column kk of Wb.
-            // When the next column is in this panel, the same pass over the panel's first kk
-            // columns also applies them to column k+1 (its step (a): rows k+1.., held by the
-            // threads that own those rows in step (b)), and the kk-th term v_k w_k[k+1] + w_k
-            // (v_k[k+1] = 1) follows once w is final.
-            const bool fuse = kk + 1 < nb;
-            if (fuse) {
-                if (tid < kk) {                     // row k+1 of the panel's V and W
-                    sv[tid] = A[(size_t)(p0 + tid) * ld + k + 1];
-                    sw[tid] = Wb[(size_t)tid * ld + k + 1];
-                }
-                __syncthreads();
-            }
-            float wr[RW], cr[RW];
-            float dpart = 0.f;
-            #pragma unroll
-            for (int i = 0; i < RW; i++) {
-                const int r = k + 1 + tid + i * NT;
-                float w = 0.f, c = 0.f;
-                if (r < n) {
-                    float y = 0.f;
-                    #pragma unroll
-                    for (int ww = 0; ww < NW; ww++) y += ywall[(size_t)ww * n32 + r];
-                    if (fuse) {
-                        c = A[(size_t)(k + 1) * ld + r];
-                        for (int jj = 0; jj < kk; jj++) {
-                            const float vj = A[(size_t)(p0 + jj) * ld + r], wj = Wb[(size_t)jj * ld + r];
-                            y -= vj * t1[jj] + wj * t2[jj];
-                            c -= vj * sw[jj] + wj * sv[jj];
-                        }
-                    } else {
-                        for (int jj = 0; jj < kk; jj++)
-                            y -= A[(size_t)(p0 + jj) * ld + r] * t1[jj] + Wb[(size_t)jj * ld + r] * t2[jj];
-                    }
-                    w = tk * y;
-                    dpart += w * x[r];
-                }
-                wr[i] = w;
-                cr[i] = c;
-            }
-            const float dot = block_sum<NT>(dpart, red);
-            const float half = -0.5f * tk * dot;
-            #pragma unroll
-            for (int i = 0; i < RW; i++) {
-                const int r = k + 1 + tid + i * NT;
-                if (r < n) {
-                    wr[i] += half * x[r];
-                    Wb[(size_t)kk * ld + r] = wr[i];
-                    if (r == k + 1) red[50] = wr[i];
-                }
-            }
-            if (fuse) {
-                __syncthreads();                   // w_k[k+1] in red[50]
-                const float wk1 = red[50];
-                float part = 0.f;
-                #pragma unroll
-                for (int i = 0; i < RW; i++) {
-                    const int r = k + 1 + tid + i * NT;
-                    if (r < n) {
-                        const float c = cr[i] - x[r] * wk1 - wr[i];
-                        if (r == k + 1) d[k + 1] = c;
-                        else if (r == k + 2) red[48] = c;
-                        else { x[r] = c; part += c * c; }
-                    }
-                }
-                xn2 = block_sum<NT>(part, red);
-            }
-            __syncthreads();
-            mark(16);
-        }
-        // (e) the trailing block beyond the panel
-        trail_update<NT>(A, Wb, n, ld, p0, nb, ywall);
-        __syncthreads();
-        mark(17);
-    }
-    if (tid == 0) {
-        d[n - 2] = A[(size_t)(n - 2) * ld + n - 2];
-        e[n - 2] = A[(size_t)(n - 2) * ld + n - 1];
-        d[n - 1] = A[(size_t)(n - 1) * ld + n - 1];
-        tau[n - 2] = 0.f;
-        e[n - 1] = 0.f;
-    }
-    __syncthreads();
-}
-
-// Phase 1 of matrix `mat` of a (the body of k_eigh_tq and of k_eigh_tq_multi).
-template <int NT, int NMAX, bool BLK>
-__device__ __forceinline__ void tq_body(const EighArgs &a, int mat) {
-    constexpr int QG = (NMAX + 4 * NT - 1) / (4 * NT); // 4-row groups per thread, phase 1
-    constexpr int NW = NT / 32;
-    extern __shared__ __align__(16) float smem[];
-    const int n = a.n, ld = a.ld;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    float *A = a.A + (size_t)mat * a.mstride;
-    float *Z = a.Z + (size_t)mat * (a.zstride ? a.zstride : a.mstride);
-
-    const int n4 = (n + 3) & ~3;
-    float *d = smem;             // [n4]
-    float *e = d + n4;           // [n4]
-    float *tau = e + n4;         // [n4]
-    float *U = tau + n4;         // union region (tq_union_floats)
-    float *red = U + tq_union_floats(n, NT, BLK);   // [64]
-
-    unsigned long long *pt = a.phase_ns ? a.phase_ns + (size_t)mat * CIR_EIG_PROF_SLOTS : nullptr;
-    if (pt && tid == 0) pt[0] = globaltimer_ns();
-    if (a.status && tid == 0) a.status[mat] = 0;
-    // ---------------- phase 1: tridiagonalisation ----------------
-    if constexpr (BLK) {
-        // W of the current panel lives in Z, which phase 2 overwrites
-        const int n32 = (n + 31) & ~31;
-        const int yws = max(n32 * NW, 2 * tb_stage(NT));
-        tridiag_blocked<NT, NMAX>(A, Z, n, ld, d, e, tau, U, U + n32, U + n32 + yws, red, pt, a.tq_order);
-    } else {
-        float *vp = U, *wp = U + n4, *vc = U + 2 * n4, *wc = U + 3 * n4;
-        // the first column reads vp / wp (scaled by zero) before any update has written them:
-        // clear them, since 0 * (a NaN or infinity left in shared memory) is NaN
-        for (int i = tid; i < 4 * n4; i += NT) U[i] = 0.f;
-        __syncthreads();
-        bool pending = false;
-        for (int k = 0; k + 2 < n; k++) {
-            // (a) column k below the diagonal with the pending rank-2 update applied
-            float part = 0.f;
-            for (int i = k + tid; i < n; i += NT) {
-                float v = A[(size_t)k * ld + i];
-                if (pending) v -= vp[i] * wp[k] + wp[i] * vp[k];
-                if (i == k) d[k] = v;
-                else if (i == k + 1) red[48] = v;   // alpha
-                else { vc[i] = v; part += v * v; }
-            }
-            const float xn2 = block_sum<NT>(part, red);
-            // (b) the reflector (slarfg convention: v[0] = 1, beta = -sign(alpha)*norm)
-            if (tid == 0) {
-                const float alpha = red[48];
-                float t = 0.f, beta = alpha, scale = 0.f;
-                if (xn2 > 0.f) {
-                    beta = -copysignf(sqrtf(alpha * alpha + xn2), alpha);
-                    t = (beta - alpha) / beta;
-                    scale = 1.f / (alpha - beta);
-                }
-                tau[k] = t;
-                e[k] = beta;
-                red[49] = scale;
-            }
-            __syncthreads();
-            const float scale = red[49];
-            const float tk = tau[k];
-            for (int i = k + 2 + tid; i < n; i += NT) {
-                const float v = vc[i] * scale;
-                vc[i] = v;
-                A[(size_t)k * ld + i] = v;
-            }
-            if (tid == 0) vc[k + 1] = 1.f;
-            __syncthreads();
-            // (c) one pass over the trailing block: apply update k-1, accumulate p = A v_k.
-            // Thread t owns the 4-row groups starting at r_al + 4*(t + q*NT).
-            const int r0 = k + 1;
-            const int r_al = r0 & ~3;
-            float p[QG][4];
-            float vr[QG][4], wr[QG][4];
-            #pragma unroll
-            for (int q = 0; q < QG; q++)
-                #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int r = r_al + 4 * (tid + q * NT) + j;
-                    const bool in = r >= r0 && r < n;
-                    p[q][j] = 0.f;
-                    vr[q][j] = (pending && in) ? vp[r] : 0.f;
-                    wr[q][j] = (pending && in) ? wp[r] : 0.f;
-                }
-            int c = r0;
-            for (; c + 3 < n; c += 4) {
-                float4 col[4][QG];
-                #pragma unroll
-                for (int cc = 0; cc < 4; cc++)
-                    #pragma unroll
-                    for (int q = 0; q < QG; q++) {
-                        const int rb = r_al + 4 * (tid + q * NT);
-                        col[cc][q] = rb < n ? *reinterpret_cast<const float4 *>(A + (size_t)(c + cc) * ld + rb)
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                #pragma unroll
-                for (int cc = 0; cc < 4; cc++) {
-                    const float vpc = vp[c + cc], wpc = wp[c + cc], vcc = vc[c + cc];
-                    #pragma unroll
-                    for (int q = 0; q < QG; q++) {
-                        const int rb = r_al + 4 * (tid + q * NT);
-                        if (rb >= n) continue;
-                        float x[4] = {col[cc][q].x, col[cc][q].y, col[cc][q].z, col[cc][q].w};
-                        #pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            const float v = x[j] - (vr[q][j] * wpc + wr[q][j] * vpc);
-                            x[j] = v;
-                            p[q][j] += v * vcc;
-                        }
-                        if (pending)
-                            *reinterpret_cast<float4 *>(A + (size_t)(c + cc) * ld + rb) = make_float4(x[0], x[1], x[2], x[3]);
-                    }
-                }
-            }
-            for (; c < n; c++) {
-                const float vpc = vp[c], wpc = wp[c], vcc = vc[c];
-                #pragma unroll
-                for (int q = 0; q < QG; q++) {
-                    const int rb = r_al + 4 * (tid + q * NT);
-                    if (rb >= n) continue;
-                    float4 v4 = *reinterpret_cast<const float4 *>(A + (size_t)c * ld + rb);
-                    float x[4] = {v4.x, v4.y, v4.z, v4.w};
-                    #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const float v = x[j] - (vr[q][j] * wpc + wr[q][j] * vpc);
-                        x[j] = v;
-                        p[q][j] += v * vcc;
-                    }
-                    if (pending) *reinterpret_cast<float4 *>(A + (size_t)c * ld + rb) = make_float4(x[0], x[1], x[2], x[3]);
-                }
-            }
-            // rows below r0 saw vr = wr = 0 and contribute nothing
-            float dpart = 0.f;
-            #pragma unroll
-            for (int q = 0; q < QG; q++)
-                #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int r = r_al + 4 * (tid + q * NT) + j;
-                    if (r >= r0 && r < n) {
-                        p[q][j] *= tk;
-                        dpart += p[q][j] * vc[r];
-                    }
-                }
-            const float dot = block_sum<NT>(dpart, red);
-            const float half = 0.5f * tk * dot;
-            #pragma unroll
-            for (int q = 0; q < QG; q++)
-                #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int r = r_al + 4 * (tid + q * NT) + j;
-                    if (r >= r0 && r < n) wc[r] = p[q][j] - half * vc[r];
-                }
-            __syncthreads();
-            float *t0 = vp; vp = vc; vc = t0;
-            float *t1 = wp; wp = wc; wc = t1;
-            pending = true;
-        }
-        if (tid == 0) {
-            if (n >= 2) {
-                float a00 = A[(size_t)(n - 2) * ld + n - 2], a10 = A[(size_t)(n - 2) * ld + n - 1];
-                float a11 = A[(size_t)(n - 1) * ld + n - 1];
-                if (pending) {
-                    a00 -= 2.f * vp[n - 2] * wp[n - 2];
-                    a10 -= vp[n - 1] * wp[n - 2] + wp[n - 1] * vp[n - 2];
-                    a11 -= 2.f * vp[n - 1] * wp[n - 1];
-                }
-                d[n - 2] = a00;
-                d[n - 1] = a11;
-                e[n - 2] = a10;
-                tau[n - 2] = 0.f;
-            } else {
-                d[0] = A[0];
-            }
-            e[n - 1] = 0.f;
-        }
-        __syncthreads();
-    }
-
-    // d, e and tau for the next two kernels
-    float *de = a.DE + (size_t)mat * 3 * ld;
-    for (int i = tid; i < n; i += NT) {
-        de[i] = d[i];
-        de[ld + i] = e[i];
-        de[2 * ld + i] = tau[i];
-    }
-    if (pt) {
-        __syncthreads();
-        if (tid == 0) pt[1] = globaltimer_ns();
-    }
-}
-
-template <int NT, int NMAX, int MINB, bool BLK>
-__global__ void __launch_bounds__(NT, MINB) k_eigh_tq(EighArgs a) {
-    tq_body<NT, NMAX, BLK>(a, blockIdx.x);
-}
-
-// Several batches of the blocked form in one launch (orders 257-1024, the order-1024
-// instantiation for all): problem p covers blocks start[p] .. start[p+1]-1, the problems in
-// descending order, so that the longest matrices start first and the shorter ones fill
-// the last wave.
-struct TqPlan {
-    EighArgs a[CIR_TQ_MAXP];
-    int start[CIR_TQ_MAXP + 1];
-    int np;
-};
-
-template <int NT, int NMAX, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_eigh_tq_multi(const __grid_constant__ TqPlan plan) {
-    int p = 0;
-    while (p + 1 < plan.np && (int)blockIdx.x >= plan.start[p + 1]) p++;
-    tq_body<NT, NMAX, true>(plan.a[p], (int)blockIdx.x - plan.start[p]);
 }
 
 // Sum NV per-lane values over the warp by halving exchanges (lane bit 4 first): lane L ends
@@ -1288,37 +623,6 @@ __global__ void __launch_bounds__(NT, 3) k_eigh_qr(EighArgs a) {
     }
 }
 
-// MINB: resident blocks per SM the register budget is fitted to (3 while the spill stays
-// negligible; the order-2048 variant is fitted to 2 blocks).
-template <int NT, int NMAX, int MINB, bool BLK>
-cudaError_t launch_tq(const EighArgs &a, int nmat, cudaStream_t s) {
-    auto kern = k_eigh_tq<NT, NMAX, MINB, BLK>;
-    const size_t smem = tq_smem_bytes(a.n, NT, BLK);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    static const int order = [] {
-        const char *v = getenv("CIR_TQ_ORDER");
-        return v ? atoi(v) : 1;
-    }();
-    EighArgs b = a;
-    b.tq_order = order;
-    size_t req = smem;
-    if (a.tq_blocks > 0 && a.tq_blocks < MINB) {
-        // fewer blocks per SM: ask for enough shared memory that only tq_blocks fit
-        int dev = 0, per_sm = 0, reserved = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess ||
-            (e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess)
-            return e;
-        const size_t want = (size_t)per_sm / (a.tq_blocks + 1) - (size_t)reserved + 1024;
-        if (want > req) req = want;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)req)) != cudaSuccess)
-            return e;
-    }
-    kern<<<nmat, NT, req, s>>>(b);
-    return cudaGetLastError();
-}
-
 template <int NT, int NMAX, int NBQ, int CB, int MINB>
 cudaError_t launch_formq(const EighArgs &a, int nmat, cudaStream_t s) {
     auto kern = k_eigh_formq<NT, NMAX, NBQ, CB, MINB>;
@@ -1348,54 +652,6 @@ size_t cir_eigh_rot_bytes(int n) { return sizeof(float2) * 2 * EIG_KS * (size_t)
 size_t cir_eigh_de_bytes(int ld) { return sizeof(float) * 3 * (size_t)ld; }
 
 int cir_eigh_max_n() { return 2048; }
-
-int cir_tridiag_blocks(int n) { return n <= 256 ? 4 : (n <= 1024 ? 3 : 2); }
-
-size_t cir_tridiag_w_floats(int ld) { return (size_t)TB_NB * ld; }
-
-cudaError_t cir_launch_tridiag_multi(const EighArgs *a, const int *nmat, int np, cudaStream_t s, int *launches) {
-    if (np < 1 || np > CIR_TQ_MAXP) return cudaErrorInvalidValue;
-    int order[CIR_TQ_MAXP];
-    for (int i = 0; i < np; i++) {
-        const EighArgs &x = a[i];
-        if (x.n <= 256 || x.n > 1024 || nmat[i] < 1 || nmat[i] > 65535 || (x.ld & 3) || x.ld < x.n || !x.DE ||
-            (reinterpret_cast<uintptr_t>(x.A) & 15) || (reinterpret_cast<uintptr_t>(x.Z) & 15))
-            return cudaErrorInvalidValue;
-        order[i] = i;
-    }
-    std::sort(order, order + np, [&](int x, int y) { return a[x].n > a[y].n; });
-    static const int tq_order = [] {
-        const char *v = getenv("CIR_TQ_ORDER");
-        return v ? atoi(v) : 1;
-    }();
-    TqPlan plan;
-    memset(&plan, 0, sizeof plan);
-    plan.np = np;
-    size_t smem = 0;
-    int total = 0;
-    for (int k = 0; k < np; k++) {
-        plan.a[k] = a[order[k]];
-        plan.a[k].tq_order = tq_order;
-        plan.start[k] = total;
-        total += nmat[order[k]];
-        smem = std::max(smem, tq_smem_bytes(plan.a[k].n, 256, true));
-    }
-    plan.start[np] = total;
-    auto kern = k_eigh_tq_multi<256, 1024, 3>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<total, 256, smem, s>>>(plan);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (launches) *launches += 1;
-    return cudaSuccess;
-}
-
-cudaError_t cir_launch_tridiag(const EighArgs &a, int nmat, cudaStream_t s) {
-    if (a.n <= 256) return launch_tq<128, 256, 4, false>(a, nmat, s);
-    if (a.n <= 512) return launch_tq<256, 512, 3, true>(a, nmat, s);
-    if (a.n <= 1024) return launch_tq<256, 1024, 3, true>(a, nmat, s);
-    return launch_tq<256, 2048, 2, true>(a, nmat, s);
-}
 
 cudaError_t cir_launch_eigh(const EighArgs &a, int nmat, cudaStream_t s, int *launches) {
     if (a.n < 1 || a.n > cir_eigh_max_n() || nmat < 1 || nmat > 65535 || (a.ld & 3) || a.ld < a.n)

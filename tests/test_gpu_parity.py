@@ -450,3 +450,24 @@ def test_lineshape_forms(lib, ntcf, nzeros):
     np.testing.assert_array_equal(om, om_ref.astype(np.float32))
     # four FP32 roundings (the sum, the axis step, the norm and the quotient), 6e-8 each
     assert O.rel_l2(val, val_ref) < 5e-7
+
+
+# every form of the tridiagonalisation and the edges between them (152 SMs): resident in shared
+# memory (n <= 128 in 4 warps for large batches, 8 warps up to 192, up to 256 for a single wave),
+# streaming with two blocks per SM or one (n <= 512), one block or a cluster per matrix (n > 512)
+@pytest.mark.parametrize("n,nmat", [(4, 305), (33, 3), (128, 305), (129, 2), (192, 2), (193, 153), (256, 2), (256, 153),
+                                    (260, 2), (353, 153), (512, 153), (512, 2), (513, 2), (642, 12), (801, 30),
+                                    (770, 60), (1025, 2), (1031, 20)])
+def test_eigh_forms(lib, n, nmat):
+    rng = np.random.default_rng(n + nmat)
+    p = lib.default_params(species="H2O")
+    base = rng.standard_normal((2, n, n)).astype(np.float32) * 5
+    base = base + base.transpose(0, 2, 1)
+    base[:, np.arange(n), np.arange(n)] += 150 * rng.standard_normal((2, n)).astype(np.float32)
+    A = np.ascontiguousarray(base[np.arange(nmat) % 2])
+    with lib.Engine(p, 8) as eng:
+        w, V = eng.eigh(A)
+    for i in sorted({0, 1, nmat - 1}):
+        _check_eig(A[i], w[i], V[i])
+    for i in range(2, nmat):      # every matrix of the batch, to the last bit
+        assert np.array_equal(w[i], w[i % 2]) and np.array_equal(V[i], V[i % 2])
