@@ -471,3 +471,16 @@ def test_eigh_forms(lib, n, nmat):
         _check_eig(A[i], w[i], V[i])
     for i in range(2, nmat):      # every matrix of the batch, to the last bit
         assert np.array_equal(w[i], w[i % 2]) and np.array_equal(V[i], V[i % 2])
+
+
+@pytest.mark.parametrize("nmol,nframes", [(8, 3), (33, 250), (100, 120)])
+def test_build_forms(lib, nmol, nframes):
+    """A batch (a thread per chromophore, four tiles of H a block) equals its frames built one by
+    one (a warp per chromophore, one tile a block) to the last bit."""
+    xyz, box = lib.synth_trajectory(nmol, nframes, seed=nmol)
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 4 * nmol) as eng:
+        batch = eng.build_hamiltonian(xyz, box)
+        for f in (0, 1, nframes // 2, nframes - 1):
+            one = eng.build_hamiltonian(xyz[f:f + 1], box)
+            for b, o in zip(batch, one):
+                np.testing.assert_array_equal(b[f], o[0])
