@@ -764,24 +764,18 @@ extern "C" int cir_spectral_density(cir_ctx *c, int n, const float *V, const flo
     if ((rc = stage_in(c, B_IN0, V, (size_t)n * n * 4, &dV, true))) return rc;
     if ((rc = stage_in(c, B_IN1, w, (size_t)n * 4, &dW, true))) return rc;
     if ((rc = stage_in(c, B_IN2, dip, (size_t)3 * n * 4, &dD, true))) return rc;
-    CK(c->buf[B_SCR].ensure((size_t)n * 4 + (size_t)nomega * 8 + 64));
-    float *mu2 = c->buf[B_SCR].as<float>();
-    double *acc = reinterpret_cast<double *>(c->buf[B_SCR].as<char>() + (((size_t)n * 4 + 15) & ~(size_t)15));
-    CK(cudaMemsetAsync(acc, 0, (size_t)nomega * 8, c->stream));
+    CK(c->buf[B_SCR].ensure((size_t)(n + nomega) * 4));
+    float *mu2 = c->buf[B_SCR].as<float>(), *sum = mu2 + n;
+    const bool dev = is_device_ptr(Sw);   // added to in place, on the stream
+    if (!dev) CK(cudaMemcpyAsync(sum, Sw, (size_t)nomega * 4, cudaMemcpyHostToDevice, c->stream));
     int launches = 0;
-    CK(cir_launch_spectral(static_cast<float *>(dV), n, static_cast<float *>(dW), static_cast<float *>(dD), n, n, mu2,
-                           acc, nomega, c->p.omegaStart, c->p.omegaStep, c->p.t1, c->p.avef, c->stream, &launches));
+    CK(cir_launch_spectral(static_cast<float *>(dV), n, 0, static_cast<float *>(dW), 0, static_cast<float *>(dD), n, 0, n, 1, 1,
+                           mu2, nullptr, dev ? Sw : sum, nomega, c->p.omegaStart, c->p.omegaStep, c->p.t1, c->p.avef,
+                           c->stream, &launches));
     count_launch(c, launches);
-    std::vector<double> h(nomega);
-    CK(cudaMemcpyAsync(h.data(), acc, (size_t)nomega * 8, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (is_device_ptr(Sw)) {
-        std::vector<float> cur(nomega);
-        CK(cudaMemcpy(cur.data(), Sw, (size_t)nomega * 4, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < nomega; i++) cur[i] += (float)h[i];
-        CK(cudaMemcpy(Sw, cur.data(), (size_t)nomega * 4, cudaMemcpyHostToDevice));
-    } else {
-        for (int i = 0; i < nomega; i++) Sw[i] += (float)h[i];
+    if (!dev) {
+        CK(cudaMemcpyAsync(Sw, sum, (size_t)nomega * 4, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
     }
     return CIR_OK;
 }
@@ -977,7 +971,7 @@ struct GroupJob {
         CK(buf[B_OOR].ensure((size_t)T * 8));
         CK(buf[B_SWEEPS].ensure(8));
         CK(buf[B_SW].ensure((size_t)T * nomega * 8));
-        CK(buf[B_MU2].ensure((size_t)ld * 4));
+        CK(buf[B_MU2].ensure((size_t)St * n * 4));
         CK(cudaMemsetAsync(buf[B_TCF].p, 0, (size_t)steps * 48, c->stream));
         CK(cudaMemsetAsync(buf[B_HCNT].p, 0, (size_t)T * nomega * 8, c->stream));
         CK(cudaMemsetAsync(buf[B_HIPR].p, 0, (size_t)T * nomega * 8, c->stream));
@@ -1239,12 +1233,10 @@ struct GroupJob {
         CK(cudaEventRecord(ev[3], c->stream));
         if (k0 == 0) {
             // spectral density at step 0 of every origin (calcIR.cu:456-482), per trajectory
-            for (int s = 0; s < St; s++) {
-                const size_t b = (size_t)base0 + (size_t)s * dlt;
-                CK(cir_launch_spectral(A + b * mstride, ld, W + b * ld, M + b * 9 * ld, ld, n, buf[B_MU2].as<float>(),
-                                       buf[B_SW].as<double>() + (size_t)(s / S) * nomega, nomega, p.omegaStart,
-                                       p.omegaStep, p.t1, p.avef, c->stream, &launches));
-            }
+            const size_t b = (size_t)base0, d = (size_t)dlt;
+            CK(cir_launch_spectral(A + b * mstride, ld, (long long)(d * mstride), W + b * ld, (long long)(d * ld), M + b * 9 * ld, ld,
+                                   (long long)(d * 9 * ld), n, S, T, buf[B_MU2].as<float>(), buf[B_SW].as<double>(), nullptr,
+                                   nomega, p.omegaStart, p.omegaStep, p.t1, p.avef, c->stream, &launches));
             // F = I and the t = 0 vectors (calcIR.cu:577-594)
             if (vectors) {
                 CK(cir_adj_psi_init(M + (size_t)base0 * 9 * ld, (long long)dlt * 9 * ld, ld, n, St,

@@ -267,10 +267,12 @@ struct TcfArgs {
 };
 cudaError_t cir_launch_tcf(const TcfArgs &t, int batch, cudaStream_t s, int *launches);
 
-// spectral density of one frame: Sw[nomega] += ...
-cudaError_t cir_launch_spectral(const float *V, int ld, const float *w, const float *dip, int ldv, int n,
-                                float *mu2_scratch, double *Sw, int nomega, float omegaStart, int omegaStep,
-                                float t1, float avef, cudaStream_t s, int *launches);
+// spectral density of S * sets frames (strides sV, sw, sdip; set q holds frames qS .. qS + S - 1):
+// Sw[set][nomega] += the set's sum, or, when Swf is given (one set), Swf[nomega] += in FP32;
+// mu2: scratch, n floats per frame
+cudaError_t cir_launch_spectral(const float *V, int ld, long long sV, const float *w, long long sw, const float *dip, int ldv,
+                                long long sdip, int n, int S, int sets, float *mu2, double *Sw, float *Swf, int nomega,
+                                float omegaStart, int omegaStep, float t1, float avef, cudaStream_t s, int *launches);
 
 // The printed rows of a lineshape: outputs i0 .. i0 + cnt1 - 1 of the transform of length n,
 // then outputs 0 .. cnt2 - 1, each over norm (cir_api.cu ls_rows).

@@ -1,11 +1,15 @@
 // Correlation-function contraction and spectral density.
 //
-// k_tcf: psi_a = F m_a(0) for the 9 dipole/polarisability vectors (one warp per row of
-// F), then the 15 unconjugated dot products with m_b(t) the reference evaluates as
-// separate magma_cgemv + magma_cdotu pairs (calcIR.cu:628-745), combined directly into
+// k_tcf: psi_a = F m_a(0) for the 9 dipole/polarisability vectors, then the 15 unconjugated dot
+// products with m_b(t) the reference evaluates as separate magma_cgemv + magma_cdotu pairs
+// (calcIR.cu:628-745), combined directly into
 //     IR = sum_a mu_a(t).F.mu_a(0)
 //     VV = (3 iiFii + iiFjj + 4 ijFij) / 15,   VH = (2 iiFii - iiFjj + 6 ijFij) / 30.
-// Row sums are accumulated in double and stay on the device.
+// A warp takes R rows of F at a time, a column per lane.  The terms are linear in psi, so a
+// lane contracts its own partial psi with m(t) and the sums over columns and rows meet in double
+// at the end (reducing the 18 partial psi of every row over the warp, and the fractions in
+// double by one lane, was 44 us of latency for n = 128 and 120 us for 10 origins at n = 1024).
+// Nothing leaves the device.
 //
 // k_spec_mu2 / k_spec_sum: M = V^T mu (calcIR.cu:462-467) and the Lorentzian sum
 // S(w_i) += sum_j |M_j|^2 g / ((w_i - l_j - avef)^2 + g^2) / pi, g = hbar/(2 T1)
@@ -15,73 +19,91 @@
 namespace {
 
 constexpr int TCF_WARPS = 8;
-constexpr int TCF_ROWS = 64;   // rows of F per block
 
-__global__ void __launch_bounds__(TCF_WARPS * 32) k_tcf(TcfArgs t) {
+// the four sums (re, im) of one row's (partial) psi with m(t): IR, iiFii, ijFij, iiFjj
+__device__ __forceinline__ void tcf_sums(const float (&pr)[9], const float (&pi)[9], const float (&c)[9], double (&acc)[8]) {
+    acc[0] += c[0] * pr[0] + c[1] * pr[1] + c[2] * pr[2];
+    acc[1] += c[0] * pi[0] + c[1] * pi[1] + c[2] * pi[2];
+    acc[2] += c[3] * pr[3] + c[4] * pr[4] + c[5] * pr[5];
+    acc[3] += c[3] * pi[3] + c[4] * pi[4] + c[5] * pi[5];
+    acc[4] += c[6] * pr[6] + c[7] * pr[7] + c[8] * pr[8];
+    acc[5] += c[6] * pi[6] + c[7] * pi[7] + c[8] * pi[8];
+    // xx->yy, xx->zz, yy->xx, yy->zz, zz->xx, zz->yy (psi index 3, 4, 5 = xx, yy, zz)
+    acc[6] += (c[4] + c[5]) * pr[3] + (c[3] + c[5]) * pr[4] + (c[3] + c[4]) * pr[5];
+    acc[7] += (c[4] + c[5]) * pi[3] + (c[3] + c[5]) * pi[4] + (c[3] + c[4]) * pi[5];
+}
+
+// the block's sums into out: IR, VV, VH (re, im)
+__device__ __forceinline__ void tcf_finish(double (&acc)[8], double *out) {
+    __shared__ double part[TCF_WARPS][8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    #pragma unroll
+    for (int q = 0; q < 8; q++) acc[q] = warp_sum_d(acc[q]);
+    if (lane == 0)
+        #pragma unroll
+        for (int q = 0; q < 8; q++) part[warp][q] = acc[q];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int im = threadIdx.x & 1;
+        double s[4] = {0, 0, 0, 0};
+        for (int w = 0; w < TCF_WARPS; w++)
+            #pragma unroll
+            for (int q = 0; q < 4; q++) s[q] += part[w][2 * q + im];
+        const double v = threadIdx.x < 2 ? s[0]
+                       : threadIdx.x < 4 ? (3.0 * s[1] + s[3] + 4.0 * s[2]) / 15.0
+                                         : (2.0 * s[1] - s[3] + 6.0 * s[2]) / 30.0;
+        atomicAdd(out + threadIdx.x, v);
+    }
+}
+
+// rows: the block's rows (a multiple of TCF_WARPS * R)
+template <int R>
+__global__ void __launch_bounds__(TCF_WARPS * 32) k_tcf(TcfArgs t, int rows) {
     extern __shared__ float m0s[];   // [9][n]
-    __shared__ double part[TCF_WARPS][6];
     const int b = blockIdx.y;
     const float *F = t.F + (size_t)b * t.sF;
     const float *m0 = t.m0 + (size_t)b * t.sm0;
     const float *mt = t.mt + (size_t)b * t.smt;
     const int n = t.n;
-    for (int i = threadIdx.x; i < 9 * n; i += blockDim.x) m0s[i] = m0[(size_t)(i / n) * t.ldv + i % n];
+    for (int a = 0; a < 9; a++)
+        for (int i = threadIdx.x; i < n; i += TCF_WARPS * 32) m0s[a * n + i] = m0[(size_t)a * t.ldv + i];
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    const int rend = min(n, (int)(blockIdx.x + 1) * TCF_ROWS);
-    for (int r = blockIdx.x * TCF_ROWS + warp; r < rend; r += TCF_WARPS) {
-        const float2 *row = reinterpret_cast<const float2 *>(F + (size_t)r * t.ldf);
-        float pr[9], pi[9];
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const int rend = min(n, ((int)blockIdx.x + 1) * rows);
+    for (int r0 = blockIdx.x * rows + warp * R; r0 < rend; r0 += TCF_WARPS * R) {
+        float pr[R][9], pi[R][9];
+        const float2 *row[R];
         #pragma unroll
-        for (int a = 0; a < 9; a++) pr[a] = pi[a] = 0.f;
+        for (int i = 0; i < R; i++) {
+            row[i] = reinterpret_cast<const float2 *>(F + (size_t)min(r0 + i, n - 1) * t.ldf);
+            #pragma unroll
+            for (int a = 0; a < 9; a++) pr[i][a] = pi[i][a] = 0.f;
+        }
         for (int q = lane; q < n; q += 32) {
-            const float2 f = row[q];
+            float2 f[R];
+            #pragma unroll
+            for (int i = 0; i < R; i++) f[i] = row[i][q];
             #pragma unroll
             for (int a = 0; a < 9; a++) {
                 const float m = m0s[a * n + q];
-                pr[a] = fmaf(f.x, m, pr[a]);
-                pi[a] = fmaf(f.y, m, pi[a]);
+                #pragma unroll
+                for (int i = 0; i < R; i++) {
+                    pr[i][a] = fmaf(f[i].x, m, pr[i][a]);
+                    pi[i][a] = fmaf(f[i].y, m, pi[i][a]);
+                }
             }
         }
         #pragma unroll
-        for (int a = 0; a < 9; a++) {
-            pr[a] = warp_sum(pr[a]);
-            pi[a] = warp_sum(pi[a]);
-        }
-        if (lane == 0) {
+        for (int i = 0; i < R; i++) {
+            if (r0 + i >= rend) break;
             float c[9];
             #pragma unroll
-            for (int a = 0; a < 9; a++) c[a] = mt[(size_t)a * t.ldv + r];
-            // IR: x, y, z
-            float ir_r = c[0] * pr[0] + c[1] * pr[1] + c[2] * pr[2];
-            float ir_i = c[0] * pi[0] + c[1] * pi[1] + c[2] * pi[2];
-            // iiFii: xx->xx, yy->yy, zz->zz (psi index 3,4,5 = xx,yy,zz)
-            float ii_r = c[3] * pr[3] + c[4] * pr[4] + c[5] * pr[5];
-            float ii_i = c[3] * pi[3] + c[4] * pi[4] + c[5] * pi[5];
-            // ijFij: xy->xy, yz->yz, zx->zx
-            float ij_r = c[6] * pr[6] + c[7] * pr[7] + c[8] * pr[8];
-            float ij_i = c[6] * pi[6] + c[7] * pi[7] + c[8] * pi[8];
-            // iiFjj: xx->yy, xx->zz, yy->xx, yy->zz, zz->xx, zz->yy
-            float jj_r = (c[4] + c[5]) * pr[3] + (c[3] + c[5]) * pr[4] + (c[3] + c[4]) * pr[5];
-            float jj_i = (c[4] + c[5]) * pi[3] + (c[3] + c[5]) * pi[4] + (c[3] + c[4]) * pi[5];
-            acc[0] += ir_r;
-            acc[1] += ir_i;
-            acc[2] += (3.0 * ii_r + jj_r + 4.0 * ij_r) / 15.0;
-            acc[3] += (3.0 * ii_i + jj_i + 4.0 * ij_i) / 15.0;
-            acc[4] += (2.0 * ii_r - jj_r + 6.0 * ij_r) / 30.0;
-            acc[5] += (2.0 * ii_i - jj_i + 6.0 * ij_i) / 30.0;
+            for (int a = 0; a < 9; a++) c[a] = mt[(size_t)a * t.ldv + r0 + i];
+            tcf_sums(pr[i], pi[i], c, acc);
         }
     }
-    if (lane == 0)
-        #pragma unroll
-        for (int q = 0; q < 6; q++) part[warp][q] = acc[q];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double s = 0;
-        for (int w = 0; w < TCF_WARPS; w++) s += part[w][threadIdx.x];
-        atomicAdd(t.out + (size_t)b * t.sout + threadIdx.x, s);
-    }
+    tcf_finish(acc, t.out + (size_t)b * t.sout);
 }
 
 // The same contraction with F stored transposed as a split BF16 pair (the mixed form's
@@ -91,27 +113,8 @@ __global__ void __launch_bounds__(TCF_WARPS * 32) k_tcf(TcfArgs t) {
 // t >> 6) handles row r = 64 blockIdx.x + rr and every fourth q of the block's range.
 constexpr int TT_ROWS = 64, TT_QSPLIT = 4;
 
-__device__ __forceinline__ void tcf_terms(const float (&pr)[9], const float (&pi)[9], const float (&c)[9],
-                                          double (&acc)[6]) {
-    const float ir_r = c[0] * pr[0] + c[1] * pr[1] + c[2] * pr[2];
-    const float ir_i = c[0] * pi[0] + c[1] * pi[1] + c[2] * pi[2];
-    const float ii_r = c[3] * pr[3] + c[4] * pr[4] + c[5] * pr[5];
-    const float ii_i = c[3] * pi[3] + c[4] * pi[4] + c[5] * pi[5];
-    const float ij_r = c[6] * pr[6] + c[7] * pr[7] + c[8] * pr[8];
-    const float ij_i = c[6] * pi[6] + c[7] * pi[7] + c[8] * pi[8];
-    const float jj_r = (c[4] + c[5]) * pr[3] + (c[3] + c[5]) * pr[4] + (c[3] + c[4]) * pr[5];
-    const float jj_i = (c[4] + c[5]) * pi[3] + (c[3] + c[5]) * pi[4] + (c[3] + c[4]) * pi[5];
-    acc[0] += ir_r;
-    acc[1] += ir_i;
-    acc[2] += (3.0 * ii_r + jj_r + 4.0 * ij_r) / 15.0;
-    acc[3] += (3.0 * ii_i + jj_i + 4.0 * ij_i) / 15.0;
-    acc[4] += (2.0 * ii_r - jj_r + 6.0 * ij_r) / 30.0;
-    acc[5] += (2.0 * ii_i - jj_i + 6.0 * ij_i) / 30.0;
-}
-
 __global__ void __launch_bounds__(256) k_tcf_t(TcfArgs t) {
     extern __shared__ float mq[];    // [9][qchunk]
-    __shared__ double part[8][6];
     const int b = blockIdx.z, n = t.n;
     const int qchunk = (n + TT_QSPLIT - 1) / TT_QSPLIT;
     const int qb = blockIdx.y * qchunk, qe = min(n, qb + qchunk);
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(256) k_tcf_t(TcfArgs t) {
     __syncthreads();
     const int rr = threadIdx.x & 63, ql = threadIdx.x >> 6;
     const int r = blockIdx.x * TT_ROWS + rr;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (r < n) {
         const __nv_bfloat16 *fh = t.Ft.hi + (size_t)b * t.sFt + r, *fl = t.Ft.lo + (size_t)b * t.sFt + r;
         float pr[9], pi[9], c[9];
@@ -143,49 +146,57 @@ __global__ void __launch_bounds__(256) k_tcf_t(TcfArgs t) {
         }
         #pragma unroll
         for (int a = 0; a < 9; a++) c[a] = mt[(size_t)a * t.ldv + r];
-        tcf_terms(pr, pi, c, acc);
+        tcf_sums(pr, pi, c, acc);
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    #pragma unroll
-    for (int q = 0; q < 6; q++) acc[q] = warp_sum_d(acc[q]);
-    if (lane == 0)
-        #pragma unroll
-        for (int q = 0; q < 6; q++) part[warp][q] = acc[q];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double s = 0;
-        for (int w = 0; w < 8; w++) s += part[w][threadIdx.x];
-        atomicAdd(t.out + (size_t)b * t.sout + threadIdx.x, s);
-    }
+    tcf_finish(acc, t.out + (size_t)b * t.sout);
 }
 
-__global__ void k_spec_mu2(const float *V, int ld, const float *dip, int ldv, int n, float *mu2) {
+// |M_j|^2 of frame blockIdx.y, a warp per eigenvector
+__global__ void k_spec_mu2(const float *V, int ld, long long sV, const float *dip, int ldv, long long sdip, int n,
+                           float *mu2) {
     const int lane = threadIdx.x & 31;
     const int j = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     if (j >= n) return;
-    const float *col = V + (size_t)j * ld;
+    const float *col = V + (size_t)blockIdx.y * sV + (size_t)j * ld, *d = dip + (size_t)blockIdx.y * sdip;
     float mx = 0, my = 0, mz = 0;
     for (int i = lane; i < n; i += 32) {
         const float v = col[i];
-        mx = fmaf(v, dip[i], mx);
-        my = fmaf(v, dip[ldv + i], my);
-        mz = fmaf(v, dip[2 * ldv + i], mz);
+        mx = fmaf(v, d[i], mx);
+        my = fmaf(v, d[ldv + i], my);
+        mz = fmaf(v, d[2 * ldv + i], mz);
     }
     mx = warp_sum(mx); my = warp_sum(my); mz = warp_sum(mz);
-    if (lane == 0) mu2[j] = mx * mx + my * my + mz * mz;
+    if (lane == 0) mu2[(size_t)blockIdx.y * n + j] = mx * mx + my * my + mz * mz;
 }
 
-__global__ void k_spec_sum(const float *mu2, const float *w, int n, double *Sw, int nomega, float omegaStart,
-                           int omegaStep, float gamma, float avef) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nomega) return;
+// Lorentzian sums of the frames of set blockIdx.y (S consecutive frames): SP_W frequencies a
+// block, the eigenvalues shared by SP_J threads each, the frames one after another, their sums
+// added in double in the frames' order.  Bound by the two divisions of a term; one thread per
+// frequency on 24 blocks, a launch per frame, was 102 us a frame at n = 1024.
+constexpr int SP_W = 32, SP_J = 16;
+__global__ void __launch_bounds__(SP_W * SP_J) k_spec_sum(const float *mu2, const float *w, long long sw, int n, int S,
+                                                          double *Sw, float *Swf, int nomega, float omegaStart,
+                                                          int omegaStep, float gamma, float avef) {
+    __shared__ float part[SP_J][SP_W + 1];
+    const int il = threadIdx.x, g = threadIdx.y, i = blockIdx.x * SP_W + il;
     const float wi = (float)(omegaStart + omegaStep * i);
-    float s = 0.f;
-    for (int j = 0; j < n; j++) {
-        const float dw = wi - (w[j] + avef);
-        s += mu2[j] * gamma / (dw * dw + gamma * gamma) / (float)CIR_PI;
+    double tot = 0.0;
+    for (int f = blockIdx.y * S; f < ((int)blockIdx.y + 1) * S; f++) {
+        const float *m = mu2 + (size_t)f * n, *l = w + (size_t)f * sw;
+        float s = 0.f;
+        for (int j = g; j < n; j += SP_J) {
+            const float dw = wi - (l[j] + avef);
+            s += m[j] * gamma / (dw * dw + gamma * gamma) / (float)CIR_PI;
+        }
+        part[g][il] = s;
+        __syncthreads();
+        if (g == 0)
+            for (int q = 0; q < SP_J; q++) tot += (double)part[q][il];
+        __syncthreads();
     }
-    Sw[i] += (double)s;
+    if (g || i >= nomega) return;
+    if (Swf) Swf[i] += (float)tot;
+    else Sw[(size_t)blockIdx.y * nomega + i] += tot;
 }
 
 }  // namespace
@@ -200,22 +211,27 @@ cudaError_t cir_launch_tcf(const TcfArgs &t, int batch, cudaStream_t s, int *lau
         return cudaGetLastError();
     }
     const size_t smem = sizeof(float) * 9 * (size_t)t.n;
-    cudaError_t e = cudaFuncSetAttribute(k_tcf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // four rows a warp at a time share the reads of m(0) where that leaves two blocks per SM,
+    // and a block takes up to 64 rows so that staging m(0) stays small beside them
+    const long long all = (long long)t.n * batch;
+    const int R = all >= 304LL * TCF_WARPS * 4 ? 4 : 1, rows = TCF_WARPS * (R == 4 && all >= 304LL * 64 ? 8 : R);
+    auto kern = R == 4 ? k_tcf<4> : k_tcf<1>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid((t.n + TCF_ROWS - 1) / TCF_ROWS, batch);
-    k_tcf<<<grid, TCF_WARPS * 32, smem, s>>>(t);
+    kern<<<dim3((t.n + rows - 1) / rows, batch), TCF_WARPS * 32, smem, s>>>(t, rows);
     if (launches) *launches += 1;
     return cudaGetLastError();
 }
 
-cudaError_t cir_launch_spectral(const float *V, int ld, const float *w, const float *dip, int ldv, int n,
-                                float *mu2, double *Sw, int nomega, float omegaStart, int omegaStep, float t1,
-                                float avef, cudaStream_t s, int *launches) {
-    k_spec_mu2<<<(n + 7) / 8, 256, 0, s>>>(V, ld, dip, ldv, n, mu2);
+cudaError_t cir_launch_spectral(const float *V, int ld, long long sV, const float *w, long long sw, const float *dip, int ldv,
+                                long long sdip, int n, int S, int sets, float *mu2, double *Sw, float *Swf, int nomega,
+                                float omegaStart, int omegaStep, float t1, float avef, cudaStream_t s, int *launches) {
+    k_spec_mu2<<<dim3((n + 7) / 8, S * sets), 256, 0, s>>>(V, ld, sV, dip, ldv, sdip, n, mu2);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const float gamma = (float)(CIR_HBAR / (t1 * 2.0));
-    k_spec_sum<<<(nomega + 127) / 128, 128, 0, s>>>(mu2, w, n, Sw, nomega, omegaStart, omegaStep, gamma, avef);
+    k_spec_sum<<<dim3((nomega + SP_W - 1) / SP_W, sets), dim3(SP_W, SP_J), 0, s>>>(mu2, w, sw, n, S, Sw, Swf, nomega,
+                                                                                 omegaStart, omegaStep, gamma, avef);
     if (launches) *launches += 2;
     return cudaGetLastError();
 }

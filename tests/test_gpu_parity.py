@@ -484,3 +484,21 @@ def test_build_forms(lib, nmol, nframes):
             one = eng.build_hamiltonian(xyz[f:f + 1], box)
             for b, o in zip(batch, one):
                 np.testing.assert_array_equal(b[f], o[0])
+
+
+@pytest.mark.parametrize("nmol,origins", [(27, 2), (33, 150), (41, 240)])
+def test_contraction_forms(lib, nmol, origins):
+    """The plain contraction with one row of F a warp and four (from 9728 rows), and blocks of 32
+    and 64 rows (from 19456), with a ragged last block; the spectral density of many origins."""
+    prm = {"natom_mol": 4, "nchrom_mol": 2, "nzeros": 64, "ntcfpoints": 3, "nsamples": origins, "sampleEvery": 0.01,
+           "dt": 0.01, "t1": 0.26, "avef": 3415.0, "omegaStart": 2000.0, "omegaStop": 5000.0, "omegaStep": 7,
+           "beginTime": 0.0, "map": 0, "imodel": 1, "ispecies": 0}
+    xyz, box = lib.synth_trajectory(nmol, origins + 2, seed=3)
+    fos = (np.arange(origins)[:, None] + np.arange(3)[None, :]).astype(np.int32).ravel()
+    p = lib.default_params(species="H2O", model="tip4p2005", nsamples=origins, ntcfpoints=3, nzeros=64, omegaStep=7,
+                           avef=3415.0, omegaStart=2000, omegaStop=5000, sampleEvery=0.01)
+    with lib.Engine(p, xyz.shape[1]) as eng:
+        out = eng.run(xyz, box, fos)
+    ref = O.run(prm, xyz, np.broadcast_to(box, (len(xyz), 3)), fos)
+    for k in ("tcf_ir", "tcf_vv", "tcf_vh", "ls_ir", "ls_vv", "ls_vh", "sw"):
+        assert O.rel_l2(out[k], ref[k]) < 1e-4, k      # the plain form's bound
