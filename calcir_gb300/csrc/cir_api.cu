@@ -74,8 +74,6 @@ struct GraphEntry {
     int launches = 0;
 };
 
-using GemmShape = std::tuple<int, int, int, int, bool, int>;   // M, N, K, batch, A column-major, epilogue
-
 struct cir_ctx {
     cir_params p;
     int natoms = 0, nmol = 0, n = 0, ld = 0;
@@ -89,7 +87,6 @@ struct cir_ctx {
     CirMaps maps;
     LsRows ls;                            // printed lineshape rows and their frequencies
     std::vector<float> ls_omega;
-    std::map<GemmShape, int> gemm_tile;   // autotuner: SIMT tile shape per product shape
     // autotuner, mixed forms: tile width of each split-BF16 product shape (M, N, K, batch,
     // epilogue, output form, fused contraction) and tridiagonalisation blocks per SM per order
     std::map<std::tuple<int, int, int, int, int, int, int>, int> split_tile;
@@ -282,15 +279,15 @@ extern "C" int cir_create(const cir_params *p, int natoms, cir_ctx **out) {
 }
 
 // The tensor-core kernels set the context's error flag when a bounded wait gives up.
+static int clear_kernel_flag(cir_ctx *c) {
+    cudaMemsetAsync(c->buf[B_ERR].p, 0, sizeof(int), c->stream);
+    return cir_fail(CIR_ERR_CUDA, "a tensor-core kernel timed out waiting on its pipeline");
+}
 static int check_kernel_flag(cir_ctx *c) {
     int flag = 0;
     CK(cudaMemcpyAsync(&flag, c->buf[B_ERR].p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (flag) {
-        cudaMemsetAsync(c->buf[B_ERR].p, 0, sizeof(int), c->stream);
-        return cir_fail(CIR_ERR_CUDA, "a tensor-core kernel timed out waiting on its pipeline");
-    }
-    return CIR_OK;
+    return flag ? clear_kernel_flag(c) : CIR_OK;
 }
 
 extern "C" int cir_destroy(cir_ctx *c) {
@@ -318,8 +315,7 @@ extern "C" int cir_set_stream(cir_ctx *c, void *s) {
 
 extern "C" int cir_synchronize(cir_ctx *c) {
     if (!c) return cir_fail(CIR_ERR_ARG, "cir_synchronize: null context");
-    CK(cudaStreamSynchronize(c->stream));
-    return CIR_OK;
+    return check_kernel_flag(c);   // of asynchronous calls as well
 }
 
 extern "C" int cir_get_stats(cir_ctx *c, cir_stats *s) {
@@ -457,11 +453,13 @@ extern "C" int cir_eigh(cir_ctx *c, int nmat, int n, float *A, float *w) {
     unsigned long long sweeps = 0;
     CK(cudaMemcpyAsync(st.data(), a.status, (size_t)nmat * 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemcpyAsync(&sweeps, a.sweeps, 8, cudaMemcpyDeviceToHost, c->stream));
+    int flag = 0;
+    CK(cudaMemcpyAsync(&flag, c->buf[B_ERR].p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->stats.eig_sweeps += (long long)sweeps;
     for (int i = 0; i < nmat; i++)
         if (st[i]) return cir_fail(CIR_ERR_NOCONVERGE, "eigensolver sweep cap reached on matrix %d", i);
-    if (a.precision != CIR_PREC_FP32 && (rc = check_kernel_flag(c))) return rc;
+    if (flag) return clear_kernel_flag(c);
     return CIR_OK;
 }
 
@@ -504,56 +502,6 @@ static int setup_refine(cir_ctx *c, EighArgs &e, int nmat) {
     e.RW = c->buf[B_RW].p;
     e.refine_iters = c->p.refine_eigen;
     e.refine_chunk = chunk;
-    return CIR_OK;
-}
-
-static GemmShape gemm_shape(const GemmArgs &g, int batch) {
-    return GemmShape(g.M, g.N, g.K, batch, g.a_colmajor, g.epilogue);
-}
-
-// The SIMT tile shape the autotuner chose for this product shape (128 x 128 if untuned).
-static int tuned_tile(cir_ctx *c, const GemmArgs &g, int batch) {
-    auto it = c->gemm_tile.find(gemm_shape(g, batch));
-    return it == c->gemm_tile.end() ? CIR_GEMM_TILE_128 : it->second;
-}
-
-// Autotuner: times both SIMT tile shapes of a product shape once per context (on scratch
-// operands of the same sizes, so the caller's data is untouched) and keeps the faster.
-// Must run outside stream capture.
-static int autotune_gemm(cir_ctx *c, const GemmArgs &g, int batch) {
-    if (!c->p.autotune || c->gemm_tile.count(gemm_shape(g, batch))) return CIR_OK;
-    const size_t a_el = (size_t)(g.a_colmajor ? g.K : g.M) * g.lda, b_el = (size_t)(g.b_kmajor ? g.N : g.K) * g.ldb,
-                 c_el = (size_t)g.M * g.ldc, w_el = g.epilogue == 1 ? (size_t)g.M : 0;
-    const size_t tot = (a_el + b_el + c_el + w_el + 16) * batch * sizeof(float);
-    CK(c->buf[B_TUNE].ensure(tot));
-    CK(cudaMemsetAsync(c->buf[B_TUNE].p, 0, tot, c->stream));
-    float *base = c->buf[B_TUNE].as<float>();
-    GemmArgs t = g;
-    t.A = base;
-    t.sA = (long long)a_el;
-    t.B = base + a_el * batch;
-    t.sB = (long long)b_el;
-    t.C = base + (a_el + b_el) * batch;
-    t.sC = (long long)c_el;
-    if (g.epilogue == 1) {
-        t.w = base + (a_el + b_el + c_el) * batch;
-        t.wstride = g.M;
-    }
-    float best = 1e30f;
-    int pick = CIR_GEMM_TILE_128;
-    for (int tile : {CIR_GEMM_TILE_128, CIR_GEMM_TILE_64}) {
-        CK(cir_launch_gemm(t, batch, c->stream, nullptr, tile));   // warm-up
-        CK(cudaEventRecord(c->ev[6], c->stream));
-        for (int r = 0; r < 3; r++) CK(cir_launch_gemm(t, batch, c->stream, nullptr, tile));
-        CK(cudaEventRecord(c->ev[7], c->stream));
-        CK(cudaEventSynchronize(c->ev[7]));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, c->ev[6], c->ev[7]));
-        if (ms < best) { best = ms; pick = tile; }
-    }
-    c->gemm_tile[gemm_shape(g, batch)] = pick;
-    if (c->p.verbose) printf("autotune: GEMM %d x %d x %d (batch %d): %s tiles\n", g.M, g.N, g.K, batch,
-                             pick == CIR_GEMM_TILE_64 ? "64 x 64" : "128 x 128");
     return CIR_OK;
 }
 
@@ -684,17 +632,16 @@ static int propagate_dev(cir_ctx *c, int nprop, int n, const float *V, int ldv, 
     g1.B = F; g1.ldb = ldf; g1.sB = sF;
     g1.C = G; g1.ldc = ldf; g1.sC = sF;
     g1.M = n; g1.N = 2 * n; g1.K = n;
+    g1.err = c->buf[B_ERR].as<int>();
     g1.epilogue = 1; g1.w = w; g1.wstride = wstride;
     g1.dt_over_hbar = (float)(dt / CIR_HBAR);
     GemmArgs g2 = g1;
     g2.A = V; g2.a_colmajor = true;                                   // V itself
     g2.B = G; g2.C = F; g2.epilogue = 0;
     if (c->p.precision == CIR_PREC_FP32) {
-        CK(cir_launch_gemm(g1, nprop, c->stream, &launches, tuned_tile(c, g1, nprop)));
-        CK(cir_launch_gemm(g2, nprop, c->stream, &launches, tuned_tile(c, g2, nprop)));
+        CK(cir_launch_gemm(g1, nprop, c->stream, &launches));
+        CK(cir_launch_gemm(g2, nprop, c->stream, &launches));
     } else {
-        CK(c->buf[B_ERR].ensure(sizeof(int)));
-        g1.err = g2.err = c->buf[B_ERR].as<int>();
         CK(cir_launch_tc_gemm(g1, nprop, c->p.precision, c->stream, &launches));
         CK(cir_launch_tc_gemm(g2, nprop, c->p.precision, c->stream, &launches));
     }
@@ -716,8 +663,8 @@ extern "C" int cir_propagate(cir_ctx *c, int nprop, int n, const float *V, const
     count_launch(c, launches);
     if (rc) return rc;
     if ((rc = stage_out(c, F, dF, nprop * mb * 2))) return rc;
-    if (!is_device_ptr(F)) CK(cudaStreamSynchronize(c->stream));
-    if (c->p.precision != CIR_PREC_FP32 && (rc = check_kernel_flag(c))) return rc;
+    // (plain form on device buffers: asynchronous, cir_synchronize reports)
+    if ((!is_device_ptr(F) || c->p.precision != CIR_PREC_FP32) && (rc = check_kernel_flag(c))) return rc;
     return CIR_OK;
 }
 
@@ -831,10 +778,10 @@ __global__ void k_copy_m0(const float *m, long long sm_origin, int rows_ld, floa
 // Launch key of a captured step loop: every shape and pointer its launches depend on.
 static std::vector<long long> step_key(const Group &g, int St, int K, int k0, int kc, int precision, const void *A,
                                        const void *W, const void *M, const void *F, const void *G, const void *M0,
-                                       const void *tcf, int tile1, int tile2, const void *VS, const void *FS) {
+                                       const void *tcf, const void *VS, const void *FS) {
     return {g.n, g.ld, St, K, k0, kc, precision, (long long)(uintptr_t)A, (long long)(uintptr_t)W,
             (long long)(uintptr_t)M, (long long)(uintptr_t)F, (long long)(uintptr_t)G, (long long)(uintptr_t)M0,
-            (long long)(uintptr_t)tcf, tile1, tile2, (long long)(uintptr_t)VS, (long long)(uintptr_t)FS};
+            (long long)(uintptr_t)tcf, (long long)(uintptr_t)VS, (long long)(uintptr_t)FS};
 }
 
 static int psi_propagate(cir_ctx *c, int S, int n, int ld, const float *V, long long sV, const float *w, long long sw,
@@ -887,7 +834,7 @@ struct GroupJob {
     __nv_bfloat16 *vs = nullptr, *fs = nullptr;
     SplitMat Vc{}, Vr{}, Ft{}, Gt{};
     double *tcf = nullptr;
-    int tile1 = 0, tile2 = 0, stile1 = 0, stile2 = 0;
+    int stile1 = 0, stile2 = 0;
     int launches = 0;
     int k0 = 0, kc = 0, nmat = 0, base0 = 0, dlt = 0;   // the chunk being run
 
@@ -997,16 +944,6 @@ struct GroupJob {
         launches = 0;
         int rc;
 
-        // the propagation products of this group, tuned before anything is timed or captured
-        GemmArgs g1{}, g2{};
-        g1.M = n; g1.N = 2 * n; g1.K = n; g1.lda = ld; g1.ldb = g1.ldc = 2 * ld; g1.a_colmajor = false; g1.epilogue = 1;
-        g2 = g1; g2.a_colmajor = true; g2.epilogue = 0;
-        if (p.precision == CIR_PREC_FP32) {
-            if ((rc = autotune_gemm(c, g1, St))) return rc;
-            if ((rc = autotune_gemm(c, g2, St))) return rc;
-        }
-        tile1 = tuned_tile(c, g1, St);
-        tile2 = tuned_tile(c, g2, St);
         // the split-BF16 products' tile widths (the shapes and strides of the step loop's two
         // products; the autotuner runs them on scratch operands)
         stile1 = stile2 = 0;
@@ -1343,7 +1280,7 @@ struct GroupJob {
 
     // the key of the chunk's captured step loop
     std::vector<long long> graph_key() const {
-        std::vector<long long> key = step_key(g, St, K, k0, kc, p.precision, A, W, M, F, G, M0, tcf, tile1, tile2, vs, fs);
+        std::vector<long long> key = step_key(g, St, K, k0, kc, p.precision, A, W, M, F, G, M0, tcf, vs, fs);
         key.insert(key.end(), {(long long)vectors, (long long)base0, (long long)dlt, (long long)stile1, (long long)stile2,
                                (long long)(uintptr_t)buf[B_PSI].p, (long long)(uintptr_t)buf[B_LAM].p});
         return key;
@@ -1368,11 +1305,13 @@ struct GroupJob {
         CK(cudaMemcpyAsync(hst.data(), buf[B_STATUS].p, (size_t)nb * 4, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaMemcpyAsync(oor.data(), buf[B_OOR].p, (size_t)T * 8, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaMemcpyAsync(&sweeps, buf[B_SWEEPS].p, 8, cudaMemcpyDeviceToHost, c->stream));
+        int flag = 0;
+        CK(cudaMemcpyAsync(&flag, c->buf[B_ERR].p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         c->stats.eig_sweeps += (long long)sweeps;
         for (int i = 0; i < nb; i++)
             if (hst[i]) return cir_fail(CIR_ERR_NOCONVERGE, "eigensolver sweep cap reached");
-        if (p.precision != CIR_PREC_FP32 && (rc = check_kernel_flag(c))) return rc;
+        if (flag) return clear_kernel_flag(c);
 
         // damped correlation sums of every trajectory, their lineshapes in one launch
         // (calcIR.cu:786-827, 890-919); the host fills the other outputs meanwhile
@@ -1872,7 +1811,7 @@ extern "C" int cir_set_coeffs(cir_ctx *c, const float *t) {
 }
 
 // x <- V_k exp(i L_k dt/hbar) V_k^T x for S origins, x n x 9 complex (row-major, 18 floats per
-// row); FP32 SIMT GEMMs.  V: origin s at V + s*sV, w likewise; tmp: S x n x 18.
+// row); FP32 GEMMs.  V: origin s at V + s*sV, w likewise; tmp: S x n x 18.
 static int psi_propagate(cir_ctx *c, int S, int n, int ld, const float *V, long long sV, const float *w, long long sw,
                          float dt, float *x, float *tmp, int &launches) {
     // X = e^{i L dt/hbar} V^T psi, then psi = V X: two streaming passes over V (k_adjoint.cu)
@@ -2077,6 +2016,7 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
             if (k >= 1) {
                 // a = V^T lambda(k), b = V^T psi(k-1); R; G = V R V^T (into R)
                 GemmArgs ga{};
+                ga.err = c->buf[B_ERR].as<int>();
                 ga.A = Vk; ga.lda = ld; ga.sA = sV; ga.a_colmajor = false;
                 ga.B = lam; ga.ldb = CIR_PSI_LD; ga.sB = (long long)n * CIR_PSI_LD;
                 ga.C = PA; ga.ldc = CIR_PSI_LD; ga.sC = (long long)n * CIR_PSI_LD;
@@ -2089,6 +2029,7 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
                 CK(cir_adj_build_R(PA, PB, W + (size_t)k * ld, sWk, n, S, tau, R, ld, mstride, c->stream));
                 launches++;
                 GemmArgs gt{};
+                gt.err = c->buf[B_ERR].as<int>();
                 gt.A = Vk; gt.lda = ld; gt.sA = sV; gt.a_colmajor = true;     // V
                 gt.B = R; gt.ldb = ld; gt.sB = mstride;                        // R row-major
                 gt.C = T; gt.ldc = ld; gt.sC = mstride;
@@ -2114,7 +2055,7 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
         }
     }
     CK(cudaMemcpyAsync(grad, dgrad, CIR_NTHETA * 8, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if ((rc = check_kernel_flag(c))) return rc;
     count_launch(c, launches);
     *loss = L;
     return CIR_OK;

@@ -160,7 +160,7 @@ cudaError_t cir_launch_refine(const float *H, float *Z, long long mstride, int l
                               int nmat, int iters, void *ws, int chunk, cudaStream_t s, int *launches);
 int cir_eigh_max_n();
 
-// batched SIMT FP32 GEMM, C = A * B (row-major B, C); A row- or column-major.
+// batched FP32 GEMM (k_gemm.cu), C = A * B (row-major B, C); A row- or column-major.
 // epilogue 1: rotate column pairs (2q, 2q+1) of row i by exp(+i w[i] dt/hbar).
 struct GemmArgs {
     const float *A, *B;
@@ -182,10 +182,8 @@ struct GemmArgs {
     // element offsets instead (batch stride 2 sC elements)
     __nv_bfloat16 *Chi, *Clo;
 };
-// SIMT tile shapes: 128 x 128 x 8, or 64 x 64 x 16 (more blocks for small products)
-constexpr int CIR_GEMM_TILE_128 = 0, CIR_GEMM_TILE_64 = 1;
-cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *launches, int tile = CIR_GEMM_TILE_128);
-// the same product on the tensor cores (tcgen05), precision CIR_PREC_TF32
+cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *launches);
+// the same product in TF32 or two-term split BF16 (k_tc_gemm.cu)
 cudaError_t cir_launch_tc_gemm(const GemmArgs &g, int batch, int precision, cudaStream_t s, int *launches);
 size_t cir_tc_gemm_smem_bytes();
 

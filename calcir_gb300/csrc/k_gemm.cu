@@ -1,202 +1,496 @@
-// Batched FP32 SIMT GEMM for the propagation step of the plain form.
-// The reference builds a dense diagonal propagator and multiplies three complex
-// matrices per frame (Pinit + 3 x magma_cgemm, calcIR.cu:596-613, 24 N^3 real flops).
-// Here the complex F is a real N x 2N matrix of interleaved (re, im) columns and one step
-// is two real GEMMs, 8 N^3 flops:
+// Batched FP32 GEMM on the tensor cores: C[b] = A[b] B[b], FP32 in and out and FP32 accuracy,
+// for the plain form: the propagation step, the eigensolver's back-transform and upper merges,
+// and the gradient.  The reference builds a dense diagonal propagator and multiplies three
+// complex matrices per frame (Pinit + 3 x magma_cgemm, calcIR.cu:596-613, 24 N^3 real flops).
+// Here the complex F is a real N x 2N matrix of interleaved (re, im) columns and one step is two
+// real GEMMs, 8 N^3 flops:
 //     G  = V^T F                  (epilogue: row j of G times exp(+i w_j dt/hbar))
 //     F' = V G
-// 128x128x8 or 64x64x16 block tiles, 256 threads, 8x8 or 4x4 outputs per thread,
-// double-buffered shared memory; edges are predicated so any N works.
+//
+// Each operand value is split into three BF16 terms, x = h + m + l (8 + 8 + 8 mantissa bits: the
+// whole of an FP32 value), and the product is six tcgen05.mma kind::f16 per 16 of K: h h into the
+// accumulator H, and h m, m h, m m, h l, l h into a second accumulator L (what is left out is
+// below 2^-24 of a product).  The tensor core drops the bits that fall below the accumulator's
+// last on every instruction, so a long sum in one accumulator drifts toward zero by half an ulp an
+// instruction; H is therefore read out every F_CHUNK slices and summed in FP32 registers with
+// rounding to nearest, and L, 2^-8 of the sum, once a tile.
+//
+// One CTA per SM walks 128 x 128 tiles (column tile fastest, then row tile, then matrix):
+//   warps 0-7   load FP32 slices 32 deep (0-3 A, 4-7 B), split them and store the three terms
+//               K-major (core matrices of 8 rows x 16 bytes, (r/8, k/8) at (r/8)*SBO + (k/8)*LBO;
+//               SBO padded so that either orientation stores without bank conflicts) into a ring;
+//               the next slice's loads are in flight while one is split;
+//   warps 8-15  sum the chunks (a thread a row and half of the columns), then the epilogue, while
+//               the next tile is loaded and multiplied (two H and two L accumulators, all 512
+//               columns of tensor memory);
+//   warp 16     issues the MMAs.
+// The loads' issue and the splitting bound it (six MMAs of 16 K take 40% of a slice's time).
+// 1024 x 2048 x 1024 in ten matrices: 859-1044 us as SIMT FFMAs (50-41 TFLOP/s), 304-378 so
+// (141-114), relative error against 64 bits 5.5e-7 before, 1.2e-7 so.  Products with too few
+// tiles for the SMs run on the SIMT kernel further down (gemm_small_wins).
+// Every wait is bounded: a timeout raises the CTA's abort flag and the error flag, every role
+// leaves its loop, and the MMAs issued are waited for before the tensor memory is freed.
 #include "cir_device.cuh"
+#include "cir_tcgen05.cuh"
+
+#include <cuda_bf16.h>
+#include <algorithm>
+#include <climits>
 
 namespace {
 
-// Tile shapes (256 threads, a 16 x 16 thread grid, TM x TN outputs per thread in 4 x 4 groups
-// 64 rows / columns apart): 128 x 128 x 8 for large products, 64 x 64 x 16 for products
-// whose 128 x 128 grid would not fill the SMs.  The autotuner of the library picks one.
-template <int BM_, int BN_, int BK_>
-struct Tile {
-    static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = BM_ / 16, TN = BN_ / 16;
-};
-using TileL = Tile<128, 128, 8>;
-using TileS = Tile<64, 64, 16>;
-constexpr int GT = 256;
+constexpr int FM = 128, FN = 128, FK = 32;     // tile, K of a slice
+constexpr int F_LBO = 128, F_SBO = 528;
+constexpr int F_PART = (FM / 8) * F_SBO;       // bytes of one term of one operand's slice
+constexpr int F_STAGE = 6 * F_PART, F_NS = 4;
+constexpr int F_CHUNK = 1;                     // slices between read-outs of H
+constexpr int F_LOAD = 8, F_ACC = 8;           // warps
+constexpr int F_NT = 32 * (F_LOAD + F_ACC + 4);   // whole warpgroups: the register split is per group
+constexpr size_t F_SMEM = (size_t)F_NS * F_STAGE + 256;
 
-template <class T, bool ACOL>
-__device__ __forceinline__ void load_a(const GemmArgs &g, const float *A, int m0, int k0, float (&ra)[4]) {
-    const int t = threadIdx.x;
-    if (ACOL) {   // element (i, k) at A[k*lda + i]; thread loads 4 consecutive i of one k
-        const int kk = t / (T::BM / 4), i = (t % (T::BM / 4)) * 4;
-        const int gk = k0 + kk, gi = m0 + i;
-        const float *p = A + (size_t)gk * g.lda + gi;
-        if (gk < g.K && gi + 3 < g.M && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-            const float4 v = *reinterpret_cast<const float4 *>(p);
-            ra[0] = v.x; ra[1] = v.y; ra[2] = v.z; ra[3] = v.w;
-        } else {
-            #pragma unroll
-            for (int q = 0; q < 4; q++) ra[q] = (gk < g.K && gi + q < g.M) ? p[q] : 0.f;
-        }
-    } else {      // element (i, k) at A[i*lda + k]; thread loads 4 consecutive k of one i
-        const int i = t / (T::BK / 4), kk = (t % (T::BK / 4)) * 4;
-        const int gi = m0 + i, gk = k0 + kk;
-        const float *p = A + (size_t)gi * g.lda + gk;
-        if (gi < g.M && gk + 3 < g.K && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-            const float4 v = *reinterpret_cast<const float4 *>(p);
-            ra[0] = v.x; ra[1] = v.y; ra[2] = v.z; ra[3] = v.w;
-        } else {
-            #pragma unroll
-            for (int q = 0; q < 4; q++) ra[q] = (gi < g.M && gk + q < g.K) ? p[q] : 0.f;
-        }
-    }
+// The warpgroups' registers: 640 threads launch with 96 each (61440); the idle three warps of
+// the MMA group give theirs to the loads in flight and the sums: 2 * 128 * 120 + 2 * 128 * 104 +
+// 128 * 24 = 60416
+template <int R>
+__device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R>
+__device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+
+__device__ __forceinline__ void mbar_arrive1(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-template <class T, bool ACOL>
-__device__ __forceinline__ void store_a(float (*As)[T::BM], const float (&ra)[4]) {
-    const int t = threadIdx.x;
-    if (ACOL) {
-        const int kk = t / (T::BM / 4), i = (t % (T::BM / 4)) * 4;
-        *reinterpret_cast<float4 *>(&As[kk][i]) = make_float4(ra[0], ra[1], ra[2], ra[3]);
-    } else {
-        const int i = t / (T::BK / 4), kk = (t % (T::BK / 4)) * 4;
-        #pragma unroll
-        for (int q = 0; q < 4; q++) As[kk + q][i] = ra[q];
-    }
-}
-
-template <class T, bool BKC>
-__device__ __forceinline__ void load_b(const GemmArgs &g, const float *B, int k0, int n0, float (&rb)[4]) {
-    const int t = threadIdx.x;
-    if (BKC) {    // element (k, j) at B[j*ldb + k]; thread loads 4 consecutive k of one j
-        const int j = t / (T::BK / 4), kk = (t % (T::BK / 4)) * 4;
-        const int gj = n0 + j, gk = k0 + kk;
-        const float *p = B + (size_t)gj * g.ldb + gk;
-        if (gj < g.N && gk + 3 < g.K && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-            const float4 v = *reinterpret_cast<const float4 *>(p);
-            rb[0] = v.x; rb[1] = v.y; rb[2] = v.z; rb[3] = v.w;
-        } else {
-            #pragma unroll
-            for (int q = 0; q < 4; q++) rb[q] = (gj < g.N && gk + q < g.K) ? p[q] : 0.f;
-        }
-        return;
-    }
-    const int kk = t / (T::BN / 4), j = (t % (T::BN / 4)) * 4;
-    const int gk = k0 + kk, gj = n0 + j;
-    const float *p = B + (size_t)gk * g.ldb + gj;
-    if (gk < g.K && gj + 3 < g.N && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-        const float4 v = *reinterpret_cast<const float4 *>(p);
-        rb[0] = v.x; rb[1] = v.y; rb[2] = v.z; rb[3] = v.w;
-    } else {
-        #pragma unroll
-        for (int q = 0; q < 4; q++) rb[q] = (gk < g.K && gj + q < g.N) ? p[q] : 0.f;
-    }
-}
-
-template <class T, bool BKC>
-__device__ __forceinline__ void store_b(float (*Bs)[T::BN], const float (&rb)[4]) {
-    const int t = threadIdx.x;
-    if (BKC) {
-        const int j = t / (T::BK / 4), kk = (t % (T::BK / 4)) * 4;
-        #pragma unroll
-        for (int q = 0; q < 4; q++) Bs[kk + q][j] = rb[q];
-    } else {
-        const int kk = t / (T::BN / 4), j = (t % (T::BN / 4)) * 4;
-        *reinterpret_cast<float4 *>(&Bs[kk][j]) = make_float4(rb[0], rb[1], rb[2], rb[3]);
-    }
-}
-
-template <class T, bool ACOL, bool BKC>
-__global__ void __launch_bounds__(GT) k_sgemm(GemmArgs g) {
-    constexpr int BM = T::BM, BN = T::BN, BK = T::BK, TM = T::TM, TN = T::TN;
-    __shared__ __align__(16) float As[2][BK][BM];
-    __shared__ __align__(16) float Bs[2][BK][BN];
-    const int bz = blockIdx.z;
-    const float *A = g.A + (size_t)bz * g.sA;
-    const float *B = g.B + (size_t)bz * g.sB;
-    float *C = g.C + (size_t)bz * g.sC;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-
-    float acc[TM][TN];
+// the three BF16 terms of eight values, as 16-byte words
+__device__ __forceinline__ void split3(const float (&x)[8], uint4 &h, uint4 &m, uint4 &l) {
+    uint32_t wh[4], wm[4], wl[4];
     #pragma unroll
-    for (int i = 0; i < TM; i++)
-        #pragma unroll
-        for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
-
-    float ra[4], rb[4];
-    load_a<T, ACOL>(g, A, m0, 0, ra);
-    load_b<T, BKC>(g, B, 0, n0, rb);
-    store_a<T, ACOL>(As[0], ra);
-    store_b<T, BKC>(Bs[0], rb);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < g.K; k0 += BK) {
-        const bool more = k0 + BK < g.K;
-        if (more) {
-            load_a<T, ACOL>(g, A, m0, k0 + BK, ra);
-            load_b<T, BKC>(g, B, k0 + BK, n0, rb);
-        }
-        #pragma unroll
-        for (int kk = 0; kk < BK; kk++) {
-            float af[TM], bf[TN];
-            #pragma unroll
-            for (int q = 0; q < TM / 4; q++) {
-                const float4 a4 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4 + 64 * q]);
-                af[4 * q] = a4.x; af[4 * q + 1] = a4.y; af[4 * q + 2] = a4.z; af[4 * q + 3] = a4.w;
-            }
-            #pragma unroll
-            for (int q = 0; q < TN / 4; q++) {
-                const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4 + 64 * q]);
-                bf[4 * q] = b4.x; bf[4 * q + 1] = b4.y; bf[4 * q + 2] = b4.z; bf[4 * q + 3] = b4.w;
-            }
-            #pragma unroll
-            for (int i = 0; i < TM; i++)
-                #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(af[i], bf[j], acc[i][j]);
-        }
-        if (more) {
-            store_a<T, ACOL>(As[buf ^ 1], ra);
-            store_b<T, BKC>(Bs[buf ^ 1], rb);
-        }
-        __syncthreads();
-        buf ^= 1;
+    for (int q = 0; q < 4; q++) {
+        const float a = x[2 * q], b = x[2 * q + 1];
+        const __nv_bfloat162 ph = __floats2bfloat162_rn(a, b);
+        wh[q] = *reinterpret_cast<const uint32_t *>(&ph);
+        const float ra = a - __uint_as_float(wh[q] << 16), rb = b - __uint_as_float(wh[q] & 0xffff0000u);
+        const __nv_bfloat162 pm = __floats2bfloat162_rn(ra, rb);
+        wm[q] = *reinterpret_cast<const uint32_t *>(&pm);
+        const __nv_bfloat162 pl = __floats2bfloat162_rn(ra - __uint_as_float(wm[q] << 16),
+                                                        rb - __uint_as_float(wm[q] & 0xffff0000u));
+        wl[q] = *reinterpret_cast<const uint32_t *>(&pl);
     }
-    // rows ty*4 + {0..3} (+ 64); columns tx*4 + {0..3} (+ 64)
-    #pragma unroll
-    for (int i = 0; i < TM; i++) {
-        const int r = m0 + 64 * (i / 4) + ty * 4 + (i % 4);
-        if (r >= g.M) continue;
-        float cph = 1.f, sph = 0.f;
-        if (g.epilogue == 1) {
-            const float ph = g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar;
-            sincosf(ph, &sph, &cph);
+    h = make_uint4(wh[0], wh[1], wh[2], wh[3]);
+    m = make_uint4(wm[0], wm[1], wm[2], wm[3]);
+    l = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+}
+
+// One thread's part of an operand slice (128 rows of the M or N dimension, 32 of K): four groups
+// of eight consecutive K of one row.  KC: K contiguous in memory (element (r, k) at p[r*ld + k]),
+// group i is row 32 i + 8 (warp & 3) + (lane & 7), K 8 (lane >> 3) ..; else rows contiguous
+// (element (r, k) at p[k*ld + r]), the groups are rows 4 lane .. + 3, K 8 (warp & 3) ...
+template <bool KC>
+struct Part {
+    float4 v[8];
+    __device__ __forceinline__ static float4 load4(const float *q, int have) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (have > 0) x.x = __ldg(q);
+        if (have > 1) x.y = __ldg(q + 1);
+        if (have > 2) x.z = __ldg(q + 2);
+        if (have > 3) x.w = __ldg(q + 3);
+        return x;
+    }
+    __device__ __forceinline__ void load(const float *p, int ld, int rdim, int kdim, int r0, int k0, int w4, int lane, bool vec) {
+        if (vec && r0 + 128 <= rdim && k0 + 32 <= kdim) {   // the whole slice inside
+            const float *q = KC ? p + (size_t)(r0 + 8 * w4 + (lane & 7)) * ld + k0 + 8 * (lane >> 3)
+                                : p + (size_t)(k0 + 8 * w4) * ld + r0 + 4 * lane;
+            const size_t st = KC ? (size_t)32 * ld : (size_t)ld;
+            #pragma unroll
+            for (int i = 0; i < 8; i++)
+                v[i] = __ldg(reinterpret_cast<const float4 *>(KC ? q + (i >> 1) * st + 4 * (i & 1) : q + i * st));
+        } else if (KC) {
+            #pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int r = r0 + 32 * i + 8 * w4 + (lane & 7), k = k0 + 8 * (lane >> 3);
+                const float *q = p + (size_t)r * ld + k;
+                const int have = r < rdim ? kdim - k : 0;
+                v[2 * i] = load4(q, have);
+                v[2 * i + 1] = load4(q + 4, have - 4);
+            }
+        } else {
+            const int r = r0 + 4 * lane;
+            #pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int k = k0 + 8 * w4 + i;
+                v[i] = load4(p + (size_t)k * ld + r, k < kdim ? rdim - r : 0);
+            }
         }
+    }
+    __device__ __forceinline__ void store(unsigned char *base, int w4, int lane) const {
         #pragma unroll
-        for (int h = 0; h < TN / 4; h++) {
-            const int c = n0 + h * 64 + tx * 4;
-            float v[4] = {acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]};
-            if (g.epilogue == 1) {   // (re, im) pairs times exp(+i ph)
-                #pragma unroll
-                for (int q = 0; q < 4; q += 2) {
-                    const float re = v[q], im = v[q + 1];
-                    v[q] = cph * re - sph * im;
-                    v[q + 1] = sph * re + cph * im;
-                }
-            }
-            if (g.epilogue == 2) {   // C = D - A B
-                const float *d = g.D + (size_t)bz * g.sD + (size_t)r * g.ldd + c;
-                #pragma unroll
-                for (int q = 0; q < 4; q++) v[q] = (c + q < g.N ? d[q] : 0.f) - v[q];
-            }
-            float *p = C + (size_t)r * g.ldc + c;
-            if (c + 3 < g.N && ((reinterpret_cast<uintptr_t>(p) & 15) == 0)) {
-                *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        for (int i = 0; i < 4; i++) {
+            float x[8];
+            uint32_t o;
+            if (KC) {
+                x[0] = v[2 * i].x; x[1] = v[2 * i].y; x[2] = v[2 * i].z; x[3] = v[2 * i].w;
+                x[4] = v[2 * i + 1].x; x[5] = v[2 * i + 1].y; x[6] = v[2 * i + 1].z; x[7] = v[2 * i + 1].w;
+                o = (4 * i + w4) * F_SBO + (lane >> 3) * F_LBO + (lane & 7) * 16;
             } else {
                 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (c + q < g.N) p[q] = v[q];
+                for (int q = 0; q < 8; q++) x[q] = i == 0 ? v[q].x : i == 1 ? v[q].y : i == 2 ? v[q].z : v[q].w;
+                const int r = 4 * lane + i;
+                o = (r >> 3) * F_SBO + w4 * F_LBO + (r & 7) * 16;
+            }
+            uint4 h, m, l;
+            split3(x, h, m, l);
+            *reinterpret_cast<uint4 *>(base + o) = h;
+            *reinterpret_cast<uint4 *>(base + F_PART + o) = m;
+            *reinterpret_cast<uint4 *>(base + 2 * F_PART + o) = l;
+        }
+    }
+};
+
+__device__ __forceinline__ uint64_t f_desc(uint32_t addr) { return smem_desc_kmajor(addr, F_LBO, F_SBO); }
+
+// vecA, vecB, vecC: every 16-byte access of the operand (C and D: both) is aligned (pointer,
+// leading dimension, stride)
+template <bool ACOL, bool BKC>
+__global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int tiles_mn, int ntiles, bool vecA, bool vecB,
+                                                   bool vecC, int *err) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)F_NS * F_STAGE);   // [F_NS]
+    uint64_t *empty = full + F_NS;                                                 // [F_NS]
+    uint64_t *hfull = empty + F_NS;                                                // [2] chunk in H
+    uint64_t *hempty = hfull + 2;                                                  // [2]
+    uint64_t *lempty = hempty + 2;                                                 // [2] L read out
+    uint64_t *drain = lempty + 2;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + 1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tslot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == F_LOAD + F_ACC) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < F_NS; s++) {
+            mbar_init(&full[s], F_LOAD);
+            mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; a++) {
+            mbar_init(&hfull[a], 1);
+            mbar_init(&hempty[a], F_ACC);
+            mbar_init(&lempty[a], F_ACC);
+        }
+        mbar_init(drain, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tslot;
+    const int KT = (g.K + FK - 1) / FK, NC = (KT + F_CHUNK - 1) / F_CHUNK;   // slices, chunks of a tile
+    auto fail = [&]() {
+        *abort_flag = 1;
+        if (err) atomicExch(err, 1);
+    };
+    auto tile = [&](int t, int &bz, int &m0, int &n0) {
+        bz = t / tiles_mn;
+        const int rem = t % tiles_mn;
+        m0 = (rem / tiles_n) * FM;
+        n0 = (rem % tiles_n) * FN;
+    };
+
+    if (warp < F_LOAD) {
+        regs_up<120>();
+        const bool isA = warp < 4;
+        const int w4 = warp & 3;
+        // (the operand's side: pointer, strides, extents)
+        auto produce = [&](auto &part, const float *base, long long sb, int ld, int rdim, bool vec) {
+            // the load side runs a slice ahead of the store side
+            int lt = blockIdx.x, lkt = 0, r0 = 0;
+            const float *src = base;
+            auto seek = [&] {
+                if (lt >= ntiles) return;
+                int bz, m0, n0;
+                tile(lt, bz, m0, n0);
+                src = base + (size_t)bz * sb;
+                r0 = isA ? m0 : n0;
+            };
+            auto load = [&](auto &p) {
+                if (lt >= ntiles) return;
+                p.load(src, ld, rdim, g.K, r0, lkt * FK, w4, lane, vec);
+                if (++lkt == KT) { lkt = 0; lt += gridDim.x; seek(); }
+            };
+            seek();
+            load(part);
+            uint32_t it = 0;
+            const uint32_t total = (uint32_t)((ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * KT;
+            bool ok = true;
+            auto step = [&] {
+                const int s = it % F_NS;
+                if (it >= F_NS && !(ok = mbar_wait(&empty[s], ((it / F_NS) & 1) ^ 1))) return;
+                if (*abort_flag) { ok = false; return; }
+                part.store(smem + (size_t)s * F_STAGE + (isA ? 0 : 3 * F_PART), w4, lane);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive1(&full[s]);
+                it++;
+                load(part);
+            };
+            while (it < total && ok) step();
+            if (!ok) fail();
+        };
+        if (isA) {
+            Part<!ACOL> part;
+            produce(part, g.A, g.sA, g.lda, g.M, vecA);
+        } else {
+            Part<BKC> part;
+            produce(part, g.B, g.sB, g.ldb, g.N, vecB);
+        }
+    } else if (warp >= F_LOAD + F_ACC) {
+        regs_down<24>();
+        if (warp == F_LOAD + F_ACC && lane == 0) {
+            constexpr uint32_t IDESC = make_idesc_mn(1u, FM, FN);
+            uint32_t it = 0, ch = 0;      // slices and chunks issued
+            bool ok = true, issued = false;
+            int li = 0;
+            for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, li++) {
+                const int a = li & 1;
+                if (li >= 2 && !(ok = mbar_wait(&lempty[a], ((li >> 1) & 1) ^ 1))) break;
+                const uint32_t dl = tmem + 256 + 128 * a;
+                for (int kt = 0; kt < KT && ok; kt++, it++) {
+                    const int s = it % F_NS, hb = ch & 1;
+                    const uint32_t dh = tmem + 128 * hb;
+                    if (kt % F_CHUNK == 0 && ch >= 2 && !(ok = mbar_wait(&hempty[hb], ((ch >> 1) & 1) ^ 1))) break;
+                    if (!(ok = mbar_wait(&full[s], (it / F_NS) & 1))) break;
+                    if (*abort_flag) { ok = false; break; }
+                    fence_after();
+                    const uint32_t st = smem_addr(smem) + s * F_STAGE;
+                    #pragma unroll
+                    for (int ks = 0; ks < FK / 16; ks++) {
+                        const uint32_t o = st + 2 * ks * F_LBO;
+                        const uint64_t ah = f_desc(o), am = f_desc(o + F_PART), al = f_desc(o + 2 * F_PART);
+                        const uint64_t bh = f_desc(o + 3 * F_PART), bm = f_desc(o + 4 * F_PART), bl = f_desc(o + 5 * F_PART);
+                        mma_f16(dh, ah, bh, IDESC, (kt % F_CHUNK | ks) != 0);
+                        mma_f16(dl, ah, bl, IDESC, (kt | ks) != 0);
+                        mma_f16(dl, al, bh, IDESC, 1u);
+                        mma_f16(dl, am, bm, IDESC, 1u);
+                        mma_f16(dl, ah, bm, IDESC, 1u);
+                        mma_f16(dl, am, bh, IDESC, 1u);
+                    }
+                    issued = true;
+                    mma_commit(&empty[s]);
+                    if (kt % F_CHUNK == F_CHUNK - 1 || kt == KT - 1) {
+                        mma_commit(&hfull[hb]);
+                        ch++;
+                    }
+                }
+            }
+            if (!ok) fail();
+            if (issued) {   // every MMA issued has completed before the accumulators are freed
+                mma_commit(drain);
+                mbar_wait(drain, 0);
+            }
+        }
+    } else {
+        regs_up<104>();
+        const int quarter = warp & 3, half = (warp - F_LOAD) >> 2, row = quarter * 32 + lane;
+        const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + 64 * half;
+        uint32_t ch = 0;
+        int li = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, li++) {
+            float acc[4][16];
+            #pragma unroll
+            for (int h = 0; h < 4; h++)
+                #pragma unroll
+                for (int q = 0; q < 16; q++) acc[h][q] = 0.f;
+            int bz, m0, n0;
+            tile(t, bz, m0, n0);
+            const int r = m0 + row;
+            const float *D = g.epilogue == 2 && r < g.M ? g.D + (size_t)bz * g.sD + (size_t)r * g.ldd : nullptr;
+            if (D) {   // the row's 256 bytes of D into L2 while the tile is multiplied
+                const int c = n0 + 64 * half;
+                if (c < g.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(D + c));
+                if (c + 32 < g.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(D + c + 32));
+            }
+            for (int c = 0; c < NC; c++, ch++) {
+                const int hb = ch & 1;
+                if (!(ok = mbar_wait(&hfull[hb], (ch >> 1) & 1)) || *abort_flag) { ok = false; break; }
+                fence_after();
+                #pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    float v[16];
+                    tmem_ld16(tl + 128 * hb + 16 * h, v);
+                    #pragma unroll
+                    for (int q = 0; q < 16; q++) acc[h][q] += v[q];
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive1(&hempty[hb]);
+            }
+            if (!ok) { fail(); break; }
+            #pragma unroll
+            for (int h = 0; h < 4; h++) {
+                float v[16];
+                tmem_ld16(tl + 256 + 128 * (li & 1) + 16 * h, v);
+                #pragma unroll
+                for (int q = 0; q < 16; q++) acc[h][q] += v[q];
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive1(&lempty[li & 1]);
+            if (r >= g.M) continue;
+            float cph = 1.f, sph = 0.f;
+            if (g.epilogue == 1) sincosf(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar, &sph, &cph);
+            float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
+            const int cb = n0 + 64 * half;
+            if (vecC && cb + 64 <= g.N) {
+                #pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    float4 d[4];
+                    if (D)
+                        #pragma unroll
+                        for (int q = 0; q < 4; q++) d[q] = *reinterpret_cast<const float4 *>(D + cb + 16 * h + 4 * q);
+                    if (g.epilogue == 1)   // (re, im) pairs times exp(+i ph)
+                        #pragma unroll
+                        for (int q = 0; q < 16; q += 2) {
+                            const float re = acc[h][q], im = acc[h][q + 1];
+                            acc[h][q] = cph * re - sph * im;
+                            acc[h][q + 1] = sph * re + cph * im;
+                        }
+                    #pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        float4 x = make_float4(acc[h][4 * q], acc[h][4 * q + 1], acc[h][4 * q + 2], acc[h][4 * q + 3]);
+                        if (D) x = make_float4(d[q].x - x.x, d[q].y - x.y, d[q].z - x.z, d[q].w - x.w);   // C = D - A B
+                        *reinterpret_cast<float4 *>(C + cb + 16 * h + 4 * q) = x;
+                    }
+                }
+            } else {
+                #pragma unroll
+                for (int h = 0; h < 4; h++)
+                    #pragma unroll
+                    for (int q = 0; q < 16; q += 2) {
+                        const int c = cb + 16 * h + q;
+                        float re = acc[h][q], im = acc[h][q + 1];
+                        if (g.epilogue == 1) {
+                            const float x = cph * re - sph * im;
+                            im = sph * re + cph * im;
+                            re = x;
+                        }
+                        if (c < g.N) C[c] = D ? D[c] - re : re;
+                        if (c + 1 < g.N) C[c + 1] = D ? D[c + 1] - im : im;
+                    }
             }
         }
     }
+    fence_before();
+    __syncthreads();
+    if (warp == F_LOAD + F_ACC) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+    }
+}
+
+int gemm_sms() {
+    static int cache[64] = {};
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!cache[dev] && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) cache[dev] = n;
+    return cache[dev] > 0 ? cache[dev] : 148;
+}
+
+// ---- small products: FP32 SIMT, 32 x 32 tiles, 64 threads of 4 x 4 outputs, K 32 at a time in
+// two buffers.  Where the 128 x 128 tiles leave most SMs idle, the tile above pays its start-up
+// and 0.8 us for every 32 of K; this one about 0.5 us on many more SMs (gemm_small_wins).
+constexpr int SB = 32, SLD = SB + 4;
+
+template <bool KC>
+__device__ __forceinline__ void small_load(const float *p, int ld, int rdim, int kdim, int r0, int k0, bool vec, float4 (&v)[4]) {
+    #pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int idx = threadIdx.x + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
+        const int r = r0 + (KC ? o : c4), k = k0 + (KC ? c4 : o);
+        const float *q = KC ? p + (size_t)r * ld + k : p + (size_t)k * ld + r;
+        const int have = KC ? (r < rdim ? kdim - k : 0) : (k < kdim ? rdim - r : 0);
+        if (vec && have >= 4) { v[i] = __ldg(reinterpret_cast<const float4 *>(q)); continue; }
+        v[i] = make_float4(have > 0 ? __ldg(q) : 0.f, have > 1 ? __ldg(q + 1) : 0.f, have > 2 ? __ldg(q + 2) : 0.f,
+                           have > 3 ? __ldg(q + 3) : 0.f);
+    }
+}
+template <bool KC>
+__device__ __forceinline__ void small_store(float (*s)[SLD], const float4 (&v)[4]) {
+    #pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int idx = threadIdx.x + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
+        if (KC) { s[c4][o] = v[i].x; s[c4 + 1][o] = v[i].y; s[c4 + 2][o] = v[i].z; s[c4 + 3][o] = v[i].w; }
+        else *reinterpret_cast<float4 *>(&s[o][c4]) = v[i];
+    }
+}
+
+template <bool ACOL, bool BKC>
+__global__ void __launch_bounds__(64) k_gemm_small(GemmArgs g, bool vecA, bool vecB) {
+    __shared__ __align__(16) float As[2][SB][SLD], Bs[2][SB][SLD];
+    const int bz = blockIdx.z, m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
+    const float *A = g.A + (size_t)bz * g.sA, *B = g.B + (size_t)bz * g.sB;
+    const int tx = 4 * (threadIdx.x & 7), ty = 4 * (threadIdx.x >> 3);
+    float acc[4][4] = {};
+    float4 ra[4], rb[4];
+    small_load<!ACOL>(A, g.lda, g.M, g.K, m0, 0, vecA, ra);
+    small_load<BKC>(B, g.ldb, g.N, g.K, n0, 0, vecB, rb);
+    small_store<!ACOL>(As[0], ra);
+    small_store<BKC>(Bs[0], rb);
+    __syncthreads();
+    for (int k0 = 0, buf = 0; k0 < g.K; k0 += SB, buf ^= 1) {
+        const bool more = k0 + SB < g.K;
+        if (more) {
+            small_load<!ACOL>(A, g.lda, g.M, g.K, m0, k0 + SB, vecA, ra);
+            small_load<BKC>(B, g.ldb, g.N, g.K, n0, k0 + SB, vecB, rb);
+        }
+        #pragma unroll 8
+        for (int k = 0; k < SB; k++) {
+            const float4 a4 = *reinterpret_cast<const float4 *>(&As[buf][k][ty]);
+            const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[buf][k][tx]);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+            #pragma unroll
+            for (int i = 0; i < 4; i++)
+                #pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        if (more) {
+            small_store<!ACOL>(As[buf ^ 1], ra);
+            small_store<BKC>(Bs[buf ^ 1], rb);
+        }
+        __syncthreads();
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int r = m0 + ty + i;
+        if (r >= g.M) continue;
+        float cph = 1.f, sph = 0.f;
+        if (g.epilogue == 1) sincosf(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar, &sph, &cph);
+        float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
+        const float *D = g.epilogue == 2 ? g.D + (size_t)bz * g.sD + (size_t)r * g.ldd : nullptr;
+        #pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+            const int c = n0 + tx + j;
+            float re = acc[i][j], im = acc[i][j + 1];
+            if (g.epilogue == 1) {   // (re, im) pairs times exp(+i ph)
+                const float x = cph * re - sph * im;
+                im = sph * re + cph * im;
+                re = x;
+            }
+            if (c < g.N) C[c] = D ? D[c] - re : re;
+            if (c + 1 < g.N) C[c + 1] = D ? D[c + 1] - im : im;
+        }
+    }
+}
+
+// Which of the two is faster, from fits in us to both over M 54..2048, K 54..2048: 8 + 1.1 per
+// 32 of K and wave of tiles for the tensor cores, 4 + (0.75 + 0.3 blocks an SM) per 32 of K here.
+// Measured, this against the tensor cores: 128 x 256 x 128 8.4 / 12.5, 512 x 18 x 512 in four
+// matrices 22.7 / 32.4, 1024 x 128 x 1024 37 / 54; 256 x 512 x 256 in four 16.6 / 16.5;
+// 512 x 1024 x 512 28.8 / 25.2, 1024 x 2048 x 1024 156 / 43.
+bool gemm_small_wins(const GemmArgs &g, long long tiles, int batch, int sms) {
+    const double kt = (g.K + 31) / 32, waves = (double)((tiles + sms - 1) / sms);
+    const double blocks = (double)((g.M + SB - 1) / SB) * ((g.N + SB - 1) / SB) * batch / sms;
+    return 4.0 + kt * (0.75 + 0.3 * blocks) < 8.0 + 1.1 * kt * waves;
 }
 
 __global__ void k_identity(float *F, int n, int ldf, long long sF) {
@@ -205,23 +499,37 @@ __global__ void k_identity(float *F, int n, int ldf, long long sF) {
     for (int c = threadIdx.x; c < 2 * n; c += blockDim.x) f[(size_t)r * ldf + c] = (c == 2 * r) ? 1.f : 0.f;
 }
 
-template <class T>
-cudaError_t launch_sgemm(const GemmArgs &g, int batch, cudaStream_t s) {
-    dim3 grid((g.N + T::BN - 1) / T::BN, (g.M + T::BM - 1) / T::BM, batch);
-    if (g.a_colmajor && g.b_kmajor) return cudaErrorInvalidValue;
-    if (g.a_colmajor) k_sgemm<T, true, false><<<grid, GT, 0, s>>>(g);
-    else if (g.b_kmajor) k_sgemm<T, false, true><<<grid, GT, 0, s>>>(g);
-    else k_sgemm<T, false, false><<<grid, GT, 0, s>>>(g);
-    return cudaGetLastError();
-}
-
 }  // namespace
 
-cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *launches, int tile) {
-    if ((g.epilogue == 1 && (g.N & 1)) || (g.epilogue == 2 && !g.D)) return cudaErrorInvalidValue;
-    if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
-    const cudaError_t e = tile == CIR_GEMM_TILE_64 ? launch_sgemm<TileS>(g, batch, s) : launch_sgemm<TileL>(g, batch, s);
-    if (launches) *launches += 1;
+cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *launches) {
+    if ((g.epilogue == 1 && (g.N & 1)) || (g.epilogue == 2 && !g.D) || (g.a_colmajor && g.b_kmajor)) return cudaErrorInvalidValue;
+    if (batch < 1 || batch > 65535 || g.M < 1 || g.N < 1 || g.K < 1) return cudaErrorInvalidValue;
+    const int tiles_n = (g.N + FN - 1) / FN;
+    const long long mn = (long long)tiles_n * ((g.M + FM - 1) / FM), nt = mn * batch;
+    if (nt > INT_MAX) return cudaErrorInvalidValue;
+    auto vec = [&](const float *p, int ld, long long st) {
+        return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld & 3) == 0 && (batch == 1 || (st & 3) == 0);
+    };
+    const int sms = gemm_sms();
+    const bool va = vec(g.A, g.lda, g.sA), vb = vec(g.B, g.ldb, g.sB),
+               vc = vec(g.C, g.ldc, g.sC) && (g.epilogue != 2 || vec(g.D, g.ldd, g.sD));
+    if (gemm_small_wins(g, nt, batch, sms)) {
+        const dim3 grid((g.N + SB - 1) / SB, (g.M + SB - 1) / SB, batch);
+        if (g.a_colmajor) k_gemm_small<true, false><<<grid, 64, 0, s>>>(g, va, vb);
+        else if (g.b_kmajor) k_gemm_small<false, true><<<grid, 64, 0, s>>>(g, va, vb);
+        else k_gemm_small<false, false><<<grid, 64, 0, s>>>(g, va, vb);
+        if (launches) *launches += 1;
+        return cudaGetLastError();
+    }
+    const int grid = (int)std::min<long long>(nt, sms);
+    auto go = [&](auto kern) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, F_NT, F_SMEM, s>>>(g, tiles_n, (int)mn, (int)nt, va, vb, vc, g.err);
+        return cudaGetLastError();
+    };
+    const cudaError_t e = g.a_colmajor ? go(k_gemm<true, false>) : g.b_kmajor ? go(k_gemm<false, true>) : go(k_gemm<false, false>);
+    if (e == cudaSuccess && launches) *launches += 1;
     return e;
 }
 

@@ -88,7 +88,8 @@ typedef struct cir_params {
     int   batch_frames;            /* frame-steps per eigensolver batch, 0 = automatic */
     int   verbose;                 /* 0 silent, 1 reference-style progress on stdout   */
     int   cuda_graphs;             /* 1: replay the per-step launches from captured CUDA graphs */
-    int   autotune;                /* 1: time the GEMM tile shapes once per problem shape      */
+    int   autotune;                /* 1: time the tile widths of the split-BF16 products and
+                                      the tridiagonalisation's blocks per SM once per shape   */
     /* options of the run that give the same results by less work; off by default, so that
        the default run does the reference's work (full F propagation, one eigensolve per
        origin and step) */
@@ -296,8 +297,8 @@ typedef struct cir_traj_in {
 /* Many independent trajectories, boxes of uneven size allowed, with the context's
  * parameters (its own natoms is not used): trajectories of equal size are batched through
  * every launch (their eigensolves, propagation steps and contractions share launches), the
- * per-step launches are replayed from captured CUDA graphs (cuda_graphs) and the SIMT GEMM
- * tile shapes come from the autotuner (autotune).  results[i] receives trajectory i's
+ * per-step launches are replayed from captured CUDA graphs (cuda_graphs) and the
+ * split-BF16 tile widths come from the autotuner (autotune).  results[i] receives trajectory i's
  * outputs exactly as cir_run would fill them.  No counterpart in the reference, which runs
  * one trajectory per process (calcIR.cu:360-839 per run). */
 int cir_run_multi(cir_ctx *c, int ntraj, const cir_traj_in *traj, cir_result *results);

@@ -502,3 +502,20 @@ def test_contraction_forms(lib, nmol, origins):
     ref = O.run(prm, xyz, np.broadcast_to(box, (len(xyz), 3)), fos)
     for k in ("tcf_ir", "tcf_vv", "tcf_vh", "ls_ir", "ls_vv", "ls_vh", "sw"):
         assert O.rel_l2(out[k], ref[k]) < 1e-4, k      # the plain form's bound
+
+
+@pytest.mark.parametrize("n,batch", [(2, 1), (19, 2), (33, 3), (128, 1), (160, 60), (255, 24), (509, 2), (512, 4), (640, 1)])
+def test_propagate_forms(lib, n, batch):
+    """The FP32 products on small tiles and on the tensor cores, whole and ragged tiles, rows that
+    are and are not 16-byte aligned, against 64 bits: 2^-23 sqrt(n) a product for the sums,
+    2^-23 of the phase (at most 8 rad)."""
+    rng = np.random.default_rng(n)
+    V = np.stack([np.linalg.qr(rng.standard_normal((n, n)))[0] for _ in range(batch)]).astype(np.float32)
+    w = rng.uniform(-400, 400, (batch, n)).astype(np.float32)
+    F = (rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))).astype(np.complex64)
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 12) as eng:
+        got = eng.propagate(V, w, 0.1, F)
+    V64 = V.astype(np.float64)
+    phase = np.exp(1j * w.astype(np.float64) * np.float32(0.1) / HBAR)
+    ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F.astype(np.complex128)))
+    assert O.rel_l2(got, ref) < 2.0 ** -23 * (2 * np.sqrt(n) + 8)
