@@ -57,7 +57,7 @@ enum {
     B_TCF, B_HCNT, B_HIPR, B_HMIPR, B_OOR, B_SW, B_MU2, B_SWEEPS, B_ROT, B_PAD,
     B_FFT0, B_FFT1, B_FFTY, B_FFTX,  // lineshape: Stockham work, adjoint, rows, input
     B_PROF, B_DE, B_ERR, B_DC, B_TUNE,
-    B_PSI, B_LAM, B_PA, B_PB, B_SEG, B_CKPT, B_R, B_T, B_GRAD,   // differentiation form
+    B_PSI, B_LAM, B_PA, B_PB, B_GRAD,   // differentiation form
     B_VS, B_FS,                                    // split-BF16 propagation operands
     B_UFR,                                         // run: distinct frames of a chunk and their multiplicity
     B_HREF, B_RW,                                  // FP64 eigenpair refinement: input copy, workspace
@@ -785,7 +785,8 @@ static std::vector<long long> step_key(const Group &g, int St, int K, int k0, in
 }
 
 static int psi_propagate(cir_ctx *c, int S, int n, int ld, const float *V, long long sV, const float *w, long long sw,
-                         float dt, float *x, float *tmp, int &launches);
+                         float dt, const float *in, float *out, float *tmp, float *raw, const PsiSource *src,
+                         int &launches);
 
 // CIR_EIG_SPLIT=0: the eigensolver batch of a chunk in one stream, not two (for comparison)
 static bool eig_split_enabled() {
@@ -1234,10 +1235,11 @@ struct GroupJob {
                 if (k > 0) {
                     const int rc2 = psi_propagate(c, St, n, ld, A + mk * mstride, (long long)dlt * mstride, W + mk * ld,
                                                   (long long)dlt * ld, p.dt, buf[B_PSI].as<float>(),
-                                                  buf[B_LAM].as<float>(), nl);
+                                                  buf[B_PSI].as<float>(), buf[B_LAM].as<float>(), nullptr,
+                                                  nullptr, nl);
                     if (rc2) return rc2;
                 }
-                CK(cir_adj_tcf(buf[B_PSI].as<float>(), M + mk * 9 * ld, (long long)dlt * 9 * ld, ld, n, St,
+                CK(cir_adj_tcf(buf[B_PSI].as<float>(), M + mk * 9 * ld, (long long)dlt * 9 * ld, ld, n, St, 1,
                                tcf + (size_t)k * 6, (long long)K * 6, c->stream));
                 nl++;
                 return CIR_OK;
@@ -1810,19 +1812,16 @@ extern "C" int cir_set_coeffs(cir_ctx *c, const float *t) {
     return CIR_OK;
 }
 
-// x <- V_k exp(i L_k dt/hbar) V_k^T x for S origins, x n x 9 complex (row-major, 18 floats per
-// row); FP32 GEMMs.  V: origin s at V + s*sV, w likewise; tmp: S x n x 18.
+// out = V_k exp(i L_k dt/hbar) V_k^T in (+ the source) for S origins, n x 9 complex each
+// (row-major, 18 floats per row).  V: origin s at V + s*sV, w likewise; tmp: S x n x 18; raw, if
+// given: V_k^T in.
 static int psi_propagate(cir_ctx *c, int S, int n, int ld, const float *V, long long sV, const float *w, long long sw,
-                         float dt, float *x, float *tmp, int &launches) {
-    // X = e^{i L dt/hbar} V^T psi, then psi = V X: two streaming passes over V (k_adjoint.cu)
-    CK(cir_psi_step(V, ld, sV, n, w, sw, (float)(dt / CIR_HBAR), x, tmp, S, c->stream));
+                         float dt, const float *in, float *out, float *tmp, float *raw, const PsiSource *src,
+                         int &launches) {
+    CK(cir_psi_step(V, ld, sV, n, w, sw, (float)(dt / CIR_HBAR), in, out, tmp, raw, src, S, c->stream));
     launches += 2;
     return CIR_OK;
 }
-
-// psi is checkpointed every CKPT steps (psi(0), then psi(j*CKPT - 1)); the backward pass
-// recomputes one segment of CKPT steps at a time from its checkpoint.
-constexpr int CKPT = 16;
 
 extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const float *box, const int *frame_of_step,
                              const float *target_ir, const float *target_vv, int nls, double *loss, double *grad) {
@@ -1858,7 +1857,6 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     if ((rc = stage_in(c, B_BOX, box, (size_t)nframes * 12, &dbox, true))) return rc;
     const int nb = (int)steps;
     const size_t psz = (size_t)S * n * CIR_PSI_LD;            // floats of one psi set
-    const int nseg = (K + CKPT - 1) / CKPT;
     CK(c->buf[B_FIDX].ensure((size_t)steps * 4));
     CK(cudaMemcpyAsync(c->buf[B_FIDX].p, fidx.data(), (size_t)steps * 4, cudaMemcpyHostToDevice, c->stream));
     CK(c->buf[B_CXYZ].ensure((size_t)nb * c->natoms * 12));
@@ -1871,24 +1869,21 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     CK(c->buf[B_W].ensure((size_t)nb * ld * 4));
     CK(c->buf[B_M].ensure((size_t)nb * 9 * ld * 4));
     CK(c->buf[B_STATUS].ensure((size_t)nb * 4));
-    CK(c->buf[B_PSI].ensure(psz * 4));
-    CK(c->buf[B_LAM].ensure(psz * 4));
-    CK(c->buf[B_PA].ensure(psz * 4));
-    CK(c->buf[B_PB].ensure(psz * 4));
-    CK(c->buf[B_SEG].ensure(psz * (CKPT + 1) * 4));
-    CK(c->buf[B_CKPT].ensure(psz * nseg * 4));
-    CK(c->buf[B_R].ensure((size_t)S * mstride * 4));
-    CK(c->buf[B_T].ensure((size_t)S * mstride * 4));
+    // psi(k), and the half-way points V_k^T psi(k-1) and V_k^T lambda(k), of every step
+    CK(c->buf[B_PSI].ensure(psz * K * 4));
+    CK(c->buf[B_PA].ensure(psz * K * 4));
+    CK(c->buf[B_PB].ensure(psz * K * 4));
+    CK(c->buf[B_LAM].ensure(psz * 2 * 4));
     CK(c->buf[B_TCF].ensure((size_t)steps * 48));
     CK(c->buf[B_GRAD].ensure(CIR_NTHETA * 8));
     CK(cudaMemsetAsync(c->buf[B_STATUS].p, 0, (size_t)nb * 4, c->stream));
     CK(cudaMemsetAsync(c->buf[B_GRAD].p, 0, CIR_NTHETA * 8, c->stream));
     float *A = c->buf[B_A].as<float>(), *W = c->buf[B_W].as<float>(), *M = c->buf[B_M].as<float>();
     float *CT = c->buf[B_CT].as<float>(), *CB = c->buf[B_CBOX].as<float>();
-    float *psi = c->buf[B_PSI].as<float>(), *lam = c->buf[B_LAM].as<float>();
+    float *psi = c->buf[B_PSI].as<float>(), *lam = c->buf[B_LAM].as<float>(), *X = lam + psz;
     float *PA = c->buf[B_PA].as<float>(), *PB = c->buf[B_PB].as<float>();
-    float *seg = c->buf[B_SEG].as<float>(), *ckpt = c->buf[B_CKPT].as<float>();
-    float *R = c->buf[B_R].as<float>(), *T = c->buf[B_T].as<float>();
+    // R and G, and V R, of every step in the eigensolver's scratch, free by then
+    float *R = c->buf[B_Z].as<float>(), *T = c->buf[B_DC].as<float>();
     double *tcf = c->buf[B_TCF].as<double>(), *dgrad = c->buf[B_GRAD].as<double>();
     int launches = 0;
     // frames, Hamiltonians and eigendecompositions of every step (origin-major: b = s*K + k)
@@ -1928,21 +1923,15 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     e.test_stall = c->p.test_stall_gemm;
     e.test_sweep_cap = c->p.test_sweep_cap;
     CK(cir_launch_eigh(e, nb, c->stream, &launches));
-    // forward: psi(0) = m(0); psi(k) = U_k psi(k-1); correlation terms per step; checkpoints
+    // forward: psi(0) = m(0); psi(k) = U_k psi(k-1); then every step's correlation terms
     const long long sV = (long long)K * mstride, sWk = (long long)K * ld, sM = (long long)K * 9 * ld;
     CK(cir_adj_psi_init(M, sM, ld, n, S, psi, c->stream));
-    launches++;
-    for (int k = 0; k < K; k++) {
-        if (k > 0 && (rc = psi_propagate(c, S, n, ld, A + (size_t)k * mstride, sV, W + (size_t)k * ld, sWk, p.dt, psi, PA,
-                                         launches)))
+    for (int k = 1; k < K; k++)
+        if ((rc = psi_propagate(c, S, n, ld, A + (size_t)k * mstride, sV, W + (size_t)k * ld, sWk, p.dt,
+                                psi + psz * (k - 1), psi + psz * k, X, PB + psz * k, nullptr, launches)))
             return rc;
-        CK(cir_adj_tcf(psi, M + (size_t)k * 9 * ld, sM, ld, n, S, tcf + (size_t)k * 6, (long long)K * 6, c->stream));
-        launches++;
-        if (k == 0 || (k + 1) % CKPT == 0) {
-            const int slot = k == 0 ? 0 : (k + 1) / CKPT;
-            if (slot < nseg) CK(cudaMemcpyAsync(ckpt + psz * slot, psi, psz * 4, cudaMemcpyDeviceToDevice, c->stream));
-        }
-    }
+    CK(cir_adj_tcf(psi, M, sM, ld, n, S, K, tcf, (long long)K * 6, c->stream));
+    launches += 2;
     // loss: lineshapes of the damped, origin-averaged IR and VV sums against the targets
     std::vector<double> htcf((size_t)steps * 6);
     std::vector<int> hst(nb);
@@ -1951,19 +1940,19 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     CK(cudaStreamSynchronize(c->stream));
     for (int i = 0; i < nb; i++)
         if (hst[i]) return cir_fail(CIR_ERR_NOCONVERGE, "eigensolver sweep cap reached");
-    std::vector<double> dcy(K), X((size_t)4 * K, 0.0);
+    std::vector<double> dcy(K), spec((size_t)4 * K, 0.0);
     for (int k = 0; k < K; k++) {
         dcy[k] = exp(-1.0 * k * p.dt / (2.0 * p.t1)) / (1. * S);
         CompSum sum[4];                              // IR (terms 0, 1) and VV (terms 2, 3)
         for (int s = 0; s < S; s++)
             for (int q = 0; q < 4; q++) sum[q].add(htcf[((size_t)s * K + k) * 6 + q]);
         for (int q = 0; q < 2; q++) {
-            X[(size_t)2 * (q * K + k)] = sum[2 * q].value() * dcy[k];
-            X[(size_t)2 * (q * K + k) + 1] = sum[2 * q + 1].value() * dcy[k];
+            spec[(size_t)2 * (q * K + k)] = sum[2 * q].value() * dcy[k];
+            spec[(size_t)2 * (q * K + k) + 1] = sum[2 * q + 1].value() * dcy[k];
         }
     }
     // the loss and dL/dX of both spectra (k_fft.cu), then through the damping and 1/nsamples
-    if ((rc = lineshape_dev(c, X.data(), 2, lr))) return rc;
+    if ((rc = lineshape_dev(c, spec.data(), 2, lr))) return rc;
     CK(c->buf[B_FFT1].ensure((size_t)nls * (16 + 8) + (size_t)(4 * K + 1) * 8));
     double *dy = c->buf[B_FFT1].as<double>(), *dl = dy + 2 * (size_t)nls, *dg = dl + 1;
     float *tgt = reinterpret_cast<float *>(dg + 4 * (size_t)K);
@@ -1974,86 +1963,64 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
     CK(cudaMemcpyAsync(lg.data(), dl, lg.size() * 8, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     const double L = lg[0];
-    std::vector<double> gre[2], gim[2];
-    for (int q = 0; q < 2; q++)
-        for (int k = 0; k < K; k++) {
-            gre[q].push_back(lg[1 + (size_t)2 * (q * K + k)] * dcy[k]);
-            gim[q].push_back(lg[2 + (size_t)2 * (q * K + k)] * dcy[k]);
-        }
-    // backward, one segment of CKPT steps at a time, last segment first
+    std::vector<double> gk((size_t)4 * K);                     // dL/dTCF: (re, im) of IR and VV
+    for (int k = 0; k < K; k++)
+        for (int q = 0; q < 4; q++) gk[4 * (size_t)k + q] = lg[1 + (size_t)2 * ((q / 2) * K + k) + (q & 1)] * dcy[k];
+    CK(cudaMemcpyAsync(dg, gk.data(), gk.size() * 8, cudaMemcpyHostToDevice, c->stream));
+    // backward: lambda(k) = w(k) + U_{k+1} lambda(k+1)
+    auto source = [&](int k) {
+        return PsiSource{M + (size_t)k * 9 * ld, sM, (float)gk[4 * (size_t)k], (float)gk[4 * (size_t)k + 1],
+                         (float)gk[4 * (size_t)k + 2], (float)gk[4 * (size_t)k + 3]};
+    };
+    CK(cir_adj_lambda_init(lam, source(K - 1), ld, n, S, c->stream));
+    launches++;
+    for (int k = K - 1; k >= 1; k--) {
+        const PsiSource src = source(k - 1);
+        if ((rc = psi_propagate(c, S, n, ld, A + (size_t)k * mstride, sV, W + (size_t)k * ld, sWk, p.dt, lam, lam, X,
+                                PA + psz * k, &src, launches)))
+            return rc;
+    }
+    // R and G = V R V^T of steps 1 .. K-1 of every origin: batches over the longer of the two
     const float tau = (float)(p.dt / CIR_HBAR);
+    const bool by_origin = K - 1 >= S;
+    for (int q = 0; q < (K < 2 ? 0 : by_origin ? S : K - 1); q++) {
+        const int s0 = by_origin ? q : 0, k0 = by_origin ? 1 : q + 1, batch = by_origin ? K - 1 : S;
+        const size_t b0 = (size_t)s0 * K + k0, p0 = ((size_t)k0 * S + s0) * n * CIR_PSI_LD;
+        const long long step = by_origin ? 1 : K;              // matrices between the batch's
+        CK(cir_adj_build_R(PA + p0, PB + p0, by_origin ? (long long)psz : (long long)n * CIR_PSI_LD, W + b0 * ld,
+                           step * ld, n, batch, tau, R + b0 * mstride, ld, step * mstride, c->stream));
+        GemmArgs gt{};
+        gt.err = c->buf[B_ERR].as<int>();
+        gt.A = A + b0 * mstride; gt.lda = ld; gt.sA = step * mstride; gt.a_colmajor = true;   // V
+        gt.B = R + b0 * mstride; gt.ldb = ld; gt.sB = step * mstride;
+        gt.C = T + b0 * mstride; gt.ldc = ld; gt.sC = step * mstride;
+        gt.M = gt.N = gt.K = n;
+        GemmArgs gg = gt;
+        gg.A = gt.C; gg.a_colmajor = false;
+        gg.B = gt.A;                                           // B(k, j) = V[j][k]
+        gg.C = R + b0 * mstride;
+        CK(cir_launch_gemm(gt, batch, c->stream, &launches));
+        CK(cir_launch_gemm(gg, batch, c->stream, &launches));
+        launches++;
+    }
     DthetaArgs dt{};
-    dt.sct = (long long)K * CT_NROW * ld;
-    dt.sbox = 3LL * K;
+    dt.ct = CT;
+    dt.box = CB;
+    dt.G = R;
     dt.ldg = ld;
     dt.sG = mstride;
+    dt.psi = psi;
+    dt.lam0 = lam;
+    dt.g = dg;
     dt.maps = c->maps;
     dt.n = n;
     dt.ld = ld;
+    dt.K = K;
     dt.nchrom_mol = p.nchrom_mol;
     dt.ispecies = p.ispecies;
     dt.out = dgrad;
-    for (int j = nseg - 1; j >= 0; j--) {
-        const int c0 = j * CKPT, c1 = std::min(K, c0 + CKPT);
-        const int base = c0 == 0 ? 0 : c0 - 1;        // seg slot q holds psi(base + q)
-        CK(cudaMemcpyAsync(seg, ckpt + psz * j, psz * 4, cudaMemcpyDeviceToDevice, c->stream));
-        for (int k = base + 1; k < c1; k++) {
-            float *dst = seg + psz * (k - base);
-            CK(cudaMemcpyAsync(dst, seg + psz * (k - 1 - base), psz * 4, cudaMemcpyDeviceToDevice, c->stream));
-            if ((rc = psi_propagate(c, S, n, ld, A + (size_t)k * mstride, sV, W + (size_t)k * ld, sWk, p.dt, dst, PA,
-                                    launches)))
-                return rc;
-        }
-        for (int k = c1 - 1; k >= c0; k--) {
-            // lambda(k) = w(k) + U_{k+1} lambda(k+1)
-            if (k < K - 1 && (rc = psi_propagate(c, S, n, ld, A + (size_t)(k + 1) * mstride, sV, W + (size_t)(k + 1) * ld,
-                                                 sWk, p.dt, lam, PA, launches)))
-                return rc;
-            CK(cir_adj_lambda_src(lam, M + (size_t)k * 9 * ld, sM, ld, n, S, (float)gre[0][k], (float)gim[0][k],
-                                  (float)gre[1][k], (float)gim[1][k], k == K - 1, c->stream));
-            launches++;
-            const float *Vk = A + (size_t)k * mstride;
-            if (k >= 1) {
-                // a = V^T lambda(k), b = V^T psi(k-1); R; G = V R V^T (into R)
-                GemmArgs ga{};
-                ga.err = c->buf[B_ERR].as<int>();
-                ga.A = Vk; ga.lda = ld; ga.sA = sV; ga.a_colmajor = false;
-                ga.B = lam; ga.ldb = CIR_PSI_LD; ga.sB = (long long)n * CIR_PSI_LD;
-                ga.C = PA; ga.ldc = CIR_PSI_LD; ga.sC = (long long)n * CIR_PSI_LD;
-                ga.M = n; ga.N = CIR_PSI_LD; ga.K = n;
-                GemmArgs gb = ga;
-                gb.B = seg + psz * (k - 1 - base);
-                gb.C = PB;
-                CK(cir_launch_gemm(ga, S, c->stream, &launches));
-                CK(cir_launch_gemm(gb, S, c->stream, &launches));
-                CK(cir_adj_build_R(PA, PB, W + (size_t)k * ld, sWk, n, S, tau, R, ld, mstride, c->stream));
-                launches++;
-                GemmArgs gt{};
-                gt.err = c->buf[B_ERR].as<int>();
-                gt.A = Vk; gt.lda = ld; gt.sA = sV; gt.a_colmajor = true;     // V
-                gt.B = R; gt.ldb = ld; gt.sB = mstride;                        // R row-major
-                gt.C = T; gt.ldc = ld; gt.sC = mstride;
-                gt.M = gt.N = gt.K = n;
-                GemmArgs gg = gt;
-                gg.A = T; gg.a_colmajor = false; gg.sA = mstride;              // T row-major
-                gg.B = Vk; gg.sB = sV;                                         // B(k, j) = V[j][k]
-                gg.C = R;
-                CK(cir_launch_gemm(gt, S, c->stream, &launches));
-                CK(cir_launch_gemm(gg, S, c->stream, &launches));
-            }
-            dt.ct = CT + (size_t)k * CT_NROW * ld;
-            dt.box = CB + 3 * (size_t)k;
-            dt.G = k >= 1 ? R : nullptr;
-            dt.psi = seg + psz * (k - base);
-            dt.lam0 = k == 0 ? lam : nullptr;
-            dt.gir_r = (float)gre[0][k];
-            dt.gir_i = (float)gim[0][k];
-            dt.gvv_r = (float)gre[1][k];
-            dt.gvv_i = (float)gim[1][k];
-            CK(cir_adj_dtheta(dt, S, c->stream));
-            launches++;
-        }
-    }
+    CK(cir_adj_dtheta(dt, S, c->stream));
+    launches++;
     CK(cudaMemcpyAsync(grad, dgrad, CIR_NTHETA * 8, cudaMemcpyDeviceToHost, c->stream));
     if ((rc = check_kernel_flag(c))) return rc;
     count_launch(c, launches);

@@ -295,31 +295,37 @@ cudaError_t cir_launch_identity(float *F, int n, int ldf, long long sF, int batc
 
 // ---- differentiation form (k_adjoint.cu) ----
 constexpr int CIR_PSI_LD = 18;   // psi / lambda: n x 9 complex, row-major (re, im) pairs
-struct DthetaArgs {
-    const float *ct;      // chromophore table of the step's frame of origin 0; origin s at + s*sct
-    long long sct;
-    const float *box;     // box of that frame; origin s at + s*sbox
-    long long sbox;
-    const float *G;       // dL/dH of the step (row-major, ldg; origin s at + s*sG), or null at step 0
+struct DthetaArgs {       // matrix b = s*K + k: step k of origin s
+    const float *ct;      // chromophore tables, CT_NROW * ld apart
+    const float *box;     // boxes, 3 apart
+    const float *G;       // dL/dH (symmetric, leading dimension ldg), sG apart; not read at step 0
     int ldg;
     long long sG;
-    const float *psi;     // psi(k), n x 18 per origin
-    const float *lam0;    // lambda(0) at step 0, else null
-    float gir_r, gir_i, gvv_r, gvv_i;   // dL/dTCF of the step (IR, VV)
+    const float *psi;     // psi(k) of origin s at (k*S + s) * n * CIR_PSI_LD
+    const float *lam0;    // lambda(0), n x CIR_PSI_LD per origin
+    const double *g;      // dL/dTCF of the steps: (re, im) of IR and of VV, 4 a step
     CirMaps maps;
-    int n, ld, nchrom_mol, ispecies;
+    int n, ld, K, nchrom_mol, ispecies;
     double *out;          // [13] accumulated
 };
-// one step psi <- V e^{i L dt/hbar} V^T psi of S origins (psi, tmp: n x CIR_PSI_LD per origin)
+// the adjoint's source w(k): m(k) of origin 0 (origin s at M + s*sM) and dL/dTCF of the step
+struct PsiSource {
+    const float *M;
+    long long sM;
+    float gir_r, gir_i, gvv_r, gvv_i;
+};
+// one step out = V e^{i L dt/hbar} V^T in (+ the source, if any) of S origins (n x CIR_PSI_LD per
+// origin each; in may be out); raw, if given, receives V^T in
 cudaError_t cir_psi_step(const float *V, int ld, long long sV, int n, const float *w, long long sw, float dt_over_hbar,
-                         float *psi, float *tmp, int S, cudaStream_t s);
+                         const float *in, float *out, float *tmp, float *raw, const PsiSource *src, int S,
+                         cudaStream_t s);
 cudaError_t cir_adj_psi_init(const float *M, long long sM, int ld, int n, int S, float *psi, cudaStream_t s);
-cudaError_t cir_adj_tcf(const float *psi, const float *M, long long sM, int ld, int n, int S, double *out, long long sout,
-                        cudaStream_t s);
-cudaError_t cir_adj_lambda_src(float *lam, const float *M, long long sM, int ld, int n, int S, float gir_r, float gir_i,
-                               float gvv_r, float gvv_i, int zero, cudaStream_t s);
-cudaError_t cir_adj_build_R(const float *a, const float *b, const float *W, long long sW, int n, int S, float tau, float *R,
-                            int ldr, long long sR, cudaStream_t s);
+// K steps: psi(k) of all origins at psi + k * S * n * CIR_PSI_LD, m(k) at M + 9 k ld
+cudaError_t cir_adj_tcf(const float *psi, const float *M, long long sM, int ld, int n, int S, int K, double *out,
+                        long long sout, cudaStream_t s);
+cudaError_t cir_adj_lambda_init(float *lam, const PsiSource &src, int ld, int n, int S, cudaStream_t s);
+cudaError_t cir_adj_build_R(const float *a, const float *b, long long sab, const float *W, long long sW, int n, int batch,
+                            float tau, float *R, int ldr, long long sR, cudaStream_t s);
 cudaError_t cir_adj_dtheta(const DthetaArgs &d, int S, cudaStream_t s);
 
 #endif

@@ -117,3 +117,32 @@ def test_loss_grad_config_size(lib):
     assert abs(L - Lref) <= BAR * Lref, (L, Lref)
     err = _close(g, z["grad"], th0, "FP64 adjoint, 256 H2O 4 x 200")
     print(f"config-size gradient: worst theta_i dL/dtheta_i error {err:.2e} of the largest")
+
+
+@pytest.mark.parametrize("nmol,S,K", [(13, 1, 2), (17, 2, 1), (19, 7, 4), (37, 3, 5), (24, 210, 2)])
+def test_loss_grad_batches(lib, nmol, S, K):
+    """Steps batched by origin and by step, the last rows of a block ragged, two rows a thread in
+    the vector steps (from 608 blocks), and no step at all."""
+    prm, p, xyz, box, fos, th0, targets = _setup(lib, nmol, S, K, 200, seed=nmol)
+    with lib.Engine(p, xyz.shape[1]) as eng:
+        L, g = eng.loss_grad(xyz, box, fos, targets[0], targets[1])
+    Lref, gref = A.adjoint_grad(prm, th0, xyz, [box] * len(xyz), fos, [t.astype(np.float64) for t in targets])
+    assert abs(L - Lref) <= BAR * Lref, (L, Lref)
+    _close(g, gref, th0, "FP64 adjoint")
+
+
+@pytest.mark.parametrize("nmol,S", [(16, 1), (257, 2), (300, 40)])
+def test_vector_steps(lib, nmol, S):
+    """psi = F m(0) propagated equals F propagated: one and two depths staged, one and two rows a
+    thread.  2^-23 sqrt(n) for each of two products in two steps, about ten for the cancellation."""
+    _, p, xyz, box, fos, _, _ = _setup(lib, 16, 1, 3, 200)
+    xyz, box = lib.synth_trajectory(nmol, S + 2, seed=nmol)
+    fos = (np.arange(S)[:, None] + np.arange(3)[None, :]).astype(np.int32).ravel()
+    out = []
+    for vec in (0, 1):
+        q = lib.default_params(model="tip4p2005", species="H2O", ntcfpoints=3, nsamples=S, sampleEvery=0.01, nzeros=200,
+                               avef=3415.0, propagate_vectors=vec)
+        with lib.Engine(q, xyz.shape[1]) as eng:
+            out.append(eng.run(xyz, box, fos))
+    for k in ("tcf_ir", "tcf_vv", "tcf_vh"):
+        assert O.rel_l2(out[1][k], out[0][k]) < 40 * 2.0 ** -23 * np.sqrt(2 * nmol), k
