@@ -519,3 +519,13 @@ def test_propagate_forms(lib, n, batch):
     phase = np.exp(1j * w.astype(np.float64) * np.float32(0.1) / HBAR)
     ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F.astype(np.complex128)))
     assert O.rel_l2(got, ref) < 2.0 ** -23 * (2 * np.sqrt(n) + 8)
+
+
+@pytest.mark.parametrize("n,batch", [(2, 3), (3, 1), (33, 5), (130, 2), (513, 1)])
+def test_unit_eigenvectors(lib, n, batch):
+    """The plain form's eigenvectors have length one to the rounding of their elements (2^-24
+    each, at most 2^-23 of the squared length, and as much again for the sum that scales them)."""
+    A = np.random.default_rng(n).standard_normal((batch, n, n)).astype(np.float32)
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 12) as eng:
+        _, V = eng.eigh(A + A.swapaxes(1, 2))
+    assert np.abs((np.asarray(V, np.float64) ** 2).sum(1) - 1).max() < 2.0 ** -22
