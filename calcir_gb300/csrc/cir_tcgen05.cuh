@@ -1,5 +1,5 @@
 // PTX wrappers for the tcgen05 tensor-core kernels: mbarriers (every wait bounded),
-// MMA issue and commit, the tcgen05 fences, and tensor-memory loads.
+// MMA issue and commit, the tcgen05 fences, and tensor-memory loads; thread-block clusters.
 #ifndef CIR_TCGEN05_CUH_
 #define CIR_TCGEN05_CUH_
 
@@ -86,6 +86,30 @@ __device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t addr, uint32_t lbo
 // instruction descriptor: D f32, A/B format, K-major A and B, N x M tile
 __host__ __device__ constexpr uint32_t make_idesc_mn(uint32_t ab_format, int m, int n) {
     return (1u << 4) | (ab_format << 7) | (ab_format << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// ---- thread-block clusters and their distributed shared memory
+__device__ __forceinline__ unsigned cl_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cl_size() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cl_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// p (this block's shared memory) in block `rank` of the cluster
+__device__ __forceinline__ unsigned cl_map(const float *p, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cl_store(unsigned addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
 }  // namespace

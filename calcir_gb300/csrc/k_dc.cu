@@ -10,7 +10,7 @@
 //   * k_dc_leaf: one warp per leaf solves its block by implicit QR (Wilkinson shift), every
 //     lane applying the rotations to its row of the leaf's eigenvector block, and writes the
 //     eigenvalues ascending with their vectors.
-//   * k_dc_merge (one block per merge): z = (last row of Q1, sign(beta) first row of Q2)/sqrt2,
+//   * k_dc_merge (a block or a cluster per merge): z = (last row of Q1, sign(beta) first row of Q2)/sqrt2,
 //     rho = 2|beta|; the two sorted eigenvalue lists are merged; small components of z and
 //     close pairs are deflated (close pairs by a Givens rotation, LAPACK laed2 rules with
 //     tol = 8 eps max(|D|, |z|)); the secular equation 1/rho + sum z_j^2/(D_j - lambda) = 0
@@ -26,6 +26,7 @@
 // applied to Q_T in compact WY blocks (k_backtransform.cu): FP32 GEMMs in the plain form,
 // the tensor-core GEMM (a.precision) in the mixed forms.
 #include "cir_device.cuh"
+#include "cir_tcgen05.cuh"
 
 #include <cstdlib>
 #include <float.h>
@@ -33,18 +34,22 @@
 namespace {
 
 constexpr int DC_LEAF = 32;
-constexpr int DC_NT = 256;          // threads of a merge block of 129-512 rows (fewer below, twice above)
 constexpr float DC_EPS = 5.9604645e-8f;   // 2^-24
 
 __host__ __device__ inline int dc_off(int level, int b, int n) { return (int)(((long long)b * n) >> level); }
 
 // ---------------------------------------------------------------------------------------
-// Leaves: warp w of the block handles leaf blockIdx.x * 4 + w of matrix blockIdx.y.
+// Leaves: warp w of the block handles leaf blockIdx.x * 4 + w of matrix blockIdx.y.  The chain
+// of a sweep's rotations bounds it: d and e stay in registers, an entry a lane, those a
+// rotation meets are fetched one rotation ahead, its (c, s) come from one refined reciprocal
+// square root, and the sweep's range from a ballot.  One matrix of order 128: 256 us with a square root,
+// two divisions and a round trip through shared memory a rotation and the range searched entry by
+// entry, 88 so; 200 of order 1024: 763, 387.
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) k_dc_leaf(EighArgs a, int depth, float *Qout) {
-    __shared__ float Zs[4][DC_LEAF][DC_LEAF + 1];
-    __shared__ float dS[4][DC_LEAF + 1], eS[4][DC_LEAF + 1];
-    __shared__ int rk[4][DC_LEAF];
+    __shared__ float Zs[4][32][DC_LEAF + 1];
+    __shared__ float dS[4][32];
+    __shared__ int rk[4][32];
     const int n = a.n, ld = a.ld;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int leaf = blockIdx.x * 4 + warp;
@@ -55,64 +60,65 @@ __global__ void __launch_bounds__(128) k_dc_leaf(EighArgs a, int depth, float *Q
     float *Q = Qout + (size_t)m * a.mstride;
     const int a0 = dc_off(depth, leaf, n), a1 = dc_off(depth, leaf + 1, n);
     const int s = a1 - a0;
-    float *d = dS[warp], *e = eS[warp];
+    float *d = dS[warp];
     float(*Z)[DC_LEAF + 1] = Zs[warp];
+    float dl = 0.f, el = 0.f;                       // lane i: d[i], e[i]
     if (lane < s) {
-        float v = dw[a0 + lane];
-        if (lane == 0 && a0 > 0) v -= fabsf(ev[a0 - 1]);
-        if (lane == s - 1 && a1 < n) v -= fabsf(ev[a1 - 1]);
-        d[lane] = v;
-        e[lane] = lane < s - 1 ? ev[a0 + lane] : 0.f;
+        dl = dw[a0 + lane];
+        if (lane == 0 && a0 > 0) dl -= fabsf(ev[a0 - 1]);
+        if (lane == s - 1 && a1 < n) dl -= fabsf(ev[a1 - 1]);
+        el = lane < s - 1 ? ev[a0 + lane] : 0.f;
     }
-    for (int c = 0; c < s; c++)
-        if (lane < s) Z[lane][c] = lane == c ? 1.f : 0.f;
-    __syncwarp();
+    for (int c = 0; c < s; c++) Z[lane][c] = lane == c ? 1.f : 0.f;
+    auto at = [](float v, int i) { return __shfl_sync(0xffffffffu, v, i); };
     // implicit QR with the Wilkinson shift; every lane runs the same scalar recurrence
-    float tn = 0.f;
-    for (int i = 0; i < s; i++) tn = fmaxf(tn, fabsf(d[i]) + 2.f * fabsf(e[i]));
+    float tn = fabsf(dl) + 2.f * fabsf(el);
+    for (int o = 16; o > 0; o >>= 1) tn = fmaxf(tn, __shfl_xor_sync(0xffffffffu, tn, o));
     const float tiny = 1e-12f * tn + FLT_MIN;
     int cm = s - 1, nsweep = 0;
     const int cap = a.test_sweep_cap > 0 ? a.test_sweep_cap : 30 * s + 30;
     while (cm > 0 && nsweep < cap) {
-        if (fabsf(e[cm - 1]) <= DC_EPS * (fabsf(d[cm - 1]) + fabsf(d[cm])) || fabsf(e[cm - 1]) <= tiny) {
-            cm--;
-            continue;
-        }
-        int l = cm - 1;
-        while (l > 0 && !(fabsf(e[l - 1]) <= DC_EPS * (fabsf(d[l - 1]) + fabsf(d[l])) || fabsf(e[l - 1]) <= tiny)) l--;
-        const float t = 0.5f * (d[cm - 1] - d[cm]);
-        const float bb = e[cm - 1];
+        // the couplings that are negligible, and the unreduced range l .. cm that ends last
+        const float du = __shfl_down_sync(0xffffffffu, dl, 1);
+        const bool neg = lane < s - 1 && (fabsf(el) <= DC_EPS * (fabsf(dl) + fabsf(du)) || fabsf(el) <= tiny);
+        const unsigned cut = __ballot_sync(0xffffffffu, neg);
+        while (cm > 0 && (cut >> (cm - 1) & 1)) cm--;
+        if (cm == 0) break;
+        const int l = 32 - __clz(cut & ((1u << (cm - 1)) - 1));
+        const float bb = at(el, cm - 1), dm = at(dl, cm);
+        const float t = 0.5f * (at(dl, cm - 1) - dm);
         const float den = t + copysignf(sqrtf(t * t + bb * bb), t);
-        const float mu = d[cm] - (den != 0.f ? bb * bb / den : 0.f);
-        float x = d[l] - mu, z = e[l];
+        const float mu = dm - (den != 0.f ? bb * bb / den : 0.f);
+        float dk = at(dl, l), ek = at(el, l), dn = at(dl, l + 1), en = at(el, l + 1);
+        float x = dk - mu, z = ek, z0 = Z[lane][l];
         for (int k = l; k < cm; k++) {
-            // every lane reads the same scalars, then lane 0 alone writes them back
-            const float dk = d[k], dk1 = d[k + 1], ek = e[k], ek1 = k + 1 < cm ? e[k + 1] : 0.f;
-            __syncwarp();
-            const float r = sqrtf(x * x + z * z);
-            const float c = r > 0.f ? x / r : 1.f, sn = r > 0.f ? z / r : 0.f;
-            const float g = sn * (dk - dk1) - 2.f * c * ek;
-            const float ekn = c * sn * (dk1 - dk) + (c * c - sn * sn) * ek;
-            if (lane == 0) {
-                if (k > l) e[k - 1] = r;
-                d[k] = dk - sn * g;
-                d[k + 1] = dk1 + sn * g;
-                e[k] = ekn;
-                if (k + 1 < cm) e[k + 1] = c * ek1;
-            }
-            if (k + 1 < cm) {
-                z = sn * ek1;
-                x = ekn;
-            }
-            if (lane < s) {
-                const float z0 = Z[lane][k], z1 = Z[lane][k + 1];
-                Z[lane][k] = c * z0 + sn * z1;
-                Z[lane][k + 1] = c * z1 - sn * z0;
-            }
-            __syncwarp();
+            const float dk1 = dn, ek1 = k + 1 < cm ? en : 0.f, z1 = Z[lane][k + 1];
+            dn = at(dl, k + 2);
+            en = at(el, k + 2);
+            const float r2 = x * x + z * z;
+            float rs = rsqrtf(r2);
+            rs = fmaf(rs, fmaf(-0.5f * r2 * rs, rs, 0.5f), rs);
+            const bool turn = r2 > 0.f;
+            const float c = turn ? x * rs : 1.f, sn = turn ? z * rs : 0.f;
+            const float dd = dk - dk1;
+            const float g = sn * dd - 2.f * c * ek;
+            x = (c * c - sn * sn) * ek - c * sn * dd;
+            if (lane == k - 1 && k > l) el = turn ? r2 * rs : 0.f;
+            if (lane == k) dl = dk - sn * g;
+            Z[lane][k] = c * z0 + sn * z1;
+            z0 = c * z1 - sn * z0;
+            dk = dk1 + sn * g;
+            ek = c * ek1;
+            z = sn * ek1;
         }
+        if (lane == cm) dl = dk;
+        if (lane == cm - 1) el = x;
+        Z[lane][cm] = z0;
         nsweep++;
     }
+    __syncwarp();
+    if (lane < s) d[lane] = dl;
+    __syncwarp();
     if (lane == 0 && nsweep >= cap && a.status) a.status[m] = 1;
     // ascending order (ties by index)
     if (lane < s) {
@@ -176,43 +182,90 @@ __device__ float dc_block_sum(float v, float *red) {
     return r;
 }
 
-// root i of 1/rho + sum_j z2_j / (Dn_j - lambda); returns the origin index, *tau = lambda - Dn[origin]
-__device__ int dc_root(int i, int Kp, const float *Dn, const float *z2, float rho, float z2sum, float *tau_out,
-                       int *iters) {
+// sum over the G lanes of a root (every lane gets the same bits)
+__device__ __forceinline__ float dc_lanes(float v, int G, unsigned mask) {
+    for (int o = G >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+    return v;
+}
+
+// root i of 1/rho + sum_j z2_j / (Dn_j - lambda); returns the origin index, *tau = lambda - Dn[origin].
+// G lanes of a warp (mask) share it, this one with the terms j = gl modulo G; ONE: G is 1 (the
+// compiler unrolls the loops and reads the terms by fours).
+template <bool ONE>
+__device__ int dc_root(int i, int Kp, const float *Dn, const float *z2, float rho, float z2sum, int gl, int lanes,
+                       unsigned mask, float *tau_out, int *iters) {
+    const int G = ONE ? 1 : lanes;
+    if (ONE) gl = 0;
     const float rinv = 1.f / rho;
     int o;
-    float lo, hi;
+    float lo, hi, t;
+    // the interval and a first value: the root of the two poles about it (the last two, for the
+    // last root) with the other terms as they are in the middle (LAPACK laed4).  Starting in the
+    // middle took 4 evaluations a root and 24 for the slowest of a merge, the last root halving its
+    // way to a small z; so it takes 3, and 9.
     if (i < Kp - 1) {
         const float gap = Dn[i + 1] - Dn[i];
         const float mid = 0.5f * gap;
         const float base = Dn[i];
-        float g = rinv;
-        for (int j = 0; j < Kp; j++) g += z2[j] / ((Dn[j] - base) - mid);
-        if (g >= 0.f) { o = i; lo = 0.f; hi = mid; }
-        else { o = i + 1; lo = mid - gap; hi = 0.f; }
+        float g = 0.f;
+        for (int j = gl; j < Kp; j += G) g += z2[j] / ((Dn[j] - base) - mid);
+        g = rinv + dc_lanes(g, G, mask);
+        const float za = z2[i], zb = z2[i + 1], c = g - (zb - za) / mid;
+        if (g >= 0.f) {
+            o = i; lo = 0.f; hi = mid;
+            const float p = fmaf(c, gap, za + zb), q = za * gap, disc = sqrtf(fabsf(p * p - 4.f * q * c));
+            t = p > 0.f ? 2.f * q / (p + disc) : (p - disc) / (2.f * c);
+        } else {
+            o = i + 1; lo = mid - gap; hi = 0.f;
+            const float p = fmaf(c, gap, -za - zb), q = zb * gap, disc = sqrtf(fabsf(p * p + 4.f * q * c));
+            t = p < 0.f ? 2.f * q / (p - disc) : -(p + disc) / (2.f * c);
+        }
     } else {
         o = i; lo = 0.f; hi = rho * z2sum;
+        t = 0.f;
+        if (Kp > 1) {
+            const float base = Dn[i], mid = 0.5f * hi, gap = base - Dn[i - 1], za = z2[i - 1], zb = z2[i];
+            float c = 0.f;
+            for (int j = gl; j < Kp - 2; j += G) c += z2[j] / ((Dn[j] - base) - mid);
+            c = rinv + dc_lanes(c, G, mask);
+            const float p = fmaf(c, gap, -za - zb), q = zb * gap, disc = sqrtf(fabsf(p * p + 4.f * q * c));
+            t = p > 0.f ? 2.f * q / (p + disc) : (disc - p) / (2.f * c);
+        }
     }
+    if (!(t > lo && t < hi)) t = 0.5f * (lo + hi);
     const float dorg = Dn[o];
     const int ip = i < Kp - 1 ? i : Kp - 2;   // poles ip, ip+1 of the local model
-    float t = 0.5f * (lo + hi);
     int it = 0;
     for (; it < 64; it++) {
-        // the poles up to ip (psi) and beyond (phi) in two loops; one reciprocal per term,
-        // approximate (1 ulp), well inside the 8 eps sum(|terms|) convergence bound below
+        // the poles up to ip (psi) and beyond (phi); one reciprocal per term, approximate (1 ulp),
+        // well inside the 8 eps sum(|terms|) convergence bound below
         float psi = 0.f, phi = 0.f, dpsi = 0.f, dphi = 0.f;
-        for (int j = 0; j <= ip; j++) {
-            const float rl = __fdividef(1.f, (Dn[j] - dorg) - t);
-            const float q = z2[j] * rl;
-            psi += q;
-            dpsi = fmaf(q, rl, dpsi);
+        if (ONE) {
+            for (int j = 0; j <= ip; j++) {
+                const float rl = __fdividef(1.f, (Dn[j] - dorg) - t);
+                const float q = z2[j] * rl;
+                psi += q;
+                dpsi = fmaf(q, rl, dpsi);
+            }
+            for (int j = ip + 1; j < Kp; j++) {
+                const float rl = __fdividef(1.f, (Dn[j] - dorg) - t);
+                const float q = z2[j] * rl;
+                phi += q;
+                dphi = fmaf(q, rl, dphi);
+            }
+        } else {   // one loop: the lanes' boundaries differ
+            #pragma unroll 4
+            for (int j = gl; j < Kp; j += G) {
+                const float rl = __fdividef(1.f, (Dn[j] - dorg) - t);
+                const float q = z2[j] * rl;
+                if (j <= ip) { psi += q; dpsi = fmaf(q, rl, dpsi); }
+                else { phi += q; dphi = fmaf(q, rl, dphi); }
+            }
         }
-        for (int j = ip + 1; j < Kp; j++) {
-            const float rl = __fdividef(1.f, (Dn[j] - dorg) - t);
-            const float q = z2[j] * rl;
-            phi += q;
-            dphi = fmaf(q, rl, dphi);
-        }
+        psi = dc_lanes(psi, G, mask);
+        phi = dc_lanes(phi, G, mask);
+        dpsi = dc_lanes(dpsi, G, mask);
+        dphi = dc_lanes(dphi, G, mask);
         const float di = ip >= 0 ? (Dn[ip] - dorg) - t : 0.f;
         const float dj = ip + 1 < Kp ? (Dn[ip + 1] - dorg) - t : 0.f;
         const float g = rinv + psi + phi;
@@ -244,7 +297,38 @@ __device__ int dc_root(int i, int Kp, const float *Dn, const float *z2, float rh
     return o;
 }
 
-template <int NT>
+// positions of the i < K with pred(i), in order: emit(i, position, pred); returns their number
+template <int NT, class P, class E>
+__device__ __forceinline__ int dc_compact(int K, int *wsum, P pred, E emit) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int i0 = 0; i0 < K; i0 += NT) {
+        const int i = i0 + threadIdx.x;
+        const bool p = i < K && pred(i);
+        const unsigned m = __ballot_sync(0xffffffffu, p);
+        if (lane == 0) wsum[warp] = __popc(m);
+        __syncthreads();
+        int off = base;
+        for (int w = 0; w < NT / 32; w++) {
+            if (w < warp) off += wsum[w];
+            base += wsum[w];
+        }
+        if (i < K) emit(i, off + __popc(m & ((1u << lane) - 1)), p);
+        __syncthreads();
+    }
+    return base;
+}
+
+// One merge per block, or per cluster of C blocks (CL): every block forms the sorted lists and
+// deflates them for itself; the roots, the recomputed z, the norms, the ranks and the columns of U
+// are dealt to all threads of the cluster, G lanes to a root where there are more threads than
+// roots, and pushed to every block.  The roots' terms bound the large merges of many matrices
+// (and 200 blocks on 152 SMs leave a second wave of 48), the serial chain (the deflation's scan, a
+// root's terms on one lane) those of few.  The scan is parallel but for the pairs that deflate.
+// Measured with a lane a root from the middle of its interval, one block a merge and a serial scan,
+// and so (us): the top three levels of one matrix of order 1024 2075, 336; one merge of 128 73, 31;
+// 200 merges of 1024 1723, 1298; 1600 of 128 308, 219.
+template <int NT, bool CL, bool ONE>
 __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, const float *Qin, float *Uout) {
     extern __shared__ __align__(16) float sm[];
     const DcSmem L(KM);
@@ -253,10 +337,12 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
     int *perm = reinterpret_cast<int *>(sm + L.perm), *kind = reinterpret_cast<int *>(sm + L.kind);
     int *nidx = reinterpret_cast<int *>(sm + L.nidx), *defl = reinterpret_cast<int *>(sm + L.defl);
     int *org = reinterpret_cast<int *>(sm + L.org), *src = reinterpret_cast<int *>(sm + L.src);
+    int *wsum = reinterpret_cast<int *>(red + 48);
     float *rot = sm + L.rot;
-    __shared__ int s_kp, s_m, s_nd;
+    __shared__ int s_m;
+    const int C = CL ? (int)cl_size() : 1, rank = CL ? (int)cl_rank() : 0;
     // optional per-phase timers of the merges (EighArgs.phase_ns slots 7-11, summed over merges)
-    unsigned long long *pt = a.phase_ns ? a.phase_ns + (size_t)blockIdx.y * CIR_EIG_PROF_SLOTS : nullptr;
+    unsigned long long *pt = a.phase_ns && rank == 0 ? a.phase_ns + (size_t)blockIdx.y * CIR_EIG_PROF_SLOTS : nullptr;
     unsigned long long tl = 0;
     auto mark = [&](int slot) {
         if (!pt) return;
@@ -270,8 +356,18 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
     };
     mark(-1);
     const int n = a.n, ld = a.ld, tid = threadIdx.x;
-    const int mat = blockIdx.y, b = blockIdx.x;
-    if (b >= (1 << level)) return;
+    const int mat = blockIdx.y, b = blockIdx.x / C;
+    const int NTT = NT * C, gid = rank * NT + tid;       // all threads of the merge
+    auto all_sync = [&] {
+        if (CL) cl_sync();
+        else __syncthreads();
+    };
+    // a word of this block's shared memory, in every block of the cluster
+    auto put = [&](float *p, float v) {
+        if (!CL) { *p = v; return; }
+        for (int c = 0; c < C; c++) cl_store(cl_map(p, c), v);
+    };
+    auto puti = [&](int *p, int v) { put(reinterpret_cast<float *>(p), __int_as_float(v)); };
     const int a0 = dc_off(level, b, n), a1 = dc_off(level, b + 1, n), mid = dc_off(level + 1, 2 * b + 1, n);
     const int K = a1 - a0, k1 = mid - a0;
     float *dw = a.DE + (size_t)mat * 3 * ld;
@@ -313,44 +409,56 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
     __syncthreads();
     for (int r = tid; r < K; r += NT) zs[r] = z2[r];
     __syncthreads();
-    // deflation (LAPACK laed2): sequential scan over the sorted entries
+    // Deflation (LAPACK laed2).  Small components leave first; the rest (lst, M of them) are scanned
+    // for close pairs |t c s| <= tol, c = z_j / tt, s = -z_pj / tt, tt^2 = z_j^2 + z_pj^2 (multiplied
+    // through by tt^2: no division unless the pair deflates).  A pair's test depends on the one
+    // before it only where that one deflated, so all pairs are tested as they stand, and one thread
+    // follows the chains that start at those that pass.
+    int *lst = org, *hot = src;          // (both free until the roots are known)
+    const int M = dc_compact<NT>(K, wsum, [&](int j) { return !(rho * fabsf(zs[j]) <= tol); }, [&](int j, int pos, bool p) {
+        kind[j] = p ? 0 : -1;
+        if (p) lst[pos] = j;
+    });
+    auto close = [&](int i) {
+        const int j = lst[i], p = lst[i - 1];
+        const float zj = zs[j], zp = zs[p], t = Ds[j] - Ds[p];
+        return fabsf(t * zj * zp) <= tol * fmaf(zj, zj, zp * zp);
+    };
+    const int nhot = dc_compact<NT>(M, wsum, [&](int i) { return i > 0 && close(i); }, [&](int i, int pos, bool p) {
+        if (p) hot[pos] = i;
+    });
     if (tid == 0) {
-        int kp = 0, nd = 0, m = 0, pj = -1;
-        for (int j = 0; j < K; j++) {
-            if (rho * fabsf(zs[j]) <= tol) { kind[j] = -1; defl[nd++] = j; continue; }
-            if (pj < 0) { pj = j; continue; }
-            // close pair test |t c s| <= tol with c = z_j / tt, s = -z_pj / tt, tt^2 = z_j^2 + z_pj^2,
-            // multiplied through by tt^2 (no division unless the pair deflates)
-            const float zj = zs[j], zp = zs[pj], t = Ds[j] - Ds[pj];
-            if (fabsf(t * zj * zp) <= tol * fmaf(zj, zj, zp * zp)) {
-                const float tt = hypotf(zj, zp);
-                const float c = zj / tt, s = -zp / tt;
+        int m = 0, next = 1;             // pairs before next are done
+        for (int q = 0; q < nhot; q++) {
+            if (hot[q] < next) continue;
+            int i = hot[q];
+            for (; i < M && close(i); i++) {
+                const int j = lst[i], p = lst[i - 1];
+                const float tt = hypotf(zs[j], zs[p]);
+                const float c = zs[j] / tt, s = -zs[p] / tt;
                 zs[j] = tt;
-                zs[pj] = 0.f;
-                reinterpret_cast<int *>(rot)[4 * m] = pj;
+                zs[p] = 0.f;
+                reinterpret_cast<int *>(rot)[4 * m] = p;
                 reinterpret_cast<int *>(rot)[4 * m + 1] = j;
                 rot[4 * m + 2] = c;
                 rot[4 * m + 3] = s;
                 m++;
-                const float t2 = Ds[pj] * c * c + Ds[j] * s * s;
-                Ds[j] = Ds[pj] * s * s + Ds[j] * c * c;
-                Ds[pj] = t2;
-                kind[pj] = -1;
-                defl[nd++] = pj;
-                pj = j;
-            } else {
-                kind[pj] = kp;
-                nidx[kp++] = pj;
-                pj = j;
+                const float t2 = Ds[p] * c * c + Ds[j] * s * s;
+                Ds[j] = Ds[p] * s * s + Ds[j] * c * c;
+                Ds[p] = t2;
+                kind[p] = -1;
             }
+            next = i + 1;
         }
-        if (pj >= 0) { kind[pj] = kp; nidx[kp++] = pj; }
-        s_kp = kp;
         s_m = m;
-        s_nd = nd;
     }
     __syncthreads();
-    const int Kp = s_kp, nrot = s_m, nd = s_nd;
+    const int nrot = s_m;
+    const int Kp = dc_compact<NT>(K, wsum, [&](int j) { return kind[j] == 0; }, [&](int j, int pos, bool p) {
+        if (p) nidx[pos] = j;
+        else defl[j - pos] = j;
+        kind[j] = p ? pos : -1;
+    });
     float zpart = 0.f;
     for (int i = tid; i < Kp; i += NT) {
         const int r = nidx[i];
@@ -363,53 +471,74 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
     const float z2sum = dc_block_sum<NT>(zpart, red);
     __syncthreads();
     mark(7);
-    // secular roots
-    int nit = 0;
-    for (int i = tid; i < Kp; i += NT) {
+    // secular roots, G lanes each
+    int lanes = 1;
+    while (!ONE && lanes < 32 && 2 * lanes * Kp <= NTT) lanes *= 2;
+    const int G = ONE ? 1 : lanes, gl = ONE ? 0 : gid & (G - 1);
+    const int gi = gid / G, ng = NTT / G;
+    const unsigned gmask = (G == 32 ? 0xffffffffu : (1u << G) - 1) << (tid & 31 & ~(G - 1));
+    if (CL) cl_sync();                   // every block has its lists: their words may be written
+    int nit = 0, nroot = 0;
+    for (int i = gi; i < Kp; i += ng) {
         float t;
         int itc;
-        org[i] = dc_root(i, Kp, Dn, z2, rho, z2sum, &t, &itc);
-        tau[i] = t;
+        const int o = dc_root<ONE>(i, Kp, Dn, z2, rho, z2sum, gl, G, gmask, &t, &itc);
+        if (gl == 0) {
+            puti(org + i, o);
+            put(tau + i, t);
+        }
         nit += itc;
+        nroot++;
     }
-    if (pt && nit) {
-        atomicAdd(pt + 18, (unsigned long long)nit);
-        atomicAdd(pt + 19, (unsigned long long)((Kp - tid + NT - 1) / NT > 0 ? (Kp - tid + NT - 1) / NT : 0));
+    if (a.phase_ns && gl == 0 && nit) {
+        unsigned long long *ps = a.phase_ns + (size_t)blockIdx.y * CIR_EIG_PROF_SLOTS;
+        atomicAdd(ps + 18, (unsigned long long)nit);
+        atomicAdd(ps + 19, (unsigned long long)nroot);
     }
-    __syncthreads();
+    all_sync();
     mark(8);
     // Gu-Eisenstat: zh_j^2 = -prod_i (Dn_j - lambda_i) / prod_{i != j} (Dn_j - Dn_i)
-    for (int j = tid; j < Kp; j += NT) {
+    for (int j = gi; j < Kp; j += ng) {
         const float dj = Dn[j];
-        float p = (dj - Dn[org[j]]) - tau[j];
-        for (int i = 0; i < Kp; i++)
+        float p = gl == 0 ? (dj - Dn[org[j]]) - tau[j] : 1.f;
+        for (int i = gl; i < Kp; i += G)
             if (i != j) p *= ((dj - Dn[org[i]]) - tau[i]) / (dj - Dn[i]);
-        vals[j] = copysignf(sqrtf(fmaxf(-p, 0.f)), zh[j]);
+        for (int o = G >> 1; o > 0; o >>= 1) p *= __shfl_xor_sync(gmask, p, o);
+        if (gl == 0) put(zh + j, copysignf(sqrtf(fmaxf(-p, 0.f)), zh[j]));
     }
-    __syncthreads();
-    for (int j = tid; j < Kp; j += NT) zh[j] = vals[j];
-    __syncthreads();
-    for (int i = tid; i < Kp; i += NT) {
+    all_sync();
+    for (int i = gi; i < Kp; i += ng) {
         const float base = Dn[org[i]], ti = tau[i];
         float sq = 0.f;
-        for (int j = 0; j < Kp; j++) {
+        for (int j = gl; j < Kp; j += G) {
             const float u = __fdividef(zh[j], (Dn[j] - base) - ti);
             sq = fmaf(u, u, sq);
         }
-        inv[i] = 1.f / sqrtf(sq);
+        sq = dc_lanes(sq, G, gmask);
+        if (gl == 0) put(inv + i, 1.f / sqrtf(sq));
     }
-    mark(9);
     // eigenvalues: roots then deflated values; ascending rank (ties by index)
     for (int q = tid; q < K; q += NT) vals[q] = q < Kp ? Dn[org[q]] + tau[q] : Ds[defl[q - Kp]];
+    int *touched = reinterpret_cast<int *>(D);   // D is free once the two lists are merged
+    const int *rotp = reinterpret_cast<const int *>(rot);
+    for (int r = tid; r < K; r += NT) touched[r] = 0;
     __syncthreads();
-    for (int q = tid; q < K; q += NT) {
+    for (int t = tid; t < nrot; t += NT) {
+        touched[rotp[4 * t]] = 1;
+        touched[rotp[4 * t + 1]] = 1;
+    }
+    mark(9);
+    for (int q = gi; q < K; q += ng) {
         const float v = vals[q];
         int r = 0;
-        for (int i = 0; i < K; i++) r += cir_before(vals[i], i, v, q);
-        src[r] = q;
-        dw[a0 + r] = v;
+        for (int i = gl; i < K; i += G) r += cir_before(vals[i], i, v, q);
+        for (int o = G >> 1; o > 0; o >>= 1) r += __shfl_xor_sync(gmask, r, o);
+        if (gl == 0) {
+            puti(src + r, q);
+            dw[a0 + r] = v;
+        }
     }
-    __syncthreads();
+    all_sync();
     mark(10);
     // U = P G W without an intermediate: G = G_0 G_1 ... G_{nrot-1} are the deflation
     // rotations (G_t mixes the sorted rows p_t, j_t: p' = c p - s j, j' = s p + c j), W the
@@ -420,16 +549,11 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
     // previous step's p row (or from W at the end of a chain); row j_t is then final, and
     // row p_t is carried to rotation t-1 or, at the start of a chain, written.  The values
     // and the order of the operations are those of applying every rotation to a full copy.
-    int *touched = reinterpret_cast<int *>(D);   // D is free once the two lists are merged
-    const int *rotp = reinterpret_cast<const int *>(rot);
-    for (int r = tid; r < K; r += NT) touched[r] = 0;
-    __syncthreads();
-    for (int t = tid; t < nrot; t += NT) {
-        touched[rotp[4 * t]] = 1;
-        touched[rotp[4 * t + 1]] = 1;
-    }
-    __syncthreads();
-    for (int c = tid; c < K; c += NT) {
+    // A warp takes 32 columns and every nr-th row of them.
+    const int nc = (K + 31) / 32, nw = NTT / 32, nr = ONE ? 1 : max(1, nw / nc);
+    for (int u = gid >> 5; u < nc * nr; u += nw) {
+        const int c = 32 * (u % nc) + (tid & 31), rg = u / nc;
+        if (c >= K) continue;
         const int q = src[c];
         const bool root = q < Kp;
         const float base = root ? Dn[org[q]] : 0.f, ti = root ? tau[q] : 0.f, sc = root ? inv[q] : 0.f;
@@ -440,8 +564,9 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
             return jn >= 0 ? zh[jn] / ((Dn[jn] - base) - ti) * sc : 0.f;
         };
         float *Uc = U + (size_t)a0 * ld + a0 + c;
-        for (int r = 0; r < K; r++)
+        for (int r = rg; r < K; r += nr)
             if (!touched[r]) Uc[(size_t)perm[r] * ld] = w(r);
+        if (rg) continue;
         float carry = 0.f;
         for (int t = nrot - 1; t >= 0; t--) {
             const int p = rotp[4 * t], j = rotp[4 * t + 1];
@@ -453,7 +578,6 @@ __global__ void __launch_bounds__(NT) k_dc_merge(EighArgs a, int level, int KM, 
         }
     }
     mark(11);
-    (void)nd;
 }
 
 // Q_new = diag(Q1, Q2) U for every merge of a level: blockIdx.y = matrix, blockIdx.x =
@@ -585,6 +709,15 @@ bool pair_q_enabled() {
     return on;
 }
 
+// Threads nt and blocks C of a merge of up to KM rows: the block that suits many merges (a thread
+// a root, small blocks so that many share an SM), widened while the merges leave threads of the
+// SMs idle, up to DC_LANES lanes a root and a block of the cluster per 128 rows.
+constexpr int DC_LANES = 16;
+void dc_shape(long long merges, int KM, int sms, int &nt, int &C) {
+    while (nt < 512 && nt < DC_LANES * KM && merges * 2 * nt <= 2048LL * sms) nt *= 2;
+    while (nt == 512 && C < 8 && 256 * C <= KM && merges * 2 * nt * C <= 2048LL * sms) C *= 2;
+}
+
 int dc_depth(int n) {
     int D = 0;
     while (((n + (1 << D) - 1) >> D) > DC_LEAF) D++;
@@ -603,9 +736,13 @@ cudaError_t cir_launch_dc(const EighArgs &a, int nmat, cudaStream_t s, int *laun
     const int D = dc_depth(n);
     float *buf[3] = {a.DC, a.DC + (size_t)nmat * a.mstride, a.DC + 2 * (size_t)nmat * a.mstride};
     const int nleaf = 1 << D;
+    int dev = 0, sms = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
     k_dc_leaf<<<dim3((nleaf + 3) / 4, nmat), 128, 0, s>>>(a, D, buf[0]);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int nl = 1;
     int cur = 0;
     // the split-BF16 back-transform takes Q_T as a BF16 pair: the top merge's tensor-core
@@ -617,23 +754,45 @@ cudaError_t cir_launch_dc(const EighArgs &a, int nmat, cudaStream_t s, int *laun
         const DcSmem L(KM);
         const size_t smem = sizeof(float) * L.total;
         const int other = cur ^ 1;
-        // small merges in small blocks, so that many of them share an SM
-        auto merge = [&](auto kern, int nt) -> cudaError_t {
+        const int base = KM <= 64 ? 64 : KM <= 128 ? 128 : KM <= 512 ? 256 : 512;
+        int nt = base, C = 1;
+        dc_shape((1 << level) * (long long)nmat, KM, sms, nt, C);
+        auto merge = [&](auto kern) -> cudaError_t {
             cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (r != cudaSuccess) return r;
-            kern<<<dim3(1 << level, nmat), nt, smem, s>>>(a, level, KM, buf[cur], buf[2]);
-            return cudaSuccess;
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at[1];
+            cfg.gridDim = dim3((unsigned)C << level, nmat);
+            cfg.blockDim = dim3(nt);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            if (C > 1) {
+                at[0].id = cudaLaunchAttributeClusterDimension;
+                at[0].val.clusterDim.x = C;
+                at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+                cfg.attrs = at;
+                cfg.numAttrs = 1;
+            }
+            return cudaLaunchKernelEx(&cfg, kern, a, level, KM, (const float *)buf[cur], buf[2]);
         };
-        e = KM <= 64 ? merge(k_dc_merge<64>, 64) : KM <= 128 ? merge(k_dc_merge<128>, 128)
-          : KM <= 512 ? merge(k_dc_merge<DC_NT>, DC_NT) : merge(k_dc_merge<2 * DC_NT>, 2 * DC_NT);
+        const bool one = nt * C < 2 * KM;      // a lane a root
+        e = C > 1 ? (one ? merge(k_dc_merge<512, true, true>) : merge(k_dc_merge<512, true, false>))
+          : nt == 64 ? merge(k_dc_merge<64, false, true>)
+          : nt == 128 ? (one ? merge(k_dc_merge<128, false, true>) : merge(k_dc_merge<128, false, false>))
+          : nt == 256 ? (one ? merge(k_dc_merge<256, false, true>) : merge(k_dc_merge<256, false, false>))
+                      : (one ? merge(k_dc_merge<512, false, true>) : merge(k_dc_merge<512, false, false>));
         if (e != cudaSuccess) return e;
-        // the top three levels on the tensor cores (plain form: FP32 through three BF16 terms,
-        // from merges of 256 rows; 200 matrices of order 1024: 10.4 -> 2.6 ms): one batched
-        // product per merge half when every offset keeps 16-byte alignment
-        bool tc = level <= 2 && (a.precision != CIR_PREC_FP32 || KM >= 256);
+        // One batched product per merge half on the tensor cores: the mixed forms' top three levels
+        // where every offset keeps 16-byte alignment, and in FP32 (three BF16 terms) every merge of
+        // 256 rows or more besides that gives a launch 32 tiles (200 matrices of order 1024, top three
+        // levels: 10.4 -> 2.6 ms; 320 each of 256, 432, 686, whose halves are odd, and 1024 in the
+        // mixed form 7.0 -> 3.8; below, k_dc_gemm's one launch a level is faster: four merges of 512
+        // rows 35 us, eight products of 8 tiles 84).
+        bool tc = level <= 2 && a.precision != CIR_PREC_FP32;
         for (int b = 0; tc && b < (1 << level); b++)
             tc = (dc_off(level, b, n) & 3) == 0 && (dc_off(level + 1, 2 * b + 1, n) & 3) == 0;
-        if (tc) {
+        const long long tiles = (long long)((KM + 127) / 128) * ((KM + 255) / 256) * nmat;
+        if (tc || (KM >= 256 && tiles >= 32)) {
             for (int b = 0; b < (1 << level); b++) {
                 const int a0 = dc_off(level, b, n), a1 = dc_off(level, b + 1, n), mid = dc_off(level + 1, 2 * b + 1, n);
                 for (int half = 0; half < 2; half++) {
@@ -652,19 +811,18 @@ cudaError_t cir_launch_dc(const EighArgs &a, int nmat, cudaStream_t s, int *laun
                     g.a_colmajor = true;
                     g.epilogue = 0;
                     g.err = a.err;
-                    if (level == 0 && q_pair) {
+                    if (tc && level == 0 && q_pair) {
                         __nv_bfloat16 *pb = reinterpret_cast<__nv_bfloat16 *>(buf[other]) + (size_t)a0 * ld + h0;
                         g.Chi = pb;
                         g.Clo = pb + a.mstride;
                     }
-                    e = a.precision == CIR_PREC_FP32 ? cir_launch_gemm(g, nmat, s, nullptr)
-                                                     : cir_launch_tc_gemm(g, nmat, a.precision, s, nullptr);
+                    e = tc ? cir_launch_tc_gemm(g, nmat, a.precision, s, nullptr) : cir_launch_gemm(g, nmat, s, nullptr);
                     if (e != cudaSuccess) return e;
                     nl++;
                 }
             }
             nl++;
-            if (level == 0 && q_pair) q_split = true;
+            if (tc && level == 0 && q_pair) q_split = true;
         } else {
             const int tiles = ((KM / 2 + 1 + 63) / 64) * ((KM + 63) / 64);
             k_dc_gemm<<<dim3(tiles * (1 << level) * 2, nmat), 256, 0, s>>>(a, level, tiles, buf[cur], buf[2], buf[other]);

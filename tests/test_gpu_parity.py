@@ -529,3 +529,26 @@ def test_unit_eigenvectors(lib, n, batch):
     with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 12) as eng:
         _, V = eng.eigh(A + A.swapaxes(1, 2))
     assert np.abs((np.asarray(V, np.float64) ** 2).sum(1) - 1).max() < 2.0 ** -22
+
+
+# the merges of the divide and conquer: one lane a root in blocks of 64 to 512 threads, several
+# lanes, clusters of 2 to 8 blocks with one lane and with several; spectra that deflate by small
+# components and by close pairs, alone and in chains
+@pytest.mark.parametrize("kind", ["pairs", "clusters", "glued", "graded"])
+@pytest.mark.parametrize("n,nmat", [(66, 1), (130, 1), (130, 700), (300, 1), (516, 1), (520, 160), (1024, 1), (1100, 1)])
+def test_merge_forms(lib, kind, n, nmat):
+    rng = np.random.default_rng(n)
+    if kind == "glued":           # equal Wilkinson blocks, weakly coupled
+        d, e = np.abs(np.arange(n) % 21 - 10.0), np.where(np.arange(n - 1) % 21 == 20, 1e-4, 1.0)
+        A = np.diag(d) + np.diag(e, 1) + np.diag(e, -1)
+    else:
+        w = {"pairs": np.repeat(rng.standard_normal((n + 1) // 2), 2)[:n], "clusters": np.round(2 * rng.standard_normal(n)),
+             "graded": 10.0 ** rng.uniform(-5, 2, n)}[kind]
+        Q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+        A = (Q * w) @ Q.T
+    A = np.broadcast_to(((A + A.T) / 2).astype(np.float32), (nmat, n, n))
+    with lib.Engine(lib.default_params(species="H2O"), 8) as eng:
+        w, V = eng.eigh(np.ascontiguousarray(A))
+    _check_eig(A[0], w[0], V[0])
+    for i in range(1, nmat):
+        assert np.array_equal(w[i], w[0]) and np.array_equal(V[i], V[0])
