@@ -6,9 +6,11 @@
 //     IR = sum_a mu_a(t).F.mu_a(0)
 //     VV = (3 iiFii + iiFjj + 4 ijFij) / 15,   VH = (2 iiFii - iiFjj + 6 ijFij) / 30.
 // A warp takes R rows of F at a time, a column per lane.  The terms are linear in psi, so a
-// lane contracts its own partial psi with m(t) and the sums over columns and rows meet in double
-// at the end (reducing the 18 partial psi of every row over the warp, and the fractions in
-// double by one lane, was 44 us of latency for n = 128 and 120 us for 10 origins at n = 1024).
+// lane contracts its own partial psi with m(t) and the sums over columns and rows meet as pairs of
+// floats, in double per block.  Few rows are bound by the chain of loads and sums, many by the loads
+// in flight (four rows a warp, two columns of each: more spill).  One matrix of order 128: 44 us
+// with the 18 partial psi of every row reduced over the warp, 13.6 with one partial psi a lane and
+// its sums in double, 5.4 so; ten of order 1024 120, 82 and 37.
 // Nothing leaves the device.
 //
 // k_spec_mu2 / k_spec_sum: M = V^T mu (calcIR.cu:462-467) and the Lorentzian sum
@@ -20,56 +22,87 @@ namespace {
 
 constexpr int TCF_WARPS = 8;
 
-// the four sums (re, im) of one row's (partial) psi with m(t): IR, iiFii, ijFij, iiFjj
-__device__ __forceinline__ void tcf_sums(const float (&pr)[9], const float (&pi)[9], const float (&c)[9], double (&acc)[8]) {
-    acc[0] += c[0] * pr[0] + c[1] * pr[1] + c[2] * pr[2];
-    acc[1] += c[0] * pi[0] + c[1] * pi[1] + c[2] * pi[2];
-    acc[2] += c[3] * pr[3] + c[4] * pr[4] + c[5] * pr[5];
-    acc[3] += c[3] * pi[3] + c[4] * pi[4] + c[5] * pi[5];
-    acc[4] += c[6] * pr[6] + c[7] * pr[7] + c[8] * pr[8];
-    acc[5] += c[6] * pi[6] + c[7] * pi[7] + c[8] * pi[8];
-    // xx->yy, xx->zz, yy->xx, yy->zz, zz->xx, zz->yy (psi index 3, 4, 5 = xx, yy, zz)
-    acc[6] += (c[4] + c[5]) * pr[3] + (c[3] + c[5]) * pr[4] + (c[3] + c[4]) * pr[5];
-    acc[7] += (c[4] + c[5]) * pi[3] + (c[3] + c[5]) * pi[4] + (c[3] + c[4]) * pi[5];
+// A sum held as an unevaluated pair of floats (Knuth's two-sum): 48 bits, on the FP32 pipe.  In
+// double the eight sums of a warp (40 adds, 16 clocks each for the warp) were most of the kernel.
+struct Pair {
+    float hi, lo;
+};
+__device__ __forceinline__ Pair pair_add(Pair a, float x) {
+    const float s = __fadd_rn(a.hi, x), v = __fsub_rn(s, a.hi);
+    return {s, __fadd_rn(a.lo, __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, v)), __fsub_rn(x, v)))};
+}
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+    Pair r = pair_add(a, b.hi);
+    r.lo = __fadd_rn(r.lo, b.lo);
+    const float s = __fadd_rn(r.hi, r.lo);
+    return {s, __fsub_rn(r.lo, __fsub_rn(s, r.hi))};
+}
+__device__ __forceinline__ Pair pair_xor(Pair a, int o) {
+    return {__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
 }
 
-// the block's sums into out: IR, VV, VH (re, im)
-__device__ __forceinline__ void tcf_finish(double (&acc)[8], double *out) {
+// the four sums (re, im) of one row's (partial) psi with m(t): IR, iiFii, ijFij, iiFjj
+__device__ __forceinline__ void tcf_sums(const float (&pr)[9], const float (&pi)[9], const float (&c)[9], Pair (&acc)[8]) {
+    acc[0] = pair_add(acc[0], c[0] * pr[0] + c[1] * pr[1] + c[2] * pr[2]);
+    acc[1] = pair_add(acc[1], c[0] * pi[0] + c[1] * pi[1] + c[2] * pi[2]);
+    acc[2] = pair_add(acc[2], c[3] * pr[3] + c[4] * pr[4] + c[5] * pr[5]);
+    acc[3] = pair_add(acc[3], c[3] * pi[3] + c[4] * pi[4] + c[5] * pi[5]);
+    acc[4] = pair_add(acc[4], c[6] * pr[6] + c[7] * pr[7] + c[8] * pr[8]);
+    acc[5] = pair_add(acc[5], c[6] * pi[6] + c[7] * pi[7] + c[8] * pi[8]);
+    // xx->yy, xx->zz, yy->xx, yy->zz, zz->xx, zz->yy (psi index 3, 4, 5 = xx, yy, zz)
+    acc[6] = pair_add(acc[6], (c[4] + c[5]) * pr[3] + (c[3] + c[5]) * pr[4] + (c[3] + c[4]) * pr[5]);
+    acc[7] = pair_add(acc[7], (c[4] + c[5]) * pi[3] + (c[3] + c[5]) * pi[4] + (c[3] + c[4]) * pi[5]);
+}
+
+// the block's sums into out: IR, VV, VH (re, im).  A warp's eight sums meet by halves: the lanes
+// whose bit is set keep the upper half of what is left, so nine exchanges do for all eight.
+__device__ __forceinline__ void tcf_finish(Pair (&acc)[8], double *out) {
     __shared__ double part[TCF_WARPS][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     #pragma unroll
-    for (int q = 0; q < 8; q++) acc[q] = warp_sum_d(acc[q]);
-    if (lane == 0)
+    for (int w = 4; w > 0; w >>= 1) {
+        const bool up = lane & (4 * w);
         #pragma unroll
-        for (int q = 0; q < 8; q++) part[warp][q] = acc[q];
+        for (int q = 0; q < w; q++) {
+            const Pair send = up ? acc[q] : acc[q + w], keep = up ? acc[q + w] : acc[q];
+            acc[q] = pair_add(keep, pair_xor(send, 4 * w));
+        }
+    }
+    acc[0] = pair_add(acc[0], pair_xor(acc[0], 2));
+    acc[0] = pair_add(acc[0], pair_xor(acc[0], 1));
+    if ((lane & 3) == 0) part[warp][lane >> 2] = (double)acc[0].hi + (double)acc[0].lo;
     __syncthreads();
-    if (threadIdx.x < 6) {
-        const int im = threadIdx.x & 1;
-        double s[4] = {0, 0, 0, 0};
-        for (int w = 0; w < TCF_WARPS; w++)
+    if (warp == 0) {
+        double s = 0.0;
+        if (lane < 8)
             #pragma unroll
-            for (int q = 0; q < 4; q++) s[q] += part[w][2 * q + im];
-        const double v = threadIdx.x < 2 ? s[0]
-                       : threadIdx.x < 4 ? (3.0 * s[1] + s[3] + 4.0 * s[2]) / 15.0
-                                         : (2.0 * s[1] - s[3] + 6.0 * s[2]) / 30.0;
-        atomicAdd(out + threadIdx.x, v);
+            for (int w = 0; w < TCF_WARPS; w++) s += part[w][lane];
+        const int im = lane & 1;
+        const double ii = __shfl_sync(0xffffffffu, s, 2 + im), ij = __shfl_sync(0xffffffffu, s, 4 + im),
+                     jj = __shfl_sync(0xffffffffu, s, 6 + im);
+        if (lane < 6)
+            atomicAdd(out + lane, lane < 2 ? s : lane < 4 ? (3.0 * ii + jj + 4.0 * ij) / 15.0 : (2.0 * ii - jj + 6.0 * ij) / 30.0);
     }
 }
 
-// rows: the block's rows (a multiple of TCF_WARPS * R)
+// rows: the block's rows (a multiple of TCF_WARPS * R).  One row a warp reads m(0) as it needs it
+// (the loads of all its columns are in flight at once), four share it in shared memory.
 template <int R>
-__global__ void __launch_bounds__(TCF_WARPS * 32) k_tcf(TcfArgs t, int rows) {
+__global__ void __launch_bounds__(TCF_WARPS * 32, 2) k_tcf(TcfArgs t, int rows) {
     extern __shared__ float m0s[];   // [9][n]
     const int b = blockIdx.y;
     const float *F = t.F + (size_t)b * t.sF;
     const float *m0 = t.m0 + (size_t)b * t.sm0;
     const float *mt = t.mt + (size_t)b * t.smt;
     const int n = t.n;
-    for (int a = 0; a < 9; a++)
-        for (int i = threadIdx.x; i < n; i += TCF_WARPS * 32) m0s[a * n + i] = m0[(size_t)a * t.ldv + i];
-    __syncthreads();
+    if (R > 1) {
+        for (int i = threadIdx.x; i < n; i += TCF_WARPS * 32)
+            #pragma unroll
+            for (int a = 0; a < 9; a++) m0s[a * n + i] = m0[(size_t)a * t.ldv + i];
+        __syncthreads();
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    Pair acc[8] = {};
     const int rend = min(n, ((int)blockIdx.x + 1) * rows);
     for (int r0 = blockIdx.x * rows + warp * R; r0 < rend; r0 += TCF_WARPS * R) {
         float pr[R][9], pi[R][9];
@@ -80,13 +113,14 @@ __global__ void __launch_bounds__(TCF_WARPS * 32) k_tcf(TcfArgs t, int rows) {
             #pragma unroll
             for (int a = 0; a < 9; a++) pr[i][a] = pi[i][a] = 0.f;
         }
+        #pragma unroll R > 1 ? 2 : 4
         for (int q = lane; q < n; q += 32) {
             float2 f[R];
             #pragma unroll
             for (int i = 0; i < R; i++) f[i] = row[i][q];
             #pragma unroll
             for (int a = 0; a < 9; a++) {
-                const float m = m0s[a * n + q];
+                const float m = R > 1 ? m0s[a * n + q] : __ldg(m0 + (size_t)a * t.ldv + q);
                 #pragma unroll
                 for (int i = 0; i < R; i++) {
                     pr[i][a] = fmaf(f[i].x, m, pr[i][a]);
@@ -127,7 +161,7 @@ __global__ void __launch_bounds__(256) k_tcf_t(TcfArgs t) {
     __syncthreads();
     const int rr = threadIdx.x & 63, ql = threadIdx.x >> 6;
     const int r = blockIdx.x * TT_ROWS + rr;
-    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    Pair acc[8] = {};
     if (r < n) {
         const __nv_bfloat16 *fh = t.Ft.hi + (size_t)b * t.sFt + r, *fl = t.Ft.lo + (size_t)b * t.sFt + r;
         float pr[9], pi[9], c[9];
@@ -210,11 +244,11 @@ cudaError_t cir_launch_tcf(const TcfArgs &t, int batch, cudaStream_t s, int *lau
         if (launches) *launches += 1;
         return cudaGetLastError();
     }
-    const size_t smem = sizeof(float) * 9 * (size_t)t.n;
     // four rows a warp at a time share the reads of m(0) where that leaves two blocks per SM,
     // and a block takes up to 64 rows so that staging m(0) stays small beside them
     const long long all = (long long)t.n * batch;
     const int R = all >= 304LL * TCF_WARPS * 4 ? 4 : 1, rows = TCF_WARPS * (R == 4 && all >= 304LL * 64 ? 8 : R);
+    const size_t smem = R == 4 ? sizeof(float) * 9 * (size_t)t.n : 0;
     auto kern = R == 4 ? k_tcf<4> : k_tcf<1>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
