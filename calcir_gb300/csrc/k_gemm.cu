@@ -396,16 +396,18 @@ int gemm_sms() {
     return cache[dev] > 0 ? cache[dev] : 148;
 }
 
-// ---- small products: FP32 SIMT, 32 x 32 tiles, 64 threads of 4 x 4 outputs, K 32 at a time in
-// two buffers.  Where the 128 x 128 tiles leave most SMs idle, the tile above pays its start-up
-// and 0.8 us for every 32 of K; this one about 0.5 us on many more SMs (gemm_small_wins).
+// ---- small products: FP32 SIMT, 32 x 32 tiles, 64 threads of 4 x 4 outputs, K 32 at a time.
+// Where the 128 x 128 tiles leave most SMs idle, the tile above pays its start-up and 0.8 us for
+// every 32 of K; this one less, on many more SMs (gemm_small_wins).  Few blocks are bound by the
+// chain of loads and sums along K: KS groups of 64 threads then take every KS-th slice and meet in
+// shared memory.
 constexpr int SB = 32, SLD = SB + 4;
 
 template <bool KC>
-__device__ __forceinline__ void small_load(const float *p, int ld, int rdim, int kdim, int r0, int k0, bool vec, float4 (&v)[4]) {
+__device__ __forceinline__ void small_load(const float *p, int ld, int rdim, int kdim, int r0, int k0, int t, bool vec, float4 (&v)[4]) {
     #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int idx = threadIdx.x + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
+        const int idx = t + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
         const int r = r0 + (KC ? o : c4), k = k0 + (KC ? c4 : o);
         const float *q = KC ? p + (size_t)r * ld + k : p + (size_t)k * ld + r;
         const int have = KC ? (r < rdim ? kdim - k : 0) : (k < kdim ? rdim - r : 0);
@@ -415,49 +417,74 @@ __device__ __forceinline__ void small_load(const float *p, int ld, int rdim, int
     }
 }
 template <bool KC>
-__device__ __forceinline__ void small_store(float (*s)[SLD], const float4 (&v)[4]) {
+__device__ __forceinline__ void small_store(float *s, int t, const float4 (&v)[4]) {
     #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int idx = threadIdx.x + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
-        if (KC) { s[c4][o] = v[i].x; s[c4 + 1][o] = v[i].y; s[c4 + 2][o] = v[i].z; s[c4 + 3][o] = v[i].w; }
-        else *reinterpret_cast<float4 *>(&s[o][c4]) = v[i];
+        const int idx = t + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
+        if (KC) {
+            s[c4 * SLD + o] = v[i].x; s[(c4 + 1) * SLD + o] = v[i].y;
+            s[(c4 + 2) * SLD + o] = v[i].z; s[(c4 + 3) * SLD + o] = v[i].w;
+        } else *reinterpret_cast<float4 *>(s + o * SLD + c4) = v[i];
     }
 }
 
-template <bool ACOL, bool BKC>
-__global__ void __launch_bounds__(64) k_gemm_small(GemmArgs g, bool vecA, bool vecB) {
-    __shared__ __align__(16) float As[2][SB][SLD], Bs[2][SB][SLD];
+template <bool ACOL, bool BKC, int KS>
+__global__ void __launch_bounds__(64 * KS) k_gemm_small(GemmArgs g, bool vecA, bool vecB) {
+    __shared__ __align__(16) float sm[KS == 1 ? 2 : KS][2][SB * SLD];   // one group: two buffers
     const int bz = blockIdx.z, m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
     const float *A = g.A + (size_t)bz * g.sA, *B = g.B + (size_t)bz * g.sB;
-    const int tx = 4 * (threadIdx.x & 7), ty = 4 * (threadIdx.x >> 3);
+    const int t = threadIdx.x & 63, grp = threadIdx.x >> 6;
+    const int tx = 4 * (t & 7), ty = 4 * (t >> 3);
+    auto group_sync = [&] {
+        if (KS == 1) __syncthreads();
+        else asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");
+    };
     float acc[4][4] = {};
     float4 ra[4], rb[4];
-    small_load<!ACOL>(A, g.lda, g.M, g.K, m0, 0, vecA, ra);
-    small_load<BKC>(B, g.ldb, g.N, g.K, n0, 0, vecB, rb);
-    small_store<!ACOL>(As[0], ra);
-    small_store<BKC>(Bs[0], rb);
-    __syncthreads();
-    for (int k0 = 0, buf = 0; k0 < g.K; k0 += SB, buf ^= 1) {
-        const bool more = k0 + SB < g.K;
-        if (more) {
-            small_load<!ACOL>(A, g.lda, g.M, g.K, m0, k0 + SB, vecA, ra);
-            small_load<BKC>(B, g.ldb, g.N, g.K, n0, k0 + SB, vecB, rb);
+    int buf = KS == 1 ? 0 : grp;
+    small_load<!ACOL>(A, g.lda, g.M, g.K, m0, SB * grp, t, vecA, ra);
+    small_load<BKC>(B, g.ldb, g.N, g.K, n0, SB * grp, t, vecB, rb);
+    small_store<!ACOL>(sm[buf][0], t, ra);
+    small_store<BKC>(sm[buf][1], t, rb);
+    group_sync();
+    for (int k0 = SB * grp; k0 < g.K; k0 += SB * KS) {
+        const int kn = k0 + SB * KS;
+        if (kn < g.K) {
+            small_load<!ACOL>(A, g.lda, g.M, g.K, m0, kn, t, vecA, ra);
+            small_load<BKC>(B, g.ldb, g.N, g.K, n0, kn, t, vecB, rb);
         }
+        const float *as = sm[buf][0] + ty, *bs = sm[buf][1] + tx;
         #pragma unroll 8
         for (int k = 0; k < SB; k++) {
-            const float4 a4 = *reinterpret_cast<const float4 *>(&As[buf][k][ty]);
-            const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[buf][k][tx]);
+            const float4 a4 = *reinterpret_cast<const float4 *>(as + k * SLD);
+            const float4 b4 = *reinterpret_cast<const float4 *>(bs + k * SLD);
             const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
             #pragma unroll
             for (int i = 0; i < 4; i++)
                 #pragma unroll
                 for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        if (more) {
-            small_store<!ACOL>(As[buf ^ 1], ra);
-            small_store<BKC>(Bs[buf ^ 1], rb);
+        if (kn < g.K) {
+            if (KS == 1) buf ^= 1;
+            else group_sync();
+            small_store<!ACOL>(sm[buf][0], t, ra);
+            small_store<BKC>(sm[buf][1], t, rb);
         }
+        group_sync();
+    }
+    if (KS > 1) {   // the first group adds the others' sums
+        float *part = sm[grp][0];
+        #pragma unroll
+        for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(part + (ty + i) * SLD + tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
         __syncthreads();
+        if (grp) return;
+        #pragma unroll
+        for (int q = 1; q < KS; q++)
+            #pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 v = *reinterpret_cast<const float4 *>(sm[q][0] + (ty + i) * SLD + tx);
+                acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
+            }
     }
     #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -482,15 +509,21 @@ __global__ void __launch_bounds__(64) k_gemm_small(GemmArgs g, bool vecA, bool v
     }
 }
 
-// Which of the two is faster, from fits in us to both over M 54..2048, K 54..2048: 8 + 1.1 per
-// 32 of K and wave of tiles for the tensor cores, 4 + (0.75 + 0.3 blocks an SM) per 32 of K here.
-// Measured, this against the tensor cores: 128 x 256 x 128 8.4 / 12.5, 512 x 18 x 512 in four
-// matrices 22.7 / 32.4, 1024 x 128 x 1024 37 / 54; 256 x 512 x 256 in four 16.6 / 16.5;
-// 512 x 1024 x 512 28.8 / 25.2, 1024 x 2048 x 1024 156 / 43.
-bool gemm_small_wins(const GemmArgs &g, long long tiles, int batch, int sms) {
-    const double kt = (g.K + 31) / 32, waves = (double)((tiles + sms - 1) / sms);
-    const double blocks = (double)((g.M + SB - 1) / SB) * ((g.N + SB - 1) / SB) * batch / sms;
-    return 4.0 + kt * (0.75 + 0.3 * blocks) < 8.0 + 1.1 * kt * waves;
+// Four groups a block while there are at most four blocks an SM (128 x 256 x 128 in one matrix
+// 10.5 us with one group, 6.2 with four; 1024 x 128 x 1024 35, 21; 1024 x 1024 x 128, 1024 blocks,
+// 16.5, 20.9).
+bool small_split(long long blocks, int K, int sms) { return K > SB && blocks <= 4LL * sms; }
+
+// Which of the two is faster, from fits in us to all three over M 54..2048, K 54..2048: 8 + 1.1 per
+// 32 of K and wave of tiles for the tensor cores, 4 + (0.75 + 0.3 blocks an SM) per 32 of K for one
+// group, 4.2 + max(2.05, 1.9 blocks an SM) per 128 of K for four.  Measured, small against tensor
+// cores: 128 x 256 x 128 6.2 / 12.5, 512 x 18 x 512 in four matrices 12.5 / 32.8, 2048 x 128 x 2048
+// 58 / 100; 256 x 512 x 256 in four 18.7 / 16.6, 512 x 1024 x 512 29 / 25, 1024 x 2048 x 1024 158 / 43.
+bool gemm_small_wins(const GemmArgs &g, long long tiles, long long blocks, int sms) {
+    const double kt = (g.K + 31) / 32, waves = (double)((tiles + sms - 1) / sms), per = (double)blocks / sms;
+    const double small = small_split(blocks, g.K, sms) ? 4.2 + ((g.K + 127) / 128) * std::max(2.05, 1.9 * per)
+                                                       : 4.0 + kt * (0.75 + 0.3 * per);
+    return small < 8.0 + 1.1 * kt * waves;
 }
 
 __global__ void k_identity(float *F, int n, int ldf, long long sF) {
@@ -513,11 +546,16 @@ cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *l
     const int sms = gemm_sms();
     const bool va = vec(g.A, g.lda, g.sA), vb = vec(g.B, g.ldb, g.sB),
                vc = vec(g.C, g.ldc, g.sC) && (g.epilogue != 2 || vec(g.D, g.ldd, g.sD));
-    if (gemm_small_wins(g, nt, batch, sms)) {
-        const dim3 grid((g.N + SB - 1) / SB, (g.M + SB - 1) / SB, batch);
-        if (g.a_colmajor) k_gemm_small<true, false><<<grid, 64, 0, s>>>(g, va, vb);
-        else if (g.b_kmajor) k_gemm_small<false, true><<<grid, 64, 0, s>>>(g, va, vb);
-        else k_gemm_small<false, false><<<grid, 64, 0, s>>>(g, va, vb);
+    const dim3 small((g.N + SB - 1) / SB, (g.M + SB - 1) / SB, batch);
+    const long long blocks = (long long)small.x * small.y * batch;
+    if (gemm_small_wins(g, nt, blocks, sms)) {
+        auto go = [&](auto one, auto four) {
+            if (small_split(blocks, g.K, sms)) four<<<small, 256, 0, s>>>(g, va, vb);
+            else one<<<small, 64, 0, s>>>(g, va, vb);
+        };
+        if (g.a_colmajor) go(k_gemm_small<true, false, 1>, k_gemm_small<true, false, 4>);
+        else if (g.b_kmajor) go(k_gemm_small<false, true, 1>, k_gemm_small<false, true, 4>);
+        else go(k_gemm_small<false, false, 1>, k_gemm_small<false, false, 4>);
         if (launches) *launches += 1;
         return cudaGetLastError();
     }
