@@ -15,10 +15,14 @@
 //
 // k_bt_prep (one thread block per reflector block and matrix) runs first: it writes the
 // implied zeros and unit of V_b into A (rows kb..k+1 of column k), forms G = V_b^T V_b,
-// T by the slarft recursion T[i][j] = -tau_j sum_{i <= l < j} T[i][l] G[l][j],
-// T[j][j] = tau_j, and Y_b into rows kb.. of Z (Y[kb+j][r] for r >= kb).
+// T (bt_triangle), and Y_b into rows kb.. of Z (Y[kb+j][r] for r >= kb).  With few blocks for the
+// SMs, each block of reflectors is given to several (blockIdx.z), which form G and T alike and
+// share the rows of Y.  Bound by T's chain and the staging for few, by the FMAs for many.  One
+// matrix of order 128: 114 us with T column by column and the zeros of its lower half
+// multiplied, 40 so; of order 1024 364, 186; 200 of 1024 2106, 1551.
 #include "cir_device.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <vector>
 
@@ -40,7 +44,7 @@ constexpr size_t bt_prep_smem() { return sizeof(float) * ((size_t)BT_NB * BT_LDM
 __device__ __forceinline__ void bt_stage(float *A, int ld, int n, int kb, int nbb, int r0, bool clean, float *Vt) {
     const int t = threadIdx.x;
     const int rr = 4 * (t & 15), r = r0 + rr;
-    #pragma unroll 2
+    #pragma unroll 4
     for (int q = 0; q < BT_NB / 16; q++) {
         const int j = (t >> 4) + 16 * q, k = kb + j;
         float x[4] = {0.f, 0.f, 0.f, 0.f};
@@ -86,6 +90,80 @@ __host__ __device__ inline long long bt_yoff2(int q, int n) {
     return 2LL * BT_NB * ((long long)q * n - 2LL * BT_NB * q * (q - 1) / 2);
 }
 
+// T^T (lower triangular, zeros above) in place of G = V^T V (its upper triangle) in M: the diagonal
+// 16 x 16 blocks by the recursion T[i][j] = -tau_j sum_{i <= l < j} T[i][l] G[l][j], T[j][j] = tau_j,
+// a warp each with a row a lane, then T_AB = -T_A (G_AB T_B) for pairs of blocks of 16, 32 and 64,
+// all pairs of a size at once.  X: scratch, 64 x (64 + 4).  Called by BT_NT threads.
+template <int H>
+__device__ __forceinline__ void bt_pairs(float *M, float *X) {
+    constexpr int NP = BT_NT / (4 * H), CR = H / 16, CG = H / 4, LX = H + 4;   // pairs, rows and column groups
+    static_assert(NP * 2 * H == BT_NB, "every pair has its threads");
+    const int t = threadIdx.x % (4 * H), pair = threadIdx.x / (4 * H), rg = t / CG, cg = t % CG;
+    float *A = M + 2 * H * pair * (BT_LDM + 1), *G = A + H, *B = A + H * (BT_LDM + 1), *Y = A + H * BT_LDM;
+    float *Xp = X + pair * H * LX;
+    float acc[CR][4] = {};
+    for (int l = 0; l < H; l += 4) {        // X^T[c][r] = sum_l T_B^T[c][l] G[r][l]: c = rg + 16 i, r = cg + CG j
+        float4 b[CR], g[4];
+        #pragma unroll
+        for (int i = 0; i < CR; i++) b[i] = *reinterpret_cast<const float4 *>(B + (rg + 16 * i) * BT_LDM + l);
+        #pragma unroll
+        for (int j = 0; j < 4; j++) g[j] = *reinterpret_cast<const float4 *>(G + (cg + CG * j) * BT_LDM + l);
+        #pragma unroll
+        for (int i = 0; i < CR; i++)
+            #pragma unroll
+            for (int j = 0; j < 4; j++)
+                acc[i][j] = fmaf(b[i].x, g[j].x, fmaf(b[i].y, g[j].y, fmaf(b[i].z, g[j].z, fmaf(b[i].w, g[j].w, acc[i][j]))));
+    }
+    #pragma unroll
+    for (int i = 0; i < CR; i++)
+        #pragma unroll
+        for (int j = 0; j < 4; j++) {
+            Xp[(rg + 16 * i) * LX + cg + CG * j] = acc[i][j];
+            acc[i][j] = 0.f;
+        }
+    __syncthreads();
+    for (int l = 0; l < H; l++) {           // T_AB^T[c][r] = -sum_l X^T[c][l] T_A^T[l][r]: r = 4 cg + j
+        const float4 v = *reinterpret_cast<const float4 *>(A + l * BT_LDM + 4 * cg);
+        #pragma unroll
+        for (int i = 0; i < CR; i++) {
+            const float x = Xp[(rg + 16 * i) * LX + l];
+            acc[i][0] = fmaf(-x, v.x, acc[i][0]);
+            acc[i][1] = fmaf(-x, v.y, acc[i][1]);
+            acc[i][2] = fmaf(-x, v.z, acc[i][2]);
+            acc[i][3] = fmaf(-x, v.w, acc[i][3]);
+        }
+    }
+    #pragma unroll
+    for (int i = 0; i < CR; i++) {
+        *reinterpret_cast<float4 *>(Y + (rg + 16 * i) * BT_LDM + 4 * cg) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        *reinterpret_cast<float4 *>(G + (rg + 16 * i) * BT_LDM + 4 * cg) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void bt_triangle(float *M, const float *tau, float *X) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, o = 16 * warp;
+    float *D = M + o * (BT_LDM + 1);
+    float row[16];
+    #pragma unroll
+    for (int j = 0; j < 16; j++) {
+        float s = 0.f;
+        #pragma unroll
+        for (int l = 0; l < j; l++) s = fmaf(row[l], D[l * BT_LDM + j], s);
+        row[j] = lane < j ? -tau[o + j] * s : lane == j ? tau[o + j] : 0.f;
+    }
+    __syncwarp();
+    if (lane < 16)
+        #pragma unroll
+        for (int j = 0; j < 16; j++) {
+            D[j * BT_LDM + lane] = lane <= j ? row[j] : 0.f;   // T^T; column `lane` of it is row `lane` of T
+        }
+    __syncthreads();
+    bt_pairs<16>(M, X);
+    bt_pairs<32>(M, X);
+    bt_pairs<64>(M, X);
+}
+
 template <bool SPLIT>
 __global__ void __launch_bounds__(BT_NT, 2) k_bt_prep(EighArgs a, BtSplit sp) {
     extern __shared__ __align__(16) float bsm[];
@@ -111,7 +189,7 @@ __global__ void __launch_bounds__(BT_NT, 2) k_bt_prep(EighArgs a, BtSplit sp) {
             for (int q = 0; q < 8; q++) acc[p][q] = 0.f;
         for (int r0 = kb; r0 < n; r0 += BT_RC) {
             __syncthreads();
-            bt_stage(A, ld, n, kb, nbb, r0, !SPLIT, Vt);
+            bt_stage(A, ld, n, kb, nbb, r0, !SPLIT && blockIdx.z == 0, Vt);
             __syncthreads();
             if (SPLIT) {   // the cleaned chunk as a split pair: column kb + j, rows r0..
                 const size_t ov = (size_t)mat * sp.sV;
@@ -146,26 +224,11 @@ __global__ void __launch_bounds__(BT_NT, 2) k_bt_prep(EighArgs a, BtSplit sp) {
             for (int q = p; q < 8; q++) M[(ty + 16 * p) * BT_LDM + tx + 16 * q] = acc[p][q];
     }
     __syncthreads();
-    // T, column by column; T[i][l] (i <= l) is kept at M[l][i], which the recursion never
-    // reads as G (it reads G[l][j], l < j, from the untouched upper part M[l][j])
-    for (int j = 0; j < BT_NB; j++) {
-        if (t < j) {
-            float s = 0.f;
-            for (int l = 0; l < j; l++) s = fmaf(l >= t ? M[l * BT_LDM + t] : 0.f, M[l * BT_LDM + j], s);
-            M[j * BT_LDM + t] = -tau[j] * s;
-        } else if (t == j) {
-            M[j * BT_LDM + j] = tau[j];
-        }
-        __syncthreads();
-    }
-    for (int idx = t; idx < BT_NB * BT_NB; idx += BT_NT) {   // T[i][j] = 0 for i > j
-        const int j = idx / BT_NB, i = idx - j * BT_NB;
-        if (i > j) M[j * BT_LDM + i] = 0.f;
-    }
+    bt_triangle(M, tau, Vt);
     // Y[kb + j][r] = sum_i T[i][j] V[r][i] = sum_i M[j][i] Vt[i][r]: thread (tr, tj) computes
     // rows j = tj + 16 q, columns r0 + 4 tr .. +3 of each chunk
     const int tr = t & 15, tj = t >> 4;
-    for (int r0 = kb; r0 < n; r0 += BT_RC) {
+    for (int r0 = kb + BT_RC * blockIdx.z; r0 < n; r0 += BT_RC * gridDim.z) {
         __syncthreads();
         bt_stage(A, ld, n, kb, nbb, r0, false, Vt);
         __syncthreads();
@@ -181,6 +244,7 @@ __global__ void __launch_bounds__(BT_NT, 2) k_bt_prep(EighArgs a, BtSplit sp) {
             for (int p = 0; p < 4; p++) v[p] = *reinterpret_cast<const float4 *>(Vt + (i + p) * BT_LDV + 4 * tr);
             #pragma unroll
             for (int q = 0; q < 8; q++) {
+                if (16 * q + 15 < i) continue;               // above T^T's diagonal
                 const float4 m = *reinterpret_cast<const float4 *>(M + (tj + 16 * q) * BT_LDM + i);
                 const float mm[4] = {m.x, m.y, m.z, m.w};
                 #pragma unroll
@@ -754,7 +818,12 @@ cudaError_t cir_launch_backtransform(const EighArgs &a, float *Q, float *P, floa
     const size_t smem = bt_prep_smem();
     cudaError_t e = cudaFuncSetAttribute(k_bt_prep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_bt_prep<false><<<dim3(nblk, nmat), BT_NT, smem, s>>>(a, BtSplit{});
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    const int share = (int)std::max(1LL, std::min({4LL, (long long)(n + BT_RC - 1) / BT_RC, (long long)sms / ((long long)nblk * nmat)}));
+    k_bt_prep<false><<<dim3(nblk, nmat, share), BT_NT, smem, s>>>(a, BtSplit{});
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int nl = 1;
     for (int b = nblk - 1; b >= 0; b--) {
