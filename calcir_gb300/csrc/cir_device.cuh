@@ -12,6 +12,34 @@
 __device__ __forceinline__ float cir_mi(float dx, float L) {
     return __fsub_rn(dx, __fmul_rn(L, roundf(__fdiv_rn(dx, L))));
 }
+// cir_mi of three components with the quotients' rounding taken from products with 1 / L.  The
+// nearest integers are the same unless a quotient lies within the products' error of a half (or
+// is large, or NaN): cir_mi3_quick says so and leaves the components, cir_mi3 asks cir_mi.
+__device__ __forceinline__ bool cir_mi3_quick(float &dx, float &dy, float &dz, float bx, float by, float bz, float rx,
+                                              float ry, float rz) {
+    const float tx = dx * rx, ty = dy * ry, tz = dz * rz;
+    constexpr float R = 12582912.f;   // 1.5 * 2^23: adding it leaves the nearest integer (|t| < 2^22)
+    const float nx = __fsub_rn(__fadd_rn(tx, R), R), ny = __fsub_rn(__fadd_rn(ty, R), R), nz = __fsub_rn(__fadd_rn(tz, R), R);
+    const float half = fmaxf(fmaxf(fabsf(tx - nx), fabsf(ty - ny)), fabsf(tz - nz));
+    const float big = fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz));
+    if (!(half < 0.49999f && big < 32.f && tx == tx && ty == ty && tz == tz)) return false;
+    dx = __fsub_rn(dx, __fmul_rn(bx, nx));
+    dy = __fsub_rn(dy, __fmul_rn(by, ny));
+    dz = __fsub_rn(dz, __fmul_rn(bz, nz));
+    return true;
+}
+__device__ __forceinline__ void cir_mi3(float &dx, float &dy, float &dz, float bx, float by, float bz, float rx, float ry,
+                                        float rz) {
+    if (cir_mi3_quick(dx, dy, dz, bx, by, bz, rx, ry, rz)) return;
+    dx = cir_mi(dx, bx);
+    dy = cir_mi(dy, by);
+    dz = cir_mi(dz, bz);
+}
+// 1 / sqrt(x), the hardware's approximation with one Newton step
+__device__ __forceinline__ float cir_rsqrt(float x) {
+    const float y = rsqrtf(x);
+    return fmaf(__fmul_rn(0.5f, y), fmaf(__fmul_rn(-x, y), y, 1.f), y);
+}
 // mag3 (calcIR.cu:1464-1476): sqrt(x*x + y*y + z*z) with the reference's order of operations
 // and one rounding each; the field's cutoff test compares it with 0.7831 nm, a discontinuous
 // decision that a contracted evaluation would take differently for pairs within an ulp of it.

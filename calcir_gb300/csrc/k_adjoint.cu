@@ -153,49 +153,50 @@ __global__ void __launch_bounds__(256) k_build_R(const float *a, const float *b,
         if (n0 + r < n && m0 + c < n) Rz[(size_t)(n0 + r) * ldr + m0 + c] = tr[c][r];
 }
 
-// the geometric factor of the transition dipole coupling between chromophore i (position t,
-// direction u) and chromophore j of a frame's table (calcIR.cu:1352-1399 without the x and mu'
-// factors)
-__device__ __forceinline__ float tdc_kappa(const float3 &t, const float3 &u, const float *ct, int ld, int j, const float3 &b) {
-    float dx = cir_mi(t.x - ct[CT_TX * ld + j], b.x);
-    float dy = cir_mi(t.y - ct[CT_TY * ld + j], b.y);
-    float dz = cir_mi(t.z - ct[CT_TZ * ld + j], b.z);
-    const float ir = 1.f / sqrtf(dx * dx + dy * dy + dz * dz);
-    dx *= ir; dy *= ir; dz *= ir;
-    const float q = ir * (1.f / CIR_BOHR_NM);
-    const float ujx = ct[CT_UX * ld + j], ujy = ct[CT_UY * ld + j], ujz = ct[CT_UZ * ld + j];
-    const float uu = u.x * ujx + u.y * ujy + u.z * ujz;
-    const float un = u.x * dx + u.y * dy + u.z * dz;
-    const float vn = ujx * dx + ujy * dy + ujz * dz;
+// The geometric factor of the transition dipole coupling between chromophore i (position t,
+// direction u) and chromophore o (position and direction) of a frame (calcIR.cu:1352-1399 without
+// the x and mu' factors); rb = 1 / b.  QUICK takes the nearest image from products with rb and
+// clears ok where cir_mi3 would ask cir_mi.
+template <bool QUICK>
+__device__ __forceinline__ float tdc_kappa(const float3 &t, const float3 &u, const float (&o)[6], const float3 &b, const float3 &rb, bool &ok) {
+    float dx = t.x - o[0], dy = t.y - o[1], dz = t.z - o[2];
+    if (QUICK) ok &= cir_mi3_quick(dx, dy, dz, b.x, b.y, b.z, rb.x, rb.y, rb.z);
+    else cir_mi3(dx, dy, dz, b.x, b.y, b.z, rb.x, rb.y, rb.z);
+    const float ir = cir_rsqrt(dx * dx + dy * dy + dz * dz), q = ir * (1.f / CIR_BOHR_NM);
+    const float uu = u.x * o[3] + u.y * o[4] + u.z * o[5];
+    const float un = (u.x * dx + u.y * dy + u.z * dz) * ir;
+    const float vn = (o[3] * dx + o[4] * dy + o[5] * dz) * ir;
     return (uu - 3.0f * un * vn) * (q * q * q) * CIR_CM_HARTREE;
 }
 
 // Contraction of the gradients of every origin and step with the map derivatives: blockIdx.y is
 // the matrix b = s*K + k (frame table, box and G of step k of origin s; psi(k) of it).
-// A warp takes DT_R rows i of one matrix at a time, its lanes the columns j: G (symmetric) is
-// read once, along its rows, and the table's values of j serve DT_R pairs.  For each i
+// A warp takes 32 rows i of one matrix, DT_R at a time, its lanes the columns j: G (symmetric) is
+// read once, along its rows, and the table's values of j serve DT_R pairs; lane l keeps the sums
+// of row l, so that the arithmetic in double is done once for 32 rows.  For each i
 //   cw = G_ii (on d omega), a_i = sum_j inter 2 G_ij kappa_ij q_j (q = mu' x),
 //   the intramolecular sums, and dL/dm_b,i (the correlation terms at this step, plus
 //   Re lambda_c(0) at step 0, where psi(0) = m(0) and there is no G),
 // folded into coefficients on d omega, d x, d p and d mu'; the 13 products with the derivatives
 // of those four maps (plus the direct intramolecular ones) are added to out[13].
 // The pair arithmetic bounds it.  Four matrices of order 512 a step, 100 steps: 49.4 ms with a
-// thread a row and a launch a step, 1.6 so.
-constexpr int DT_R = 4, DT_W = 8;             // rows a warp, warps
+// thread a row and a launch a step, 0.37 so (1.6 with the branches of the image and of the
+// intramolecular pairs in the loop).
+constexpr int DT_R = 4, DT_W = 4;             // rows at a time, warps
 __global__ void __launch_bounds__(32 * DT_W) k_dtheta(DthetaArgs d) {
     __shared__ double tot[DT_W][13];
     const int s = blockIdx.y / d.K, k = blockIdx.y - s * d.K, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = d.n, ld = d.ld, i0 = (blockIdx.x * DT_W + warp) * DT_R;
+    const int n = d.n, ld = d.ld, nc = d.nchrom_mol, w0 = (blockIdx.x * DT_W + warp) * 32;
     const float *ct = d.ct + (size_t)blockIdx.y * CT_NROW * ld;
     const float *b = d.box + 3 * (size_t)blockIdx.y;
-    const float3 box = make_float3(b[0], b[1], b[2]);
+    const float3 box = make_float3(b[0], b[1], b[2]), rbox = make_float3(1.f / b[0], 1.f / b[1], 1.f / b[2]);
     const CirMaps &mp = d.maps;
     const bool pairs = k > 0 && d.ispecies != 1 && d.ispecies != 2;
     const float *G = d.G + (size_t)blockIdx.y * d.sG;
-    float a[DT_R] = {}, ax[DT_R] = {}, bp[DT_R] = {}, d10[DT_R] = {}, d11[DT_R] = {}, d12[DT_R] = {};
-    if (pairs && i0 < n) {
+    float sa = 0.f;                                          // row w0 + lane's
+    for (int i0 = w0; pairs && i0 < min(n, w0 + 32); i0 += DT_R) {
+        float a[DT_R] = {};
         float3 t[DT_R], u[DT_R];
-        float E[DT_R], x[DT_R], p[DT_R];
         const float *Gr[DT_R];
         int mol[DT_R];
         #pragma unroll
@@ -203,41 +204,47 @@ __global__ void __launch_bounds__(32 * DT_W) k_dtheta(DthetaArgs d) {
             const int i = min(i0 + r, n - 1);
             t[r] = make_float3(ct[CT_TX * ld + i], ct[CT_TY * ld + i], ct[CT_TZ * ld + i]);
             u[r] = make_float3(ct[CT_UX * ld + i], ct[CT_UY * ld + i], ct[CT_UZ * ld + i]);
-            E[r] = ct[CT_E * ld + i];
-            x[r] = ct[CT_X * ld + i];
-            p[r] = ct[CT_P * ld + i];
             Gr[r] = G + (size_t)i * d.ldg;
-            mol[r] = i / d.nchrom_mol;
+            mol[r] = i / nc * nc;                            // the molecule's first chromophore
         }
         for (int j = lane; j < n; j += 32) {
-            const float xj = ct[CT_X * ld + j], qj = ct[CT_MUP * ld + j] * xj;
-            const int mj = j / d.nchrom_mol;
+            const float qj = 2.f * ct[CT_MUP * ld + j] * ct[CT_X * ld + j];
+            const float o[6] = {ct[CT_TX * ld + j], ct[CT_TY * ld + j], ct[CT_TZ * ld + j],
+                                ct[CT_UX * ld + j], ct[CT_UY * ld + j], ct[CT_UZ * ld + j]};
+            float g[DT_R], kap[DT_R];
+            bool ok = true;
             #pragma unroll
-            for (int r = 0; r < DT_R; r++) {
-                const float g = Gr[r][j], gs = 2.f * g;
-                if (mj != mol[r]) {                          // transition dipole coupling
-                    a[r] += gs * tdc_kappa(t[r], u[r], ct, ld, j, box) * qj;
-                } else if (j != min(i0 + r, n - 1)) {        // intramolecular map (calcIR.cu:1339)
-                    const float Ej = ct[CT_E * ld + j], pj = ct[CT_P * ld + j];
-                    ax[r] += gs * (mp.wi[0] + mp.wi[1] * (E[r] + Ej)) * xj;
-                    bp[r] += gs * mp.wi[2] * pj;
-                    d10[r] += g * x[r] * xj;
-                    d11[r] += g * (E[r] + Ej) * x[r] * xj;
-                    d12[r] += g * p[r] * pj;
-                }
-            }
+            for (int r = 0; r < DT_R; r++) g[r] = Gr[r][j] * qj;
+            #pragma unroll
+            for (int r = 0; r < DT_R; r++) kap[r] = tdc_kappa<true>(t[r], u[r], o, box, rbox, ok);
+            if (!ok)
+                for (int r = 0; r < DT_R; r++) kap[r] = tdc_kappa<false>(t[r], u[r], o, box, rbox, ok);
+            #pragma unroll
+            for (int r = 0; r < DT_R; r++)
+                a[r] += (unsigned)(j - mol[r]) >= (unsigned)nc ? g[r] * kap[r] : 0.f;
+        }
+        #pragma unroll
+        for (int r = 0; r < DT_R; r++) {
+            const float v = warp_sum(a[r]);
+            if (lane == i0 - w0 + r) sa = v;
         }
     }
     double th[13] = {};
-    #pragma unroll
-    for (int r = 0; r < DT_R; r++) {
-        const float sa = warp_sum(a[r]), sax = warp_sum(ax[r]), sbp = warp_sum(bp[r]);
-        const float s10 = warp_sum(d10[r]), s11 = warp_sum(d11[r]), s12 = warp_sum(d12[r]);
-        const int i = i0 + r;
-        if (lane != r || i >= n) continue;                   // row r's tail is lane r's
+    const int i = w0 + lane;
+    if (i < n) {
         const float Ei = ct[CT_E * ld + i], w = ct[CT_W * ld + i], xi = ct[CT_X * ld + i], mup = ct[CT_MUP * ld + i];
         const float ux = ct[CT_UX * ld + i], uy = ct[CT_UY * ld + i], uz = ct[CT_UZ * ld + i];
         const float cw = k > 0 ? G[(size_t)i * d.ldg + i] : 0.f;
+        float sax = 0.f, sbp = 0.f, s10 = 0.f, s11 = 0.f, s12 = 0.f;   // intramolecular map (calcIR.cu:1339)
+        for (int j = i / nc * nc; pairs && j < min(n, i / nc * nc + nc); j++) {
+            if (j == i) continue;
+            const float g = G[(size_t)i * d.ldg + j], xj = ct[CT_X * ld + j], pj = ct[CT_P * ld + j], ee = Ei + ct[CT_E * ld + j];
+            sax += 2.f * g * (mp.wi[0] + mp.wi[1] * ee) * xj;
+            sbp += 2.f * g * mp.wi[2] * pj;
+            s10 += g * xi * xj;
+            s11 += g * ee * xi * xj;
+            s12 += g * ct[CT_P * ld + i] * pj;
+        }
         // dL/dm_b,i: the correlation terms of this step, plus Re lambda(0) at step 0
         const int S = gridDim.y / d.K;
         const float *ps = d.psi + (((size_t)k * S + s) * n + i) * PSI_LD;
@@ -278,8 +285,7 @@ __global__ void __launch_bounds__(32 * DT_W) k_dtheta(DthetaArgs d) {
     }
     #pragma unroll
     for (int q = 0; q < 13; q++) {
-        double v = th[q];                                    // lanes 0..DT_R-1 hold the rows
-        for (int o = DT_R / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const double v = warp_sum_d(th[q]);
         if (lane == 0) tot[warp][q] = v;
     }
     __syncthreads();
@@ -501,7 +507,7 @@ cudaError_t cir_adj_build_R(const float *a, const float *b, long long sab, const
 }
 
 cudaError_t cir_adj_dtheta(const DthetaArgs &d, int S, cudaStream_t s) {
-    const int rows = DT_R * DT_W;
+    const int rows = 32 * DT_W;
     k_dtheta<<<dim3((d.n + rows - 1) / rows, (unsigned)(S * d.K)), 32 * DT_W, 0, s>>>(d);
     return cudaGetLastError();
 }

@@ -28,33 +28,6 @@ namespace {
 constexpr int CHROM_NT = 64;        // threads of a block: 64 chromophores, or 2 (WIDE)
 constexpr int MOL_F = 12;           // floats of a staged molecule: H1, H2, M, O
 
-// cir_mi of three components with the quotients' rounding taken from products with 1 / L: the
-// nearest integers are the same unless a quotient lies within the products' error of a half (or
-// is large, or NaN), where cir_mi decides.
-__device__ __forceinline__ void mi3(float &dx, float &dy, float &dz, float bx, float by, float bz, float rx, float ry,
-                                    float rz) {
-    const float tx = dx * rx, ty = dy * ry, tz = dz * rz;
-    constexpr float R = 12582912.f;   // 1.5 * 2^23: adding it leaves the nearest integer (|t| < 2^22)
-    const float nx = __fsub_rn(__fadd_rn(tx, R), R), ny = __fsub_rn(__fadd_rn(ty, R), R), nz = __fsub_rn(__fadd_rn(tz, R), R);
-    const float half = fmaxf(fmaxf(fabsf(tx - nx), fabsf(ty - ny)), fabsf(tz - nz));
-    const float big = fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz));
-    if (half < 0.49999f && big < 32.f && tx == tx && ty == ty && tz == tz) {
-        dx = __fsub_rn(dx, __fmul_rn(bx, nx));
-        dy = __fsub_rn(dy, __fmul_rn(by, ny));
-        dz = __fsub_rn(dz, __fmul_rn(bz, nz));
-    } else {
-        dx = cir_mi(dx, bx);
-        dy = cir_mi(dy, by);
-        dz = cir_mi(dz, bz);
-    }
-}
-
-// 1 / sqrt(x), the hardware's approximation with one Newton step
-__device__ __forceinline__ float rsqrt_newton(float x) {
-    const float y = rsqrtf(x);
-    return fmaf(__fmul_rn(0.5f, y), fmaf(__fmul_rn(-x, y), y, 1.f), y);
-}
-
 // (the roundings are written out wherever the compiler could contract two copies of the code
 // differently: both forms of k_chromophore give the same bits)
 __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz) {
@@ -65,7 +38,7 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
 __device__ __forceinline__ float4 site_term(float hx, float hy, float hz, float sx, float sy, float sz, float q, float bx,
                                             float by, float bz, float rx, float ry, float rz) {
     float qx = hx - sx, qy = hy - sy, qz = hz - sz;
-    mi3(qx, qy, qz, bx, by, bz, rx, ry, rz);
+    cir_mi3(qx, qy, qz, bx, by, bz, rx, ry, rz);
     qx = qx * CIR_BOHR_NM;
     qy = qy * CIR_BOHR_NM;
     qz = qz * CIR_BOHR_NM;
@@ -118,7 +91,7 @@ __global__ void __launch_bounds__(CHROM_NT) k_chromophore(BuildArgs a, float cut
             const int n = (c0 + q) / a.nchrom_mol;
             const float *h = sm_mol + n * MOL_F + 3 * ((c0 + q) % 2);   // chrom%2 selects HW1/HW2 (calcIR.cu:1061-1072)
             float dx = ox - h[0], dy = oy - h[1], dz = oz - h[2];
-            mi3(dx, dy, dz, bx, by, bz, rx, ry, rz);
+            cir_mi3(dx, dy, dz, bx, by, bz, rx, ry, rz);
             // calcIR.cu:1106-1113 (a NaN distance is not beyond the cutoff)
             const bool in = !(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)) > cut2);
             const unsigned b = __ballot_sync(0xffffffffu, in && m < a.nmol && m != n);
@@ -238,8 +211,8 @@ __device__ __forceinline__ float pair_coupling(const Chrom &lo, const Chrom &hi,
                     __fmul_rn(mp.wi[2], __fmul_rn(lo.p, hi.p)));
     // transition dipole coupling (calcIR.cu:1352-1399)
     float dx = lo.tx - hi.tx, dy = lo.ty - hi.ty, dz = lo.tz - hi.tz;
-    mi3(dx, dy, dz, bx, by, bz, rx, ry, rz);
-    const float ri = rsqrt_newton(dot3(dx, dy, dz, dx, dy, dz)), rb = __fmul_rn(ri, 1.f / CIR_BOHR_NM);
+    cir_mi3(dx, dy, dz, bx, by, bz, rx, ry, rz);
+    const float ri = cir_rsqrt(dot3(dx, dy, dz, dx, dy, dz)), rb = __fmul_rn(ri, 1.f / CIR_BOHR_NM);
     const float uu = dot3(lo.ux, lo.uy, lo.uz, hi.ux, hi.uy, hi.uz);
     const float un = __fmul_rn(dot3(lo.ux, lo.uy, lo.uz, dx, dy, dz), ri);
     const float vn = __fmul_rn(dot3(hi.ux, hi.uy, hi.uz, dx, dy, dz), ri);
