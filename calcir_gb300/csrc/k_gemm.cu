@@ -16,17 +16,18 @@
 // rounding to nearest, and L, 2^-8 of the sum, once a tile.
 //
 // One CTA per SM walks 128 x 128 tiles (column tile fastest, then row tile, then matrix):
-//   warps 0-7   load FP32 slices 32 deep (0-3 A, 4-7 B), split them and store the three terms
-//               K-major (core matrices of 8 rows x 16 bytes, (r/8, k/8) at (r/8)*SBO + (k/8)*LBO;
-//               SBO padded so that either orientation stores without bank conflicts) into a ring;
-//               the next slice's loads are in flight while one is split;
+//   warps 0-7   copy FP32 slices 32 deep (0-3 A, 4-7 B) into shared memory, F_RAW slices ahead,
+//               split them and store the three terms K-major (core matrices of 8 rows x 16 bytes,
+//               (r/8, k/8) at (r/8)*SBO + (k/8)*LBO; SBO padded so that either orientation stores
+//               without bank conflicts) into a ring;
 //   warps 8-15  sum the chunks (a thread a row and half of the columns), then the epilogue, while
 //               the next tile is loaded and multiplied (two H and two L accumulators, all 512
 //               columns of tensor memory);
 //   warp 16     issues the MMAs.
-// The loads' issue and the splitting bound it (six MMAs of 16 K take 40% of a slice's time).
-// 1024 x 2048 x 1024 in ten matrices: 859-1044 us as SIMT FFMAs (50-41 TFLOP/s), 304-378 so
-// (141-114), relative error against 64 bits 5.5e-7 before, 1.2e-7 so.  Products with too few
+// The splitting bounds it (the six MMAs of 16 K take half of a slice's time).  1024 x 2048 x 1024
+// in ten matrices: 859-1044 us as SIMT FFMAs (50-41 TFLOP/s), 306-380 with the next slice in
+// registers, 283-331 so (152-130), relative error against 64 bits 5.5e-7 before, 1.2e-7 so.  Not
+// taken: 16 splitting warps (403-432: the copies of 8 bytes that rows contiguous then need).  Products with too few
 // tiles for the SMs run on the SIMT kernel further down (gemm_small_wins).
 // Every wait is bounded: a timeout raises the CTA's abort flag and the error flag, every role
 // leaves its loop, and the MMAs issued are waited for before the tensor memory is freed.
@@ -42,11 +43,12 @@ namespace {
 constexpr int FM = 128, FN = 128, FK = 32;     // tile, K of a slice
 constexpr int F_LBO = 128, F_SBO = 528;
 constexpr int F_PART = (FM / 8) * F_SBO;       // bytes of one term of one operand's slice
-constexpr int F_STAGE = 6 * F_PART, F_NS = 4;
+constexpr int F_STAGE = 6 * F_PART, F_NS = 3, F_RAW = 2;
 constexpr int F_CHUNK = 1;                     // slices between read-outs of H
 constexpr int F_LOAD = 8, F_ACC = 8;           // warps
 constexpr int F_NT = 32 * (F_LOAD + F_ACC + 4);   // whole warpgroups: the register split is per group
-constexpr size_t F_SMEM = (size_t)F_NS * F_STAGE + 256;
+constexpr size_t F_RAWB = (size_t)F_LOAD * 32 * 128;   // bytes of an FP32 slice of both operands
+constexpr size_t F_SMEM = (size_t)F_NS * F_STAGE + F_RAW * F_RAWB + 256;
 
 // The warpgroups' registers: 640 threads launch with 96 each (61440); the idle three warps of
 // the MMA group give theirs to the loads in flight and the sums: 2 * 128 * 120 + 2 * 128 * 104 +
@@ -84,44 +86,59 @@ __device__ __forceinline__ void split3(const float (&x)[8], uint4 &h, uint4 &m, 
 // of eight consecutive K of one row.  KC: K contiguous in memory (element (r, k) at p[r*ld + k]),
 // group i is row 32 i + 8 (warp & 3) + (lane & 7), K 8 (lane >> 3) ..; else rows contiguous
 // (element (r, k) at p[k*ld + r]), the groups are rows 4 lane .. + 3, K 8 (warp & 3) ...
+// The values wait in shared memory, each thread's own eight 16-byte words (raw, RAW_ST apart),
+// which no other thread reads: an asynchronous copy needs no register and no barrier.
+constexpr int RAW_ST = F_LOAD * 32 * 16;
+
 template <bool KC>
 struct Part {
-    float4 v[8];
-    __device__ __forceinline__ static float4 load4(const float *q, int have) {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (have > 0) x.x = __ldg(q);
-        if (have > 1) x.y = __ldg(q + 1);
-        if (have > 2) x.z = __ldg(q + 2);
-        if (have > 3) x.w = __ldg(q + 3);
-        return x;
+    // four values at q, of which the first `have` exist; the others are zero (p: any address of the
+    // operand, for what is not read)
+    __device__ __forceinline__ static void load4(unsigned char *raw, const float *q, int have, const float *p, bool vec) {
+        const uint32_t dst = smem_addr(raw);
+        if (vec) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(have > 0 ? q : p),
+                         "r"(4 * max(0, min(have, 4))) : "memory");
+            return;
+        }
+        #pragma unroll
+        for (int e = 0; e < 4; e++)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4 * e), "l"(have > e ? q + e : p),
+                         "r"(have > e ? 4 : 0) : "memory");
     }
-    __device__ __forceinline__ void load(const float *p, int ld, int rdim, int kdim, int r0, int k0, int w4, int lane, bool vec) {
+    __device__ __forceinline__ static void load(unsigned char *raw, const float *p, int ld, int rdim, int kdim, int r0, int k0,
+                                                int w4, int lane, bool vec) {
         if (vec && r0 + 128 <= rdim && k0 + 32 <= kdim) {   // the whole slice inside
             const float *q = KC ? p + (size_t)(r0 + 8 * w4 + (lane & 7)) * ld + k0 + 8 * (lane >> 3)
                                 : p + (size_t)(k0 + 8 * w4) * ld + r0 + 4 * lane;
             const size_t st = KC ? (size_t)32 * ld : (size_t)ld;
             #pragma unroll
             for (int i = 0; i < 8; i++)
-                v[i] = __ldg(reinterpret_cast<const float4 *>(KC ? q + (i >> 1) * st + 4 * (i & 1) : q + i * st));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(raw + i * RAW_ST)),
+                             "l"(KC ? q + (i >> 1) * st + 4 * (i & 1) : q + i * st)
+                             : "memory");
         } else if (KC) {
             #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int r = r0 + 32 * i + 8 * w4 + (lane & 7), k = k0 + 8 * (lane >> 3);
                 const float *q = p + (size_t)r * ld + k;
                 const int have = r < rdim ? kdim - k : 0;
-                v[2 * i] = load4(q, have);
-                v[2 * i + 1] = load4(q + 4, have - 4);
+                load4(raw + 2 * i * RAW_ST, q, have, p, vec);
+                load4(raw + (2 * i + 1) * RAW_ST, q + 4, have - 4, p, vec);
             }
         } else {
             const int r = r0 + 4 * lane;
             #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int k = k0 + 8 * w4 + i;
-                v[i] = load4(p + (size_t)k * ld + r, k < kdim ? rdim - r : 0);
+                load4(raw + i * RAW_ST, p + (size_t)k * ld + r, k < kdim ? rdim - r : 0, p, vec);
             }
         }
     }
-    __device__ __forceinline__ void store(unsigned char *base, int w4, int lane) const {
+    __device__ __forceinline__ static void store(const unsigned char *raw, unsigned char *base, int w4, int lane) {
+        float4 v[8];
+        #pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = *reinterpret_cast<const float4 *>(raw + i * RAW_ST);
         #pragma unroll
         for (int i = 0; i < 4; i++) {
             float x[8];
@@ -153,7 +170,7 @@ template <bool ACOL, bool BKC>
 __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int tiles_mn, int ntiles, bool vecA, bool vecB,
                                                    bool vecC, int *err) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)F_NS * F_STAGE);   // [F_NS]
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)F_NS * F_STAGE + F_RAW * F_RAWB);   // [F_NS]
     uint64_t *empty = full + F_NS;                                                 // [F_NS]
     uint64_t *hfull = empty + F_NS;                                                // [2] chunk in H
     uint64_t *hempty = hfull + 2;                                                  // [2]
@@ -201,10 +218,11 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
         const bool isA = warp < 4;
         const int w4 = warp & 3;
         // (the operand's side: pointer, strides, extents)
-        auto produce = [&](auto &part, const float *base, long long sb, int ld, int rdim, bool vec) {
-            // the load side runs a slice ahead of the store side
+        auto produce = [&](auto part, const float *base, long long sb, int ld, int rdim, bool vec) {
+            // the load side runs F_RAW slices ahead of the store side
             int lt = blockIdx.x, lkt = 0, r0 = 0;
             const float *src = base;
+            unsigned char *raw = smem + (size_t)F_NS * F_STAGE + 16 * tid;
             auto seek = [&] {
                 if (lt >= ntiles) return;
                 int bz, m0, n0;
@@ -212,13 +230,15 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                 src = base + (size_t)bz * sb;
                 r0 = isA ? m0 : n0;
             };
-            auto load = [&](auto &p) {
-                if (lt >= ntiles) return;
-                p.load(src, ld, rdim, g.K, r0, lkt * FK, w4, lane, vec);
-                if (++lkt == KT) { lkt = 0; lt += gridDim.x; seek(); }
+            auto load = [&](uint32_t slot) {
+                if (lt < ntiles) {
+                    part.load(raw + slot * F_RAWB, src, ld, rdim, g.K, r0, lkt * FK, w4, lane, vec);
+                    if (++lkt == KT) { lkt = 0; lt += gridDim.x; seek(); }
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
             };
             seek();
-            load(part);
+            for (int i = 0; i < F_RAW; i++) load(i);
             uint32_t it = 0;
             const uint32_t total = (uint32_t)((ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * KT;
             bool ok = true;
@@ -226,23 +246,20 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                 const int s = it % F_NS;
                 if (it >= F_NS && !(ok = mbar_wait(&empty[s], ((it / F_NS) & 1) ^ 1))) return;
                 if (*abort_flag) { ok = false; return; }
-                part.store(smem + (size_t)s * F_STAGE + (isA ? 0 : 3 * F_PART), w4, lane);
+                asm volatile("cp.async.wait_group %0;" ::"n"(F_RAW - 1) : "memory");
+                part.store(raw + it % F_RAW * F_RAWB, smem + (size_t)s * F_STAGE + (isA ? 0 : 3 * F_PART), w4, lane);
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive1(&full[s]);
+                load(it % F_RAW);
                 it++;
-                load(part);
             };
             while (it < total && ok) step();
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
             if (!ok) fail();
         };
-        if (isA) {
-            Part<!ACOL> part;
-            produce(part, g.A, g.sA, g.lda, g.M, vecA);
-        } else {
-            Part<BKC> part;
-            produce(part, g.B, g.sB, g.ldb, g.N, vecB);
-        }
+        if (isA) produce(Part<!ACOL>(), g.A, g.sA, g.lda, g.M, vecA);
+        else produce(Part<BKC>(), g.B, g.sB, g.ldb, g.N, vecB);
     } else if (warp >= F_LOAD + F_ACC) {
         regs_down<24>();
         if (warp == F_LOAD + F_ACC && lane == 0) {
