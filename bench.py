@@ -130,21 +130,21 @@ def gpu_identifier():
 
 
 # DRAM bytes (read + write) per 1024 x 1024 matrix of the tridiagonalisation kernel, from one
-# ncu capture of k_eigh_tq on 152 matrices of order 1024 (dram__bytes_read.sum +
-# dram__bytes_write.sum over the launch, / 152: 86.17 GB + 3.48 GB read and written, with
-# the tiles of the matrix-vector products walked in alternating order):
+# ncu capture of k_tridiag on 152 matrices of order 1024 (dram__bytes_read.sum +
+# dram__bytes_write.sum over the launch, / 152):
 #   python -m calcir_gb300.profile eigh --nmol 512 --batch 152 && \
-#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:k_eigh_tq -c 1 \
+#   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:k_tridiag -c 1 \
 #       python -m calcir_gb300.profile eigh --nmol 512 --batch 152
 TRIDIAG_DRAM_BYTES_PER_MATRIX = 0.590e9
 
 
-def tridiag_bytes(n, nb=32):
+def tridiag_bytes(n, nb=8):
     """Algorithmic DRAM bytes of the blocked tridiagonalisation of one order-n matrix: each
     column's matrix-vector product reads the lower triangle of its trailing block once, and
-    each panel of nb columns reads and writes the lower triangle beyond the panel once."""
+    each panel of nb columns writes the lower triangle beyond the panel once (the pass of the
+    next column reads it, updates it and multiplies)."""
     sym = sum(4.0 * m * (m + 1) / 2 for m in range(1, n - 1))
-    upd = sum(8.0 * (n - q0) * (n - q0 + 1) / 2 for q0 in range(nb, n - 1, nb))
+    upd = sum(4.0 * (n - q0) * (n - q0 + 1) / 2 for q0 in range(nb, n - 1, nb))
     return sym + upd + 8.0 * 2 * 2   # + the final 2 x 2 block
 
 
@@ -245,8 +245,8 @@ def run_batching(args):
     """The batching configuration: 32 seeded trajectories of each of 128, 216, 343 and 512
     TIP4P/2005 molecules (256-1024 chromophores), 200 correlation points at 10 fs each, one
     time origin per trajectory, all in one cir_run_multi job (equal sizes batched through
-    every launch, step loops replayed from captured CUDA graphs, SIMT tile shapes from the
-    autotuner).  One bench step is the whole job; positions resident in HBM."""
+    every launch, step loops replayed from captured CUDA graphs, tcgen05 tile widths from
+    the autotuner).  One bench step is the whole job; positions resident in HBM."""
     import torch
     torch.cuda.set_device(0)
     from calcir_gb300 import build
@@ -365,8 +365,8 @@ def run_differentiation(args):
     """The differentiation configuration: 256 TIP4P/2005 molecules (512 chromophores), 4 time
     origins x 200 points; the loss is the IR + VV lineshape mismatch against targets made by
     the same code with the map coefficients perturbed by seeded +-2% noise.  One bench step is
-    one loss + gradient evaluation (cir_loss_grad: forward, psi checkpoints every 16 steps,
-    adjoint backward).  The gradient is checked against GPU central differences (relative
+    one loss + gradient evaluation (cir_loss_grad: forward, adjoint
+    backward).  The gradient is checked against GPU central differences (relative
     step 1e-4) on the three coefficients the loss is most sensitive to."""
     import torch
     torch.cuda.set_device(0)
@@ -421,8 +421,7 @@ def run_differentiation(args):
         "ms_per_step": sec * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic",
         "config": {"workload": "256 TIP4P/2005 molecules (512 chromophores), 4 origins 2 ps apart x 200 points; "
-                               "targets from map coefficients perturbed by seeded +-2% noise; psi checkpoints every "
-                               "16 steps", "loss": L},
+                               "targets from map coefficients perturbed by seeded +-2% noise", "loss": L},
         "gradient_checks": checks, "gpu_launches": int(st["kernel_launches"]), "clocks": clk,
     }
     print(json.dumps(line), flush=True)
@@ -557,7 +556,7 @@ def main():
     nomega = 3001
     h2d = xyz.nbytes + xyz.shape[0] * 12 + fos.nbytes
     d2h = steps_per_job * 48 + nomega * 8 * 4 + 3 * nfft * 8
-    form = {"fp32": "plain FP32 (SIMT GEMMs)", "tf32": "mixed: TF32 tcgen05 propagation GEMMs",
+    form = {"fp32": "plain FP32 (three-term BF16 tcgen05 and SIMT GEMMs)", "tf32": "mixed: TF32 tcgen05 propagation GEMMs",
             "bf16x3": "mixed: 3-pass split-BF16 tcgen05 propagation GEMMs"}[args.precision]
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -568,12 +567,12 @@ def main():
         "stages_ms_per_step": {k: st[k] / args.steps for k in ("ms_build", "ms_eig", "ms_prop")},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
         "gpu_launches": int(st["kernel_launches"]),
-        "roofline": {"kernel": "k_eigh_tq (blocked lower-storage tridiagonalisation; the job's 2500 matrices in "
+        "roofline": {"kernel": "k_tridiag (blocked lower-storage tridiagonalisation; the job's 2500 matrices in "
                                "two launches on two streams, timed together)",
                      "bound": "hbm", "achieved": tq_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
                      "frac": tq_gbs / pk["hbm_gbs"], "peak_kind": f"{pk_kind} copy bandwidth (burst)",
                      "work": "algorithmic bytes: per column the lower triangle of the trailing block, per "
-                             "32-column panel one read and write of the trailing lower triangle; "
+                             "8-column panel one write of the trailing lower triangle; "
                              f"{tridiag_bytes(n) / 1e9:.3f} GB per 1024 x 1024 matrix x 2500 matrices per job",
                      "ms_per_launch": tq_ms,
                      "traffic": TRIDIAG_DRAM_BYTES_PER_MATRIX * steps_per_job,
@@ -615,7 +614,7 @@ def main():
         if plain is not None and "fp32_simt_tflops" in extra:
             plain_prop = prop_flops / (plain["stats"]["ms_prop"] / args.steps * 1e-3) / 1e12
             line["plain_fp32"]["roofline_propagation"] = {
-                "kernel": "k_sgemm (SIMT FP32 propagation GEMMs)", "bound": "fp32 simt", "achieved": plain_prop,
+                "kernel": "k_gemm (FP32 propagation GEMMs as six BF16 tcgen05 products)", "bound": "fp32 simt", "achieved": plain_prop,
                 "peak": extra["fp32_simt_tflops"], "unit": "TFLOP/s", "frac": plain_prop / extra["fp32_simt_tflops"],
                 "peak_kind": "measured cuBLAS SGEMM, TF32 off (peaks_probe)"}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:

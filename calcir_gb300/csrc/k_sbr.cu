@@ -1,6 +1,6 @@
 // Two-stage reduction of the batched symmetric eigenproblem to tridiagonal form (the
 // successive band reduction of ELPA / MAGMA's two-stage ssyevd; the one-stage path is
-// k_eigh_tq, which replaces the sytrd step of magma_ssyevd_gpu, calcIR.cu:420-448):
+// k_tridiag, which replaces the sytrd step of magma_ssyevd_gpu, calcIR.cu:420-448):
 //
 //  stage 1, dense -> band of width SB_B, by panels of SB_B columns: the panel below the band
 //   is factored by Householder QR (k_sb_panel, one thread per panel row, the panel in

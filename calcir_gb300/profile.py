@@ -88,7 +88,7 @@ def sbr(nmol: int, nb: int, reps: int = 3) -> None:
 
 def noalloc(nmol: int, nb: int) -> None:
     """cir_eigh_noalloc on device copies of water Hamiltonians (the implicit-QR eigensolver
-    path: k_eigh_tq, k_eigh_formq, k_eigh_qr)."""
+    path: k_tridiag, k_eigh_formq, k_eigh_qr)."""
     import ctypes as C
     import torch
     from calcir_gb300._lib import check, load
