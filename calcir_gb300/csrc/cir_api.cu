@@ -625,7 +625,8 @@ static int autotune_tridiag(cir_ctx *c, const EighArgs &e, int nmat) {
 
 // F <- V diag(exp(+i w dt/hbar)) V^T F for `nprop` chains; all pointers on the device.
 static int propagate_dev(cir_ctx *c, int nprop, int n, const float *V, int ldv, long long sV, const float *w,
-                         int wstride, float dt, float *F, int ldf, long long sF, float *G, int &launches) {
+                         int wstride, float dt, float *F, int ldf, long long sF, float *G, int &launches,
+                         const TcfArgs *tcf = nullptr, bool *fused = nullptr) {
     GemmArgs g1;
     memset(&g1, 0, sizeof g1);
     g1.A = V; g1.lda = ldv; g1.sA = sV; g1.a_colmajor = false;      // V^T as a row-major view of V
@@ -640,7 +641,7 @@ static int propagate_dev(cir_ctx *c, int nprop, int n, const float *V, int ldv, 
     g2.B = G; g2.C = F; g2.epilogue = 0;
     if (c->p.precision == CIR_PREC_FP32) {
         CK(cir_launch_gemm(g1, nprop, c->stream, &launches));
-        CK(cir_launch_gemm(g2, nprop, c->stream, &launches));
+        CK(cir_launch_gemm(g2, nprop, c->stream, &launches, tcf, fused));
     } else {
         CK(cir_launch_tc_gemm(g1, nprop, c->p.precision, c->stream, &launches));
         CK(cir_launch_tc_gemm(g2, nprop, c->p.precision, c->stream, &launches));
@@ -1252,12 +1253,8 @@ struct GroupJob {
                 CK(cir_launch_split_gemm(s1, St, c->stream, &nl));
                 CK(cir_launch_split_gemm(s2, St, c->stream, &nl));
                 return CIR_OK;
-            } else if (k > 0) {
-                int rc2 = propagate_dev(c, St, n, A + mk * mstride, ld, (long long)dlt * mstride,
-                                        W + mk * ld, dlt * ld, p.dt, F, 2 * ld, (long long)n * 2 * ld, G, nl);
-                if (rc2) return rc2;
             }
-            TcfArgs t;
+            TcfArgs t;   // the step's correlation terms
             memset(&t, 0, sizeof t);
             t.F = F;
             t.sF = (long long)n * 2 * ld;
@@ -1275,6 +1272,13 @@ struct GroupJob {
                 t.sFt = fs_el;
                 t.ldft = ldh;
             }
+            bool done = false;
+            if (k > 0 && !split) {
+                int rc2 = propagate_dev(c, St, n, A + mk * mstride, ld, (long long)dlt * mstride,
+                                        W + mk * ld, dlt * ld, p.dt, F, 2 * ld, (long long)n * 2 * ld, G, nl, &t, &done);
+                if (rc2) return rc2;
+            }
+            if (done) return CIR_OK;
             CK(cir_launch_tcf(t, St, c->stream, &nl));
         }
         return CIR_OK;

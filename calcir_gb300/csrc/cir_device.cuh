@@ -210,7 +210,11 @@ struct GemmArgs {
     // element offsets instead (batch stride 2 sC elements)
     __nv_bfloat16 *Chi, *Clo;
 };
-cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *launches);
+struct TcfArgs;
+// tcf: the product is the propagated F whose contraction is wanted; *fused is set where the launch
+// has done it (small products), and is otherwise left
+cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *launches, const TcfArgs *tcf = nullptr,
+                            bool *fused = nullptr);
 // the same product in TF32 or two-term split BF16 (k_tc_gemm.cu)
 cudaError_t cir_launch_tc_gemm(const GemmArgs &g, int batch, int precision, cudaStream_t s, int *launches);
 size_t cir_tc_gemm_smem_bytes();

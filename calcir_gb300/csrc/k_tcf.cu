@@ -17,71 +17,25 @@
 // S(w_i) += sum_j |M_j|^2 g / ((w_i - l_j - avef)^2 + g^2) / pi, g = hbar/(2 T1)
 // (get_spectral_density, calcIR.cu:1414-1444).
 #include "cir_device.cuh"
+#include "cir_tcf.cuh"
 
 namespace {
 
 constexpr int TCF_WARPS = 8;
 
-// A sum held as an unevaluated pair of floats (Knuth's two-sum): 48 bits, on the FP32 pipe.  In
-// double the eight sums of a warp (40 adds, 16 clocks each for the warp) were most of the kernel.
-struct Pair {
-    float hi, lo;
-};
-__device__ __forceinline__ Pair pair_add(Pair a, float x) {
-    const float s = __fadd_rn(a.hi, x), v = __fsub_rn(s, a.hi);
-    return {s, __fadd_rn(a.lo, __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, v)), __fsub_rn(x, v)))};
-}
-__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
-    Pair r = pair_add(a, b.hi);
-    r.lo = __fadd_rn(r.lo, b.lo);
-    const float s = __fadd_rn(r.hi, r.lo);
-    return {s, __fsub_rn(r.lo, __fsub_rn(s, r.hi))};
-}
-__device__ __forceinline__ Pair pair_xor(Pair a, int o) {
-    return {__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-}
-
-// the four sums (re, im) of one row's (partial) psi with m(t): IR, iiFii, ijFij, iiFjj
-__device__ __forceinline__ void tcf_sums(const float (&pr)[9], const float (&pi)[9], const float (&c)[9], Pair (&acc)[8]) {
-    acc[0] = pair_add(acc[0], c[0] * pr[0] + c[1] * pr[1] + c[2] * pr[2]);
-    acc[1] = pair_add(acc[1], c[0] * pi[0] + c[1] * pi[1] + c[2] * pi[2]);
-    acc[2] = pair_add(acc[2], c[3] * pr[3] + c[4] * pr[4] + c[5] * pr[5]);
-    acc[3] = pair_add(acc[3], c[3] * pi[3] + c[4] * pi[4] + c[5] * pi[5]);
-    acc[4] = pair_add(acc[4], c[6] * pr[6] + c[7] * pr[7] + c[8] * pr[8]);
-    acc[5] = pair_add(acc[5], c[6] * pi[6] + c[7] * pi[7] + c[8] * pi[8]);
-    // xx->yy, xx->zz, yy->xx, yy->zz, zz->xx, zz->yy (psi index 3, 4, 5 = xx, yy, zz)
-    acc[6] = pair_add(acc[6], (c[4] + c[5]) * pr[3] + (c[3] + c[5]) * pr[4] + (c[3] + c[4]) * pr[5]);
-    acc[7] = pair_add(acc[7], (c[4] + c[5]) * pi[3] + (c[3] + c[5]) * pi[4] + (c[3] + c[4]) * pi[5]);
-}
-
-// the block's sums into out: IR, VV, VH (re, im).  A warp's eight sums meet by halves: the lanes
-// whose bit is set keep the upper half of what is left, so nine exchanges do for all eight.
+// the block's sums into out
 __device__ __forceinline__ void tcf_finish(Pair (&acc)[8], double *out) {
     __shared__ double part[TCF_WARPS][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    #pragma unroll
-    for (int w = 4; w > 0; w >>= 1) {
-        const bool up = lane & (4 * w);
-        #pragma unroll
-        for (int q = 0; q < w; q++) {
-            const Pair send = up ? acc[q] : acc[q + w], keep = up ? acc[q + w] : acc[q];
-            acc[q] = pair_add(keep, pair_xor(send, 4 * w));
-        }
-    }
-    acc[0] = pair_add(acc[0], pair_xor(acc[0], 2));
-    acc[0] = pair_add(acc[0], pair_xor(acc[0], 1));
-    if ((lane & 3) == 0) part[warp][lane >> 2] = (double)acc[0].hi + (double)acc[0].lo;
+    const double v = tcf_reduce(acc);
+    if ((lane & 3) == 0) part[warp][lane >> 2] = v;
     __syncthreads();
     if (warp == 0) {
         double s = 0.0;
         if (lane < 8)
             #pragma unroll
             for (int w = 0; w < TCF_WARPS; w++) s += part[w][lane];
-        const int im = lane & 1;
-        const double ii = __shfl_sync(0xffffffffu, s, 2 + im), ij = __shfl_sync(0xffffffffu, s, 4 + im),
-                     jj = __shfl_sync(0xffffffffu, s, 6 + im);
-        if (lane < 6)
-            atomicAdd(out + lane, lane < 2 ? s : lane < 4 ? (3.0 * ii + jj + 4.0 * ij) / 15.0 : (2.0 * ii - jj + 6.0 * ij) / 30.0);
+        tcf_add(s, out);
     }
 }
 

@@ -552,3 +552,11 @@ def test_merge_forms(lib, kind, n, nmat):
     _check_eig(A[0], w[0], V[0])
     for i in range(1, nmat):
         assert np.array_equal(w[i], w[0]) and np.array_equal(V[i], V[0])
+
+
+@pytest.mark.parametrize("nmol,origins", [(10, 1), (17, 9), (40, 3), (64, 1), (100, 4), (100, 40)])
+def test_contraction_in_product(lib, nmol, origins):
+    """The correlation terms added by the small products' epilogue (one group of threads up to order
+    32, four above; ragged tiles), and by the contraction where the product is large, against the
+    oracle."""
+    test_contraction_forms(lib, nmol, origins)
