@@ -33,6 +33,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
     return false;
 }
 
+// The outcome of a wait as the whole warp's: lanes that saw it differently would part before the
+// tensor-memory loads and shuffles that follow, which all 32 lanes have to reach together.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
 __device__ __forceinline__ void mma_tf32(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -64,9 +68,11 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
     return r;
 }
 
-// 16 consecutive fp32 columns of this thread's TMEM lane
+// 16 consecutive fp32 columns of this thread's TMEM lane.  The load is one instruction of the whole
+// warp: lanes that a ragged tile sent past the last epilogue meet the others first.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),

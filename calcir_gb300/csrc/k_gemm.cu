@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
             bool ok = true;
             auto step = [&] {
                 const int s = it % F_NS;
-                if (it >= F_NS && !(ok = mbar_wait(&empty[s], ((it / F_NS) & 1) ^ 1))) return;
-                if (*abort_flag) { ok = false; return; }
+                if (it >= F_NS && !(ok = warp_agrees(mbar_wait(&empty[s], ((it / F_NS) & 1) ^ 1)))) return;
+                if (!(ok = warp_agrees(!*abort_flag))) return;
                 asm volatile("cp.async.wait_group %0;" ::"n"(F_RAW - 1) : "memory");
                 part.store(raw + it % F_RAW * F_RAWB, smem + (size_t)s * F_STAGE + (isA ? 0 : 3 * F_PART), w4, lane);
                 fence_proxy_async();
@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                 mbar_wait(drain, 0);
             }
         }
+        __syncwarp();
     } else {
         regs_up<104>();
         const int quarter = warp & 3, half = (warp - F_LOAD) >> 2, row = quarter * 32 + lane;
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
             }
             for (int c = 0; c < NC; c++, ch++) {
                 const int hb = ch & 1;
-                if (!(ok = mbar_wait(&hfull[hb], (ch >> 1) & 1)) || *abort_flag) { ok = false; break; }
+                if (!(ok = warp_agrees(mbar_wait(&hfull[hb], (ch >> 1) & 1) && !*abort_flag))) break;
                 fence_after();
                 #pragma unroll
                 for (int h = 0; h < 4; h++) {

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(NTHREADS) k_tc_gemm(GemmArgs g) {
     }
     {   // the last commit covers every MMA issued before it
         const int last = KT - 1;
-        ok = mbar_wait(&bar[last & 1], (last >> 1) & 1) && ok;
+        ok = warp_agrees(mbar_wait(&bar[last & 1], (last >> 1) & 1) && ok);
     }
     fence_after();
     if (!ok) {

@@ -489,11 +489,11 @@ __global__ void __launch_bounds__(PT, 1) k_tc_persist(const __grid_constant__ Pe
         int li = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, li++) {
             const int a = li & 1;
-            if (!mbar_wait(&tfull[a], (li >> 1) & 1, lim)) {
+            if (!warp_agrees(mbar_wait(&tfull[a], (li >> 1) & 1, lim))) {
                 fail();
                 break;
             }
-            if (*abort_flag) break;
+            if (!warp_agrees(!*abort_flag)) break;
             fence_after();
             int bz, m0, n0;
             const SplitGemmArgs &g = plan.g[plan_tile(plan, t, bz, m0, n0, QN)];

@@ -560,3 +560,22 @@ def test_contraction_in_product(lib, nmol, origins):
     32, four above; ragged tiles), and by the contraction where the product is large, against the
     oracle."""
     test_contraction_forms(lib, nmol, origins)
+
+
+@pytest.mark.parametrize("precision,tol", [("fp32", None), ("tf32", 2e-3), ("bf16x3", 5e-5)])
+@pytest.mark.parametrize("n,batch", [(129, 60), (250, 40)])
+def test_propagate_ragged_tiles(lib, precision, tol, n, batch):
+    """More tiles than SMs whose last rows are missing: in every tensor-core product lanes of a warp
+    leave the epilogue early, and all have to meet again for the next tile's loads.  Bounds as
+    for one step in each form above."""
+    rng = np.random.default_rng(n)
+    V = np.stack([np.linalg.qr(rng.standard_normal((n, n)))[0] for _ in range(batch)]).astype(np.float32)
+    w = rng.uniform(-400, 400, (batch, n)).astype(np.float32)
+    F = (rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))).astype(np.complex64)
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005", precision=precision), 12) as eng:
+        got = eng.propagate(V, w, 0.1, F)
+    V64 = V.astype(np.float64)
+    phase = np.exp(1j * w.astype(np.float64) * np.float32(0.1) / HBAR)
+    ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F.astype(np.complex128)))
+    for b in range(batch):
+        assert O.rel_l2(got[b], ref[b]) < (tol or 2.0 ** -23 * (2 * np.sqrt(n) + 8)), b
