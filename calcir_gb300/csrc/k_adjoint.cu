@@ -400,12 +400,11 @@ __global__ void __launch_bounds__(PSI_B * PSI_G) k_psi_rows(const float *V, int 
     for (int t = threadIdx.x; t < NR * (PSI_LD / 2); t += PSI_B * PSI_G) {
         const int row = t / (PSI_LD / 2), q = 2 * (t - row * (PSI_LD / 2)), j = j0 + row;
         if (j >= n) continue;
-        const float re = psi_total<RP>(sm, row, q), im = psi_total<RP>(sm, row, q + 1);
-        float sn, cs;
-        sincosf(w[(size_t)b * sw + j] * dtoh, &sn, &cs);
+        float re = psi_total<RP>(sm, row, q), im = psi_total<RP>(sm, row, q + 1);
         const size_t o = ((size_t)b * n + j) * PSI_LD + q;
-        *reinterpret_cast<float2 *>(X + o) = make_float2(cs * re - sn * im, sn * re + cs * im);
         if (raw) *reinterpret_cast<float2 *>(raw + o) = make_float2(re, im);
+        cir_rotate(cir_phase(w[(size_t)b * sw + j] * dtoh), re, im);
+        *reinterpret_cast<float2 *>(X + o) = make_float2(re, im);
     }
 }
 

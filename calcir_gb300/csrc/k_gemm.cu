@@ -356,8 +356,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
             __syncwarp();
             if (lane == 0) mbar_arrive1(&lempty[li & 1]);
             if (r >= g.M) continue;
-            float cph = 1.f, sph = 0.f;
-            if (g.epilogue == 1) sincosf(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar, &sph, &cph);
+            const CirPhase ph = g.epilogue == 1 ? cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar) : CirPhase{};
             float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
             const int cb = n0 + 64 * half;
             if (vecC && cb + 64 <= g.N) {
@@ -369,11 +368,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                         for (int q = 0; q < 4; q++) d[q] = *reinterpret_cast<const float4 *>(D + cb + 16 * h + 4 * q);
                     if (g.epilogue == 1)   // (re, im) pairs times exp(+i ph)
                         #pragma unroll
-                        for (int q = 0; q < 16; q += 2) {
-                            const float re = acc[h][q], im = acc[h][q + 1];
-                            acc[h][q] = cph * re - sph * im;
-                            acc[h][q + 1] = sph * re + cph * im;
-                        }
+                        for (int q = 0; q < 16; q += 2) cir_rotate(ph, acc[h][q], acc[h][q + 1]);
                     #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         float4 x = make_float4(acc[h][4 * q], acc[h][4 * q + 1], acc[h][4 * q + 2], acc[h][4 * q + 3]);
@@ -388,11 +383,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                     for (int q = 0; q < 16; q += 2) {
                         const int c = cb + 16 * h + q;
                         float re = acc[h][q], im = acc[h][q + 1];
-                        if (g.epilogue == 1) {
-                            const float x = cph * re - sph * im;
-                            im = sph * re + cph * im;
-                            re = x;
-                        }
+                        if (g.epilogue == 1) cir_rotate(ph, re, im);
                         if (c < g.N) C[c] = D ? D[c] - re : re;
                         if (c + 1 < g.N) C[c + 1] = D ? D[c + 1] - im : im;
                     }
@@ -533,19 +524,14 @@ __global__ void __launch_bounds__(64 * KS) k_gemm_small(GemmArgs g, bool vecA, b
             }
             tcf_sums(pr, pi, c, sum);
         }
-        float cph = 1.f, sph = 0.f;
-        if (g.epilogue == 1) sincosf(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar, &sph, &cph);
+        const CirPhase ph = g.epilogue == 1 ? cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar) : CirPhase{};
         float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
         const float *D = g.epilogue == 2 ? g.D + (size_t)bz * g.sD + (size_t)r * g.ldd : nullptr;
         #pragma unroll
         for (int j = 0; j < 4; j += 2) {
             const int c = n0 + tx + j;
             float re = acc[i][j], im = acc[i][j + 1];
-            if (g.epilogue == 1) {   // (re, im) pairs times exp(+i ph)
-                const float x = cph * re - sph * im;
-                im = sph * re + cph * im;
-                re = x;
-            }
+            if (g.epilogue == 1) cir_rotate(ph, re, im);   // (re, im) pairs times exp(+i ph)
             if (c < g.N) C[c] = D ? D[c] - re : re;
             if (c + 1 < g.N) C[c + 1] = D ? D[c + 1] - im : im;
         }

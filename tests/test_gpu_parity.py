@@ -579,3 +579,26 @@ def test_propagate_ragged_tiles(lib, precision, tol, n, batch):
     ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F.astype(np.complex128)))
     for b in range(batch):
         assert O.rel_l2(got[b], ref[b]) < (tol or 2.0 ** -23 * (2 * np.sqrt(n) + 8)), b
+
+
+@pytest.mark.parametrize("n,steps", [(256, 150), (320, 250)])
+def test_propagate_chain_keeps_length(lib, n, steps):
+    """A long chain of plain steps neither shrinks nor stretches F: its projection on the same chain in
+    64 bits stays at one.  Rounding to nearest leaves no more than 2^-28 of a fixed sign a step
+    (1e-6 in 250); sums cut off toward zero lost 2^-23 each (3e-5)."""
+    rng = np.random.default_rng(n)
+    V = np.linalg.qr(rng.standard_normal((n, n)))[0].astype(np.float32)
+    w = rng.uniform(-400, 400, n).astype(np.float32)
+    F = np.eye(n, dtype=np.complex64)[None]
+    V64 = V.astype(np.float64)
+    ph = np.exp(1j * w.astype(np.float64) * np.float32(0.010) / HBAR)[:, None]
+    ref = F[0].astype(np.complex128)
+    mul = lambda a, z: (a @ z.view(np.float64).reshape(n, 2 * n)).view(np.complex128)
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 12) as eng:
+        for _ in range(steps):
+            F = eng.propagate(V[None], w[None], 0.010, F)
+            ref = mul(V64, np.ascontiguousarray(ph * mul(np.ascontiguousarray(V64.T), ref)))
+    got = F[0].astype(np.complex128)
+    drift = np.vdot(ref, got).real / np.vdot(ref, ref).real - 1
+    print(f"n={n}, {steps} steps: projection - 1 {drift:.1e}, relative error {O.rel_l2(got, ref):.1e}")
+    assert abs(drift) < steps * 2.0 ** -28
