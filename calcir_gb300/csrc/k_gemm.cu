@@ -7,27 +7,33 @@
 //     G  = V^T F                  (epilogue: row j of G times exp(+i w_j dt/hbar))
 //     F' = V G
 //
-// Each operand value is split into three BF16 terms, x = h + m + l (8 + 8 + 8 mantissa bits: the
-// whole of an FP32 value), and the product is six tcgen05.mma kind::f16 per 16 of K: h h into the
-// accumulator H, and h m, m h, m m, h l, l h into a second accumulator L (what is left out is
-// below 2^-24 of a product).  The tensor core drops the bits that fall below the accumulator's
-// last on every instruction, so a long sum in one accumulator drifts toward zero by half an ulp an
-// instruction; H is therefore read out every F_CHUNK slices and summed in FP32 registers with
-// rounding to nearest, and L, 2^-8 of the sum, once a tile.
+// Each operand value is split into three BF16 terms, x = h + m + l, on grids common to the 32 values
+// of a row (column) of a slice: h is x rounded to 2^(e-8), 2^e above the largest of them, m the rest
+// rounded to 2^(e-16), l what is left (the error-free splitting of Ozaki, Ogita, Oishi and Rump,
+// Numer. Algorithms 59, 2012).  The product is eight tcgen05.mma kind::f16 per 16 of K: h h into
+// the accumulator H, and h m, m h, m m, h l, l h, m l, l m into a second accumulator L (l l, below
+// 2^-34 of the slices' largest product, is left out).  The tensor core drops the bits that fall below the
+// accumulator's last on every instruction, always toward zero.  In H there are none: h is at most
+// 256 steps of its grid, 32 products at most 2^21 steps of theirs, so a slice's sum is exact; H
+// is read out every slice and summed in FP32 registers with rounding to nearest.  L, 2^-8 of the sum
+// and of no fixed sign against it, is read out once a tile.  (With h, m, l rounded value by value the
+// sums of h h lost a part of a bit every instruction: F shrank by 1.3e-7 a step, 1.9e-5 in 146 steps of
+// 244 chromophores.)
 //
 // One CTA per SM walks 128 x 128 tiles (column tile fastest, then row tile, then matrix):
 //   warps 0-7   copy FP32 slices 32 deep (0-3 A, 4-7 B) into shared memory, F_RAW slices ahead,
 //               split them and store the three terms K-major (core matrices of 8 rows x 16 bytes,
 //               (r/8, k/8) at (r/8)*SBO + (k/8)*LBO; SBO padded so that either orientation stores
 //               without bank conflicts) into a ring;
-//   warps 8-15  sum the chunks (a thread a row and half of the columns), then the epilogue, while
+//   warps 8-15  sum the slices (a thread a row and half of the columns), then the epilogue, while
 //               the next tile is loaded and multiplied (two H and two L accumulators, all 512
 //               columns of tensor memory);
 //   warp 16     issues the MMAs.
-// The splitting bounds it (the six MMAs of 16 K take half of a slice's time).  1024 x 2048 x 1024
-// in ten matrices: 859-1044 us as SIMT FFMAs (50-41 TFLOP/s), 306-380 with the next slice in
-// registers, 283-331 so (152-130), relative error against 64 bits 5.5e-7 before, 1.2e-7 so.  Not
-// taken: 16 splitting warps (403-432: the copies of 8 bytes that rows contiguous then need).  Products with too few
+// The splitting bounds it (with the two products of m and l left out 314-391 us below, without the
+// slices' maxima 303-361).  1024 x 2048 x 1024 in ten matrices: 859-1044 us as SIMT FFMAs (50-41
+// TFLOP/s), 323-386 so (133-111), error against 64 bits 5.7e-7 and 6e-8; with the terms rounded
+// value by value and six products 283-331 us, 1.2e-7 and the drift above.  Not taken: 16 splitting
+// warps (403-432: the copies of 8 bytes that rows contiguous then need).  Products with too few
 // tiles for the SMs run on the SIMT kernel further down (gemm_small_wins).
 // Every wait is bounded: a timeout raises the CTA's abort flag and the error flag, every role
 // leaves its loop, and the MMAs issued are waited for before the tensor memory is freed.
@@ -45,7 +51,6 @@ constexpr int FM = 128, FN = 128, FK = 32;     // tile, K of a slice
 constexpr int F_LBO = 128, F_SBO = 528;
 constexpr int F_PART = (FM / 8) * F_SBO;       // bytes of one term of one operand's slice
 constexpr int F_STAGE = 6 * F_PART, F_NS = 3, F_RAW = 2;
-constexpr int F_CHUNK = 1;                     // slices between read-outs of H
 constexpr int F_LOAD = 8, F_ACC = 8;           // warps
 constexpr int F_NT = 32 * (F_LOAD + F_ACC + 4);   // whole warpgroups: the register split is per group
 constexpr size_t F_RAWB = (size_t)F_LOAD * 32 * 128;   // bytes of an FP32 slice of both operands
@@ -63,19 +68,44 @@ __device__ __forceinline__ void mbar_arrive1(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
-// the three BF16 terms of eight values, as 16-byte words
-__device__ __forceinline__ void split3(const float (&x)[8], uint4 &h, uint4 &m, uint4 &l) {
+// The constants that round to the grids 2^(e-8) and 2^(e-16) by being added and taken away, 2^e the
+// power of two above mx: 1.5 * 2^(e+15) and 1.5 * 2^(e+7).  Within e's range below the grids are BF16 numbers
+// and the constants finite.
+__device__ __forceinline__ float2 split_grids(float mx) {
+    const uint32_t e = min(max(__float_as_uint(mx) & 0x7f800000u, 10u << 23), 238u << 23);
+    return make_float2(__uint_as_float(e + ((16u << 23) | 0x400000u)), __uint_as_float(e + ((8u << 23) | 0x400000u)));
+}
+
+// two FP32 operations an instruction
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {   // a - b
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+    return r;
+}
+
+// the three BF16 terms of eight values on the grids c, as 16-byte words
+__device__ __forceinline__ void split3(const float (&x)[8], float2 c, uint4 &h, uint4 &m, uint4 &l) {
+    const uint64_t ch = pair_of(c.x, c.x), chn = pair_of(-c.x, -c.x), cm = pair_of(c.y, c.y), cmn = pair_of(-c.y, -c.y);
     uint32_t wh[4], wm[4], wl[4];
     #pragma unroll
     for (int q = 0; q < 4; q++) {
-        const float a = x[2 * q], b = x[2 * q + 1];
-        const __nv_bfloat162 ph = __floats2bfloat162_rn(a, b);
-        wh[q] = *reinterpret_cast<const uint32_t *>(&ph);
-        const float ra = a - __uint_as_float(wh[q] << 16), rb = b - __uint_as_float(wh[q] & 0xffff0000u);
-        const __nv_bfloat162 pm = __floats2bfloat162_rn(ra, rb);
-        wm[q] = *reinterpret_cast<const uint32_t *>(&pm);
-        const __nv_bfloat162 pl = __floats2bfloat162_rn(ra - __uint_as_float(wm[q] << 16),
-                                                        rb - __uint_as_float(wm[q] & 0xffff0000u));
+        const uint64_t v = pair_of(x[2 * q], x[2 * q + 1]);
+        const uint64_t hv = add2(add2(v, ch), chn), r = sub2(v, hv);
+        const uint64_t mv = add2(add2(r, cm), cmn), lv = sub2(r, mv);
+        // h and m have eight significant bits: their upper halves are the BF16 numbers
+        wh[q] = __byte_perm((uint32_t)hv, (uint32_t)(hv >> 32), 0x7632);
+        wm[q] = __byte_perm((uint32_t)mv, (uint32_t)(mv >> 32), 0x7632);
+        const __nv_bfloat162 pl = __floats2bfloat162_rn(__uint_as_float((uint32_t)lv), __uint_as_float((uint32_t)(lv >> 32)));
         wl[q] = *reinterpret_cast<const uint32_t *>(&pl);
     }
     h = make_uint4(wh[0], wh[1], wh[2], wh[3]);
@@ -86,7 +116,8 @@ __device__ __forceinline__ void split3(const float (&x)[8], uint4 &h, uint4 &m, 
 // One thread's part of an operand slice (128 rows of the M or N dimension, 32 of K): four groups
 // of eight consecutive K of one row.  KC: K contiguous in memory (element (r, k) at p[r*ld + k]),
 // group i is row 32 i + 8 (warp & 3) + (lane & 7), K 8 (lane >> 3) ..; else rows contiguous
-// (element (r, k) at p[k*ld + r]), the groups are rows 4 lane .. + 3, K 8 (warp & 3) ...
+// (element (r, k) at p[k*ld + r]), group i is row 32 (warp & 3) + 4 (lane & 7) + i, K 8 (lane >> 3) ...
+// Either way four lanes of a warp, 8 apart, hold the 32 values of a row.
 // The values wait in shared memory, each thread's own eight 16-byte words (raw, RAW_ST apart),
 // which no other thread reads: an asynchronous copy needs no register and no barrier.
 constexpr int RAW_ST = F_LOAD * 32 * 16;
@@ -111,7 +142,7 @@ struct Part {
                                                 int w4, int lane, bool vec) {
         if (vec && r0 + 128 <= rdim && k0 + 32 <= kdim) {   // the whole slice inside
             const float *q = KC ? p + (size_t)(r0 + 8 * w4 + (lane & 7)) * ld + k0 + 8 * (lane >> 3)
-                                : p + (size_t)(k0 + 8 * w4) * ld + r0 + 4 * lane;
+                                : p + (size_t)(k0 + 8 * (lane >> 3)) * ld + r0 + 32 * w4 + 4 * (lane & 7);
             const size_t st = KC ? (size_t)32 * ld : (size_t)ld;
             #pragma unroll
             for (int i = 0; i < 8; i++)
@@ -128,10 +159,10 @@ struct Part {
                 load4(raw + (2 * i + 1) * RAW_ST, q + 4, have - 4, p, vec);
             }
         } else {
-            const int r = r0 + 4 * lane;
+            const int r = r0 + 32 * w4 + 4 * (lane & 7);
             #pragma unroll
             for (int i = 0; i < 8; i++) {
-                const int k = k0 + 8 * w4 + i;
+                const int k = k0 + 8 * (lane >> 3) + i;
                 load4(raw + i * RAW_ST, p + (size_t)k * ld + r, k < kdim ? rdim - r : 0, p, vec);
             }
         }
@@ -151,11 +182,16 @@ struct Part {
             } else {
                 #pragma unroll
                 for (int q = 0; q < 8; q++) x[q] = i == 0 ? v[q].x : i == 1 ? v[q].y : i == 2 ? v[q].z : v[q].w;
-                const int r = 4 * lane + i;
-                o = (r >> 3) * F_SBO + w4 * F_LBO + (r & 7) * 16;
+                const int r = 32 * w4 + 4 * (lane & 7) + i;
+                o = (r >> 3) * F_SBO + (lane >> 3) * F_LBO + (r & 7) * 16;
             }
+            float mx = 0.f;
+            #pragma unroll
+            for (int q = 0; q < 8; q++) mx = fmaxf(mx, fabsf(x[q]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
             uint4 h, m, l;
-            split3(x, h, m, l);
+            split3(x, split_grids(mx), h, m, l);
             *reinterpret_cast<uint4 *>(base + o) = h;
             *reinterpret_cast<uint4 *>(base + F_PART + o) = m;
             *reinterpret_cast<uint4 *>(base + 2 * F_PART + o) = l;
@@ -173,7 +209,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + (size_t)F_NS * F_STAGE + F_RAW * F_RAWB);   // [F_NS]
     uint64_t *empty = full + F_NS;                                                 // [F_NS]
-    uint64_t *hfull = empty + F_NS;                                                // [2] chunk in H
+    uint64_t *hfull = empty + F_NS;                                                // [2] slice in H
     uint64_t *hempty = hfull + 2;                                                  // [2]
     uint64_t *lempty = hempty + 2;                                                 // [2] L read out
     uint64_t *drain = lempty + 2;
@@ -202,7 +238,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
-    const int KT = (g.K + FK - 1) / FK, NC = (KT + F_CHUNK - 1) / F_CHUNK;   // slices, chunks of a tile
+    const int KT = (g.K + FK - 1) / FK;      // slices of a tile
     auto fail = [&]() {
         *abort_flag = 1;
         if (err) atomicExch(err, 1);
@@ -265,7 +301,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
         regs_down<24>();
         if (warp == F_LOAD + F_ACC && lane == 0) {
             constexpr uint32_t IDESC = make_idesc_mn(1u, FM, FN);
-            uint32_t it = 0, ch = 0;      // slices and chunks issued
+            uint32_t it = 0;              // slices issued
             bool ok = true, issued = false;
             int li = 0;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, li++) {
@@ -273,9 +309,9 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                 if (li >= 2 && !(ok = mbar_wait(&lempty[a], ((li >> 1) & 1) ^ 1))) break;
                 const uint32_t dl = tmem + 256 + 128 * a;
                 for (int kt = 0; kt < KT && ok; kt++, it++) {
-                    const int s = it % F_NS, hb = ch & 1;
+                    const int s = it % F_NS, hb = it & 1;
                     const uint32_t dh = tmem + 128 * hb;
-                    if (kt % F_CHUNK == 0 && ch >= 2 && !(ok = mbar_wait(&hempty[hb], ((ch >> 1) & 1) ^ 1))) break;
+                    if (it >= 2 && !(ok = mbar_wait(&hempty[hb], ((it >> 1) & 1) ^ 1))) break;
                     if (!(ok = mbar_wait(&full[s], (it / F_NS) & 1))) break;
                     if (*abort_flag) { ok = false; break; }
                     fence_after();
@@ -285,8 +321,10 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                         const uint32_t o = st + 2 * ks * F_LBO;
                         const uint64_t ah = f_desc(o), am = f_desc(o + F_PART), al = f_desc(o + 2 * F_PART);
                         const uint64_t bh = f_desc(o + 3 * F_PART), bm = f_desc(o + 4 * F_PART), bl = f_desc(o + 5 * F_PART);
-                        mma_f16(dh, ah, bh, IDESC, (kt % F_CHUNK | ks) != 0);
-                        mma_f16(dl, ah, bl, IDESC, (kt | ks) != 0);
+                        mma_f16(dh, ah, bh, IDESC, ks != 0);
+                        mma_f16(dl, am, bl, IDESC, (kt | ks) != 0);
+                        mma_f16(dl, al, bm, IDESC, 1u);
+                        mma_f16(dl, ah, bl, IDESC, 1u);
                         mma_f16(dl, al, bh, IDESC, 1u);
                         mma_f16(dl, am, bm, IDESC, 1u);
                         mma_f16(dl, ah, bm, IDESC, 1u);
@@ -294,10 +332,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                     }
                     issued = true;
                     mma_commit(&empty[s]);
-                    if (kt % F_CHUNK == F_CHUNK - 1 || kt == KT - 1) {
-                        mma_commit(&hfull[hb]);
-                        ch++;
-                    }
+                    mma_commit(&hfull[hb]);
                 }
             }
             if (!ok) fail();
@@ -311,7 +346,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
         regs_up<104>();
         const int quarter = warp & 3, half = (warp - F_LOAD) >> 2, row = quarter * 32 + lane;
         const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + 64 * half;
-        uint32_t ch = 0;
+        uint32_t it = 0;
         int li = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, li++) {
@@ -329,9 +364,9 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                 if (c < g.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(D + c));
                 if (c + 32 < g.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(D + c + 32));
             }
-            for (int c = 0; c < NC; c++, ch++) {
-                const int hb = ch & 1;
-                if (!(ok = warp_agrees(mbar_wait(&hfull[hb], (ch >> 1) & 1) && !*abort_flag))) break;
+            for (int kt = 0; kt < KT; kt++, it++) {
+                const int hb = it & 1;
+                if (!(ok = warp_agrees(mbar_wait(&hfull[hb], (it >> 1) & 1) && !*abort_flag))) break;
                 fence_after();
                 #pragma unroll
                 for (int h = 0; h < 4; h++) {
@@ -550,16 +585,16 @@ __global__ void __launch_bounds__(64 * KS) k_gemm_small(GemmArgs g, bool vecA, b
 // 16.5, 20.9).
 bool small_split(long long blocks, int K, int sms) { return K > SB && blocks <= 4LL * sms; }
 
-// Which of the two is faster, from fits in us to all three over M 54..2048, K 54..2048: 8 + 1.1 per
+// Which of the two is faster, from fits in us to all three over M 54..2048, K 54..2048: 8 + 1.3 per
 // 32 of K and wave of tiles for the tensor cores, 4 + (0.75 + 0.3 blocks an SM) per 32 of K for one
 // group, 4.2 + max(2.05, 1.9 blocks an SM) per 128 of K for four.  Measured, small against tensor
-// cores: 128 x 256 x 128 6.2 / 12.5, 512 x 18 x 512 in four matrices 12.5 / 32.8, 2048 x 128 x 2048
-// 58 / 100; 256 x 512 x 256 in four 18.7 / 16.6, 512 x 1024 x 512 29 / 25, 1024 x 2048 x 1024 158 / 43.
+// cores: 128 x 256 x 128 6.2 / 13, 512 x 18 x 512 in four matrices 12.5 / 35, 256 x 512 x 256 in four
+// 18.6 / 19.2; 512 x 1024 x 512 28.8 / 28.9, 300 x 600 x 300 in twenty 96 / 45, 1024 x 2048 x 1024 152 / 49.
 bool gemm_small_wins(const GemmArgs &g, long long tiles, long long blocks, int sms) {
     const double kt = (g.K + 31) / 32, waves = (double)((tiles + sms - 1) / sms), per = (double)blocks / sms;
     const double small = small_split(blocks, g.K, sms) ? 4.2 + ((g.K + 127) / 128) * std::max(2.05, 1.9 * per)
                                                        : 4.0 + kt * (0.75 + 0.3 * per);
-    return small < 8.0 + 1.1 * kt * waves;
+    return small < 8.0 + 1.3 * kt * waves;
 }
 
 __global__ void k_identity(float *F, int n, int ldf, long long sF) {

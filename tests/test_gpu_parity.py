@@ -581,7 +581,7 @@ def test_propagate_ragged_tiles(lib, precision, tol, n, batch):
         assert O.rel_l2(got[b], ref[b]) < (tol or 2.0 ** -23 * (2 * np.sqrt(n) + 8)), b
 
 
-@pytest.mark.parametrize("n,steps", [(256, 150), (320, 250)])
+@pytest.mark.parametrize("n,steps", [(256, 150), (320, 250), (512, 150), (1024, 250)])
 def test_propagate_chain_keeps_length(lib, n, steps):
     """A long chain of plain steps neither shrinks nor stretches F: its projection on the same chain in
     64 bits stays at one.  Rounding to nearest leaves no more than 2^-28 of a fixed sign a step
@@ -602,3 +602,21 @@ def test_propagate_chain_keeps_length(lib, n, steps):
     drift = np.vdot(ref, got).real / np.vdot(ref, ref).real - 1
     print(f"n={n}, {steps} steps: projection - 1 {drift:.1e}, relative error {O.rel_l2(got, ref):.1e}")
     assert abs(drift) < steps * 2.0 ** -28
+
+
+@pytest.mark.parametrize("n,batch", [(256, 24), (509, 2), (640, 1)])
+def test_propagate_graded(lib, n, batch):
+    """Rows and columns of F over nine orders of magnitude: every column is as exact as one of
+    equal elements (the bound of test_propagate_forms)."""
+    rng = np.random.default_rng(n)
+    V = np.stack([np.linalg.qr(rng.standard_normal((n, n)))[0] for _ in range(batch)]).astype(np.float32)
+    w = rng.uniform(-400, 400, (batch, n)).astype(np.float32)
+    F = rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))
+    F = (F * 10.0 ** rng.uniform(-9, 0, (batch, n, 1)) * 10.0 ** rng.uniform(-9, 0, (batch, 1, n))).astype(np.complex64)
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 12) as eng:
+        got = eng.propagate(V, w, 0.1, F)
+    V64 = V.astype(np.float64)
+    phase = np.exp(1j * w.astype(np.float64) * np.float32(0.1) / HBAR)
+    ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F.astype(np.complex128)))
+    err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < 2.0 ** -23 * (2 * np.sqrt(n) + 8)
