@@ -634,6 +634,7 @@ static int propagate_dev(cir_ctx *c, int nprop, int n, const float *V, int ldv, 
     g1.C = G; g1.ldc = ldf; g1.sC = sF;
     g1.M = n; g1.N = 2 * n; g1.K = n;
     g1.err = c->buf[B_ERR].as<int>();
+    g1.full_range = true;
     g1.epilogue = 1; g1.w = w; g1.wstride = wstride;
     g1.dt_over_hbar = (float)(dt / CIR_HBAR);
     GemmArgs g2 = g1;
@@ -1995,6 +1996,7 @@ extern "C" int cir_loss_grad(cir_ctx *c, int nframes, const float *xyz, const fl
                            step * ld, n, batch, tau, R + b0 * mstride, ld, step * mstride, c->stream));
         GemmArgs gt{};
         gt.err = c->buf[B_ERR].as<int>();
+        gt.full_range = true;
         gt.A = A + b0 * mstride; gt.lda = ld; gt.sA = step * mstride; gt.a_colmajor = true;   // V
         gt.B = R + b0 * mstride; gt.ldb = ld; gt.sB = step * mstride;
         gt.C = T + b0 * mstride; gt.ldc = ld; gt.sC = step * mstride;

@@ -227,6 +227,8 @@ struct GemmArgs {
     long long sA, sB, sC;  // batch strides (elements)
     bool a_colmajor;
     bool b_kmajor;         // B element (k, n) at B[n*ldb + k] instead of B[k*ldb + n]
+    bool full_range;       // k_gemm: infinite, very large and very small values as exact as FFMAs (C is
+                           // neither A nor B); the eigensolver's products, of vectors, go without
     int epilogue;          // 0 none, 1 phase rotation, 2 C = D - A B
     const float *D;        // epilogue 2 (may equal C)
     int ldd;

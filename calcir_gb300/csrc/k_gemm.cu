@@ -20,6 +20,11 @@
 // sums of h h lost a part of a bit every instruction: F shrank by 1.3e-7 a step, 1.9e-5 in 146 steps of
 // 244 chromophores.)
 //
+// BF16 numbers have FP32's range, but not all three terms of a value near its ends, and infinite
+// terms do not add up.  Where the caller's values may be anything (full_range), the loaders watch the
+// largest magnitude of every row and column of a tile, and a tile with one outside F_TINY .. F_HUGE
+// is summed again by FFMAs in its epilogue.
+//
 // One CTA per SM walks 128 x 128 tiles (column tile fastest, then row tile, then matrix):
 //   warps 0-7   copy FP32 slices 32 deep (0-3 A, 4-7 B) into shared memory, F_RAW slices ahead,
 //               split them and store the three terms K-major (core matrices of 8 rows x 16 bytes,
@@ -53,6 +58,8 @@ constexpr int F_PART = (FM / 8) * F_SBO;       // bytes of one term of one opera
 constexpr int F_STAGE = 6 * F_PART, F_NS = 3, F_RAW = 2;
 constexpr int F_LOAD = 8, F_ACC = 8;           // warps
 constexpr int F_NT = 32 * (F_LOAD + F_ACC + 4);   // whole warpgroups: the register split is per group
+constexpr float F_TINY = 0x1p-110f, F_HUGE = 0x1p112f;   // below: l under BF16's smallest number; from here: grids' constants
+constexpr int F_ODD = 8;                       // tiles the loaders' notes reach back: they are at most 5 ahead of the epilogue
 constexpr size_t F_RAWB = (size_t)F_LOAD * 32 * 128;   // bytes of an FP32 slice of both operands
 constexpr size_t F_SMEM = (size_t)F_NS * F_STAGE + F_RAW * F_RAWB + 256;
 
@@ -167,7 +174,8 @@ struct Part {
             }
         }
     }
-    __device__ __forceinline__ static void store(const unsigned char *raw, unsigned char *base, int w4, int lane) {
+    // rmx: the largest magnitude so far of each group's row
+    __device__ __forceinline__ static void store(const unsigned char *raw, unsigned char *base, int w4, int lane, float (&rmx)[4]) {
         float4 v[8];
         #pragma unroll
         for (int i = 0; i < 8; i++) v[i] = *reinterpret_cast<const float4 *>(raw + i * RAW_ST);
@@ -190,6 +198,7 @@ struct Part {
             for (int q = 0; q < 8; q++) mx = fmaxf(mx, fabsf(x[q]));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            rmx[i] = fmaxf(rmx[i], mx);
             uint4 h, m, l;
             split3(x, split_grids(mx), h, m, l);
             *reinterpret_cast<uint4 *>(base + o) = h;
@@ -200,6 +209,27 @@ struct Part {
 };
 
 __device__ __forceinline__ uint64_t f_desc(uint32_t addr) { return smem_desc_kmajor(addr, F_LBO, F_SBO); }
+
+// 64 columns from c0 of row r by FFMAs (out of line: no registers of the tile's sums held for it)
+template <bool ACOL, bool BKC>
+__device__ __noinline__ void f_row_again(const GemmArgs &g, int bz, int r, int c0) {
+    const float *A = g.A + (size_t)bz * g.sA + (ACOL ? (size_t)r : (size_t)r * g.lda), *B = g.B + (size_t)bz * g.sB;
+    const size_t as = ACOL ? g.lda : 1, bs = BKC ? 1 : g.ldb, bc = BKC ? g.ldb : 1;
+    float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
+    for (int c = c0; c < min(c0 + 64, g.N); c += 2) {
+        const bool two = c + 1 < g.N;
+        const float *b = B + c * bc;
+        float re = 0.f, im = 0.f;
+        for (int k = 0; k < g.K; k++, b += bs) {
+            const float a = A[k * as];
+            re = fmaf(a, b[0], re);
+            if (two) im = fmaf(a, b[bc], im);
+        }
+        if (g.epilogue == 1) cir_rotate(cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar), re, im);
+        C[c] = re;
+        if (two) C[c + 1] = im;
+    }
+}
 
 // vecA, vecB, vecC: every 16-byte access of the operand (C and D: both) is aligned (pointer,
 // leading dimension, stride)
@@ -215,6 +245,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
     uint64_t *drain = lempty + 2;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tslot + 1);
+    volatile int *odd = abort_flag + 1;                                            // [F_ODD]: t + 1: the CTA's tile t is out of range
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == F_LOAD + F_ACC) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tslot)), "r"(512));
@@ -232,6 +263,7 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
         }
         mbar_init(drain, 1);
         *abort_flag = 0;
+        for (int i = 0; i < F_ODD; i++) odd[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     fence_before();
@@ -279,12 +311,27 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
             uint32_t it = 0;
             const uint32_t total = (uint32_t)((ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * KT;
             bool ok = true;
+            float rmx[4] = {};
+            int skt = 0, sli = 0;                // slice and tile stored
             auto step = [&] {
                 const int s = it % F_NS;
                 if (it >= F_NS && !(ok = warp_agrees(mbar_wait(&empty[s], ((it / F_NS) & 1) ^ 1)))) return;
                 if (!(ok = warp_agrees(!*abort_flag))) return;
                 asm volatile("cp.async.wait_group %0;" ::"n"(F_RAW - 1) : "memory");
-                part.store(raw + it % F_RAW * F_RAWB, smem + (size_t)s * F_STAGE + (isA ? 0 : 3 * F_PART), w4, lane);
+                part.store(raw + it % F_RAW * F_RAWB, smem + (size_t)s * F_STAGE + (isA ? 0 : 3 * F_PART), w4, lane, rmx);
+                if (++skt == KT) {
+                    if (g.full_range) {
+                        bool out = false;
+                        #pragma unroll
+                        for (int i = 0; i < 4; i++) out |= rmx[i] >= F_HUGE || (rmx[i] > 0.f && rmx[i] < F_TINY);
+                        if (out) odd[sli % F_ODD] = sli + 1;
+                        __threadfence_block();
+                    }
+                    #pragma unroll
+                    for (int i = 0; i < 4; i++) rmx[i] = 0.f;
+                    skt = 0;
+                    sli++;
+                }
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive1(&full[s]);
@@ -387,10 +434,15 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
                 #pragma unroll
                 for (int q = 0; q < 16; q++) acc[h][q] += v[q];
             }
+            const bool again = g.full_range && odd[li % F_ODD] == li + 1;
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive1(&lempty[li & 1]);
             if (r >= g.M) continue;
+            if (again) {
+                f_row_again<ACOL, BKC>(g, bz, r, n0 + 64 * half);
+                continue;
+            }
             const CirPhase ph = g.epilogue == 1 ? cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar) : CirPhase{};
             float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
             const int cb = n0 + 64 * half;

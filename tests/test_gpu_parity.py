@@ -620,3 +620,30 @@ def test_propagate_graded(lib, n, batch):
     ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F.astype(np.complex128)))
     err = np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)
     assert err.max() < 2.0 ** -23 * (2 * np.sqrt(n) + 8)
+
+
+@pytest.mark.parametrize("n,batch", [(64, 2), (300, 8), (509, 2)])
+@pytest.mark.parametrize("value", [np.inf, 2e38, 3e-36, 1e-33])
+def test_propagate_range(lib, n, batch, value):
+    """A column of F of infinite, very large or very small values beside ordinary ones, in the small
+    products and on the tensor cores: infinities come out as FP32 sums give them, the other columns'
+    errors stay those of test_propagate_forms, also where BF16 terms would run out of their range."""
+    rng = np.random.default_rng(n)
+    V = (rng.uniform(0.5, 1.0, (batch, n, n)) / n).astype(np.float32)      # positive: no Inf - Inf, no 0 * Inf
+    w = rng.uniform(50, 400, (batch, n)).astype(np.float32)                # phases in the first quadrant
+    F = (rng.uniform(0.5, 1.0, (batch, n, n)) + 0.01j).astype(np.complex64)
+    j = n // 2
+    F[:, :, j] = (value if np.isfinite(value) else 1.0) * rng.uniform(0.5, 1.0, (batch, n))
+    if not np.isfinite(value):
+        F[:, n - 1, j] = np.inf
+    with lib.Engine(lib.default_params(species="H2O", model="tip4p2005"), 12) as eng:
+        got = eng.propagate(V, w, 0.010, F)
+    keep = [c for c in range(n) if c != j or np.isfinite(value)]
+    V64 = V.astype(np.float64)
+    phase = np.exp(1j * w.astype(np.float64) * np.float32(0.010) / HBAR)
+    F64 = F[:, :, keep].astype(np.complex128)
+    ref = V64 @ (phase[:, :, None] * (V64.swapaxes(1, 2) @ F64))
+    err = np.linalg.norm(got[:, :, keep] - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() < 2.0 ** -23 * (2 * np.sqrt(n) + 8)
+    if not np.isfinite(value):
+        assert np.all(got[:, :, j].real == np.inf) and np.all(got[:, :, j].imag == np.inf)
