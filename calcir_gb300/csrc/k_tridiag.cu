@@ -163,6 +163,10 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
     auto own_row = [&](int l) { return CL ? (((l >> 5) * C + rank) << 5) + (l & 31) : l; };
 
     for (int i = tid; i < L.T; i += NT) smem[i] = 0.f;   // V, W, partial products, vectors: rows >= n stay zero
+    // and the panel's W in the scratch, read in whole tiles from the first update on but written only below
+    // each column's reflector: what a call before left there (a NaN times the zeros of c is a NaN)
+    if (CL)
+        for (int i = rank * NT + tid; i < NB * ld; i += C * NT) Wg[i] = 0.f;
     if (RES) {
         for (int J = 0, q = 0; J < tn; J++)
             for (int I = J; I < tn; I++, q++) {
@@ -240,7 +244,7 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
             for (int t = 0; t < 8; t++) yc[t] = 0.f;
             // lane (g, h): rows 32I + 4g .. + 3 of columns 32J + 8h .. + 7
             // (rows and columns past the end are read at the last ones: the zeros of c beyond row n - 1
-            // discard them)
+            // discard them, so whatever a tile can meet there has to be finite where the matrix is)
             auto load = [&](float4 (&v)[8], int I, int J) {
                 if (RES) {
                     const float *t = tile_ptr(I, J) + 4 * g + 32 * 8 * h;
