@@ -236,7 +236,8 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
         };
         if (!RES && !upd) fetch();
         mark(13);
-        // (1) y' = A c (after a panel: with its update), c.y', and the panel's dot products
+        // (1) y' = A c (after a panel: with its update), scale c.y' (c.y' itself, a product of three factors
+        // of the matrix's size, leaves FP32's range from 1e12 on), and the panel's dot products
         {
             const bool rev = (k & 1) != 0;
             float cac = 0.f, yc[8];
@@ -284,12 +285,15 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
                     if (CL) {
                         const float *vg = A + (size_t)(o0 + j) * ld, *wg = Wg + (size_t)j * ld;
                         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                        vr = r0 < n ? __ldcg(reinterpret_cast<const float4 *>(vg + r0)) : z;
-                        wr = r0 < n ? __ldcg(reinterpret_cast<const float4 *>(wg + r0)) : z;
-                        vc0 = c0 < n ? __ldcg(reinterpret_cast<const float4 *>(vg + c0)) : z;
-                        vc1 = c0 + 4 < n ? __ldcg(reinterpret_cast<const float4 *>(vg + c0 + 4)) : z;
-                        wc0 = c0 < n ? __ldcg(reinterpret_cast<const float4 *>(wg + c0)) : z;
-                        wc1 = c0 + 4 < n ? __ldcg(reinterpret_cast<const float4 *>(wg + c0 + 4)) : z;
+                        // (finished rows and columns, where V holds what the matrix does above the
+                        // reflectors, stay as they are: what is multiplied by zeros must not overflow)
+                        const bool ri = r0 >= p0 && r0 < n, c0i = c0 >= p0 && c0 < n, c4i = c0 >= p0 && c0 + 4 < n;
+                        vr = ri ? __ldcg(reinterpret_cast<const float4 *>(vg + r0)) : z;
+                        wr = ri ? __ldcg(reinterpret_cast<const float4 *>(wg + r0)) : z;
+                        vc0 = c0i ? __ldcg(reinterpret_cast<const float4 *>(vg + c0)) : z;
+                        vc1 = c4i ? __ldcg(reinterpret_cast<const float4 *>(vg + c0 + 4)) : z;
+                        wc0 = c0i ? __ldcg(reinterpret_cast<const float4 *>(wg + c0)) : z;
+                        wc1 = c4i ? __ldcg(reinterpret_cast<const float4 *>(wg + c0 + 4)) : z;
                     } else {
                         const float *vs = VS + (size_t)j * R, *ws = WS + (size_t)j * R;
                         vr = *reinterpret_cast<const float4 *>(vs + r0);
@@ -346,7 +350,7 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
                                 fmaf(c < 2 ? e2 : 0.f, xr.z, fmaf(c < 3 ? e3 : 0.f, xr.w, yc[q]))));
                     }
                 }
-                cac = fmaf(yr[0], xr.x, fmaf(yr[1], xr.y, fmaf(yr[2], xr.z, fmaf(yr[3], xr.w, cac))));
+                cac = fmaf(yr[0], scale * xr.x, fmaf(yr[1], scale * xr.y, fmaf(yr[2], scale * xr.z, fmaf(yr[3], scale * xr.w, cac))));
                 // row sums over h (lane bits 3-4): lane (g, h) keeps row 4g + h
                 #pragma unroll
                 for (int i = 0; i < 2; i++) {
@@ -376,7 +380,7 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
                 const float y = keep + __shfl_xor_sync(0xffffffffu, send, 1);
                 const int c = 32 * J + 8 * h + g;
                 ycol[c] += y;
-                cac = fmaf(y, X[c], cac);
+                cac = fmaf(y, scale * X[c], cac);
                 #pragma unroll
                 for (int t = 0; t < 8; t++) yc[t] = 0.f;
             };
@@ -490,7 +494,7 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
                 cy += __shfl_xor_sync(0xffffffffu, cy, o);
             }
             if (lane < NB) Tq[lane] = make_float4(t1, t2, w1, v1);
-            const float vay = scale * scale * (cy - 2.f * beta * y1 + beta * beta * a11);
+            const float sb = scale * beta, vay = scale * cy - sb * (2.f * scale * y1 - sb * a11);
             half = -0.5f * tk * tk * (vay - 2.f * tt);
             wk1 = tk * (scale * (y1 - beta * a11) - wk) + half;
             __syncwarp();

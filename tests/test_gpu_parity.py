@@ -647,3 +647,24 @@ def test_propagate_range(lib, n, batch, value):
     assert err.max() < 2.0 ** -23 * (2 * np.sqrt(n) + 8)
     if not np.isfinite(value):
         assert np.all(got[:, :, j].real == np.inf) and np.all(got[:, :, j].imag == np.inf)
+
+
+@pytest.mark.parametrize("n", [64, 100, 200, 300, 600])
+@pytest.mark.parametrize("scale", [1e12, 1e17])
+def test_eigh_large_matrices(lib, n, scale):
+    """Matrices whose squares are in FP32's range but whose cubes are not."""
+    A = (_sym(np.random.default_rng(n), n, 1.0) * np.float32(scale)).astype(np.float32)
+    with lib.Engine(lib.default_params(species="H2O"), 8) as eng:
+        w, V = eng.eigh(A[None])
+    _check_eig(A / np.float32(scale), w[0] / np.float32(scale), V[0])
+
+
+@pytest.mark.parametrize("n", [64, 100, 200, 300, 600])
+@pytest.mark.parametrize("coupling", [1e-18, 1e-19])
+def test_eigh_weak_couplings(lib, n, coupling):
+    """Columns so short that the square of a reflector's scale overflows."""
+    A = _sym(np.random.default_rng(n), n, coupling)
+    A[np.arange(n), np.arange(n)] = np.arange(1, n + 1)
+    with lib.Engine(lib.default_params(species="H2O"), 8) as eng:
+        w, V = eng.eigh(A[None])
+    _check_eig(A, w[0], V[0])
