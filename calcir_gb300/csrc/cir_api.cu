@@ -579,7 +579,7 @@ static int autotune_tridiag(cir_ctx *c, const EighArgs &e, int nmat) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int sample = std::min(nmat, 6 * sms);
-    if (def < 2 || sample < 2 * sms) {   // too few matrices to tell the variants apart
+    if (def < 2 || sample <= 2 * sms) {   // too few matrices to tell the variants apart
         c->tq_blocks[e.n] = 0;
         return CIR_OK;
     }
@@ -799,7 +799,9 @@ static bool eig_split_enabled() {
     return on;
 }
 
-// Thread blocks of the tridiagonalisation of order n resident at a time (one per matrix).
+// Matrices of order n that the tridiagonalisation of a large batch holds at a time, one thread block
+// each.  (Orders above 1024 run as clusters of 2 to 16 blocks: their waves divide this one.  Batches of
+// less than two waves, which the launcher may give to clusters at lower orders too, are not split.)
 static int tridiag_wave(cir_ctx *c, int n) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)

@@ -38,3 +38,21 @@ inline int cir_split_first_part(int nmat, int wave) {
     wave = std::max(1, wave);
     return nmat >= 2 * wave ? (nmat / wave - 1) * wave : 0;
 }
+
+// The tridiagonalisation's kernel, by order and number of matrices alone: what the autotuner measured
+// on other batches of that order changes neither a batch's kernel nor its bits.  Orders up to 192, and
+// up to 256 in a single wave, stay in shared memory, the more warps per matrix the fewer matrices there
+// are (n = 128: 0.25 ms a matrix in 8 warps; n = 256, 320 matrices: 2.1 ms resident, one per SM, 2.0
+// ms streaming, two per SM).  Above, two blocks of 8 warps per SM fill each other's barriers (512: 5.5
+// ms per 304 matrices, one block of 16 warps 6.3), a single wave is better off with 16 warps (3.1
+// against 3.6 ms); orders above 512 take a block of 16 warps or a cluster of them.
+enum CirTridiagForm { CIR_TRI_RES4, CIR_TRI_RES8, CIR_TRI_STREAM8, CIR_TRI_WIDE };
+inline CirTridiagForm cir_tridiag_form(int n, int nmat, int sms) {
+    if (n <= 128 && nmat > 2 * sms) return CIR_TRI_RES4;
+    if (n <= 192 || (n <= 256 && nmat <= sms)) return CIR_TRI_RES8;
+    return n <= 512 && nmat > sms ? CIR_TRI_STREAM8 : CIR_TRI_WIDE;
+}
+
+// The autotuner's blocks per SM, measured on more than two waves of one block per SM, where a batch
+// is as large; else 0, the kernel's own number.
+inline int cir_tridiag_limit(int tuned, int nmat, int sms) { return nmat > 2 * sms ? tuned : 0; }

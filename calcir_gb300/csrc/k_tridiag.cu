@@ -35,6 +35,7 @@
 // (91 ms per 608: the copies of 128-byte rows run at 24 bytes a clock), tile rows unrolled with
 // their sums in registers and packed FMAs (80 ms: the code no longer fits the registers).
 #include "cir_device.cuh"
+#include "cir_plan.h"
 #include "cir_tcgen05.cuh"
 
 #include <algorithm>
@@ -646,9 +647,6 @@ cudaError_t launch(K kern, const EighArgs &a, int nmat, int nt, bool res, int C,
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
-constexpr int TQ_RES = 192;     // orders kept in shared memory with two blocks or more per SM
-constexpr int TQ_RES1 = 256;    // and with one
-
 // clusters of C blocks (one block per SM) that run at a time; a fact of the device, asked once
 int cluster_slots(int C) {
     static std::mutex mu;
@@ -714,18 +712,17 @@ cudaError_t cir_launch_tridiag(const EighArgs &a, int nmat, cudaStream_t s) {
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    // small orders in shared memory, the more warps per matrix the fewer matrices there are
-    // (n = 128: 0.25 ms a matrix in 8 warps; n = 256, 320 matrices: 2.1 ms resident, one per SM,
-    // 2.0 ms streaming, two per SM)
-    if (a.n <= 128 && (nmat > 2 * sms || a.tq_blocks > 0)) return launch(k_tridiag<128, 4, true, false, 1>, a, nmat, 128, true, 1, 4, s);
-    if (a.n <= TQ_RES || (a.n <= TQ_RES1 && nmat <= sms))
-        return launch(k_tridiag<256, 2, true, false, 1>, a, nmat, 256, true, 1, 2, s);
-    // two blocks of 8 warps per SM fill each other's barriers (512: 5.5 ms per 304 matrices, one
-    // block of 16 warps 6.3), a single wave is better off with 16 warps (3.1 against 3.6 ms)
-    if (a.n <= 512 && nmat > sms) return launch(k_tridiag<256, 2, false, false, 1>, a, nmat, 256, false, 1, 2, s);
+    EighArgs b = a;
+    b.tq_blocks = cir_tridiag_limit(a.tq_blocks, nmat, sms);
+    switch (cir_tridiag_form(a.n, nmat, sms)) {
+    case CIR_TRI_RES4: return launch(k_tridiag<128, 4, true, false, 1>, b, nmat, 128, true, 1, 4, s);
+    case CIR_TRI_RES8: return launch(k_tridiag<256, 2, true, false, 1>, b, nmat, 256, true, 1, 2, s);
+    case CIR_TRI_STREAM8: return launch(k_tridiag<256, 2, false, false, 1>, b, nmat, 256, false, 1, 2, s);
+    case CIR_TRI_WIDE: break;
+    }
     const int C = cluster_size(a.n, nmat, sms);
-    if (C > 1) return launch(k_tridiag<512, 1, false, true, 2>, a, nmat, 512, false, C, 1, s);
-    return launch(k_tridiag<512, 1, false, false, 2>, a, nmat, 512, false, 1, 1, s);
+    if (C > 1) return launch(k_tridiag<512, 1, false, true, 2>, b, nmat, 512, false, C, 1, s);
+    return launch(k_tridiag<512, 1, false, false, 2>, b, nmat, 512, false, 1, 1, s);
 }
 
 cudaError_t cir_launch_tridiag_multi(const EighArgs *a, const int *nmat, int np, cudaStream_t s, int *launches) {

@@ -198,3 +198,21 @@ def test_run_multi_joint_tridiagonalisation_matches_single_runs(lib):
         with lib.Engine(p, xyz.shape[1]) as eng:
             single = eng.run(xyz, box, fos)
         _same(multi[i], single, 1e-5, f"trajectory {i} ({sizes[i]} molecules), joint tridiagonalisation")
+
+
+@pytest.mark.parametrize("nmol", [40, 64, 100])
+def test_small_batch_after_a_tuned_one(lib, nmol):
+    """A small job after a large one of the same order that the autotuner measured gives the same
+    eigenpairs' densities as in a context of its own, to the last bit."""
+    _, p = _params(lib, nsamples=40, ntcfpoints=2, autotune=1)
+    fos = (np.arange(40)[:, None] + np.arange(2)[None, :]).astype(np.int32).ravel()
+    xyz, box = lib.synth_trajectory(nmol, 41, seed=nmol)
+    bx = np.tile(np.asarray(box, np.float32), (41, 1))
+    traj = (xyz, bx, fos)
+    with lib.Engine(p, xyz.shape[1]) as eng:
+        eng.run_multi([traj] * 5)                     # 400 matrices in one batch
+        after = eng.run_multi([traj])[0]              # 80
+    with lib.Engine(p, xyz.shape[1]) as eng:
+        alone = eng.run_multi([traj])[0]
+    np.testing.assert_array_equal(after["sw"], alone["sw"])
+    np.testing.assert_array_equal(after["pw"], alone["pw"])

@@ -69,3 +69,39 @@ def test_split_first_part_is_whole_waves_but_the_last(planner):
     assert res[1][1] == 0            # fewer than two waves: one stream
     assert res[2][1] == 456
     assert res[3][1] == 912          # order 2048, two blocks per SM
+
+
+FORM_DRIVER = r"""
+#include <cstdio>
+#include "cir_plan.h"
+int main() {
+    int n, nmat, tuned;
+    while (std::scanf("%d %d %d", &n, &nmat, &tuned) == 3)
+        std::printf("%d %d\n", (int)cir_tridiag_form(n, nmat, 152), cir_tridiag_limit(tuned, nmat, 152));
+    return 0;
+}
+"""
+
+
+def test_tridiagonalisation_form(tmp_path):
+    """The kernel follows from the order and the number of matrices; what the autotuner found for an
+    order limits the blocks per SM of batches of the size it measured, and of no smaller ones."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no host C++ compiler")
+    src, exe = str(tmp_path / "form.cpp"), str(tmp_path / "form")
+    with open(src, "w") as f:
+        f.write(FORM_DRIVER)
+    subprocess.run([cxx, "-std=c++17", "-O1", "-I", HEADER_DIR, src, "-o", exe], check=True)
+
+    def run(cases):
+        inp = "".join("%d %d %d\n" % c for c in cases)
+        out = subprocess.run([exe], input=inp, capture_output=True, text=True, check=True).stdout.split()
+        return [(int(out[2 * i]), int(out[2 * i + 1])) for i in range(len(cases))]
+    forms = [((3, 1), 1), ((128, 304), 1), ((128, 305), 0), ((129, 305), 1), ((192, 1000), 1), ((193, 152), 1),
+             ((193, 153), 2), ((256, 152), 1), ((257, 152), 3), ((257, 153), 2), ((512, 153), 2), ((512, 152), 3),
+             ((513, 1000), 3), ((2048, 1), 3)]
+    for tuned in (0, 1, 3):
+        for ((n, nmat), form), (got, limit) in zip(forms, run([(n, nmat, tuned) for (n, nmat), _ in forms])):
+            assert got == form, (n, nmat, tuned)
+            assert limit == (tuned if nmat > 304 else 0)
