@@ -3,10 +3,16 @@
 #ifndef CIR_TCF_CUH_
 #define CIR_TCF_CUH_
 
+#include <float.h>
+
 namespace {
 
-// A sum held as an unevaluated pair of floats (Knuth's two-sum): 48 bits, on the FP32 pipe.  In
-// double the eight sums of a warp (40 adds, 16 clocks each for the warp) were most of the kernel.
+// A sum held as an unevaluated pair of floats (Knuth's two-sum), on the FP32 pipe: in double the eight
+// sums of a warp (40 adds, 16 clocks each for the warp) were most of the kernel.  48 bits for sums of FP32
+// products: IR, VV and VH of random F, against 64 bits and relative to the vectors' norms, 3.1e-9,
+// 7.5e-10 and 4.2e-10 at order 100, 1.8e-9, 4.0e-10 and 1.8e-10 at 2048 (with sums in double, in
+// the order of the rows, 4.1e-9, 1.2e-9 and 5.4e-10; 2.0e-9, 4.6e-10 and 1.8e-10): the products' rounding.
+// hi is the plain FP32 sum; where it is not finite, lo is NaN and hi is the sum (pair_value).
 struct Pair {
     float hi, lo;
 };
@@ -17,8 +23,10 @@ __device__ __forceinline__ Pair pair_add(Pair a, float x) {
 __device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
     Pair r = pair_add(a, b.hi);
     r.lo = __fadd_rn(r.lo, b.lo);
-    const float s = __fadd_rn(r.hi, r.lo);
-    return {s, __fsub_rn(r.lo, __fsub_rn(s, r.hi))};
+    return r;
+}
+__device__ __forceinline__ double pair_value(Pair a) {
+    return (double)a.hi + (fabsf(a.hi) <= FLT_MAX ? (double)a.lo : 0.0);
 }
 __device__ __forceinline__ Pair pair_xor(Pair a, int o) {
     return {__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
@@ -52,7 +60,7 @@ __device__ __forceinline__ double tcf_reduce(Pair (&acc)[8]) {
     }
     acc[0] = pair_add(acc[0], pair_xor(acc[0], 2));
     acc[0] = pair_add(acc[0], pair_xor(acc[0], 1));
-    return (double)acc[0].hi + (double)acc[0].lo;
+    return pair_value(acc[0]);
 }
 
 // a warp whose lane l < 8 holds sum l adds IR, VV, VH (re, im) to out

@@ -668,3 +668,26 @@ def test_eigh_weak_couplings(lib, n, coupling):
     with lib.Engine(lib.default_params(species="H2O"), 8) as eng:
         w, V = eng.eigh(A[None])
     _check_eig(A, w[0], V[0])
+
+
+@pytest.mark.parametrize("n", [40, 129, 400, 1030])
+def test_tcf_terms_infinite(lib, n):
+    """An infinite dipole gives an infinite IR term, and the other terms as without it (2^-23 sqrt(n)
+    for psi and its product with m(t), all terms being positive; five roundings more in VV)."""
+    rng = np.random.default_rng(n)
+    F = (rng.uniform(0.5, 1, (n, n)) + 1j * rng.uniform(0.5, 1, (n, n))).astype(np.complex64)
+    d0, d1 = rng.uniform(0.5, 1, (2, 3, n)).astype(np.float32)
+    p0, p1 = rng.uniform(0.5, 1, (2, 6, n)).astype(np.float32)
+    d1[1, n // 2] = np.inf
+    with lib.Engine(lib.default_params(species="H2O"), 8) as eng:
+        out = np.zeros(6)      # (the wrapper's a + 1j b makes a NaN of an infinite b)
+        lib.check(eng.lib.cir_tcf_terms(eng.h, n, *[lib.ptr(x) for x in (F.view(np.float32), d0, p0, d1, p1, out)]))
+    assert out[0] == np.inf and out[1] == np.inf
+    vv, vh = out[2] + 1j * out[3], out[4] + 1j * out[5]
+    psi = F.astype(np.complex128) @ p0.astype(np.float64).T          # [n][6]
+    P = p1.astype(np.float64) @ psi                                    # [b][a] = m_b . psi_a
+    ii, ij = P[0, 0] + P[1, 1] + P[2, 2], P[3, 3] + P[4, 4] + P[5, 5]
+    jj = P[:3, :3].sum() - ii
+    tol = 2.0 ** -23 * (np.sqrt(n) + 5)
+    assert abs(vv - (3 * ii + jj + 4 * ij) / 15) < tol * abs(vv)
+    assert abs(vh - (2 * ii - jj + 6 * ij) / 30) < tol * abs(vv)
