@@ -85,8 +85,7 @@ struct cir_ctx {
     cir_stats stats;
     cudaEvent_t ev[8];
     CirMaps maps;
-    LsRows ls;                            // printed lineshape rows and their frequencies
-    std::vector<float> ls_omega;
+    LsRows ls;                            // printed lineshape rows
     // autotuner, mixed forms: tile width of each split-BF16 product shape (M, N, K, batch,
     // epilogue, output form, fused contraction) and tridiagonalisation blocks per SM per order
     std::map<std::tuple<int, int, int, int, int, int, int>, int> split_tile;
@@ -205,19 +204,24 @@ static bool all_finite(const float *x, size_t n) {
     return true;
 }
 
+// Frequency of output i of the transform as the two parts of the selection print it
+static float ls_freq1(const cir_params *p, float factor, int i) { return -1 * (i - p->ntcfpoints - p->nzeros) * factor + p->avef; }
+static float ls_freq2(const cir_params *p, float factor, int i) { return -1 * i * factor + p->avef; }
+static float ls_factor(const cir_params *p) {
+    return (float)(2 * CIR_PI * CIR_HBAR / (p->dt * (float)(p->ntcfpoints + p->nzeros)));
+}
+
 // The rows of the three lineshape files (calcIR.cu:890-919).  Each part of the selection runs
 // over falling frequencies, so it keeps an end of its range: the first from i0 up, the second
-// below cnt2.  Fixed by the parameters: made once per context, with their frequencies.
-static LsRows ls_rows(const cir_params *p, std::vector<float> &omega) {
+// below cnt2.  Fixed by the parameters: made once per context.
+static LsRows ls_rows(const cir_params *p) {
     const int n = p->ntcfpoints + p->nzeros;
-    const float factor = (float)(2 * CIR_PI * CIR_HBAR / (p->dt * (float)n));
+    const float factor = ls_factor(p);
     LsRows r{n, n, 0, 0, factor * (float)n};
-    auto freq1 = [&](int i) { return -1 * (i - p->ntcfpoints - p->nzeros) * factor + p->avef; };
-    auto freq2 = [&](int i) { return -1 * i * factor + p->avef; };
     int lo = n / 2, hi = n;                       // the first i with freq1(i) <= omegaStop
     while (lo < hi) {
-        const int mid = (lo + hi) / 2;
-        if (freq1(mid) <= (float)p->omegaStop) hi = mid;
+        const int mid = lo + (hi - lo) / 2;
+        if (ls_freq1(p, factor, mid) <= (float)p->omegaStop) hi = mid;
         else lo = mid + 1;
     }
     r.i0 = lo;
@@ -225,15 +229,19 @@ static LsRows ls_rows(const cir_params *p, std::vector<float> &omega) {
     lo = 0;                                       // the first i with freq2(i) < omegaStart
     hi = p->ntcfpoints + p->nzeros / 2;
     while (lo < hi) {
-        const int mid = (lo + hi) / 2;
-        if (freq2(mid) >= (float)p->omegaStart) lo = mid + 1;
+        const int mid = lo + (hi - lo) / 2;
+        if (ls_freq2(p, factor, mid) >= (float)p->omegaStart) lo = mid + 1;
         else hi = mid;
     }
     r.cnt2 = lo;
-    omega.resize(r.cnt1 + r.cnt2);
-    for (int i = 0; i < r.cnt1; i++) omega[i] = freq1(r.i0 + i);
-    for (int i = 0; i < r.cnt2; i++) omega[r.cnt1 + i] = freq2(i);
     return r;
+}
+
+// their frequencies
+static void ls_omega(const cir_params *p, const LsRows &r, float *omega) {
+    const float factor = ls_factor(p);
+    for (int i = 0; i < r.cnt1; i++) omega[i] = ls_freq1(p, factor, r.i0 + i);
+    for (int i = 0; i < r.cnt2; i++) omega[r.cnt1 + i] = ls_freq2(p, factor, i);
 }
 
 extern "C" int cir_create(const cir_params *p, int natoms, cir_ctx **out) {
@@ -260,7 +268,7 @@ extern "C" int cir_create(const cir_params *p, int natoms, cir_ctx **out) {
     c->n = n;
     c->ld = (n + 3) & ~3;
     cir_maps(q.map, q.ispecies, &c->maps);
-    c->ls = ls_rows(&c->p, c->ls_omega);
+    c->ls = ls_rows(&c->p);
     memset(&c->stats, 0, sizeof c->stats);
     cudaError_t e = cudaGetDevice(&c->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
@@ -750,7 +758,7 @@ extern "C" int cir_lineshape(cir_ctx *c, const double *tcf, float *omega, float 
     const int cnt = r.cnt1 + r.cnt2;
     int rc = lineshape_dev(c, tcf, 1, r);
     if (rc) return rc;
-    if (omega && cnt) memcpy(omega, c->ls_omega.data(), (size_t)cnt * 4);   // while the kernel runs
+    if (omega) ls_omega(&c->p, r, omega);         // while the kernel runs
     if (intensity && cnt)
         CK(cudaMemcpyAsync(intensity, c->buf[B_FFTY].p, (size_t)cnt * 4, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1362,7 +1370,7 @@ struct GroupJob {
                 if (r->rmw) r->rmw[i] = ((float)(mipr_t[i] / p.omegaStep) / norm) / pw;
             }
             r->nls = nls;
-            if (r->ls_omega && nls) memcpy(r->ls_omega, c->ls_omega.data(), (size_t)nls * 4);
+            if (r->ls_omega) ls_omega(&p, lr, r->ls_omega);
             r->bins_out_of_range = (long long)oor[tr];
             r->frame_steps_per_s = ms_total > 0 ? steps / (ms_total * 1e-3) : 0.0;
         }

@@ -691,3 +691,22 @@ def test_tcf_terms_infinite(lib, n):
     tol = 2.0 ** -23 * (np.sqrt(n) + 5)
     assert abs(vv - (3 * ii + jj + 4 * ij) / 15) < tol * abs(vv)
     assert abs(vh - (2 * ii - jj + 6 * ij) / 30) < tol * abs(vv)
+
+
+@pytest.mark.parametrize("start,stop", [(2000, 5000), (3415, 3415), (3000, 3200), (3600, 3700), (6000, 7000), (1, 900)])
+def test_lineshape_rows(lib, start, stop):
+    """The rows selected, for windows about, beside and beyond the axis, are those of cir_result_sizes."""
+    p = lib.default_params(species="H2O", ntcfpoints=150, nzeros=2500, omegaStart=start, omegaStop=stop, avef=3415.0)
+    prm = {"ntcfpoints": 150, "nzeros": 2500, "dt": 0.010, "avef": 3415.0, "omegaStart": start, "omegaStop": stop}
+    tcf = np.exp(-np.arange(150) / 40.0) * (1 + 1j)
+    with lib.Engine(p, 8) as eng:
+        om, _ = eng.lineshape(tcf)
+    ref, _ = O.lineshape_rows(prm, O.c2r(tcf, 2650))
+    assert len(om) == lib.result_sizes(p)[2]
+    np.testing.assert_array_equal(om, ref.astype(np.float32))
+
+
+def test_create_with_very_long_padding(lib):
+    """A context for a transform of more than 2^30 points is made without working through them."""
+    with lib.Engine(lib.default_params(species="H2O", nzeros=1_900_000_000), 8):
+        pass
