@@ -11,6 +11,8 @@
 #define CIR_PI          3.14159265359
 #define CIR_BOHR_NM     18.8973f         // bohr per nm
 #define CIR_CM_HARTREE  2.1947463E5f     // cm^-1 per hartree
+// dipole coupling of distances in nm, cm^-1 nm^3: the two above in one rounding
+#define CIR_TDC ((float)((double)CIR_CM_HARTREE / ((double)CIR_BOHR_NM * (double)CIR_BOHR_NM * (double)CIR_BOHR_NM)))
 #define CIR_CUTOFF      0.7831f          // nm, O(m) .. H(n) cutoff of the field sum
 #define CIR_TDM_OFFSET  0.067f           // nm, transition dipole position along OH
 #define CIR_OM_TIP4P    0.0150f          // nm, M-site distance used with imodel 1

@@ -162,11 +162,11 @@ __device__ __forceinline__ float tdc_kappa(const float3 &t, const float3 &u, con
     float dx = t.x - o[0], dy = t.y - o[1], dz = t.z - o[2];
     if (QUICK) ok &= cir_mi3_quick(dx, dy, dz, b.x, b.y, b.z, rb.x, rb.y, rb.z);
     else cir_mi3(dx, dy, dz, b.x, b.y, b.z, rb.x, rb.y, rb.z);
-    const float ir = cir_rsqrt(dx * dx + dy * dy + dz * dz), q = ir * (1.f / CIR_BOHR_NM);
+    const float ir = cir_rsqrt(dx * dx + dy * dy + dz * dz);
     const float uu = u.x * o[3] + u.y * o[4] + u.z * o[5];
     const float un = (u.x * dx + u.y * dy + u.z * dz) * ir;
     const float vn = (o[3] * dx + o[4] * dy + o[5] * dz) * ir;
-    return (uu - 3.0f * un * vn) * (q * q * q) * CIR_CM_HARTREE;
+    return (uu - 3.0f * un * vn) * (ir * ir * ir) * CIR_TDC;
 }
 
 // Contraction of the gradients of every origin and step with the map derivatives: blockIdx.y is

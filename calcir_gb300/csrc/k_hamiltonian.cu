@@ -212,12 +212,12 @@ __device__ __forceinline__ float pair_coupling(const Chrom &lo, const Chrom &hi,
     // transition dipole coupling (calcIR.cu:1352-1399)
     float dx = lo.tx - hi.tx, dy = lo.ty - hi.ty, dz = lo.tz - hi.tz;
     cir_mi3(dx, dy, dz, bx, by, bz, rx, ry, rz);
-    const float ri = cir_rsqrt(dot3(dx, dy, dz, dx, dy, dz)), rb = __fmul_rn(ri, 1.f / CIR_BOHR_NM);
+    const float ri = cir_rsqrt(dot3(dx, dy, dz, dx, dy, dz));
     const float uu = dot3(lo.ux, lo.uy, lo.uz, hi.ux, hi.uy, hi.uz);
     const float un = __fmul_rn(dot3(lo.ux, lo.uy, lo.uz, dx, dy, dz), ri);
     const float vn = __fmul_rn(dot3(hi.ux, hi.uy, hi.uz, dx, dy, dz), ri);
-    const float k = __fmul_rn(fmaf(-3.f, __fmul_rn(un, vn), uu), __fmul_rn(__fmul_rn(rb, rb), rb));
-    return __fmul_rn(__fmul_rn(k, __fmul_rn(lo.xm, hi.xm)), CIR_CM_HARTREE);
+    const float k = __fmul_rn(fmaf(-3.f, __fmul_rn(un, vn), uu), __fmul_rn(__fmul_rn(ri, ri), ri));
+    return __fmul_rn(__fmul_rn(k, __fmul_rn(lo.xm, hi.xm)), CIR_TDC);
 }
 
 constexpr int HT = 32;   // tile edge
