@@ -5,7 +5,19 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <float.h>
+#include <atomic>
 #include "cir_internal.h"
+
+// SMs of the current device (asked once per device)
+inline int cir_sms() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 152;
+    if ((n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 152;
+    known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
 
 // minImage (calcIR.cu:1459-1463): dx - L*round(dx/L), round half away from zero, evaluated
 // as the reference's float expression is, one rounding per operation (no fused multiply-add),

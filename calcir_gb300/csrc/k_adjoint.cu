@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(32 * DT_W) k_dtheta(DthetaArgs d) {
 // twenty of order 1024 184, 120 so.
 constexpr int PSI_B = 16, PSI_G = 16;        // rows or columns (of a thread's RP), slices of the sum
 constexpr int PSI_KC = 512;                  // depth staged at a time
-constexpr int PSI_TWO = 608;                 // blocks from which two rows a thread (four origins of order 512,
-                                             // 128 blocks: 18.5 / 24.6 us; twenty, 640: 45.2 / 44.4)
+constexpr int PSI_TWO = 4;                   // blocks an SM above which two rows a thread (four origins of order
+                                             // 512, 128 blocks on 152 SMs: 18.5 / 24.6 us; twenty, 640: 45.2 / 44.4)
 constexpr int PSI_SX = 20;                   // shared stride of a row of vectors: 16-byte reads
 __host__ __device__ inline int psi_kc(int n) { return n < PSI_KC ? (n + 63) & ~63 : PSI_KC; }
 
@@ -477,7 +477,7 @@ cudaError_t cir_psi_step(const float *V, int ld, long long sV, int n, const floa
     if (n < 1 || S < 1 || S > 65535 || ld < n || (ld & 3) || (sV & 3) || (reinterpret_cast<uintptr_t>(V) & 15))
         return cudaErrorInvalidValue;
     const PsiSource q = src ? *src : PsiSource{};
-    const bool two = (long long)S * ((n + PSI_B - 1) / PSI_B) > PSI_TWO;
+    const bool two = (long long)S * ((n + PSI_B - 1) / PSI_B) > (long long)PSI_TWO * cir_sms();
     return two ? psi_launch<2>(V, ld, sV, n, w, sw, dt_over_hbar, in, out, tmp, raw, q, S, s)
                : psi_launch<1>(V, ld, sV, n, w, sw, dt_over_hbar, in, out, tmp, raw, q, S, s);
 }

@@ -485,14 +485,6 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
     }
 }
 
-int gemm_sms() {
-    static int cache[64] = {};
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (!cache[dev] && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) cache[dev] = n;
-    return cache[dev] > 0 ? cache[dev] : 148;
-}
-
 // ---- small products: FP32 SIMT, 32 x 32 tiles, 64 threads of 4 x 4 outputs, K 32 at a time.
 // Where the 128 x 128 tiles leave most SMs idle, the tile above pays its start-up and 0.8 us for
 // every 32 of K; this one less, on many more SMs (gemm_small_wins).  Few blocks are bound by the
@@ -666,7 +658,7 @@ cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *l
     auto vec = [&](const float *p, int ld, long long st) {
         return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld & 3) == 0 && (batch == 1 || (st & 3) == 0);
     };
-    const int sms = gemm_sms();
+    const int sms = cir_sms();
     const bool va = vec(g.A, g.lda, g.sA), vb = vec(g.B, g.ldb, g.sB),
                vc = vec(g.C, g.ldc, g.sC) && (g.epilogue != 2 || vec(g.D, g.ldd, g.sD));
     const dim3 small((g.N + SB - 1) / SB, (g.M + SB - 1) / SB, batch);

@@ -200,8 +200,8 @@ cudaError_t cir_launch_tcf(const TcfArgs &t, int batch, cudaStream_t s, int *lau
     }
     // four rows a warp at a time share the reads of m(0) where that leaves two blocks per SM,
     // and a block takes up to 64 rows so that staging m(0) stays small beside them
-    const long long all = (long long)t.n * batch;
-    const int R = all >= 304LL * TCF_WARPS * 4 ? 4 : 1, rows = TCF_WARPS * (R == 4 && all >= 304LL * 64 ? 8 : R);
+    const long long all = (long long)t.n * batch, two = 2LL * cir_sms();
+    const int R = all >= two * TCF_WARPS * 4 ? 4 : 1, rows = TCF_WARPS * (R == 4 && all >= two * 64 ? 8 : R);
     const size_t smem = R == 4 ? sizeof(float) * 9 * (size_t)t.n : 0;
     auto kern = R == 4 ? k_tcf<4> : k_tcf<1>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
