@@ -61,7 +61,6 @@ enum {
     B_VS, B_FS,                                    // split-BF16 propagation operands
     B_UFR,                                         // run: distinct frames of a chunk and their multiplicity
     B_HREF, B_RW,                                  // FP64 eigenpair refinement: input copy, workspace
-    B_TQW,                                         // the panels' W of a joint tridiagonalisation
     B_COUNT
 };
 
@@ -1482,10 +1481,10 @@ static bool joint_tq_enabled() {
 }
 
 // The preparations of the groups whose chunks start at step k0.  When two or more of them
-// have orders 257-1024 (the blocked tridiagonalisation), their Hamiltonians are built one
+// have orders 257-1024, their Hamiltonians are built one
 // group after another and tridiagonalised in one launch (cir_launch_tridiag_multi: the
-// longest matrices first, the shorter ones filling the last wave, each group's panel W in
-// one shared area), then each group's eigensolver goes on from its d, e and reflectors;
+// longest matrices first, the shorter ones filling the last wave), then each group's
+// eigensolver goes on from its d, e and reflectors;
 // otherwise group by group.  The build time counted includes the autotuner's trials of the
 // first chunk.
 static int prepare_segment(cir_ctx *c, std::vector<std::unique_ptr<GroupJob>> &jobs, const std::vector<int> &prep,
@@ -1512,19 +1511,11 @@ static int prepare_segment(cir_ctx *c, std::vector<std::unique_ptr<GroupJob>> &j
         j.eg.tq_done = nullptr;
     }
     CK(cudaEventRecord(ev[2], c->stream));
-    size_t wf = 0;
-    for (int i : jt) wf += (size_t)jobs[i]->nmat * cir_tridiag_w_floats(jobs[i]->ld);
-    CK(c->buf[B_TQW].ensure(wf * 4));
     EighArgs a[CIR_TQ_MAXP];
     int nm[CIR_TQ_MAXP];
-    size_t off = 0;
     for (size_t q = 0; q < jt.size(); q++) {
-        GroupJob &j = *jobs[jt[q]];
-        a[q] = j.eg;
-        a[q].Z = c->buf[B_TQW].as<float>() + off;
-        a[q].zstride = (long long)cir_tridiag_w_floats(j.ld);
-        nm[q] = j.nmat;
-        off += (size_t)j.nmat * a[q].zstride;
+        a[q] = jobs[jt[q]]->eg;
+        nm[q] = jobs[jt[q]]->nmat;
     }
     CK(cir_launch_tridiag_multi(a, nm, (int)jt.size(), c->stream, &jobs[jt[0]]->launches));
     CK(cudaEventRecord(ev[5], c->stream));

@@ -7,8 +7,8 @@
 
 // Chunk length for K steps of St origins, at most kn_max steps a chunk.  The
 // tridiagonalisation runs `wave` matrices at a time, and a chunk whose last wave is nearly
-// empty pays for about a third of a wave while its few blocks run alone (order 1024 at 456
-// resident blocks: 3232 matrices, 7.09 waves, 525 ms; 3168 matrices, 6.95 waves, 501 ms).
+// empty pays for about a third of a wave while its few blocks run alone (measured with 456
+// blocks resident: 3232 matrices of order 1024, 7.09 waves, 525 ms; 3168, 6.95 waves, 501 ms).
 // Of the chunkings into as few chunks as kn_max allows, equal in length but the last, the
 // one with the least estimated time is taken: whole waves, a part-filled last wave counted
 // as at least 0.3 of one; ties go to the longer chunks.

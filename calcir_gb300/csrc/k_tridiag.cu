@@ -129,7 +129,7 @@ __device__ __forceinline__ void tridiag(const EighArgs &a, int mat) {
     float4 *Tq = reinterpret_cast<float4 *>(smem + L.TQ) + NB * warp;   // this warp's (t1, t2, W[k+1], V[k+1])
     float *X = smem + L.X;
     float *A = a.A + (size_t)mat * a.mstride;
-    float *Wg = a.Z + (size_t)mat * (a.zstride ? a.zstride : a.mstride);   // the panel's W (clusters)
+    float *Wg = a.Z + (size_t)mat * a.mstride;                              // the panel's W (clusters)
     float *dd = a.DE + (size_t)mat * 3 * ld, *ee = dd + ld, *tau = dd + 2 * ld;
     // this warp's tiles
     const int Ca = CL ? tq_cluster_rows(C) : 1, Cb = C / Ca;
@@ -704,8 +704,6 @@ int cluster_size(int n, int nmat, int sms) {
 
 int cir_tridiag_blocks(int n) { return n <= 128 ? 4 : (n <= 512 ? 2 : 1); }
 
-size_t cir_tridiag_w_floats(int ld) { return (size_t)TQ_NB * ld; }
-
 cudaError_t cir_launch_tridiag(const EighArgs &a, int nmat, cudaStream_t s) {
     int dev = 0, sms = 0;
     cudaError_t e;
@@ -731,7 +729,7 @@ cudaError_t cir_launch_tridiag_multi(const EighArgs *a, const int *nmat, int np,
     for (int i = 0; i < np; i++) {
         const EighArgs &x = a[i];
         if (x.n <= 256 || x.n > 1024 || nmat[i] < 1 || nmat[i] > 65535 || (x.ld & 3) || x.ld < x.n || !x.DE ||
-            (reinterpret_cast<uintptr_t>(x.A) & 15) || (reinterpret_cast<uintptr_t>(x.Z) & 15))
+            (reinterpret_cast<uintptr_t>(x.A) & 15))
             return cudaErrorInvalidValue;
         order[i] = i;
     }
