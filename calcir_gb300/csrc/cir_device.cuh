@@ -6,6 +6,9 @@
 #include <cuda_bf16.h>
 #include <float.h>
 #include <atomic>
+#include <map>
+#include <mutex>
+#include <utility>
 #include "cir_internal.h"
 
 // SMs of the current device (asked once per device)
@@ -17,6 +20,23 @@ inline int cir_sms() {
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 152;
     known[dev].store(n, std::memory_order_relaxed);
     return n;
+}
+
+// Lets kern be launched with that much dynamic shared memory.  The limit belongs to the kernel, whichever
+// thread or context launches it, so it is only ever raised: another thread's smaller launch must not take it
+// back between this call and the launch.
+template <class K>
+inline cudaError_t cir_allow_smem(K kern, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limits;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    size_t &limit = limits[{dev, reinterpret_cast<const void *>(kern)}];
+    if (limit >= bytes) return cudaSuccess;
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) == cudaSuccess) limit = bytes;
+    return e;
 }
 
 // minImage (calcIR.cu:1459-1463): dx - L*round(dx/L), round half away from zero, evaluated

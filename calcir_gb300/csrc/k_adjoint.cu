@@ -461,8 +461,8 @@ cudaError_t psi_launch(const float *V, int ld, long long sV, int n, const float 
     const size_t part = (size_t)PSI_G * NR * (PSI_LD + 1);
     const size_t smem_r = 4 * std::max((size_t)NR * (kcm + 4) + (size_t)kcm * PSI_SX, part);
     const size_t smem_c = 4 * std::max((size_t)kcm * PSI_SX, part);
-    cudaError_t e = cudaFuncSetAttribute(k_psi_rows<RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_psi_cols<RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c);
+    cudaError_t e = cir_allow_smem(k_psi_rows<RP>, smem_r);
+    if (e == cudaSuccess) e = cir_allow_smem(k_psi_cols<RP>, smem_c);
     if (e != cudaSuccess) return e;
     k_psi_rows<RP><<<dim3(grid, S), PSI_B * PSI_G, smem_r, s>>>(V, ld, sV, n, w, sw, dtoh, in, X, raw);
     k_psi_cols<RP><<<dim3(grid, S), PSI_B * PSI_G, smem_c, s>>>(V, ld, sV, n, X, out, src);

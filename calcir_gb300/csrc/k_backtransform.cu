@@ -622,13 +622,13 @@ static cudaError_t backtransform_paired(const EighArgs &a, const SplitMat &Qs, c
     }
     if ((e = multi_gemm(gx, nmat, s, nl)) != cudaSuccess) return e;
     const size_t tsm = bt_tmat_smem();
-    if ((e = cudaFuncSetAttribute(k_bt_tmat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm)) != cudaSuccess)
+    if ((e = cir_allow_smem(k_bt_tmat, tsm)) != cudaSuccess)
         return e;
     k_bt_tmat<<<dim3(nblk, nmat), BT_NB, tsm, s>>>(a, Gb, Tt, ms, ss);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     nl += 1;
     if (npf > 0) {
-        if ((e = cudaFuncSetAttribute(k_bt_cross, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_cross_smem())) !=
+        if ((e = cir_allow_smem(k_bt_cross, bt_cross_smem())) !=
             cudaSuccess)
             return e;
         k_bt_cross<<<dim3(npf, nmat), BT_CX_NT, bt_cross_smem(), s>>>(a, Xq, Tt, Cs, ms, ss);
@@ -750,7 +750,7 @@ static cudaError_t backtransform_split(const EighArgs &a, float *Q, float *P, fl
             if ((e = cir_launch_split_gemm_multi(gs.data() + b0, batch.data() + b0, np, s, &nl)) != cudaSuccess) return e;
         }
         const size_t tsm = bt_tmat_smem();
-        if ((e = cudaFuncSetAttribute(k_bt_tmat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm)) != cudaSuccess)
+        if ((e = cir_allow_smem(k_bt_tmat, tsm)) != cudaSuccess)
             return e;
         k_bt_tmat<<<dim3(nblk, nmat), BT_NB, tsm, s>>>(a, Gb, Tt, ms, ss);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -761,7 +761,7 @@ static cudaError_t backtransform_split(const EighArgs &a, float *Q, float *P, fl
         }
     } else {
         const size_t smem = bt_prep_smem();
-        if ((e = cudaFuncSetAttribute(k_bt_prep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+        if ((e = cir_allow_smem(k_bt_prep<true>, smem)) !=
             cudaSuccess)
             return e;
         k_bt_prep<true><<<dim3(nblk, nmat), BT_NT, smem, s>>>(a, sp);
@@ -816,7 +816,7 @@ cudaError_t cir_launch_backtransform(const EighArgs &a, float *Q, float *P, floa
     }
     const int pld = min(BT_NB, (nrefl + 3) & ~3);   // P: n x pld, pld <= ld
     const size_t smem = bt_prep_smem();
-    cudaError_t e = cudaFuncSetAttribute(k_bt_prep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(k_bt_prep<false>, smem);
     if (e != cudaSuccess) return e;
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||

@@ -758,7 +758,7 @@ cudaError_t cir_launch_dc(const EighArgs &a, int nmat, cudaStream_t s, int *laun
         int nt = base, C = 1;
         dc_shape((1 << level) * (long long)nmat, KM, sms, nt, C);
         auto merge = [&](auto kern) -> cudaError_t {
-            cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaError_t r = cir_allow_smem(kern, smem);
             if (r != cudaSuccess) return r;
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute at[1];

@@ -627,7 +627,7 @@ template <int NT, int NMAX, int NBQ, int CB, int MINB>
 cudaError_t launch_formq(const EighArgs &a, int nmat, cudaStream_t s) {
     auto kern = k_eigh_formq<NT, NMAX, NBQ, CB, MINB>;
     const size_t smem = sizeof(float) * fq_smem_floats<NT, NMAX, NBQ, CB>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<nmat, NT, smem, s>>>(a);
     return cudaGetLastError();
@@ -639,7 +639,7 @@ constexpr int QR_ROWS = 3;   // rows per applying thread; 3 blocks per SM withou
 cudaError_t launch_qr(const EighArgs &a, int nmat, cudaStream_t s) {
     auto kern = k_eigh_qr<QR_THREADS, QR_ROWS>;
     const size_t smem = qr_smem_bytes(a.n, QR_THREADS, QR_ROWS);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<nmat, QR_THREADS, smem, s>>>(a);
     return cudaGetLastError();

@@ -680,7 +680,7 @@ cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *l
     }
     const int grid = (int)std::min<long long>(nt, sms);
     auto go = [&](auto kern) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F_SMEM);
+        cudaError_t e = cir_allow_smem(kern, F_SMEM);
         if (e != cudaSuccess) return e;
         kern<<<grid, F_NT, F_SMEM, s>>>(g, tiles_n, (int)mn, (int)nt, va, vb, vc, g.err);
         return cudaGetLastError();

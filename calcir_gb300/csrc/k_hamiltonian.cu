@@ -296,7 +296,7 @@ cudaError_t cir_launch_build(const BuildArgs &a, int nframes, cudaStream_t s, in
     const int per_block = wide ? CHROM_NT / 32 : CHROM_NT;
     auto kern = wide ? k_chromophore<true> : k_chromophore<false>;
     const size_t smem = sizeof(float) * MOL_F * (size_t)a.nmol + sizeof(unsigned) * per_block * (size_t)(((a.nmol + 31) / 32) | 1);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<dim3((a.n + per_block - 1) / per_block, nframes), CHROM_NT, smem, s>>>(a, cut2);
     e = cudaGetLastError();

@@ -485,7 +485,7 @@ cudaError_t cir_launch_refine(const float *H, float *Z, long long mstride, int l
         return cudaErrorInvalidValue;
     const long long sM = (long long)n * n;
     const size_t smem = (size_t)3 * n * 8;
-    cudaError_t e0 = cudaFuncSetAttribute(k_rf_coef, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e0 = cir_allow_smem(k_rf_coef, smem);
     if (e0 != cudaSuccess) return e0;
     int nl = 0;
     for (int m0 = 0; m0 < nmat; m0 += chunk) {

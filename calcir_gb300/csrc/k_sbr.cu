@@ -464,7 +464,7 @@ cudaError_t cir_launch_sbr(const float *H, long long sH, int nmat, int n, int ld
     k_sb_shift<<<nmat, 256, 0, s>>>(H, sH, g);
     k_sb_split<<<dim3((n + 7) / 8, nmat), 256, 0, s>>>(H, sH, g);
     nl += 2;
-    if ((e0 = cudaFuncSetAttribute(k_sb_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb_w_smem())) != cudaSuccess)
+    if ((e0 = cir_allow_smem(k_sb_w, sb_w_smem())) != cudaSuccess)
         return fin(e0);
     for (int k = 0;; k += SB_B) {
         const int m = n - k - SB_B;

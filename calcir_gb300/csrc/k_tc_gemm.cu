@@ -320,7 +320,7 @@ template <bool ACOL, bool BKC, int MODE>
 cudaError_t launch(const GemmArgs &g, int batch, cudaStream_t s) {
     const size_t smem = smem_bytes<MODE>();
     dim3 grid((g.N + TN - 1) / TN, (g.M + TM - 1) / TM, batch);
-    cudaError_t e = cudaFuncSetAttribute(k_tc_gemm<ACOL, BKC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(k_tc_gemm<ACOL, BKC, MODE>, smem);
     if (e != cudaSuccess) return e;
     k_tc_gemm<ACOL, BKC, MODE><<<grid, NTHREADS, smem, s>>>(g);
     return cudaGetLastError();

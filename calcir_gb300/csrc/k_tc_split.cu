@@ -756,7 +756,7 @@ size_t cir_split_ld(int n) { return (size_t)((n + 7) & ~7); }
 template <int QK, int QS, int QN>
 static cudaError_t launch_split(const SplitMaps &maps, const SplitGemmArgs &g, int batch, cudaStream_t s) {
     constexpr size_t smem = QCfg<QK, QS, QN>::SMEM;
-    cudaError_t e = cudaFuncSetAttribute(k_tc_split<QK, QS, QN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(k_tc_split<QK, QS, QN>, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((g.N + QN - 1) / QN, (g.M + QM - 1) / QM, batch);
     k_tc_split<QK, QS, QN><<<grid, QT, smem, s>>>(maps, g);
@@ -864,7 +864,7 @@ static cudaError_t launch_persist(const SplitGemmArgs *g, const int *batch, int 
     plan.first[np] = (int)ntl;
     const int grid = (int)std::min<long long>(ntl, sm_count());
     auto go = [&](auto kern, size_t smem) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cir_allow_smem(kern, smem);
         if (e != cudaSuccess) return e;
         kern<<<grid, PT, smem, s>>>(plan);
         return cudaGetLastError();

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(SP_W * SP_J) k_spec_sum(const float *mu2, cons
 cudaError_t cir_launch_tcf(const TcfArgs &t, int batch, cudaStream_t s, int *launches) {
     if (t.Ft.hi) {
         const size_t sm = sizeof(float) * 9 * (size_t)((t.n + TT_QSPLIT - 1) / TT_QSPLIT);
-        cudaError_t e = cudaFuncSetAttribute(k_tcf_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = cir_allow_smem(k_tcf_t, sm);
         if (e != cudaSuccess) return e;
         k_tcf_t<<<dim3((t.n + TT_ROWS - 1) / TT_ROWS, TT_QSPLIT, batch), 256, sm, s>>>(t);
         if (launches) *launches += 1;
@@ -204,7 +204,7 @@ cudaError_t cir_launch_tcf(const TcfArgs &t, int batch, cudaStream_t s, int *lau
     const int R = all >= two * TCF_WARPS * 4 ? 4 : 1, rows = TCF_WARPS * (R == 4 && all >= two * 64 ? 8 : R);
     const size_t smem = R == 4 ? sizeof(float) * 9 * (size_t)t.n : 0;
     auto kern = R == 4 ? k_tcf<4> : k_tcf<1>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<dim3((t.n + rows - 1) / rows, batch), TCF_WARPS * 32, smem, s>>>(t, rows);
     if (launches) *launches += 1;

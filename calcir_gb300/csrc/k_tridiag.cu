@@ -631,7 +631,7 @@ cudaError_t launch(K kern, const EighArgs &a, int nmat, int nt, bool res, int C,
             return e;
         smem = std::max(smem, (size_t)per_sm / (a.tq_blocks + 1) - (size_t)reserved + 1024);
     }
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    if ((e = cir_allow_smem(kern, smem)) != cudaSuccess) return e;
     cfg.gridDim = dim3(nmat * C);
     cfg.blockDim = dim3(nt);
     cfg.dynamicSmemBytes = smem;
@@ -669,7 +669,7 @@ int cluster_slots(int C) {
     cfg.numAttrs = 1;
     int k = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cir_allow_smem(kern, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&k, kern, &cfg) != cudaSuccess) {
         cudaGetLastError();
         k = 0;
@@ -747,7 +747,7 @@ cudaError_t cir_launch_tridiag_multi(const EighArgs *a, const int *nmat, int np,
     }
     plan.start[np] = total;
     auto kern = k_tridiag_multi<512, 1, 2>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cir_allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     kern<<<total, 512, smem, s>>>(plan);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
