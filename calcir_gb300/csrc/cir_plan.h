@@ -56,3 +56,14 @@ inline CirTridiagForm cir_tridiag_form(int n, int nmat, int sms) {
 // The autotuner's blocks per SM, measured on more than two waves of one block per SM, where a batch
 // is as large; else 0, the kernel's own number.
 inline int cir_tridiag_limit(int tuned, int nmat, int sms) { return nmat > 2 * sms ? tuned : 0; }
+
+// Whether the field's sums take a warp per chromophore (wide) or a thread.  In us: the wide form by
+// the chromophores on the whole device (each block stages all molecules, so that large boxes leave few
+// blocks an SM), the other as long as one thread's run over its molecules until it fills the device.
+// Fits to 1..1000 molecules and 1..3000 frames; measured, wide against narrow: 5 x 1000 14.5 / 10.4,
+// 40 x 100 21 / 29, 100 x 30 34 / 56, 100 x 100 82 / 63, 343 x 10 65 / 109, 343 x 30 168 / 119, 1000 x 2
+// 160 / 234, 1000 x 4 280 / 236, 1000 x 30 1958 / 500.
+inline bool cir_build_wide(int n, int nmol, int nframes, int sms) {
+    const double m = nmol, wide = 5.0 + 1e-3 * n * nframes * (1.0 + 0.02 * m + 1.2e-5 * m * m) * 152.0 / sms;
+    return wide < 8.0 + std::min(0.42 * m, 42.0 + 0.18 * m);
+}

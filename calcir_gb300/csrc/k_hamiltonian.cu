@@ -20,6 +20,7 @@
 // depend on the order of the two, so H is exactly symmetric; both triangles are written with
 // coalesced stores.
 #include "cir_device.cuh"
+#include "cir_plan.h"
 
 #include <cmath>
 
@@ -290,9 +291,7 @@ cudaError_t cir_launch_build(const BuildArgs &a, int nframes, cudaStream_t s, in
         while (sqrtf(s) > CIR_CUTOFF) s = nextafterf(s, 0.f);
         return s;
     }();
-    // the wide form takes about 2 us per 1000 chromophores on the whole device, the other as long
-    // as one thread's run over its molecules, 20 + 0.2 nmol us, until it fills the device
-    const bool wide = (long long)a.n * nframes <= 10000 + 100LL * a.nmol;
+    const bool wide = cir_build_wide(a.n, a.nmol, nframes, cir_sms());
     const int per_block = wide ? CHROM_NT / 32 : CHROM_NT;
     auto kern = wide ? k_chromophore<true> : k_chromophore<false>;
     const size_t smem = sizeof(float) * MOL_F * (size_t)a.nmol + sizeof(unsigned) * per_block * (size_t)(((a.nmol + 31) / 32) | 1);

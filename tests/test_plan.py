@@ -105,3 +105,34 @@ def test_tridiagonalisation_form(tmp_path):
         for ((n, nmat), form), (got, limit) in zip(forms, run([(n, nmat, tuned) for (n, nmat), _ in forms])):
             assert got == form, (n, nmat, tuned)
             assert limit == (tuned if nmat > 304 else 0)
+
+
+WIDE_DRIVER = r"""
+#include <cstdio>
+#include "cir_plan.h"
+int main() {
+    int nmol, nf;
+    while (std::scanf("%d %d", &nmol, &nf) == 2) std::printf("%d\n", cir_build_wide(2 * nmol, nmol, nf, 152) ? 1 : 0);
+    return 0;
+}
+"""
+
+
+def test_build_form(tmp_path):
+    """A warp or a thread per chromophore: the form that measured at least 15% faster (GB300), over box
+    sizes and batches, large boxes of few frames among them."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no host C++ compiler")
+    src, exe = str(tmp_path / "wide.cpp"), str(tmp_path / "wide")
+    with open(src, "w") as f:
+        f.write(WIDE_DRIVER)
+    subprocess.run([cxx, "-std=c++17", "-O1", "-I", HEADER_DIR, src, "-o", exe], check=True)
+    wide = [(1, 1), (5, 100), (12, 200), (24, 1), (24, 100), (40, 100), (64, 1), (64, 30), (100, 30), (150, 30), (250, 10),
+            (343, 1), (343, 10), (512, 4), (700, 1), (700, 4), (1000, 1), (1000, 2)]
+    narrow = [(2, 3000), (5, 1000), (12, 1000), (24, 500), (40, 500), (64, 200), (100, 100), (150, 100), (250, 100),
+              (343, 30), (343, 200), (512, 30), (700, 10), (1000, 4), (1000, 30)]
+    cases = wide + narrow
+    out = subprocess.run([exe], input="".join("%d %d\n" % c for c in cases), capture_output=True, text=True,
+                         check=True).stdout.split()
+    assert [int(x) for x in out] == [1] * len(wide) + [0] * len(narrow)
