@@ -67,3 +67,25 @@ inline bool cir_build_wide(int n, int nmol, int nframes, int sms) {
     const double m = nmol, wide = 5.0 + 1e-3 * n * nframes * (1.0 + 0.02 * m + 1.2e-5 * m * m) * 152.0 / sms;
     return wide < 8.0 + std::min(0.42 * m, 42.0 + 0.18 * m);
 }
+
+// The FP32 product's kernel (k_gemm.cu): the least of four fits in us to 1800 measurements on 152 SMs
+// (M, N, K 8..2048, batches 1..600, operands' and outputs' rows aligned to 16 bytes and not, with and without C = D - A B; within
+// 6% of the fastest in 95% of them).  Tiles of 32 with four groups along K while there are few, of 64 for
+// many products of order 24 to about 110 and for short K, of 128 for some of order 65 to 112 in large
+// batches, and the tensor cores.  Measured (small, 64, 128, tensor cores): 128 x 256 x 128 6.6, 10, 25,
+// 15; 65 x 130 x 65 in 150, rows not aligned, 30, 28, 22, 29; 50 x 100 x 50 in 300 31, 15, 19, 21; 686 x 686 x
+// 128 in 64, C = D - A B, not aligned, 514, 297, 324, 739; aligned 474, 244, 282, 175; 512 x 1024 x 512 29, 27,
+// 76, 29; 1024 x 2048 x 1024 154, 138, 146, 50.
+enum CirGemmForm { CIR_GEMM_SMALL, CIR_GEMM_TILE64, CIR_GEMM_TILE128, CIR_GEMM_TC };
+inline CirGemmForm cir_gemm_form(int M, int N, int K, int batch, int epilogue, bool in16, bool out16, int sms) {
+    auto tiles = [&](int t) { return (double)((M + t - 1) / t) * ((N + t - 1) / t) * batch; };
+    auto slices = [&](int k) { return (double)((K + k - 1) / k); };
+    const double b32 = tiles(32) / sms, b64 = tiles(64) / sms, t128 = tiles(128), sub = epilogue == 2 ? 1.0 : 0.0;
+    const double t[4] = {
+        4.4 + slices(128) * std::max(1.92, 1.14 * b32) + 0.46 * b32,
+        4.9 + slices(16) * std::max(0.63, 0.556 * b64) * (in16 ? 1.0 : 1.09) + 0.24 * sub * b64,
+        2.7 + std::ceil(t128 / (2 * sms)) * (1.054 * slices(8) * (t128 > sms ? 1.57 : 1.0) * (in16 ? 1.0 : 1.035) + 2.76),
+        3.5 + std::ceil(t128 / sms) * (std::max((in16 ? 1.44 : 1.75) * slices(32) + 4.8, out16 ? 0.0 : 17.0) +
+                                       sub * (out16 ? 2.0 : 38.0))};
+    return static_cast<CirGemmForm>(std::min_element(t, t + 4) - t);
+}

@@ -38,11 +38,12 @@
 // slices' maxima 303-361).  1024 x 2048 x 1024 in ten matrices: 859-1044 us as SIMT FFMAs (50-41
 // TFLOP/s), 323-386 so (133-111), error against 64 bits 5.7e-7 and 6e-8; with the terms rounded
 // value by value and six products 283-331 us, 1.2e-7 and the drift above.  Not taken: 16 splitting
-// warps (403-432: the copies of 8 bytes that rows contiguous then need).  Products with too few
-// tiles for the SMs run on the SIMT kernel further down (gemm_small_wins).
+// warps (403-432: the copies of 8 bytes that rows contiguous then need).  Smaller products
+// run on the SIMT kernels further down (cir_gemm_form).
 // Every wait is bounded: a timeout raises the CTA's abort flag and the error flag, every role
 // leaves its loop, and the MMAs issued are waited for before the tensor memory is freed.
 #include "cir_device.cuh"
+#include "cir_plan.h"
 #include "cir_tcf.cuh"
 #include "cir_tcgen05.cuh"
 
@@ -446,34 +447,28 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
             const CirPhase ph = g.epilogue == 1 ? cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar) : CirPhase{};
             float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
             const int cb = n0 + 64 * half;
-            if (vecC && cb + 64 <= g.N) {
-                #pragma unroll
-                for (int h = 0; h < 4; h++) {
+            #pragma unroll
+            for (int h = 0; h < 4; h++) {
+                const int c0 = cb + 16 * h;
+                if (g.epilogue == 1)   // (re, im) pairs times exp(+i ph)
+                    #pragma unroll
+                    for (int q = 0; q < 16; q += 2) cir_rotate(ph, acc[h][q], acc[h][q + 1]);
+                if (vecC && c0 + 16 <= g.N) {
                     float4 d[4];
                     if (D)
                         #pragma unroll
-                        for (int q = 0; q < 4; q++) d[q] = *reinterpret_cast<const float4 *>(D + cb + 16 * h + 4 * q);
-                    if (g.epilogue == 1)   // (re, im) pairs times exp(+i ph)
-                        #pragma unroll
-                        for (int q = 0; q < 16; q += 2) cir_rotate(ph, acc[h][q], acc[h][q + 1]);
+                        for (int q = 0; q < 4; q++) d[q] = *reinterpret_cast<const float4 *>(D + c0 + 4 * q);
                     #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         float4 x = make_float4(acc[h][4 * q], acc[h][4 * q + 1], acc[h][4 * q + 2], acc[h][4 * q + 3]);
                         if (D) x = make_float4(d[q].x - x.x, d[q].y - x.y, d[q].z - x.z, d[q].w - x.w);   // C = D - A B
-                        *reinterpret_cast<float4 *>(C + cb + 16 * h + 4 * q) = x;
+                        *reinterpret_cast<float4 *>(C + c0 + 4 * q) = x;
                     }
-                }
-            } else {
-                #pragma unroll
-                for (int h = 0; h < 4; h++)
+                } else {
                     #pragma unroll
-                    for (int q = 0; q < 16; q += 2) {
-                        const int c = cb + 16 * h + q;
-                        float re = acc[h][q], im = acc[h][q + 1];
-                        if (g.epilogue == 1) cir_rotate(ph, re, im);
-                        if (c < g.N) C[c] = D ? D[c] - re : re;
-                        if (c + 1 < g.N) C[c + 1] = D ? D[c + 1] - im : im;
-                    }
+                    for (int q = 0; q < 16; q++)
+                        if (c0 + q < g.N) C[c0 + q] = D ? D[c0 + q] - acc[h][q] : acc[h][q];
+                }
             }
         }
     }
@@ -485,24 +480,81 @@ __global__ void __launch_bounds__(F_NT, 1) k_gemm(GemmArgs g, int tiles_n, int t
     }
 }
 
-// ---- small products: FP32 SIMT, 32 x 32 tiles, 64 threads of 4 x 4 outputs, K 32 at a time.
-// Where the 128 x 128 tiles leave most SMs idle, the tile above pays its start-up and 0.8 us for
-// every 32 of K; this one less, on many more SMs (gemm_small_wins).  Few blocks are bound by the
-// chain of loads and sums along K: KS groups of 64 threads then take every KS-th slice and meet in
-// shared memory.
-constexpr int SB = 32, SLD = SB + 4;
+// ---- smaller products: FP32 SIMT.  Where the 128 x 128 tiles above leave most SMs idle or K gives them
+// little to do, their start-up and read-out are most of the time (cir_gemm_form).
+
+// four values at q, of which the first `have` exist (one load where the address allows it: of rows that are
+// not aligned some still start on 16 bytes)
+__device__ __forceinline__ bool at16(const float *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+__device__ __forceinline__ float4 simt_load4(const float *q, int have) {
+    if (have >= 4 && at16(q)) return __ldg(reinterpret_cast<const float4 *>(q));
+    return make_float4(have > 0 ? __ldg(q) : 0.f, have > 1 ? __ldg(q + 1) : 0.f, have > 2 ? __ldg(q + 2) : 0.f,
+                       have > 3 ? __ldg(q + 3) : 0.f);
+}
+// row r, columns c .. c + 3 of a product: the phase or C = D - A B, stored
+__device__ __forceinline__ void simt_store(const GemmArgs &g, int bz, int r, int c, float4 v, const CirPhase &ph) {
+    float x[4] = {v.x, v.y, v.z, v.w};
+    if (g.epilogue == 1) {   // (re, im) pairs times exp(+i ph)
+        cir_rotate(ph, x[0], x[1]);
+        cir_rotate(ph, x[2], x[3]);
+    }
+    float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc + c;
+    const float *D = g.epilogue == 2 ? g.D + (size_t)bz * g.sD + (size_t)r * g.ldd + c : nullptr;
+    if (c + 3 < g.N && at16(C) && at16(D)) {
+        if (D) {
+            const float4 d = *reinterpret_cast<const float4 *>(D);
+            x[0] = d.x - x[0]; x[1] = d.y - x[1]; x[2] = d.z - x[2]; x[3] = d.w - x[3];
+        }
+        *reinterpret_cast<float4 *>(C) = make_float4(x[0], x[1], x[2], x[3]);
+        return;
+    }
+    #pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (c + q < g.N) C[q] = D ? D[q] - x[q] : x[q];
+}
+__device__ __forceinline__ CirPhase simt_phase(const GemmArgs &g, int bz, int r) {
+    return g.epilogue == 1 ? cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar) : CirPhase{};
+}
+
+// The correlation terms of the propagated F (interleaved complex columns) from the patches that a
+// thread holds: m(0) at its two complex columns, and a row's four values added to the sums.  150
+// steps at n = 128: 3050 us with a launch of k_tcf a step, 2820 so.
+struct TcfCols {
+    float a[9], b[9];
+    TcfCols() = default;
+    __device__ __forceinline__ TcfCols(const TcfArgs &tc, int bz, int c) {
+        const float *m = tc.m0 + (size_t)bz * tc.sm0;
+        const int q = c >> 1;
+        #pragma unroll
+        for (int u = 0; u < 9; u++) {
+            a[u] = q < tc.n ? __ldg(m + (size_t)u * tc.ldv + q) : 0.f;
+            b[u] = q + 1 < tc.n ? __ldg(m + (size_t)u * tc.ldv + q + 1) : 0.f;
+        }
+    }
+};
+__device__ __forceinline__ void tcf_row(const TcfArgs &tc, int bz, int r, const TcfCols &m0, float4 v, Pair (&sum)[8]) {
+    float pr[9], pi[9], c[9];
+    const float *m = tc.mt + (size_t)bz * tc.smt + r;
+    #pragma unroll
+    for (int u = 0; u < 9; u++) {
+        pr[u] = fmaf(v.z, m0.b[u], v.x * m0.a[u]);
+        pi[u] = fmaf(v.w, m0.b[u], v.y * m0.a[u]);
+        c[u] = __ldg(m + (size_t)u * tc.ldv);
+    }
+    tcf_sums(pr, pi, c, sum);
+}
+
+// Few tiles, bound by the chain of loads and sums along K: 32 x 32 tiles, SK groups of 64 threads (4 x 4
+// outputs each) take every SK-th slice of 32 of K and meet in shared memory.
+constexpr int SB = 32, SLD = SB + 4, SK = 4;
 
 template <bool KC>
-__device__ __forceinline__ void small_load(const float *p, int ld, int rdim, int kdim, int r0, int k0, int t, bool vec, float4 (&v)[4]) {
+__device__ __forceinline__ void small_load(const float *p, int ld, int rdim, int kdim, int r0, int k0, int t, float4 (&v)[4]) {
     #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int idx = t + 64 * i, o = idx >> 3, c4 = 4 * (idx & 7);
         const int r = r0 + (KC ? o : c4), k = k0 + (KC ? c4 : o);
-        const float *q = KC ? p + (size_t)r * ld + k : p + (size_t)k * ld + r;
-        const int have = KC ? (r < rdim ? kdim - k : 0) : (k < kdim ? rdim - r : 0);
-        if (vec && have >= 4) { v[i] = __ldg(reinterpret_cast<const float4 *>(q)); continue; }
-        v[i] = make_float4(have > 0 ? __ldg(q) : 0.f, have > 1 ? __ldg(q + 1) : 0.f, have > 2 ? __ldg(q + 2) : 0.f,
-                           have > 3 ? __ldg(q + 3) : 0.f);
+        v[i] = simt_load4(KC ? p + (size_t)r * ld + k : p + (size_t)k * ld + r, KC ? (r < rdim ? kdim - k : 0) : (k < kdim ? rdim - r : 0));
     }
 }
 template <bool KC>
@@ -517,34 +569,28 @@ __device__ __forceinline__ void small_store(float *s, int t, const float4 (&v)[4
     }
 }
 
-// TCF: the product is the propagated F (interleaved complex columns), and the block adds its tile's
-// correlation terms to tc.out: 150 steps at n = 128 3050 us with a launch of k_tcf a step, 2820 so.
-template <bool ACOL, bool BKC, int KS, bool TCF>
-__global__ void __launch_bounds__(64 * KS) k_gemm_small(GemmArgs g, bool vecA, bool vecB, TcfArgs tc) {
-    __shared__ __align__(16) float sm[KS == 1 ? 2 : KS][2][SB * SLD];   // one group: two buffers
+template <bool ACOL, bool BKC, bool TCF>
+__global__ void __launch_bounds__(64 * SK) k_gemm_small(GemmArgs g, TcfArgs tc) {
+    __shared__ __align__(16) float sm[SK][2][SB * SLD];
     const int bz = blockIdx.z, m0 = blockIdx.y * SB, n0 = blockIdx.x * SB;
     const float *A = g.A + (size_t)bz * g.sA, *B = g.B + (size_t)bz * g.sB;
     const int t = threadIdx.x & 63, grp = threadIdx.x >> 6;
     const int tx = 4 * (t & 7), ty = 4 * (t >> 3);
-    auto group_sync = [&] {
-        if (KS == 1) __syncthreads();
-        else asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory");
-    };
+    auto group_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(grp + 1) : "memory"); };
     float acc[4][4] = {};
     float4 ra[4], rb[4];
-    int buf = KS == 1 ? 0 : grp;
-    small_load<!ACOL>(A, g.lda, g.M, g.K, m0, SB * grp, t, vecA, ra);
-    small_load<BKC>(B, g.ldb, g.N, g.K, n0, SB * grp, t, vecB, rb);
-    small_store<!ACOL>(sm[buf][0], t, ra);
-    small_store<BKC>(sm[buf][1], t, rb);
+    small_load<!ACOL>(A, g.lda, g.M, g.K, m0, SB * grp, t, ra);
+    small_load<BKC>(B, g.ldb, g.N, g.K, n0, SB * grp, t, rb);
+    small_store<!ACOL>(sm[grp][0], t, ra);
+    small_store<BKC>(sm[grp][1], t, rb);
     group_sync();
-    for (int k0 = SB * grp; k0 < g.K; k0 += SB * KS) {
-        const int kn = k0 + SB * KS;
+    for (int k0 = SB * grp; k0 < g.K; k0 += SB * SK) {
+        const int kn = k0 + SB * SK;
         if (kn < g.K) {
-            small_load<!ACOL>(A, g.lda, g.M, g.K, m0, kn, t, vecA, ra);
-            small_load<BKC>(B, g.ldb, g.N, g.K, n0, kn, t, vecB, rb);
+            small_load<!ACOL>(A, g.lda, g.M, g.K, m0, kn, t, ra);
+            small_load<BKC>(B, g.ldb, g.N, g.K, n0, kn, t, rb);
         }
-        const float *as = sm[buf][0] + ty, *bs = sm[buf][1] + tx;
+        const float *as = sm[grp][0] + ty, *bs = sm[grp][1] + tx;
         #pragma unroll 8
         for (int k = 0; k < SB; k++) {
             const float4 a4 = *reinterpret_cast<const float4 *>(as + k * SLD);
@@ -556,89 +602,131 @@ __global__ void __launch_bounds__(64 * KS) k_gemm_small(GemmArgs g, bool vecA, b
                 for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         if (kn < g.K) {
-            if (KS == 1) buf ^= 1;
-            else group_sync();
-            small_store<!ACOL>(sm[buf][0], t, ra);
-            small_store<BKC>(sm[buf][1], t, rb);
+            group_sync();
+            small_store<!ACOL>(sm[grp][0], t, ra);
+            small_store<BKC>(sm[grp][1], t, rb);
         }
         group_sync();
     }
-    if (KS > 1) {   // the first group adds the others' sums
-        float *part = sm[grp][0];
+    // the first group adds the others' sums
+    float *part = sm[grp][0];
+    #pragma unroll
+    for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(part + (ty + i) * SLD + tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    __syncthreads();
+    if (grp) return;
+    #pragma unroll
+    for (int q = 1; q < SK; q++)
         #pragma unroll
-        for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(part + (ty + i) * SLD + tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        __syncthreads();
-        if (grp) return;
-        #pragma unroll
-        for (int q = 1; q < KS; q++)
-            #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 v = *reinterpret_cast<const float4 *>(sm[q][0] + (ty + i) * SLD + tx);
-                acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
-            }
-    }
-    Pair sum[8] = {};
-    float ma[9], mb[9];                  // m(0) at the thread's two complex columns
-    if (TCF) {
-        const float *m = tc.m0 + (size_t)bz * tc.sm0;
-        const int q = (n0 + tx) >> 1;
-        #pragma unroll
-        for (int a = 0; a < 9; a++) {
-            ma[a] = q < tc.n ? __ldg(m + (size_t)a * tc.ldv + q) : 0.f;
-            mb[a] = q + 1 < tc.n ? __ldg(m + (size_t)a * tc.ldv + q + 1) : 0.f;
+        for (int i = 0; i < 4; i++) {
+            const float4 v = *reinterpret_cast<const float4 *>(sm[q][0] + (ty + i) * SLD + tx);
+            acc[i][0] += v.x; acc[i][1] += v.y; acc[i][2] += v.z; acc[i][3] += v.w;
         }
-    }
+    Pair sum[8] = {};
+    const TcfCols mc = TCF ? TcfCols(tc, bz, n0 + tx) : TcfCols();
     #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int r = m0 + ty + i;
         if (r >= g.M) continue;
-        if (TCF) {
-            float pr[9], pi[9], c[9];
-            const float *m = tc.mt + (size_t)bz * tc.smt + r;
-            #pragma unroll
-            for (int a = 0; a < 9; a++) {
-                pr[a] = fmaf(acc[i][2], mb[a], acc[i][0] * ma[a]);
-                pi[a] = fmaf(acc[i][3], mb[a], acc[i][1] * ma[a]);
-                c[a] = __ldg(m + (size_t)a * tc.ldv);
-            }
-            tcf_sums(pr, pi, c, sum);
-        }
-        const CirPhase ph = g.epilogue == 1 ? cir_phase(g.w[(size_t)bz * g.wstride + r] * g.dt_over_hbar) : CirPhase{};
-        float *C = g.C + (size_t)bz * g.sC + (size_t)r * g.ldc;
-        const float *D = g.epilogue == 2 ? g.D + (size_t)bz * g.sD + (size_t)r * g.ldd : nullptr;
-        #pragma unroll
-        for (int j = 0; j < 4; j += 2) {
-            const int c = n0 + tx + j;
-            float re = acc[i][j], im = acc[i][j + 1];
-            if (g.epilogue == 1) cir_rotate(ph, re, im);   // (re, im) pairs times exp(+i ph)
-            if (c < g.N) C[c] = D ? D[c] - re : re;
-            if (c + 1 < g.N) C[c + 1] = D ? D[c + 1] - im : im;
-        }
+        const float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        if (TCF) tcf_row(tc, bz, r, mc, v, sum);
+        simt_store(g, bz, r, n0 + tx, v, simt_phase(g, bz, r));
     }
     if (TCF) {
-        __shared__ double part[8];
+        __shared__ double psum[8];
         const double v = tcf_reduce(sum);
-        if (t >= 32 && (t & 3) == 0) part[(t & 31) >> 2] = v;
+        if (t >= 32 && (t & 3) == 0) psum[(t & 31) >> 2] = v;
         group_sync();
-        if (t < 32) tcf_add(__shfl_sync(0xffffffffu, v, (4 * t) & 31) + (t < 8 ? part[t] : 0.0), tc.out + (size_t)bz * tc.sout);
+        if (t < 32) tcf_add(__shfl_sync(0xffffffffu, v, (4 * t) & 31) + (t < 8 ? psum[t] : 0.0), tc.out + (size_t)bz * tc.sout);
     }
 }
 
-// Four groups a block while there are at most four blocks an SM (128 x 256 x 128 in one matrix
-// 10.5 us with one group, 6.2 with four; 1024 x 128 x 1024 35, 21; 1024 x 1024 x 128, 1024 blocks,
-// 16.5, 20.9).
-bool small_split(long long blocks, int K, int sms) { return K > SB && blocks <= 4LL * sms; }
+// Many tiles: T x T tiles of 256 threads, 4 x 4 outputs in each quarter of 64, TK of K at a time, double
+// buffered: 64 x 64 x 16 and 128 x 128 x 8.
+template <int T, int TK, bool KC>
+__device__ __forceinline__ float4 tile_load(const float *p, int ld, int rdim, int kdim, int r0, int k0) {
+    constexpr int W = KC ? TK / 4 : T / 4;
+    const int t = threadIdx.x, r = r0 + (KC ? t / W : 4 * (t % W)), k = k0 + (KC ? 4 * (t % W) : t / W);
+    return simt_load4(KC ? p + (size_t)r * ld + k : p + (size_t)k * ld + r, KC ? (r < rdim ? kdim - k : 0) : (k < kdim ? rdim - r : 0));
+}
+template <int T, int TK, bool KC>
+__device__ __forceinline__ void tile_store(float (*s)[T], float4 v) {
+    constexpr int W = KC ? TK / 4 : T / 4;
+    const int t = threadIdx.x;
+    if (KC) {
+        const int r = t / W, k = 4 * (t % W);
+        s[k][r] = v.x; s[k + 1][r] = v.y; s[k + 2][r] = v.z; s[k + 3][r] = v.w;
+    } else *reinterpret_cast<float4 *>(&s[t / W][4 * (t % W)]) = v;
+}
 
-// Which of the two is faster, from fits in us to all three over M 54..2048, K 54..2048: 8 + 1.3 per
-// 32 of K and wave of tiles for the tensor cores, 4 + (0.75 + 0.3 blocks an SM) per 32 of K for one
-// group, 4.2 + max(2.05, 1.9 blocks an SM) per 128 of K for four.  Measured, small against tensor
-// cores: 128 x 256 x 128 6.2 / 13, 512 x 18 x 512 in four matrices 12.5 / 35, 256 x 512 x 256 in four
-// 18.6 / 19.2; 512 x 1024 x 512 28.8 / 28.9, 300 x 600 x 300 in twenty 96 / 45, 1024 x 2048 x 1024 152 / 49.
-bool gemm_small_wins(const GemmArgs &g, long long tiles, long long blocks, int sms) {
-    const double kt = (g.K + 31) / 32, waves = (double)((tiles + sms - 1) / sms), per = (double)blocks / sms;
-    const double small = small_split(blocks, g.K, sms) ? 4.2 + ((g.K + 127) / 128) * std::max(2.05, 1.9 * per)
-                                                       : 4.0 + kt * (0.75 + 0.3 * per);
-    return small < 8.0 + 1.3 * kt * waves;
+template <int T, int TK, bool ACOL, bool BKC, bool TCF>
+__global__ void __launch_bounds__(256) k_gemm_tile(GemmArgs g, TcfArgs tc) {
+    static_assert(T * TK == 1024, "four values a thread");
+    constexpr int Q = T / 64;
+    __shared__ __align__(16) float As[2][TK][T], Bs[2][TK][T];
+    const int bz = blockIdx.z, m0 = blockIdx.y * T, n0 = blockIdx.x * T;
+    const float *A = g.A + (size_t)bz * g.sA, *B = g.B + (size_t)bz * g.sB;
+    const int tx = 4 * (threadIdx.x % 16), ty = 4 * (threadIdx.x / 16);
+    float acc[4 * Q][4 * Q] = {};
+    float4 ra = tile_load<T, TK, !ACOL>(A, g.lda, g.M, g.K, m0, 0), rb = tile_load<T, TK, BKC>(B, g.ldb, g.N, g.K, n0, 0);
+    tile_store<T, TK, !ACOL>(As[0], ra);
+    tile_store<T, TK, BKC>(Bs[0], rb);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < g.K; k0 += TK) {
+        const bool more = k0 + TK < g.K;
+        if (more) {
+            ra = tile_load<T, TK, !ACOL>(A, g.lda, g.M, g.K, m0, k0 + TK);
+            rb = tile_load<T, TK, BKC>(B, g.ldb, g.N, g.K, n0, k0 + TK);
+        }
+        #pragma unroll
+        for (int k = 0; k < TK; k++) {
+            float a[4 * Q], b[4 * Q];
+            #pragma unroll
+            for (int q = 0; q < Q; q++) {
+                *reinterpret_cast<float4 *>(a + 4 * q) = *reinterpret_cast<const float4 *>(&As[buf][k][ty + 64 * q]);
+                *reinterpret_cast<float4 *>(b + 4 * q) = *reinterpret_cast<const float4 *>(&Bs[buf][k][tx + 64 * q]);
+            }
+            #pragma unroll
+            for (int i = 0; i < 4 * Q; i++)
+                #pragma unroll
+                for (int j = 0; j < 4 * Q; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        if (more) {
+            tile_store<T, TK, !ACOL>(As[buf ^ 1], ra);
+            tile_store<T, TK, BKC>(Bs[buf ^ 1], rb);
+        }
+        __syncthreads();
+        buf ^= 1;
+    }
+    Pair sum[8] = {};
+    const TcfCols mc = TCF ? TcfCols(tc, bz, n0 + tx) : TcfCols();
+    #pragma unroll
+    for (int i = 0; i < 4 * Q; i++) {
+        const int r = m0 + ty + 64 * (i / 4) + i % 4;
+        if (r >= g.M) continue;
+        const CirPhase ph = simt_phase(g, bz, r);
+        #pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const float4 v = make_float4(acc[i][4 * q], acc[i][4 * q + 1], acc[i][4 * q + 2], acc[i][4 * q + 3]);
+            if (TCF) tcf_row(tc, bz, r, mc, v, sum);
+            simt_store(g, bz, r, n0 + tx + 64 * q, v, ph);
+        }
+    }
+    if (TCF) {
+        static_assert(!TCF || Q == 1, "one column group a thread");
+        __shared__ double psum[8][8];
+        const int lane = threadIdx.x & 31;
+        const double v = tcf_reduce(sum);
+        if ((lane & 3) == 0) psum[threadIdx.x >> 5][lane >> 2] = v;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            double s = 0.0;
+            if (lane < 8)
+                #pragma unroll
+                for (int w = 0; w < 8; w++) s += psum[w][lane];
+            tcf_add(s, tc.out + (size_t)bz * tc.sout);
+        }
+    }
 }
 
 __global__ void k_identity(float *F, int n, int ldf, long long sF) {
@@ -658,23 +746,29 @@ cudaError_t cir_launch_gemm(const GemmArgs &g, int batch, cudaStream_t s, int *l
     auto vec = [&](const float *p, int ld, long long st) {
         return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld & 3) == 0 && (batch == 1 || (st & 3) == 0);
     };
-    const int sms = cir_sms();
     const bool va = vec(g.A, g.lda, g.sA), vb = vec(g.B, g.ldb, g.sB),
                vc = vec(g.C, g.ldc, g.sC) && (g.epilogue != 2 || vec(g.D, g.ldd, g.sD));
-    const dim3 small((g.N + SB - 1) / SB, (g.M + SB - 1) / SB, batch);
-    const long long blocks = (long long)small.x * small.y * batch;
-    if (gemm_small_wins(g, nt, blocks, sms)) {
+    const int sms = cir_sms();
+    const CirGemmForm form = cir_gemm_form(g.M, g.N, g.K, batch, g.epilogue, va && vb, vc, sms);
+    if (form != CIR_GEMM_TC) {
+        const bool fuse = tcf && g.a_colmajor && g.epilogue == 0 && form != CIR_GEMM_TILE128;
         const TcfArgs tc = tcf ? *tcf : TcfArgs{};
-        auto go = [&](auto one, auto four) {
-            if (small_split(blocks, g.K, sms)) four<<<small, 256, 0, s>>>(g, va, vb, tc);
-            else one<<<small, 64, 0, s>>>(g, va, vb, tc);
+        const int T = form == CIR_GEMM_SMALL ? SB : form == CIR_GEMM_TILE64 ? 64 : 128;
+        const dim3 grid((g.N + T - 1) / T, (g.M + T - 1) / T, batch);
+        auto go = [&](auto small, auto t64, auto t128) {
+            if (form == CIR_GEMM_SMALL) small<<<grid, 64 * SK, 0, s>>>(g, tc);
+            else if (form == CIR_GEMM_TILE64) t64<<<grid, 256, 0, s>>>(g, tc);
+            else t128<<<grid, 256, 0, s>>>(g, tc);
         };
-        if (tcf && g.a_colmajor && g.epilogue == 0) {
-            go(k_gemm_small<true, false, 1, true>, k_gemm_small<true, false, 4, true>);
+        if (fuse) {
+            go(k_gemm_small<true, false, true>, k_gemm_tile<64, 16, true, false, true>, k_gemm_tile<128, 8, true, false, false>);
             *fused = true;
-        } else if (g.a_colmajor) go(k_gemm_small<true, false, 1, false>, k_gemm_small<true, false, 4, false>);
-        else if (g.b_kmajor) go(k_gemm_small<false, true, 1, false>, k_gemm_small<false, true, 4, false>);
-        else go(k_gemm_small<false, false, 1, false>, k_gemm_small<false, false, 4, false>);
+        } else if (g.a_colmajor)
+            go(k_gemm_small<true, false, false>, k_gemm_tile<64, 16, true, false, false>, k_gemm_tile<128, 8, true, false, false>);
+        else if (g.b_kmajor)
+            go(k_gemm_small<false, true, false>, k_gemm_tile<64, 16, false, true, false>, k_gemm_tile<128, 8, false, true, false>);
+        else
+            go(k_gemm_small<false, false, false>, k_gemm_tile<64, 16, false, false, false>, k_gemm_tile<128, 8, false, false, false>);
         if (launches) *launches += 1;
         return cudaGetLastError();
     }

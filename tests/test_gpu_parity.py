@@ -710,3 +710,15 @@ def test_create_with_very_long_padding(lib):
     """A context for a transform of more than 2^30 points is made without working through them."""
     with lib.Engine(lib.default_params(species="H2O", nzeros=1_900_000_000), 8):
         pass
+
+
+@pytest.mark.parametrize("n,batch", [(1, 3), (24, 40), (32, 100), (33, 150), (63, 64), (65, 150), (66, 152), (98, 64), (113, 16)])
+def test_propagate_tile_forms(lib, n, batch):
+    """The products of many small matrices on tiles of 64 and 128, whole and ragged, aligned rows and not."""
+    test_propagate_forms(lib, n, batch)
+
+
+@pytest.mark.parametrize("nmol,origins", [(12, 60), (25, 100), (32, 64), (33, 160), (49, 60)])
+def test_contraction_in_tiles(lib, nmol, origins):
+    """The correlation terms from tiles of 64, and by their own launch after tiles of 128."""
+    test_contraction_forms(lib, nmol, origins)

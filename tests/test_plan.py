@@ -136,3 +136,39 @@ def test_build_form(tmp_path):
     out = subprocess.run([exe], input="".join("%d %d\n" % c for c in cases), capture_output=True, text=True,
                          check=True).stdout.split()
     assert [int(x) for x in out] == [1] * len(wide) + [0] * len(narrow)
+
+
+GEMM_DRIVER = r"""
+#include <cstdio>
+#include "cir_plan.h"
+int main() {
+    int M, N, K, b, e, a;
+    while (std::scanf("%d %d %d %d %d %d", &M, &N, &K, &b, &e, &a) == 6)
+        std::printf("%d\n", (int)cir_gemm_form(M, N, K, b, e, (a & 1) != 0, (a & 2) != 0, 152));
+    return 0;
+}
+"""
+
+
+def test_product_form(tmp_path):
+    """The FP32 product's kernel: the one that measured fastest by 10% or more (GB300), or either of two
+    that are level."""
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no host C++ compiler")
+    src, exe = str(tmp_path / "gemm.cpp"), str(tmp_path / "gemm")
+    with open(src, "w") as f:
+        f.write(GEMM_DRIVER)
+    subprocess.run([cxx, "-std=c++17", "-O1", "-I", HEADER_DIR, src, "-o", exe], check=True)
+    small, t64, t128, tc = 0, 1, 2, 3
+    # the last number: 3: rows of operands and output start on 16 bytes, 2: the output's alone, 0: neither
+    cases = [((128, 256, 128, 1, 1, 3), {small}), ((200, 400, 200, 1, 1, 3), {small}), ((64, 128, 64, 16, 1, 3), {small, t64}),
+             ((33, 66, 33, 300, 1, 0), {t64}), ((50, 100, 50, 300, 1, 3), {t64}), ((56, 112, 56, 600, 0, 3), {t64}),
+             ((65, 130, 65, 300, 1, 0), {t128, t64}), ((66, 132, 66, 152, 0, 3), {t128, t64}), ((97, 194, 97, 150, 1, 0), {t128}),
+             ((128, 256, 128, 300, 1, 3), {tc}), ((256, 512, 256, 16, 1, 3), {tc}), ((1024, 2048, 1024, 1, 1, 3), {tc}),
+             ((1024, 2048, 1024, 200, 0, 3), {tc}), ((686, 686, 128, 64, 2, 0), {t64, t128}), ((1024, 1024, 128, 64, 2, 3), {tc}),
+             ((432, 432, 128, 64, 2, 3), {tc}), ((343, 686, 128, 16, 2, 0), {t64, t128})]
+    inp = "".join("%d %d %d %d %d %d\n" % c for c, _ in cases)
+    out = subprocess.run([exe], input=inp, capture_output=True, text=True, check=True).stdout.split()
+    for (c, forms), got in zip(cases, out):
+        assert int(got) in forms, (c, got)
