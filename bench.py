@@ -42,6 +42,10 @@ WORKLOAD = ("512 TIP4P/2005 molecules (1024 chromophores, box 2.4834 nm), 10 tim
             "correlation points at 10 fs = 2500 frame-steps per step")
 
 
+# tensor-pipe work of a product in units of a BF16 product
+TENSOR_PRODUCTS = {"fp32": 8.0, "tf32": 2.0, "bf16x3": 3.0}
+
+
 def dist_env():
     return int(os.environ.get("RANK", 0)), int(os.environ.get("WORLD_SIZE", 1)), int(os.environ.get("LOCAL_RANK", 0))
 
@@ -49,22 +53,19 @@ def dist_env():
 def job_roofline(n, fps, pk, precision):
     """The whole job against a time-weighted peak: W = 12.67 N^3 flops per frame-step (8 N^3
     propagation, 2 N^3 back-transform, 4/3 N^3 tridiagonalisation, 4/3 N^3 divide and conquer);
-    in the mixed forms the propagation and back-transform on the tensor cores (BF16 peak / 3
-    passes for split-BF16), the rest at the FP32 SIMT rate; in the plain form everything at
-    the FP32 SIMT rate.  The SIMT rate is the nominal 152 SMs x 128 lanes x 2 flops x 2.07 GHz
-    (80.5 TFLOP/s); the measured SGEMM rate is in peaks_probe."""
+    the propagation and back-transform on the tensor cores (BF16 peak / 3 products for
+    split-BF16, / 8 for the plain form's three terms), the rest at the FP32 SIMT rate.  The SIMT
+    rate is the nominal 152 SMs x 128 lanes x 2 flops x 2.07 GHz (80.5 TFLOP/s); the measured
+    SGEMM rate is in peaks_probe."""
     simt = 152 * 128 * 2 * 2.07e9 / 1e12
     w_tc, w_simt = 10.0, 8.0 / 3.0
-    if precision == "fp32":
-        peak = simt
-    else:
-        tc = pk["bf16_tflops"] / (3.0 if precision == "bf16x3" else 2.0)
-        peak = (w_tc + w_simt) / (w_tc / tc + w_simt / simt)
+    tc = pk["bf16_tflops"] / TENSOR_PRODUCTS[precision]
+    peak = (w_tc + w_simt) / (w_tc / tc + w_simt / simt)
     achieved = 12.67 * n ** 3 * fps / 1e12
     return {"achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
             "work": "12.67 N^3 flops per frame-step (propagation 8, back-transform 2, tridiagonalisation 4/3, "
                     "divide and conquer 4/3)",
-            "peak_kind": "time-weighted: tensor share at the measured BF16 peak / passes (TF32 at half the BF16 "
+            "peak_kind": "time-weighted: tensor share at the measured BF16 peak / products (TF32 at half the BF16 "
                          "rate), the rest at the nominal FP32 SIMT rate"}
 
 
@@ -549,13 +550,15 @@ def main():
                                                            # end of the later of its two launches (two streams)
     tq_bytes = tridiag_bytes(n) * steps_per_job
     tq_gbs = tq_bytes / (tq_ms * 1e-3) / 1e9
+    tq_dram_gbs = TRIDIAG_DRAM_BYTES_PER_MATRIX * steps_per_job / (tq_ms * 1e-3) / 1e9
     prop_flops = 8.0 * n ** 3 * JOB["nsamples"] * (JOB["ntcfpoints"] - 1)
     prop_tflops = prop_flops / (st["ms_prop"] / args.steps * 1e-3) / 1e12
-    passes = {"fp32": 1, "tf32": 1, "bf16x3": 3}[args.precision]   # tensor-pipe passes per product
-    nfft = JOB["ntcfpoints"] + JOB["nzeros"]
-    nomega = 3001
-    h2d = xyz.nbytes + xyz.shape[0] * 12 + fos.nbytes
-    d2h = steps_per_job * 48 + nomega * 8 * 4 + 3 * nfft * 8
+    passes = {"fp32": 8, "tf32": 1, "bf16x3": 3}[args.precision]   # tensor-pipe passes per product
+    _, nomega, nls = cg.result_sizes(p)
+    # positions, boxes, frame table, damped correlation sums; correlation terms and statuses, four
+    # histograms, three lineshapes' printed rows, three counters
+    h2d = xyz.nbytes + xyz.shape[0] * 12 + fos.nbytes + 3 * JOB["ntcfpoints"] * 16
+    d2h = steps_per_job * (48 + 4) + nomega * 8 * 4 + 3 * nls * 4 + 20
     form = {"fp32": "plain FP32 (three-term BF16 tcgen05 and SIMT GEMMs)", "tf32": "mixed: TF32 tcgen05 propagation GEMMs",
             "bf16x3": "mixed: 3-pass split-BF16 tcgen05 propagation GEMMs"}[args.precision]
     line = {
@@ -569,14 +572,16 @@ def main():
         "gpu_launches": int(st["kernel_launches"]),
         "roofline": {"kernel": "k_tridiag (blocked lower-storage tridiagonalisation; the job's 2500 matrices in "
                                "two launches on two streams, timed together)",
-                     "bound": "hbm", "achieved": tq_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
-                     "frac": tq_gbs / pk["hbm_gbs"], "peak_kind": f"{pk_kind} copy bandwidth (burst)",
-                     "work": "algorithmic bytes: per column the lower triangle of the trailing block, per "
-                             "8-column panel one write of the trailing lower triangle; "
-                             f"{tridiag_bytes(n) / 1e9:.3f} GB per 1024 x 1024 matrix x 2500 matrices per job",
+                     "bound": "instruction issue (profiles/k_tridiag_n1024.md); HBM beside it",
+                     "achieved": tq_dram_gbs, "peak": pk["hbm_gbs"], "unit": "GB/s",
+                     "frac": tq_dram_gbs / pk["hbm_gbs"], "peak_kind": f"{pk_kind} copy bandwidth (burst)",
+                     "work": "bytes that reach HBM: ncu dram__bytes_read.sum + dram__bytes_write.sum per matrix x 2500",
                      "ms_per_launch": tq_ms,
                      "traffic": TRIDIAG_DRAM_BYTES_PER_MATRIX * steps_per_job,
-                     "traffic_note": "ncu dram__bytes_read.sum + dram__bytes_write.sum per matrix x 2500"},
+                     "algorithmic_gbs": tq_gbs,
+                     "algorithmic_note": "per column the lower triangle of the trailing block, per 8-column panel one "
+                                         "write of it, the L2's share included; "
+                                         f"{tridiag_bytes(n) / 1e9:.3f} GB per 1024 x 1024 matrix x 2500 matrices per job"},
         "roofline_eigensolver": {"kernels": "tridiagonalisation, divide and conquer, blocked Householder "
                                             "back-transform V = Q_H Q_T",
                                  "achieved": eig_tflops, "unit": "TFLOP/s",
@@ -602,21 +607,21 @@ def main():
                               "ms_per_step": plain["ms"] / args.steps,
                               "stages_ms_per_step": {k: plain["stats"][k] / args.steps for k in ("ms_build", "ms_eig", "ms_prop")},
                               "mixed_over_plain": plain["ms"] / ms}
+        plain_prop = prop_flops / (plain["stats"]["ms_prop"] / args.steps * 1e-3) / 1e12
+        line["plain_fp32"]["roofline_propagation"] = {
+            "kernel": "k_gemm (FP32 propagation GEMMs as eight BF16 tcgen05 products)", "bound": "tensor",
+            "achieved": plain_prop * 8, "peak": pk["bf16_tflops"], "unit": "TFLOP/s",
+            "frac": plain_prop * 8 / pk["bf16_tflops"], "algorithmic_tflops": plain_prop,
+            "note": "the loaders' splitting into three terms bounds it; time includes the correlation contraction"}
     if rank == 0:
         # FP32-SIMT / TF32 / FP64 cuBLAS peaks (not in the peak file), measured after the timed
-        # regions: the denominators of the plain form's SIMT propagation roofline
+        # regions, for comparison
         try:
             from calcir_gb300 import peaks as peak_probe
             extra = peak_probe.measure(quick=True)
         except Exception as exc:        # a probe failure must not lose the bench line
             extra = {"error": f"{type(exc).__name__}: {exc}"}
         line["peaks_probe"] = extra
-        if plain is not None and "fp32_simt_tflops" in extra:
-            plain_prop = prop_flops / (plain["stats"]["ms_prop"] / args.steps * 1e-3) / 1e12
-            line["plain_fp32"]["roofline_propagation"] = {
-                "kernel": "k_gemm (FP32 propagation GEMMs as six BF16 tcgen05 products)", "bound": "fp32 simt", "achieved": plain_prop,
-                "peak": extra["fp32_simt_tflops"], "unit": "TFLOP/s", "frac": plain_prop / extra["fp32_simt_tflops"],
-                "peak_kind": "measured cuBLAS SGEMM, TF32 off (peaks_probe)"}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         port = CpuPort(args.seed, args.cpu_sample)
         port.sample()                                   # warm-up (threads, page faults)
