@@ -8,8 +8,9 @@
 //     y_j, y_{n-j} = a_0 + sum_k a_k cos(k t_j) -+ b_k sin(k t_j),  t_j = 2 pi j / n,
 // a_k = 2 Re X_k, b_k = 2 Im X_k, so a thread gives two outputs of up to three spectra for one
 // cosine and one sine per k, each by the three-term recurrence (one FMA), restarted from
-// sincospi every LS_SEG terms (rounding grows with the square of the terms since a restart:
-// 64^2 eps = 5e-13).  Bound by the FP64 pipe (two FMAs per SM and clock).  A whole lineshape
+// sincospi every LS_SEG terms (rounding grows with the square of the terms since a restart, at
+// most 64^2 eps = 5e-13 of the terms' sum; 4e-15 to 7e-15 for n 2650 to 40040, so that the FP32 rows round
+// as the FFT's).  Bound by the FP64 pipe (two FMAs per SM and clock).  A whole lineshape
 // call at 150 points and n = 25750: 528 -> 84 us, of which the seven launches of the FFT were
 // 437 us; the twelve transforms of a job with n = 25624 = 8 * 3203 took the FFT 33 ms.
 //

@@ -254,7 +254,7 @@ int cir_spectral_density(cir_ctx *c, int n, const float *V, const float *w, cons
                          float *Sw);
 
 /* Lineshape of a damped TCF [ntcf][2] (re,im): the unnormalised inverse real DFT of the
- * zero-padded TCF (hand-written mixed-radix FFT), mapped to descending frequencies in
+ * zero-padded TCF (its unpadded terms summed, or a mixed-radix FFT), mapped to descending frequencies in
  * [omegaStart, omegaStop]; writes nls rows.  Replaces cufftExecC2R + the output mapping
  * (calcIR.cu:772-827, 890-919). */
 int cir_lineshape(cir_ctx *c, const double *tcf, float *omega, float *intensity, int *nls);
@@ -278,7 +278,7 @@ int cir_set_coeffs(cir_ctx *c, const float *theta);
 /* The backward entry: L = sum over the printed lineshape rows of (IR - target_ir)^2 +
  * (VV - target_vv)^2 for the job cir_run would compute on these frames, and dL/dtheta
  * (grad [CIR_NTHETA], double).  The adjoint runs through the propagation (psi_c = F m_c(0),
- * checkpointed every 16 steps and recomputed in the backward pass) and the eigendecompositions
+ * kept for every step) and the eigendecompositions
  * (the Daleckii-Krein divided difference of exp(i L dt/hbar), finite for equal eigenvalues),
  * then through the maps.  FP32 with FP64 sums; nls must equal the lineshape's row count.
  * Extends cir_run (calcIR.cu:360-839); the reference has no gradient. */
