@@ -23,20 +23,30 @@ inline int cir_sms() {
 }
 
 // Lets kern be launched with that much dynamic shared memory.  The limit belongs to the kernel, whichever
-// thread or context launches it, so it is only ever raised: another thread's smaller launch must not take it
-// back between this call and the launch.
+// thread or context launches it, so it is only ever set to the most the device gives a block: another
+// thread's smaller launch must not take it back between this call and the launch.
 template <class K>
 inline cudaError_t cir_allow_smem(K kern, size_t bytes) {
     static std::mutex mu;
-    static std::map<std::pair<int, const void *>, size_t> limits;
-    int dev = 0;
+    static std::map<const void *, size_t> own;     // the kernels' static shared memory
+    size_t fixed = 0;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        auto it = own.find(reinterpret_cast<const void *>(kern));
+        if (it == own.end()) {
+            cudaFuncAttributes a;
+            const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+            if (e != cudaSuccess) return e;
+            it = own.emplace(reinterpret_cast<const void *>(kern), a.sharedSizeBytes).first;
+        }
+        fixed = it->second;
+    }
+    if (bytes + fixed <= 48 * 1024) return cudaSuccess;     // what every kernel may have unasked
+    int dev = 0, most = 0;
     cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(mu);
-    size_t &limit = limits[{dev, reinterpret_cast<const void *>(kern)}];
-    if (limit >= bytes) return cudaSuccess;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) == cudaSuccess) limit = bytes;
-    return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fixed);
 }
 
 // minImage (calcIR.cu:1459-1463): dx - L*round(dx/L), round half away from zero, evaluated
