@@ -85,7 +85,6 @@ inline CirGemmForm cir_gemm_form(int M, int N, int K, int batch, int epilogue, b
         4.4 + slices(128) * std::max(1.92, 1.14 * b32) + 0.46 * b32,
         4.9 + slices(16) * std::max(0.63, 0.556 * b64) * (in16 ? 1.0 : 1.09) + 0.24 * sub * b64,
         2.7 + std::ceil(t128 / (2 * sms)) * (1.054 * slices(8) * (t128 > sms ? 1.57 : 1.0) * (in16 ? 1.0 : 1.035) + 2.76),
-        3.5 + std::ceil(t128 / sms) * (std::max((in16 ? 1.44 : 1.75) * slices(32) + 4.8, out16 ? 0.0 : 17.0) +
-                                       sub * (out16 ? 2.0 : 38.0))};
+        3.5 + std::ceil(t128 / sms) * (out16 ? (in16 ? 1.44 : 1.75) * slices(32) + 4.8 + 2.0 * sub : 2.3 * slices(32) + 8.5 + 38.0 * sub)};
     return static_cast<CirGemmForm>(std::min_element(t, t + 4) - t);
 }
