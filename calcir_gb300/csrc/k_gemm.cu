@@ -59,7 +59,8 @@ constexpr int F_PART = (FM / 8) * F_SBO;       // bytes of one term of one opera
 constexpr int F_STAGE = 6 * F_PART, F_NS = 3, F_RAW = 2;
 constexpr int F_LOAD = 8, F_ACC = 8;           // warps
 constexpr int F_NT = 32 * (F_LOAD + F_ACC + 4);   // whole warpgroups: the register split is per group
-constexpr float F_TINY = 0x1p-110f, F_HUGE = 0x1p112f;   // below: l under BF16's smallest number; from here: grids' constants
+// below F_TINY l reaches under BF16's smallest normal number; from F_HUGE the grids' constants would overflow
+constexpr float F_TINY = 0x1p-100f, F_HUGE = 0x1p112f;
 constexpr int F_ODD = 8;                       // tiles the loaders' notes reach back: they are at most 5 ahead of the epilogue
 constexpr size_t F_RAWB = (size_t)F_LOAD * 32 * 128;   // bytes of an FP32 slice of both operands
 constexpr size_t F_SMEM = (size_t)F_NS * F_STAGE + F_RAW * F_RAWB + 256;

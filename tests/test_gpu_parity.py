@@ -623,7 +623,7 @@ def test_propagate_graded(lib, n, batch):
 
 
 @pytest.mark.parametrize("n,batch", [(64, 2), (300, 8), (509, 2)])
-@pytest.mark.parametrize("value", [np.inf, 2e38, 3e-36, 1e-33])
+@pytest.mark.parametrize("value", [np.inf, 2e38, 4e33, 3e-36, 1e-33, 1e-30])
 def test_propagate_range(lib, n, batch, value):
     """A column of F of infinite, very large or very small values beside ordinary ones, in the small
     products and on the tensor cores: infinities come out as FP32 sums give them, the other columns'
